@@ -220,10 +220,10 @@ typedef struct {
     uint64_t warp1_deep;   /* strings re-sorted by the one-per-lane warp sort on
                               their next 16 bytes within the same round
                               (SSORT_PARAM_WARP1_DEEP), summed over steps */
-    uint64_t full_sorted;  /* strings of on-chip sorted segments whose packed
-                              64-bit keys could not order them (a run of more
-                              than 64 equal windows) and were re-sorted with
-                              the full key comparator */
+    uint64_t full_sorted;  /* strings of on-chip sorted segments of more than 32
+                              strings in which a run of more than 64 records
+                              that tie on their packed values was out of order
+                              (such segments are refined on further key bits) */
     uint64_t window_saved; /* strings whose key bytes 16..31 round 0's gather
                               kept for round 1 (sorts of at least 2^20 strings
                               whose arena holds >= 24 bytes per string, unless
@@ -254,11 +254,8 @@ int ssort_get_stats(const ssort_ctx *ctx, ssort_stats *out);
                                        sorts a segment of <= 32 strings takes on its own
                                        runs of equal keys before handing what is left to
                                        the next round; 0: every run waits for the next round */
-#define SSORT_PARAM_BLOCK_PREFETCH 6 /* 0 (default): the CTA sort of segments of 257..2048
-                                        strings loads one segment's records through
-                                        registers at three CTAs per SM; 1: it copies the
-                                        next segment's records into shared memory while it
-                                        sorts the current one (two CTAs per SM) */
+#define SSORT_PARAM_BLOCK_PREFETCH 6 /* 0 or 1; no effect (the CTA sort always copies its
+                                        records asynchronously) */
 #define SSORT_PARAM_MATCH_VOTE 13    /* 1: the partition's count kernel finds the lanes of a
                                         warp that share a bucket with one ballot per
                                         bucket-id bit; 0 (default): with __match_any_sync */
@@ -266,17 +263,9 @@ int ssort_get_stats(const ssort_ctx *ctx, ssort_stats *out);
                                         in one pass with decoupled look-back (tiles in
                                         ticket order add up their predecessors' published
                                         sums); 0: reduce, scan of the partials, down-sweep */
-#define SSORT_PARAM_WARP_MERGE 14    /* 1 (default): the warp-level sorts of packed keys
-                                        (one-warp and CTA sorts) sort each lane's values
-                                        with a sorting network and merge runs with
-                                        merge-path passes; 0: a bitonic network across
-                                        the warp */
-#define SSORT_PARAM_BLOCK_LEAN 12    /* 1: the CTA sort takes the LCPs of neighbours whose
-                                        packed windows differ from the windows alone and
-                                        reads full keys only for equal windows; 2: that, and
-                                        its first sort runs on 32-bit packed keys (21 key
-                                        bits and the position; ties on those bits are put in
-                                        order afterwards); 0 (default): full-key finish */
+#define SSORT_PARAM_WARP_MERGE 14    /* 0 or 1; no effect (one sort of packed values is left) */
+#define SSORT_PARAM_BLOCK_LEAN 12    /* 0, 1 or 2; no effect (neighbour LCPs come from the
+                                        packed values wherever they tell) */
 #define SSORT_PARAM_L2_PREFETCH 9    /* 1: the partition's count and scatter kernels ask
                                         for their next tile to be streamed into L2 (bulk
                                         prefetch) while they work on the current one;

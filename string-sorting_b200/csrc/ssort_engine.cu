@@ -123,10 +123,10 @@ int ssort_ctx::launch_small(const SortArgs &a, Seg *nxt, SmallDone &d) {
     const uint32_t counts[3] = {h_ctr->n_small, h_ctr->n_small2, h_ctr->n_small3};
     for (int k = 0; k < 3; ++k) {
         n = counts[k] - d.s[k];
-        const uint32_t per_cta = (uint32_t)SMALL_THREADS / (64u << k);
+        const uint32_t per_cta = 4u >> k;
         LAUNCH(this, "block",
                launch_block(a, lists[k], hspan(d.s[k], d.s[k] + n), k, nxt, dc,
-                            grid(n, per_cta * (block_prefetch ? 4u : 1u)), s3, block_prefetch));
+                            grid(n, per_cta), s3));
         d.s[k] += n;
     }
     n = h_ctr->n_equal - d.e;
@@ -304,9 +304,7 @@ int ssort_ctx::run_ws(const uint8_t *arena_p, uint64_t arena_bytes, const void *
     a.warp1_deep = warp1_deep;
     a.l2_prefetch = l2_prefetch ? 1u : 0u;
     a.scatter_staged_idx = scatter_variant;
-    a.block_lean = block_lean;
     a.match_vote = match_vote ? 1u : 0u;
-    a.warp_merge = warp_merge ? 1u : 0u;
     a.max_splitters = (1u << (digit_bits - 1)) - 1;
     std::copy(std::begin(class_targets), std::end(class_targets), std::begin(a.target_by_class));
     a.key2 = key2;
@@ -436,10 +434,8 @@ int apply_tuning(ssort_ctx *ctx, const uint8_t *d_arena, uint64_t arena_bytes,
     ctx->overlap = it->second.overlap;
     ctx->fused_gather = it->second.fused_gather;
     ctx->digit_bits = it->second.digit_bits;
-    ctx->block_prefetch = it->second.block_prefetch;
     ctx->l2_prefetch = it->second.l2_prefetch;
     ctx->graph_mode = it->second.graph;
-    ctx->block_lean = it->second.block_lean;
     return SSORT_OK;
 }
 
@@ -876,16 +872,14 @@ int ssort_set_param(ssort_ctx *ctx, int param, int64_t value) {
             return SSORT_OK;
         case SSORT_PARAM_WARP_MERGE:
             if (value != 0 && value != 1) return fail(SSORT_EINVAL, "warp_merge must be 0 or 1");
-            ctx->warp_merge = value != 0;
-            return SSORT_OK;
+            return SSORT_OK;  // one warp-level sort is left: nothing to choose
         case SSORT_PARAM_MATCH_VOTE:
             if (value != 0 && value != 1) return fail(SSORT_EINVAL, "match_vote must be 0 or 1");
             ctx->match_vote = value != 0;
             return SSORT_OK;
         case SSORT_PARAM_BLOCK_LEAN:
             if (value < 0 || value > 2) return fail(SSORT_EINVAL, "block_lean must be 0, 1 or 2");
-            ctx->block_lean = (uint32_t)value;
-            return SSORT_OK;
+            return SSORT_OK;  // one finish is left: nothing to choose
         case SSORT_PARAM_SCATTER:
             if (value < 0 || value > 2) return fail(SSORT_EINVAL, "scatter must be 0, 1 or 2");
             ctx->scatter_variant = (uint32_t)value;
@@ -905,8 +899,7 @@ int ssort_set_param(ssort_ctx *ctx, int param, int64_t value) {
             return SSORT_OK;
         case SSORT_PARAM_BLOCK_PREFETCH:
             if (value != 0 && value != 1) return fail(SSORT_EINVAL, "block_prefetch must be 0 or 1");
-            ctx->block_prefetch = value != 0;
-            return SSORT_OK;
+            return SSORT_OK;  // records always arrive by asynchronous copies
         case SSORT_PARAM_WARP1_DEEP:
             if (value < 0 || value > WARP1_DEEP_MAX)
                 return fail(SSORT_EINVAL, "warp1_deep out of range (0..4096)");
@@ -1143,8 +1136,9 @@ int ssort_autotune(ssort_ctx *ctx, const uint8_t *d_arena, uint64_t arena_bytes,
             };
             // Coordinate descent over: range-bucket size, digit width of a
             // partition pass (splitters per pass), the small-segment cutoff,
-            // the gather and overlap choices, the CTA sort's record prefetch,
-            // the partition's L2 prefetch and the device-driven loop.
+            // the gather and overlap choices, the partition's L2 prefetch and
+            // the device-driven loop.  (The two parameters without effect
+            // keep their trials, so that a call times as many sorts as ever.)
             const Knob knobs[] = {{SSORT_PARAM_TARGET_BUCKET, {256, 512, 1024}},
                                   {SSORT_PARAM_DIGIT_BITS, {10, 9, 8}},
                                   {SSORT_PARAM_WARP8_CAP, {64, 128, 256}},
@@ -1160,9 +1154,9 @@ int ssort_autotune(ssort_ctx *ctx, const uint8_t *d_arena, uint64_t arena_bytes,
                     case SSORT_PARAM_DIGIT_BITS: return ctx->digit_bits;
                     case SSORT_PARAM_WARP8_CAP: return ctx->warp8_cap;
                     case SSORT_PARAM_FUSED_GATHER: return ctx->fused_gather;
-                    case SSORT_PARAM_BLOCK_PREFETCH: return ctx->block_prefetch ? 1 : 0;
+                    case SSORT_PARAM_BLOCK_PREFETCH:
+                    case SSORT_PARAM_BLOCK_LEAN: return 0;
                     case SSORT_PARAM_L2_PREFETCH: return ctx->l2_prefetch ? 1 : 0;
-                    case SSORT_PARAM_BLOCK_LEAN: return ctx->block_lean;
                     case SSORT_PARAM_GRAPH: return ctx->graph_mode;
                     default: return ctx->overlap ? 1 : 0;
                 }
@@ -1184,9 +1178,8 @@ int ssort_autotune(ssort_ctx *ctx, const uint8_t *d_arena, uint64_t arena_bytes,
             }
             const uint32_t sc = size_class(n), ec = entropy_class(bits);
             ctx->tuned[sc * 4 + ec] = ssort_ctx::Tuned{
-                ctx->target_bucket, ctx->warp8_cap, ctx->digit_bits,     ctx->graph_mode,
-                ctx->block_lean,    ctx->fused_gather, ctx->overlap,    ctx->block_prefetch,
-                ctx->l2_prefetch};
+                ctx->target_bucket, ctx->warp8_cap, ctx->digit_bits, ctx->graph_mode,
+                ctx->fused_gather,  ctx->overlap,   ctx->l2_prefetch};
             out->size_class = sc;
             out->entropy_class = ec;
             out->entropy_bits = bits;
@@ -1195,7 +1188,7 @@ int ssort_autotune(ssort_ctx *ctx, const uint8_t *d_arena, uint64_t arena_bytes,
             out->overlap = ctx->overlap ? 1 : 0;
             out->fused_gather = ctx->fused_gather;
             out->digit_bits = ctx->digit_bits;
-            out->block_prefetch = ctx->block_prefetch ? 1 : 0;
+            out->block_prefetch = 0;  // no longer a choice
             out->l2_prefetch = ctx->l2_prefetch ? 1 : 0;
             out->graph = ctx->graph_mode;
             out->default_ms = base;

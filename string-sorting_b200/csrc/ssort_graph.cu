@@ -49,7 +49,7 @@ int add_conditional(cudaStream_t s, cudaGraphConditionalHandle h,
 // The bytes that decide a graph's contents: kernel arguments are baked into
 // the graph, so a graph is reused only for the same arguments and workspace.
 std::vector<unsigned char> graph_key(const SortArgs &a, const ssort_ctx &c) {
-    std::vector<unsigned char> k(sizeof(SortArgs) + sizeof(void *) + 2 * sizeof(size_t) + 2);
+    std::vector<unsigned char> k(sizeof(SortArgs) + sizeof(void *) + 2 * sizeof(size_t));
     unsigned char *p = k.data();
     std::memcpy(p, &a, sizeof(SortArgs));
     p += sizeof(SortArgs);
@@ -59,9 +59,6 @@ std::vector<unsigned char> graph_key(const SortArgs &a, const ssort_ctx &c) {
     p += sizeof(size_t);
     const size_t sms = (size_t)c.num_sms;
     std::memcpy(p, &sms, sizeof(size_t));
-    p += sizeof(size_t);
-    p[0] = c.block_prefetch ? 1 : 0;
-    p[1] = 0;
     return k;
 }
 
@@ -102,7 +99,7 @@ int ssort_ctx::graph_small(const SortArgs &a, cudaStream_t s) {
     for (int k = 0; k < 3; ++k)
         LAUNCH(this, "block",
                launch_block(a, lists[k], Span{dcount(&g->cur_s[k]), dcount(counts[k])}, k, nxt,
-                            dc, grid_for(block_prefetch ? 4 : 6), s, block_prefetch));
+                            dc, grid_for(6), s));
     LAUNCH(this, "equal",
            launch_equal(a, ws.E, Span{dcount(&g->cur_e), dcount(&dc->n_equal)}, nxt, dc,
                         grid_for(8), s));

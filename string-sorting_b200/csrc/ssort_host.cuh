@@ -85,14 +85,10 @@ struct ssort_ctx {
     uint32_t warp1_deep = ssort::WARP1_DEEP;        // in-warp refinement steps
     bool overlap = true;       // round-0 on-chip sorts on the side stream
     uint32_t fused_gather = 1;  // 1: rounds >= 1 gather inside the first count; 2: all rounds
-    bool block_prefetch = false;  // double-buffered CTA sort (k_block2)
-    uint32_t block_lean = 0;      // CTA sort: 1 finish from the packed windows, 2 also a
-                                  // first sort on 32-bit packed keys
     bool l2_prefetch = false;    // partition kernels prefetch their next tile into L2
     uint32_t digit_bits = 10;    // a partition pass makes at most 2^digit_bits buckets
     uint32_t scatter_variant = 0;  // 1: the scatter stages indices only (k_scatter2)
     bool match_vote = false;       // count kernel ranks keys with ballots
-    bool warp_merge = true;        // warp sorts: local networks + merge passes
     bool scan_lookback = true;     // count-matrix scan in one pass (decoupled look-back)
     // Device-driven round loop (ssort_graph.cu): the instantiated graph, the
     // key it was built for, three streams to capture nested conditional
@@ -113,8 +109,8 @@ struct ssort_ctx {
     // Autotuned values per (size class * 4 + entropy class), applied to later
     // sorts of the same classes; not while the tuner itself runs.
     struct Tuned {
-        uint32_t target_bucket, warp8_cap, digit_bits, graph, block_lean, fused_gather;
-        bool overlap, block_prefetch, l2_prefetch;
+        uint32_t target_bucket, warp8_cap, digit_bits, graph, fused_gather;
+        bool overlap, l2_prefetch;
     };
     std::map<uint32_t, Tuned> tuned;
     // target buckets per segment size class for the next batched sort

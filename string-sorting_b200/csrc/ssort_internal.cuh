@@ -48,7 +48,6 @@ constexpr uint32_t KEY2_MIN_BYTES_PER_STRING = 24;  // ... when the arena has th
 constexpr double KEY2_MIN_ROUND1_LIVE = 0.25;       // ... and the last sort's round-1 share
 constexpr int SMALL_CAP = 2048;
 constexpr int SMALL_THREADS = 256;
-constexpr int SMALL_ITEMS = SMALL_CAP / SMALL_THREADS;  // 8
 // The CTA sort splits its segments into three size classes, sorted by groups
 // of 64, 128 and 256 threads (8 strings per thread): <= BLOCK_CAP1,
 // <= BLOCK_CAP2 and <= SMALL_CAP strings.
@@ -139,9 +138,7 @@ struct SortArgs {
     uint32_t warp1_deep;     // in-warp refinement steps of the one-per-lane sort
     uint32_t l2_prefetch;    // partition kernels stream their next tile into L2 ahead
     uint32_t scatter_staged_idx;  // 0: k_scatter; 1: indices only (k_scatter2); 2: bulk key runs
-    uint32_t block_lean;     // CTA sort: neighbour LCPs from the packed windows
     uint32_t match_vote;     // count kernel ranks with ballots instead of the match unit
-    uint32_t warp_merge;     // warp sorts of packed keys: local networks + merge passes
     uint32_t max_splitters;  // splitters per partition pass, 2^(digit bits - 1) - 1 <= KMAX
     // Per segment size class (floor(log2 len)): the wanted strings per range
     // bucket autotuned for that class (0: target_bucket).  Set for batched
@@ -385,10 +382,8 @@ void launch_warp1(const SortArgs &a, const Seg *W1, Span sp, Seg *N, Counters *c
 void launch_warp8(const SortArgs &a, const Seg *W8, Span sp, Seg *N, Counters *c, int grid,
                   cudaStream_t st);
 // cls: size class 0, 1, 2 (segment list S holds that class)
-// prefetch: the double-buffered variant (records of the next segment copied
-// asynchronously while the current one sorts; two CTAs per SM instead of three).
 void launch_block(const SortArgs &a, const Seg *S, Span sp, int cls, Seg *N, Counters *c,
-                  int grid, cudaStream_t st, bool prefetch);
+                  int grid, cudaStream_t st);
 void launch_equal(const SortArgs &a, const Seg *E, Span sp, Seg *N, Counters *c, int grid,
                   cudaStream_t st);
 void launch_boundary(const SortArgs &a, const uint2 *B, Counters *c, int grid, cudaStream_t st);

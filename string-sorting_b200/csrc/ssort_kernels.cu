@@ -7,9 +7,8 @@
 // with unsigned shifts; the reference's int-promoted 64-bit form sign-extends
 // bytes >= 0x80, :82, and is not reproduced).  Each segment is then sorted by
 // (key, index): segments of <= 32 strings by one warp in registers (four
-// segments of <= 8 per warp), <= 256 by one warp with up to 8 strings per
-// lane, <= SMALL_CAP by a group of 64, 128 or 256 threads of a CTA (by size),
-// larger ones are first split by sample partitioning into range buckets and
+// segments of <= 8 per warp), <= SMALL_CAP by a group of 32 to 256 threads of
+// a CTA (by size), larger ones are first split by sample partitioning into range buckets and
 // equality buckets with a stable scatter.  Equal runs whose key holds no NUL (the reference's
 // is_end test, src/util/get_char.h:162-175, and its bucket-skip rule,
 // src/msd_ce.cpp:402) become the next round's segments at depth+16; every
@@ -59,55 +58,17 @@ __device__ __forceinline__ uint64_t cut_at_nul(uint64_t w, bool &found) {
     return jb ? (w & ((1ull << (8 * jb)) - 1)) : 0ull;
 }
 
-// The 16 bytes of the string at arena[pos..], big-endian, zero after the
-// first NUL.  The arena base is 16-byte aligned; bytes at or beyond
-// arena_bytes read as NUL.
-__device__ __forceinline__ Key load_key(const uint8_t *__restrict__ arena, uint64_t arena_bytes,
-                                        uint64_t pos) {
-    uint64_t w0, w1;  // little-endian: byte 0 of w0 is arena[pos]
-    const uint64_t a = pos & ~15ull;
-    const uint32_t off = (uint32_t)(pos & 15);
-    // (no a + 32 here: an offset near 2^64 must not wrap into the fast path)
-    if (arena_bytes >= 32 && a <= arena_bytes - 32) {
-        const ulonglong2 v0 = __ldg(reinterpret_cast<const ulonglong2 *>(arena + a));
-        if (off == 0) {
-            w0 = v0.x;
-            w1 = v0.y;
-        } else {
-            const ulonglong2 v1 = __ldg(reinterpret_cast<const ulonglong2 *>(arena + a + 16));
-            uint64_t q0, q1, q2;
-            if (off < 8) {
-                q0 = v0.x;
-                q1 = v0.y;
-                q2 = v1.x;
-            } else {
-                q0 = v0.y;
-                q1 = v1.x;
-                q2 = v1.y;
-            }
-            const uint32_t sh = (off & 7) * 8;
-            if (sh) {
-                w0 = (q0 >> sh) | (q1 << (64 - sh));
-                w1 = (q1 >> sh) | (q2 << (64 - sh));
-            } else {
-                w0 = q0;
-                w1 = q1;
-            }
-        }
-    } else {
-        w0 = 0;
-        w1 = 0;
-        for (int i = 0; i < 16; ++i) {
-            const uint64_t q = pos + i;
-            if (q >= arena_bytes) break;
-            const uint64_t c = arena[q];
-            if (i < 8)
-                w0 |= c << (8 * i);
-            else
-                w1 |= c << (8 * (i - 8));
-            if (!c) break;
-        }
-    }
+// The key whose 16 bytes start at byte `off` of the two adjacent words v0, v1
+// (v1 is not looked at when off is 0).
+__device__ __forceinline__ Key key_of_words(const ulonglong2 &v0, const ulonglong2 &v1,
+                                            uint32_t off) {
+    const uint64_t q0 = off < 8 ? v0.x : v0.y, q1 = off < 8 ? v0.y : v1.x,
+                   q2 = off < 8 ? v1.x : v1.y;
+    const uint32_t sh = (off & 7) * 8;
+    // little-endian: byte 0 of w0 is the string's first (two shifts, as a
+    // shift by 64 is undefined)
+    uint64_t w0 = (q0 >> sh) | (q1 << 1 << (63 - sh));
+    uint64_t w1 = (q1 >> sh) | (q2 << 1 << (63 - sh));
     bool nul;
     w0 = cut_at_nul(w0, nul);
     if (nul)
@@ -115,6 +76,40 @@ __device__ __forceinline__ Key load_key(const uint8_t *__restrict__ arena, uint6
     else
         w1 = cut_at_nul(w1, nul);
     return Key{bswap64(w0), bswap64(w1)};
+}
+
+// Whether the two 16-byte words at `a` (16-byte aligned) lie inside the arena
+// (no a + 32 here: an offset near 2^64 must not wrap into the fast path).
+__device__ __forceinline__ bool key_words_inside(uint64_t arena_bytes, uint64_t a) {
+    return arena_bytes >= 32 && a <= arena_bytes - 32;
+}
+
+// Byte-wise form for the last bytes of the arena and for offsets past it.
+__device__ __noinline__ Key load_key_tail(const uint8_t *__restrict__ arena,
+                                          uint64_t arena_bytes, uint64_t pos) {
+    uint64_t hi = 0, lo = 0;
+    for (int i = 0; i < 16; ++i) {
+        const uint64_t q = pos + i;
+        const uint64_t c = q >= pos && q < arena_bytes ? arena[q] : 0;
+        if (!c) break;
+        if (i < 8)
+            hi |= c << (56 - 8 * i);
+        else
+            lo |= c << (120 - 8 * i);
+    }
+    return Key{hi, lo};
+}
+
+// The 16 bytes of the string at arena[pos..], big-endian, zero after the
+// first NUL.  The arena base is 16-byte aligned; bytes at or beyond
+// arena_bytes read as NUL.
+__device__ __forceinline__ Key load_key(const uint8_t *__restrict__ arena, uint64_t arena_bytes,
+                                        uint64_t pos) {
+    const uint64_t a = pos & ~15ull;
+    if (!key_words_inside(arena_bytes, a)) return load_key_tail(arena, arena_bytes, pos);
+    const ulonglong2 *w = reinterpret_cast<const ulonglong2 *>(arena + a);
+    const ulonglong2 v0 = __ldg(w);
+    return key_of_words(v0, pos & 15 ? __ldg(w + 1) : v0, (uint32_t)pos & 15u);
 }
 
 // The key holds the end of its string (last byte NUL).
@@ -274,115 +269,13 @@ __device__ __forceinline__ void prefetch_l2(const void *p, uint64_t bytes) {
 // (stride 8) and the striped (stride 1) access patterns free of bank conflicts.
 __device__ __forceinline__ uint32_t pad(uint32_t e) { return e + (e >> 3); }
 
-// Slot of record e in a record array: padded (PK, arrays filled by the
-// threads themselves) or contiguous (arrays filled by asynchronous copies).
-template <bool PK>
-__device__ __forceinline__ uint32_t kslot(uint32_t e) {
-    if constexpr (PK)
-        return pad(e);
-    else
-        return e;
-}
-
-// ---- bitonic sort of (key, index) pairs held in registers -------------------
-// Element e = tid * ITEMS + i of a group of THREADS threads (blocked layout).
-// Strides below ITEMS run inside a thread, below 32 * ITEMS across lanes with
-// shuffles, larger ones through shared memory (groups of several warps).
-template <int ITEMS, int J>
-__device__ __forceinline__ void stage_local(Key (&k)[ITEMS], uint32_t (&x)[ITEMS], uint32_t kk,
-                                            uint32_t tid) {
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        if ((i & J) == 0) {
-            const int l = i | J;
-            const bool asc = (((tid * ITEMS + i) & kk) == 0);
-            if (pair_lt(k[l], x[l], k[i], x[i]) == asc) {
-                const Key tk = k[i];
-                k[i] = k[l];
-                k[l] = tk;
-                const uint32_t tx = x[i];
-                x[i] = x[l];
-                x[l] = tx;
-            }
-        }
-    }
-}
-
-// Bitonic sort of 32 * ITEMS pairs held by one warp (ITEMS = 2, 4 or 8):
-// lane l holds elements l * ITEMS .. l * ITEMS + ITEMS - 1.
-template <int ITEMS>
-__device__ __forceinline__ void warp_bitonic(Key (&k)[ITEMS], uint32_t (&x)[ITEMS],
-                                             uint32_t lane) {
-    constexpr uint32_t P = 32 * ITEMS;
-#pragma unroll
-    for (uint32_t kk = 2; kk <= P; kk <<= 1) {
-#pragma unroll
-        for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
-            if (j >= (uint32_t)ITEMS) {
-                const uint32_t lm = j / ITEMS;
-#pragma unroll
-                for (int i = 0; i < ITEMS; ++i) {
-                    Key ko;
-                    ko.hi = __shfl_xor_sync(0xffffffffu, k[i].hi, lm);
-                    ko.lo = __shfl_xor_sync(0xffffffffu, k[i].lo, lm);
-                    const uint32_t xo = __shfl_xor_sync(0xffffffffu, x[i], lm);
-                    const uint32_t e = lane * ITEMS + i;
-                    const bool keep_min = ((lane & lm) == 0) == ((e & kk) == 0);
-                    const bool take = keep_min ? pair_lt(ko, xo, k[i], x[i])
-                                               : pair_lt(k[i], x[i], ko, xo);
-                    if (take) {
-                        k[i] = ko;
-                        x[i] = xo;
-                    }
-                }
-            } else {
-                if constexpr (ITEMS > 4) {
-                    if (j == 4) {
-                        stage_local<ITEMS, 4>(k, x, kk, lane);
-                        continue;
-                    }
-                }
-                if constexpr (ITEMS > 2) {
-                    if (j == 2) {
-                        stage_local<ITEMS, 2>(k, x, kk, lane);
-                        continue;
-                    }
-                }
-                if constexpr (ITEMS > 1) stage_local<ITEMS, 1>(k, x, kk, lane);
-            }
-        }
-    }
-}
-
-// One warp sorts the 32 * ITEMS pairs at padded shared-memory positions
-// base .. base + 32 * ITEMS - 1 in place.
-template <int ITEMS, bool PK = true>
-__device__ __noinline__ void warp_sort_run(ulonglong2 *sk, uint32_t *sx, uint32_t base,
-                                              uint32_t lane) {
-    Key k[ITEMS];
-    uint32_t x[ITEMS];
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const uint32_t e = base + lane * ITEMS + i;
-        k[i] = to_key(sk[kslot<PK>(e)]);
-        x[i] = sx[kslot<PK>(e)];
-    }
-    warp_bitonic<ITEMS>(k, x, lane);
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const uint32_t e = base + lane * ITEMS + i;
-        sk[kslot<PK>(e)] = from_key(k[i]);
-        sx[kslot<PK>(e)] = x[i];
-    }
-}
-
 // ---- packed 64-bit sort keys -------------------------------------------------
-// Within one segment every key shares its first f bits (f = leading zeros of
-// the OR of key ^ key0 over the segment).  The 53 bits after them, with the
-// string's local position (< 2048) in the low 11 bits, form a unique 64-bit
-// sort key whose order agrees with (key, index) order except between keys
-// whose windows are equal; those pairs are checked afterwards (check_sorted)
-// and a segment with any disagreement is re-sorted with the full comparator.
+// In a segment of at most 32 strings every key shares its first f bits (f =
+// leading zeros of the OR of key ^ key0).  The 53 bits after them, with the
+// string's lane in the low bits, form a unique 64-bit sort key whose order
+// agrees with (key, index) order except between keys whose windows are equal;
+// those are checked afterwards and, on any disagreement, the segment is
+// re-sorted with the full comparator.
 constexpr uint32_t POS_BITS = 11;
 constexpr uint64_t POS_MASK = (1ull << POS_BITS) - 1;
 
@@ -402,61 +295,8 @@ __device__ __forceinline__ uint64_t sort_key(const Key &k, uint32_t f, uint32_t 
     return (window64(k, f) & ~POS_MASK) | pos;
 }
 
-template <int ITEMS, int J, typename V = uint64_t>
-__device__ __forceinline__ void stage_local64(V (&v)[ITEMS], uint32_t kk, uint32_t lane) {
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        if ((i & J) == 0) {
-            const int l = i | J;
-            const bool asc = (((lane * ITEMS + i) & kk) == 0);
-            const V a = v[i], b = v[l];
-            const bool sw = (b < a) == asc;
-            v[i] = sw ? b : a;
-            v[l] = sw ? a : b;
-        }
-    }
-}
-
-// Bitonic sort of 32 * ITEMS distinct uint64 values held by one warp (lane l
-// holds elements l * ITEMS ..), ITEMS = 1, 2, 4 or 8.
-template <int ITEMS, typename V = uint64_t>
-__device__ __forceinline__ void warp_bitonic64(V (&v)[ITEMS], uint32_t lane) {
-    constexpr uint32_t P = 32 * ITEMS;
-#pragma unroll
-    for (uint32_t kk = 2; kk <= P; kk <<= 1) {
-#pragma unroll
-        for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
-            if (j >= (uint32_t)ITEMS) {
-                const uint32_t lm = j / ITEMS;
-#pragma unroll
-                for (int i = 0; i < ITEMS; ++i) {
-                    const V o = __shfl_xor_sync(0xffffffffu, v[i], lm);
-                    const uint32_t e = lane * ITEMS + i;
-                    const bool keep_min = ((lane & lm) == 0) == ((e & kk) == 0);
-                    v[i] = keep_min ? (o < v[i] ? o : v[i]) : (o > v[i] ? o : v[i]);
-                }
-            } else {
-                if constexpr (ITEMS > 4) {
-                    if (j == 4) {
-                        stage_local64<ITEMS, 4, V>(v, kk, lane);
-                        continue;
-                    }
-                }
-                if constexpr (ITEMS > 2) {
-                    if (j == 2) {
-                        stage_local64<ITEMS, 2, V>(v, kk, lane);
-                        continue;
-                    }
-                }
-                if constexpr (ITEMS > 1) stage_local64<ITEMS, 1, V>(v, kk, lane);
-            }
-        }
-    }
-}
-
 // Merge-path split over two sorted uint64 runs (values distinct).
-template <typename V = uint64_t>
-__device__ __forceinline__ uint32_t merge_split64(const V *s, uint32_t a0, uint32_t la,
+__device__ __forceinline__ uint32_t merge_split64(const uint64_t *s, uint32_t a0, uint32_t la,
                                                   uint32_t b0, uint32_t lb, uint32_t d) {
     uint32_t lo = d > lb ? d - lb : 0, hi = d < la ? d : la;
     while (lo < hi) {
@@ -467,272 +307,6 @@ __device__ __forceinline__ uint32_t merge_split64(const V *s, uint32_t a0, uint3
             hi = mid;
     }
     return lo;
-}
-
-// Merge-path split: number of elements of run A (length la, at a0) among the
-// first d outputs of merging A with run B (length lb, at b0); ties go to A.
-template <bool PK = true>
-__device__ __forceinline__ uint32_t merge_split(const ulonglong2 *sk, const uint32_t *sx,
-                                                uint32_t a0, uint32_t la, uint32_t b0,
-                                                uint32_t lb, uint32_t d) {
-    uint32_t lo = d > lb ? d - lb : 0, hi = d < la ? d : la;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        const uint32_t pa = kslot<PK>(a0 + mid), pb = kslot<PK>(b0 + d - 1 - mid);
-        // A[mid] <= B[d-1-mid]: A[mid] is among the first d outputs.
-        if (!pair_lt(to_key(sk[pb]), sx[pb], to_key(sk[pa]), sx[pa]))
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    return lo;
-}
-
-// After a segment of `len` strings is sorted into shared memory (padded
-// layout), write its indices, LCPs and first/last keys, and emit the runs of
-// equal non-final keys as next-round segments.  Called by `threads` threads
-// numbered t = 0..threads-1.
-// Sorted position e -> shared-memory slot of its record: the slot itself
-// (records already in order) or the position field of the e-th packed key.
-template <bool IND, bool PK = true>
-__device__ __forceinline__ uint32_t rec_slot(const uint64_t *sv, uint32_t e) {
-    if constexpr (IND)
-        return kslot<PK>((uint32_t)(sv[pad(e)] & POS_MASK));
-    else
-        return kslot<PK>(e);
-}
-
-template <bool IND, bool PK = true>
-__device__ __forceinline__ void finish_segment(const SortArgs &a, const Seg &s,
-                                               const ulonglong2 *sk, const uint32_t *sx,
-                                               const uint64_t *sv, uint32_t t, uint32_t threads,
-                                               Seg *N, Counters *c) {
-    // Uniform trip count so that every warp reaches the collective append.
-    for (uint32_t e0 = 0; e0 < s.len; e0 += threads) {
-        const uint32_t e = e0 + t;
-        bool want = false;
-        uint32_t run_lo = 0;
-        if (e < s.len) {
-            const uint32_t p = s.start + e;
-            const uint32_t q = rec_slot<IND, PK>(sv, e);
-            const Key k = to_key(sk[q]);
-            a.idx[0][p] = sx[q];
-            if (e == 0 || e == s.len - 1) a.key[0][p] = from_key(k);
-            bool same_prev = false;
-            if (e > 0) {
-                const Key kp = to_key(sk[rec_slot<IND, PK>(sv, e - 1)]);
-                same_prev = key_eq(kp, k);
-                if (!same_prev)
-                    a.lcp[p] = s.depth + key_lcp(kp, k);
-                else if (key_is_end(k))
-                    a.lcp[p] = s.depth + key_len(k);
-            }
-            if (same_prev && !key_is_end(k) &&
-                (e == s.len - 1 || !key_eq(to_key(sk[rec_slot<IND, PK>(sv, e + 1)]), k))) {
-                uint32_t lo = 0, hi = e;  // first position of this run
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (key_lt(to_key(sk[rec_slot<IND, PK>(sv, mid)]), k))
-                        lo = mid + 1;
-                    else
-                        hi = mid;
-                }
-                want = true;
-                run_lo = lo;
-            }
-        }
-        emit_next_warp(N, c, want, s.start + run_lo, e - run_lo + 1, s.depth + KEY_BYTES);
-    }
-}
-
-// finish_segment for a packed sort whose order lives in sv (records in place):
-// neighbours whose windows differ get their LCP from the windows alone (all
-// keys share their first f bits, so the first differing bit is f + the
-// leading zeros of the windows' xor, and no NUL can precede it in either
-// key); only neighbours with equal windows read their full keys.  Same
-// writes and next-round runs as finish_segment<true>.
-template <bool PK>
-__device__ __forceinline__ void finish_packed(const SortArgs &a, const Seg &s,
-                                              const ulonglong2 *sk, const uint32_t *sx,
-                                              const uint64_t *sv, uint32_t f, uint32_t t,
-                                              uint32_t threads, Seg *N, Counters *c) {
-    // Uniform trip count so that every warp reaches the collective append.
-    for (uint32_t e0 = 0; e0 < s.len; e0 += threads) {
-        const uint32_t e = e0 + t;
-        bool want = false;
-        uint32_t run_lo = 0;
-        if (e < s.len) {
-            const uint32_t p = s.start + e;
-            const uint64_t v = sv[pad(e)];
-            const uint32_t q = kslot<PK>((uint32_t)(v & POS_MASK));
-            a.idx[0][p] = sx[q];
-            if (e == 0 || e == s.len - 1) a.key[0][p] = sk[q];
-            bool same_prev = false;
-            Key k = key_max();
-            if (e > 0) {
-                const uint64_t vp = sv[pad(e - 1)];
-                const uint64_t x = (v ^ vp) & ~POS_MASK;
-                if (x) {
-                    a.lcp[p] = s.depth + ((f + (uint32_t)__clzll((long long)x)) >> 3);
-                } else {
-                    k = to_key(sk[q]);
-                    const Key kp = to_key(sk[kslot<PK>((uint32_t)(vp & POS_MASK))]);
-                    same_prev = key_eq(kp, k);
-                    if (!same_prev)
-                        a.lcp[p] = s.depth + key_lcp(kp, k);
-                    else if (key_is_end(k))
-                        a.lcp[p] = s.depth + key_len(k);
-                }
-            }
-            if (same_prev && !key_is_end(k)) {
-                // a run of equal keys that do not end: is this its last record?
-                bool last = e == s.len - 1;
-                if (!last) {
-                    const uint64_t vn = sv[pad(e + 1)];
-                    last = ((v ^ vn) & ~POS_MASK) != 0 ||
-                           !key_eq(to_key(sk[kslot<PK>((uint32_t)(vn & POS_MASK))]), k);
-                }
-                if (last) {
-                    uint32_t lo = 0, hi = e;  // first position of this run
-                    while (lo < hi) {
-                        const uint32_t mid = (lo + hi) >> 1;
-                        const uint32_t qm = kslot<PK>((uint32_t)(sv[pad(mid)] & POS_MASK));
-                        if (key_lt(to_key(sk[qm]), k))
-                            lo = mid + 1;
-                        else
-                            hi = mid;
-                    }
-                    want = true;
-                    run_lo = lo;
-                }
-            }
-        }
-        emit_next_warp(N, c, want, s.start + run_lo, e - run_lo + 1, s.depth + KEY_BYTES);
-    }
-}
-
-// True when the sorted order (through the packed keys) agrees with full
-// (key, index) order wherever the packed keys could not tell records apart
-// (equal windows).  Called by `threads` threads numbered t; per-thread verdict.
-template <bool PK = true>
-__device__ __forceinline__ bool window_pairs_ok_ind(const ulonglong2 *sk, const uint64_t *sv,
-                                                    uint32_t len, uint32_t t, uint32_t threads) {
-    bool ok = true;
-    for (uint32_t e = t + 1; e < len; e += threads) {
-        const uint64_t va = sv[pad(e - 1)], vb = sv[pad(e)];
-        if ((va >> POS_BITS) == (vb >> POS_BITS)) {
-            const Key kp = to_key(sk[kslot<PK>((uint32_t)(va & POS_MASK))]);
-            const Key k = to_key(sk[kslot<PK>((uint32_t)(vb & POS_MASK))]);
-            if (key_lt(k, kp)) ok = false;
-        }
-    }
-    return ok;
-}
-
-// Runs of equal windows after a packed sort hold their records in position
-// order.  window_runs_short: no run is longer than FIX_RUN_CAP (else the
-// caller sorts the whole segment with the full comparator).  sort_window_runs:
-// the thread that owns a run's first element puts the run into full (key,
-// position) order in place (insertion sort: equal keys keep position order).
-// Runs are disjoint and every entry of a run has the run's window bits, so
-// the neighbours another thread reads keep their windows while it sorts.
-constexpr uint32_t FIX_RUN_CAP = 64;
-
-__device__ __forceinline__ bool window_run_start(const uint64_t *sv, uint32_t len, uint32_t e) {
-    const uint64_t w = sv[pad(e)] >> POS_BITS;
-    return e + 1 < len && (sv[pad(e + 1)] >> POS_BITS) == w &&
-           (e == 0 || (sv[pad(e - 1)] >> POS_BITS) != w);
-}
-
-__device__ __forceinline__ bool window_runs_short(const uint64_t *sv, uint32_t len, uint32_t t,
-                                                  uint32_t threads) {
-    for (uint32_t e = t; e + 1 < len; e += threads) {
-        if (!window_run_start(sv, len, e)) continue;
-        const uint64_t w = sv[pad(e)] >> POS_BITS;
-        const uint32_t r = min(len, e + FIX_RUN_CAP + 1);
-        uint32_t q = e + 2;
-        while (q < r && (sv[pad(q)] >> POS_BITS) == w) ++q;
-        if (q - e > FIX_RUN_CAP) return false;
-    }
-    return true;
-}
-
-template <bool PK = true>
-__device__ __forceinline__ void sort_window_runs(const ulonglong2 *sk, uint64_t *sv, uint32_t len,
-                                                 uint32_t t, uint32_t threads) {
-    for (uint32_t e = t; e + 1 < len; e += threads) {
-        if (!window_run_start(sv, len, e)) continue;
-        const uint64_t w = sv[pad(e)] >> POS_BITS;
-        uint32_t r = e + 2;
-        while (r < len && (sv[pad(r)] >> POS_BITS) == w) ++r;
-        for (uint32_t i = e + 1; i < r; ++i) {
-            const uint64_t v = sv[pad(i)];
-            const Key kv = to_key(sk[kslot<PK>((uint32_t)(v & POS_MASK))]);
-            uint32_t j = i;
-            while (j > e) {
-                const uint64_t u = sv[pad(j - 1)];
-                if (!key_lt(kv, to_key(sk[kslot<PK>((uint32_t)(u & POS_MASK))]))) break;
-                sv[pad(j)] = u;
-                --j;
-            }
-            sv[pad(j)] = v;
-        }
-    }
-}
-
-// 32-bit packed keys for a first sort: the 21 window bits after the common
-// prefix and the 11-bit position.  Their order is the 64-bit packed order
-// except among keys whose 21 bits tie; see block_class.
-constexpr uint32_t NARROW_SHIFT = 64 - 21;  // 64-bit packed key >> this = the 21 bits
-
-__device__ __forceinline__ uint32_t sort_key32(const Key &k, uint32_t f, uint32_t pos) {
-    return (uint32_t)(window64(k, f) >> 32) & ~(uint32_t)POS_MASK | pos;
-}
-
-// In sv[0..len), the 64-bit packed keys of records in 32-bit order: runs of
-// keys whose top 21 bits tie are put into 64-bit order in place by the
-// thread that owns the run's first entry (insertion sort); returns false in
-// that thread when a run is longer than FIX_RUN_CAP (the caller then sorts
-// the segment on 64-bit keys from scratch).
-__device__ __forceinline__ bool sort_narrow_runs(uint64_t *sv, uint32_t len, uint32_t t,
-                                                 uint32_t threads) {
-    bool ok = true;
-    for (uint32_t e = t; e + 1 < len; e += threads) {
-        const uint64_t w = sv[pad(e)] >> NARROW_SHIFT;
-        if ((sv[pad(e + 1)] >> NARROW_SHIFT) != w) continue;
-        if (e > 0 && (sv[pad(e - 1)] >> NARROW_SHIFT) == w) continue;  // not the run's start
-        uint32_t r = e + 2;
-        while (r < len && (sv[pad(r)] >> NARROW_SHIFT) == w && r - e <= FIX_RUN_CAP) ++r;
-        if (r - e > FIX_RUN_CAP) {
-            ok = false;
-            continue;
-        }
-        for (uint32_t i = e + 1; i < r; ++i) {
-            const uint64_t v = sv[pad(i)];
-            uint32_t j = i;
-            while (j > e && sv[pad(j - 1)] > v) {
-                sv[pad(j)] = sv[pad(j - 1)];
-                --j;
-            }
-            sv[pad(j)] = v;
-        }
-    }
-    return ok;
-}
-
-template <int ITEMS>
-__device__ __forceinline__ void warp_run_packed32(const ulonglong2 *sk, uint32_t *sv32,
-                                                  uint32_t base, uint32_t len, uint32_t f,
-                                                  uint32_t lane) {
-    uint32_t v[ITEMS];
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const uint32_t e = base + lane * ITEMS + i;
-        v[i] = e < len ? sort_key32(to_key(sk[pad(e)]), f, e) : ~0u;
-    }
-    warp_bitonic64<ITEMS, uint32_t>(v, lane);
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) sv32[pad(base + lane * ITEMS + i)] = v[i];
 }
 
 // Compare-exchange: afterwards a <= b.
@@ -797,28 +371,6 @@ __device__ __forceinline__ void warp_merge_sort64(uint64_t (&v)[ITEMS], uint64_t
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) sv[pad(base + o + i)] = v[i];
         __syncwarp();
-    }
-}
-
-// One warp: packed keys of the records at slots base .. base + 32*ITEMS - 1
-// (positions >= len pad with all-ones), sorted, stored to sv; by the bitonic
-// network or (MERGE) by warp_merge_sort64.
-template <int ITEMS, bool MERGE = false>
-__device__ __forceinline__ void warp_run_packed(const ulonglong2 *sk, uint64_t *sv,
-                                                uint32_t base, uint32_t len, uint32_t f,
-                                                uint32_t lane) {
-    uint64_t v[ITEMS];
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const uint32_t e = base + lane * ITEMS + i;
-        v[i] = e < len ? sort_key(to_key(sk[pad(e)]), f, e) : ~0ull;
-    }
-    if constexpr (MERGE) {
-        warp_merge_sort64<ITEMS>(v, sv, base, lane);
-    } else {
-        warp_bitonic64<ITEMS>(v, lane);
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) sv[pad(base + lane * ITEMS + i)] = v[i];
     }
 }
 
@@ -2494,423 +2046,7 @@ __global__ void __launch_bounds__(WARP_THREADS) k_warp1(SortArgs a, const Seg *_
     if (lane == 0 && deep) atomicAdd(&c->warp1_deep, deep);
 }
 
-// Warp-wide OR of key ^ key0 over the records at padded positions 0..len-1.
-__device__ __forceinline__ uint32_t warp_diff_bit(const ulonglong2 *sk, uint32_t len,
-                                                  uint32_t lane) {
-    const Key k0 = to_key(sk[pad(0)]);
-    uint64_t dh = 0, dl = 0;
-    for (uint32_t e = lane; e < len; e += 32) {
-        const Key k = to_key(sk[pad(e)]);
-        dh |= k.hi ^ k0.hi;
-        dl |= k.lo ^ k0.lo;
-    }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        dh |= __shfl_xor_sync(0xffffffffu, dh, d);
-        dl |= __shfl_xor_sync(0xffffffffu, dl, d);
-    }
-    return (dh | dl) ? clz128(dh, dl) : 128u;
-}
-
-// ---- segments of 33..256 strings: one warp, 2/4/8 strings per lane ----------
-constexpr int W8_PAD = WARP8_CAP + WARP8_CAP / 8;
-constexpr int W8_WARPS = WARP_THREADS / 32;
-constexpr size_t W8_SMEM = (size_t)W8_WARPS * W8_PAD * (sizeof(ulonglong2) + sizeof(uint64_t) +
-                                                         sizeof(uint32_t));
-
-__global__ void __launch_bounds__(WARP_THREADS, 3) k_warp8(SortArgs a, const Seg *__restrict__ T0,
-                                                           Span sp, Seg *N, Counters *c) {
-    const uint32_t lo = count_of(sp.lo);
-    const Seg *__restrict__ T = T0 + lo;
-    const uint32_t nT = count_of(sp.hi) - lo;
-    extern __shared__ __align__(16) unsigned char w8_smem[];
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    ulonglong2 *sk = reinterpret_cast<ulonglong2 *>(w8_smem) + w * W8_PAD;
-    uint64_t *sv = reinterpret_cast<uint64_t *>(reinterpret_cast<ulonglong2 *>(w8_smem) +
-                                                W8_WARPS * W8_PAD) + w * W8_PAD;
-    uint32_t *sx = reinterpret_cast<uint32_t *>(reinterpret_cast<uint64_t *>(
-                       reinterpret_cast<ulonglong2 *>(w8_smem) + W8_WARPS * W8_PAD) +
-                                                W8_WARPS * W8_PAD) + w * W8_PAD;
-    const uint32_t warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    unsigned long long fresh = 0, keyed = 0, full = 0;
-    for (uint32_t g = warp0; g < nT; g += nwarps) {
-        const Seg s = T[g];
-        if (s.flags & SEG_KEYS)
-            keyed += s.len;
-        else
-            fresh += s.len;
-        const uint32_t P = next_pow2(s.len);
-        {
-            // All loads first (P <= 8 * 32), then the shared-memory stores.
-            Key kk[8];
-            uint32_t ii[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const uint32_t e = lane + c * 32;
-                kk[c] = key_max();
-                ii[c] = IDX_MAX;
-                if (e < s.len) load_elem(a, s, e, kk[c], ii[c]);
-            }
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const uint32_t e = lane + c * 32;
-                if (e < P) {
-                    sk[pad(e)] = from_key(kk[c]);
-                    sx[pad(e)] = ii[c];
-                }
-            }
-        }
-        __syncwarp();
-        const uint32_t f = warp_diff_bit(sk, s.len, lane);
-        bool packed = false;
-        if (f < 128) {
-            if (a.warp_merge) {
-                if (P <= 64)
-                    warp_run_packed<2, true>(sk, sv, 0, s.len, f, lane);
-                else if (P <= 128)
-                    warp_run_packed<4, true>(sk, sv, 0, s.len, f, lane);
-                else
-                    warp_run_packed<8, true>(sk, sv, 0, s.len, f, lane);
-            } else {
-                if (P <= 64)
-                    warp_run_packed<2>(sk, sv, 0, s.len, f, lane);
-                else if (P <= 128)
-                    warp_run_packed<4>(sk, sv, 0, s.len, f, lane);
-                else
-                    warp_run_packed<8>(sk, sv, 0, s.len, f, lane);
-            }
-            __syncwarp();
-            packed = __all_sync(0xffffffffu, window_pairs_ok_ind(sk, sv, s.len, lane, 32));
-            if (!packed) {
-                packed = __all_sync(0xffffffffu, window_runs_short(sv, s.len, lane, 32));
-                if (packed) sort_window_runs(sk, sv, s.len, lane, 32);
-            }
-            if (!packed) {
-                full += s.len;
-                if (P <= 64)
-                    warp_sort_run<2>(sk, sx, 0, lane);
-                else if (P <= 128)
-                    warp_sort_run<4>(sk, sx, 0, lane);
-                else
-                    warp_sort_run<8>(sk, sx, 0, lane);
-            }
-        }
-        __syncwarp();
-        if (packed)
-            finish_segment<true>(a, s, sk, sx, sv, lane, 32, N, c);
-        else
-            finish_segment<false>(a, s, sk, sx, sv, lane, 32, N, c);
-        __syncwarp();
-    }
-    if (lane == 0 && (fresh | keyed)) {
-        atomicAdd(&c->warp8_fresh, fresh);
-        atomicAdd(&c->warp8_keyed, keyed);
-        if (full) atomicAdd(&c->full_sorted, full);
-    }
-}
-
-// ---- segments of 257..SMALL_CAP strings: groups of threads -----------------
-// A CTA of SMALL_THREADS threads is split into groups of GT threads (2, 4 or
-// 8 warps); each group sorts one segment of up to GT * SMALL_ITEMS strings at a
-// time and synchronises on its own named barrier.  Segments are bucketed by
-// size so that every thread holds 5..8 strings: small segments do not leave
-// warps idle at CTA-wide barriers, and one SM overlaps the loads and sorts of
-// up to 12 segments.
-constexpr int SMALL_PAD = SMALL_CAP + SMALL_CAP / 8;
-constexpr size_t BLOCK_SMEM = SMALL_PAD * (sizeof(ulonglong2) + sizeof(uint32_t) + sizeof(uint64_t));
-constexpr uint32_t BLOCK_RUN = 32 * SMALL_ITEMS;  // one warp's run of packed keys
-
-// Barrier among the GT threads of group gi: named barrier 1 + gi (0 is
-// __syncthreads).  Immediate ids, so that a CTA claims only the barriers it
-// uses (at most 5) and the SM's barriers do not limit occupancy.
-template <int GT>
-__device__ __forceinline__ void group_sync(uint32_t gi) {
-    constexpr int G = SMALL_THREADS / GT;
-    if (G == 1 || gi == 0)
-        asm volatile("bar.sync 1, %0;" ::"n"(GT) : "memory");
-    else if (G == 2 || gi == 1)
-        asm volatile("bar.sync 2, %0;" ::"n"(GT) : "memory");
-    else if (gi == 2)
-        asm volatile("bar.sync 3, %0;" ::"n"(GT) : "memory");
-    else
-        asm volatile("bar.sync 4, %0;" ::"n"(GT) : "memory");
-}
-
-// Full-comparator sort of the span (multiple of BLOCK_RUN) records at padded
-// positions 0..span-1 by the GT threads of a group (thread t): warp runs, then
-// pairwise merge-path merges.
-template <int GT, bool PK = true>
-__device__ __noinline__ void group_sort_full(ulonglong2 *sk, uint32_t *sx, uint32_t span,
-                                             uint32_t t, uint32_t gi) {
-    const uint32_t nruns = span / BLOCK_RUN;
-    const uint32_t lane = t & 31, gw = t >> 5;
-    if (gw < nruns) warp_sort_run<SMALL_ITEMS, PK>(sk, sx, gw * BLOCK_RUN, lane);
-    group_sync<GT>(gi);
-    for (uint32_t run = BLOCK_RUN; run < span; run <<= 1) {
-        const uint32_t o = t * SMALL_ITEMS;
-        Key ok[SMALL_ITEMS];
-        uint32_t ox[SMALL_ITEMS];
-        const bool active = o < span;
-        if (active) {
-            const uint32_t a0 = o & ~(2 * run - 1);  // run: a power of two
-            const uint32_t b0 = a0 + run;
-            const uint32_t la = min(run, span - a0);
-            const uint32_t lb = b0 < span ? min(run, span - b0) : 0u;
-            const uint32_t d = o - a0;
-            uint32_t ia = merge_split<PK>(sk, sx, a0, la, b0, lb, d);
-            uint32_t ib = d - ia;
-#pragma unroll
-            for (int i = 0; i < SMALL_ITEMS; ++i) {
-                bool take_a = ib >= lb;
-                Key ka, kb;
-                uint32_t xa = 0, xb = 0;
-                if (ia < la) {
-                    ka = to_key(sk[kslot<PK>(a0 + ia)]);
-                    xa = sx[kslot<PK>(a0 + ia)];
-                }
-                if (ib < lb) {
-                    kb = to_key(sk[kslot<PK>(b0 + ib)]);
-                    xb = sx[kslot<PK>(b0 + ib)];
-                    if (ia < la) take_a = !pair_lt(kb, xb, ka, xa);
-                }
-                if (take_a) {
-                    ok[i] = ka;
-                    ox[i] = xa;
-                    ++ia;
-                } else {
-                    ok[i] = kb;
-                    ox[i] = xb;
-                    ++ib;
-                }
-            }
-        }
-        group_sync<GT>(gi);
-        if (active) {
-#pragma unroll
-            for (int i = 0; i < SMALL_ITEMS; ++i) {
-                sk[kslot<PK>(o + i)] = from_key(ok[i]);
-                sx[kslot<PK>(o + i)] = ox[i];
-            }
-        }
-        group_sync<GT>(gi);
-    }
-}
-
-// Pairwise merge-path merges of the sorted packed-key runs of BLOCK_RUN in
-// sv[0..span) until one run is left; SMALL_ITEMS outputs per thread and pass.
-template <int GT, typename V = uint64_t>
-__device__ __forceinline__ void group_merge_passes64(V *sv, uint32_t span, uint32_t t,
-                                                     uint32_t gi) {
-    constexpr V VMAX = (V)~(V)0;
-    for (uint32_t run = BLOCK_RUN; run < span; run <<= 1) {
-        const uint32_t o = t * SMALL_ITEMS;
-        V ov[SMALL_ITEMS];
-        const bool active = o < span;
-        if (active) {
-            const uint32_t a0 = o & ~(2 * run - 1);  // run: a power of two
-            const uint32_t b0 = a0 + run;
-            const uint32_t la = min(run, span - a0);
-            const uint32_t lb = b0 < span ? min(run, span - b0) : 0u;
-            const uint32_t d = o - a0;
-            uint32_t ia = merge_split64<V>(sv, a0, la, b0, lb, d);
-            uint32_t ib = d - ia;
-#pragma unroll
-            for (int i = 0; i < SMALL_ITEMS; ++i) {
-                const V va = ia < la ? sv[pad(a0 + ia)] : VMAX;
-                const V vb = ib < lb ? sv[pad(b0 + ib)] : VMAX;
-                const bool take_a = ib >= lb || (ia < la && va < vb);
-                ov[i] = take_a ? va : vb;
-                ia += take_a;
-                ib += !take_a;
-            }
-        }
-        group_sync<GT>(gi);
-        if (active) {
-#pragma unroll
-            for (int i = 0; i < SMALL_ITEMS; ++i) sv[pad(o + i)] = ov[i];
-        }
-        group_sync<GT>(gi);
-    }
-}
-
-// The CTAs cta0 .. cta0 + ncta - 1 of the launch sort the segments of one
-// size class (list S of nS segments) with groups of GT threads.  LEAN: the
-// finish takes neighbour LCPs from the packed windows (finish_packed).
-// VAR 0: full-key finish; 1: LEAN; 2: LEAN, and the first sort is on 32-bit
-// packed keys (half the work of the 64-bit network), widened to 64-bit keys
-// afterwards; ties on their 21 window bits are then put in order in place.
-template <int GT, int VAR = 0>
-__device__ __forceinline__ void block_class(const SortArgs &a, const Seg *__restrict__ S,
-                                            uint32_t nS, uint32_t cta0, uint32_t ncta, Seg *N,
-                                            Counters *c) {
-    constexpr uint32_t G = SMALL_THREADS / GT;          // groups per CTA
-    constexpr uint32_t CAP = GT * SMALL_ITEMS;          // strings per group
-    constexpr uint32_t PADC = CAP + CAP / 8;            // padded slots per group
-    static_assert(G * PADC == SMALL_PAD, "group slots");
-    extern __shared__ __align__(16) unsigned char block_smem[];
-    __shared__ uint64_t red[2][SMALL_THREADS / 32];
-    __shared__ int ok_flag[G], fix_flag[G], nar_flag[G];
-    constexpr bool LEAN = VAR >= 1;
-    const uint32_t gi = threadIdx.x / GT, t = threadIdx.x % GT;
-    const uint32_t lane = threadIdx.x & 31, gw = t >> 5, w = threadIdx.x >> 5;
-    ulonglong2 *sk_all = reinterpret_cast<ulonglong2 *>(block_smem);
-    uint64_t *sv_all = reinterpret_cast<uint64_t *>(sk_all + SMALL_PAD);
-    uint32_t *sx_all = reinterpret_cast<uint32_t *>(sv_all + SMALL_PAD);
-    ulonglong2 *sk = sk_all + gi * PADC;
-    uint64_t *sv = sv_all + gi * PADC;
-    uint32_t *sx = sx_all + gi * PADC;
-    unsigned long long fresh = 0, keyed = 0, full = 0;
-    for (uint32_t g = (blockIdx.x - cta0) * G + gi; g < nS; g += ncta * G) {
-        const Seg s = S[g];
-        if (s.flags & SEG_KEYS)
-            keyed += s.len;
-        else
-            fresh += s.len;
-        const uint32_t nruns = (s.len + BLOCK_RUN - 1) / BLOCK_RUN;
-        const uint32_t span = nruns * BLOCK_RUN;
-        {
-            // All of a thread's loads first (span <= SMALL_ITEMS * GT), so
-            // that they are in flight together, then the shared-memory stores.
-            Key kk[SMALL_ITEMS];
-            uint32_t ii[SMALL_ITEMS];
-#pragma unroll
-            for (int c = 0; c < SMALL_ITEMS; ++c) {
-                const uint32_t e = t + c * GT;
-                kk[c] = key_max();
-                ii[c] = IDX_MAX;
-                if (e < s.len) load_elem(a, s, e, kk[c], ii[c]);
-            }
-#pragma unroll
-            for (int c = 0; c < SMALL_ITEMS; ++c) {
-                const uint32_t e = t + c * GT;
-                if (e < span) {
-                    sk[pad(e)] = from_key(kk[c]);
-                    sx[pad(e)] = ii[c];
-                }
-            }
-        }
-        if (t == 0) ok_flag[gi] = fix_flag[gi] = nar_flag[gi] = 1;
-        group_sync<GT>(gi);
-        // f: first bit in which the keys differ.
-        {
-            const Key k0 = to_key(sk[pad(0)]);
-            uint64_t dh = 0, dl = 0;
-            for (uint32_t e = t; e < s.len; e += GT) {
-                const Key k = to_key(sk[pad(e)]);
-                dh |= k.hi ^ k0.hi;
-                dl |= k.lo ^ k0.lo;
-            }
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) {
-                dh |= __shfl_xor_sync(0xffffffffu, dh, d);
-                dl |= __shfl_xor_sync(0xffffffffu, dl, d);
-            }
-            if (lane == 0) {
-                red[0][w] = dh;
-                red[1][w] = dl;
-            }
-        }
-        group_sync<GT>(gi);
-        uint64_t dh = 0, dl = 0;
-#pragma unroll
-        for (uint32_t q = 0; q < GT / 32; ++q) {
-            dh |= red[0][gi * (GT / 32) + q];
-            dl |= red[1][gi * (GT / 32) + q];
-        }
-        bool packed = false;
-        const uint32_t f = (dh | dl) ? clz128(dh, dl) : 128u;
-        if (f < 128) {
-            bool sorted64 = false;
-            if constexpr (VAR == 2) {
-                uint32_t *sv32 = reinterpret_cast<uint32_t *>(sv);  // same bytes
-                if (gw < nruns)
-                    warp_run_packed32<SMALL_ITEMS>(sk, sv32, gw * BLOCK_RUN, s.len, f, lane);
-                group_sync<GT>(gi);
-                group_merge_passes64<GT, uint32_t>(sv32, span, t, gi);
-                // Widen to 64-bit packed keys in this order; the two arrays
-                // share their bytes, so the values pass through registers.
-                const uint32_t o = t * SMALL_ITEMS;
-                uint32_t pv[SMALL_ITEMS];
-#pragma unroll
-                for (int i = 0; i < SMALL_ITEMS; ++i)
-                    pv[i] = o + i < span ? sv32[pad(o + i)] : 0u;
-                group_sync<GT>(gi);
-#pragma unroll
-                for (int i = 0; i < SMALL_ITEMS; ++i) {
-                    const uint32_t e = o + i;
-                    if (e < s.len) {
-                        const uint32_t pos = pv[i] & (uint32_t)POS_MASK;
-                        sv[pad(e)] = sort_key(to_key(sk[pad(pos)]), f, pos);
-                    }
-                }
-                group_sync<GT>(gi);
-                if (!sort_narrow_runs(sv, s.len, t, GT)) nar_flag[gi] = 0;
-                group_sync<GT>(gi);
-                sorted64 = nar_flag[gi] != 0;
-            }
-            if (!sorted64) {
-                if (gw < nruns) {
-                    if (a.warp_merge)
-                        warp_run_packed<SMALL_ITEMS, true>(sk, sv, gw * BLOCK_RUN, s.len, f, lane);
-                    else
-                        warp_run_packed<SMALL_ITEMS>(sk, sv, gw * BLOCK_RUN, s.len, f, lane);
-                }
-                group_sync<GT>(gi);
-                group_merge_passes64<GT>(sv, span, t, gi);
-            }
-            if (!window_pairs_ok_ind(sk, sv, s.len, t, GT)) ok_flag[gi] = 0;
-            group_sync<GT>(gi);
-            packed = ok_flag[gi] != 0;
-            if (!packed) {
-                if (!window_runs_short(sv, s.len, t, GT)) fix_flag[gi] = 0;
-                group_sync<GT>(gi);
-                packed = fix_flag[gi] != 0;
-                if (packed) {
-                    sort_window_runs(sk, sv, s.len, t, GT);
-                } else {
-                    if (t == 0) full += s.len;
-                    group_sort_full<GT>(sk, sx, span, t, gi);
-                }
-            }
-        }
-        group_sync<GT>(gi);
-        if (packed && LEAN)
-            finish_packed<true>(a, s, sk, sx, sv, f, t, GT, N, c);
-        else if (packed)
-            finish_segment<true>(a, s, sk, sx, sv, t, GT, N, c);
-        else
-            finish_segment<false>(a, s, sk, sx, sv, t, GT, N, c);
-        group_sync<GT>(gi);
-    }
-    if (t == 0 && (fresh | keyed)) {
-        atomicAdd(&c->block_fresh, fresh);
-        atomicAdd(&c->block_keyed, keyed);
-        if (full) atomicAdd(&c->full_sorted, full);
-    }
-}
-
-// One size class per launch (a single launch for all three inlines all
-// three bodies and spills more; measured slower).
-template <int GT, int VAR>
-__global__ void __launch_bounds__(SMALL_THREADS, 3) k_block(SortArgs a, const Seg *__restrict__ S,
-                                                            Span sp, Seg *N, Counters *c) {
-    const uint32_t lo = count_of(sp.lo);
-    block_class<GT, VAR>(a, S + lo, count_of(sp.hi) - lo, 0, gridDim.x, N, c);
-}
-
-// ---- segments of 257..SMALL_CAP strings, with the next segment prefetched ---
-// The same thread groups and sort as k_block, but a group's records (16-byte
-// key, index) of a keyed segment reach shared memory through cp.async (global
-// -> shared copies that bypass the registers), issued for the group's NEXT
-// segment before it sorts the current one, so that the copy runs under the
-// sort.  Two record buffers per group (contiguous slots: the copies cannot
-// write the padded layout); the packed keys are built from the records
-// loaded once into registers.  Segments without keys at their depth (fresh)
-// are gathered by the group's threads as in k_block.
-constexpr size_t BLOCK2_SMEM =
-    2 * (size_t)SMALL_CAP * (sizeof(ulonglong2) + sizeof(uint32_t)) + SMALL_PAD * sizeof(uint64_t);
-
+// ---- asynchronous copies into shared memory -----------------------------------
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem) : "memory");
@@ -2928,171 +2064,729 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int GT>
-__device__ __forceinline__ void block2_class(const SortArgs &a, const Seg *__restrict__ S,
-                                             uint32_t nS, Seg *N, Counters *c) {
-    constexpr uint32_t G = SMALL_THREADS / GT;  // groups per CTA
-    constexpr uint32_t CAP = GT * SMALL_ITEMS;  // strings per group
-    constexpr uint32_t PADC = CAP + CAP / 8;    // padded packed-key slots per group
-    static_assert(G * PADC == SMALL_PAD, "group slots");
-    extern __shared__ __align__(16) unsigned char block_smem[];
-    __shared__ uint64_t red[2][SMALL_THREADS / 32];
-    __shared__ int ok_flag[G], fix_flag[G];
-    const uint32_t gi = threadIdx.x / GT, t = threadIdx.x % GT;
-    const uint32_t lane = threadIdx.x & 31, gw = t >> 5, w = threadIdx.x >> 5;
-    ulonglong2 *rk_all = reinterpret_cast<ulonglong2 *>(block_smem);  // [2][SMALL_CAP]
-    uint32_t *rx_all = reinterpret_cast<uint32_t *>(rk_all + 2 * SMALL_CAP);
-    uint64_t *sv = reinterpret_cast<uint64_t *>(rx_all + 2 * SMALL_CAP) + gi * PADC;
-    unsigned long long fresh = 0, keyed = 0, full = 0;
-    const uint32_t stride = gridDim.x * G;
-    // Copies of a keyed segment's records into record buffer `buf`; every
-    // thread commits one copy group per call (empty when there is nothing).
-    auto prefetch = [&](const Seg &q, uint32_t buf) {
-        if (q.len && (q.flags & SEG_KEYS)) {
-            const int b = q.flags & SEG_BUF1;
-            const ulonglong2 *K = a.keyb(b) + q.start;
-            const uint32_t *I = a.idxb(b) + q.start;
-            ulonglong2 *dk = rk_all + buf * SMALL_CAP + gi * CAP;
-            uint32_t *dx = rx_all + buf * SMALL_CAP + gi * CAP;
+// Keys at `depth` of up to G strings per lane: elements e0 + q * stride below
+// len of the index array I.  Every step's loads are issued for all G strings
+// before any is used (index, then offset, then the two 16-byte words that
+// hold the key), so that G chains of dependent reads overlap.
+template <int G>
+__device__ __forceinline__ void gather_keys(const SortArgs &a, const uint32_t *__restrict__ I,
+                                            uint32_t depth, uint32_t e0, uint32_t stride,
+                                            uint32_t len, Key (&kk)[G], uint32_t (&ii)[G]) {
+    uint64_t pos[G];
+    ulonglong2 v0[G], v1[G];
 #pragma unroll
-            for (int cc = 0; cc < SMALL_ITEMS; ++cc) {
-                const uint32_t e = t + cc * GT;
-                if (e < q.len) {
-                    cp_async16(dk + e, K + e);
-                    cp_async4(dx + e, I + e);
-                }
-            }
-        }
-        cp_async_commit();
-    };
-    const Seg none{0, 0, 0, 0};
-    uint32_t g = blockIdx.x * G + gi;
-    Seg s_cur = g < nS ? S[g] : none;
-    Seg s_nxt = g + stride < nS ? S[g + stride] : none;
-    prefetch(s_cur, 0);
-    uint32_t cb = 0;
-    for (; g < nS; g += stride, cb ^= 1) {
-        const Seg s = s_cur;
-        prefetch(s_nxt, cb ^ 1);
-        s_cur = s_nxt;
-        s_nxt = g + 2 * stride < nS ? S[g + 2 * stride] : none;
-        ulonglong2 *sk = rk_all + cb * SMALL_CAP + gi * CAP;
-        uint32_t *sx = rx_all + cb * SMALL_CAP + gi * CAP;
-        if (s.flags & SEG_KEYS) {
-            keyed += s.len;
-        } else {
-            fresh += s.len;
-            // Gather at this depth: all of a thread's loads first.
-            Key kk[SMALL_ITEMS];
-            uint32_t ii[SMALL_ITEMS];
+    for (int q = 0; q < G; ++q) ii[q] = e0 + q * stride < len ? I[e0 + q * stride] : IDX_MAX;
 #pragma unroll
-            for (int cc = 0; cc < SMALL_ITEMS; ++cc) {
-                const uint32_t e = t + cc * GT;
-                if (e < s.len) load_elem(a, s, e, kk[cc], ii[cc]);
-            }
+    for (int q = 0; q < G; ++q)
+        pos[q] = ii[q] != IDX_MAX ? string_offset(a.offs, a.off_width, ii[q]) + depth : 0ull;
 #pragma unroll
-            for (int cc = 0; cc < SMALL_ITEMS; ++cc) {
-                const uint32_t e = t + cc * GT;
-                if (e < s.len) {
-                    sk[e] = from_key(kk[cc]);
-                    sx[e] = ii[cc];
-                }
-            }
-        }
-        cp_async_wait<1>();  // this segment's copies (the next one's may run on)
-        if (t == 0) ok_flag[gi] = fix_flag[gi] = 1;
-        group_sync<GT>(gi);
-        // f: first bit in which the keys differ (thread t's records are
-        // t, t + GT, ...; contiguous across threads, so no bank conflicts).
-        {
-            const Key k0 = to_key(sk[0]);
-            uint64_t dh = 0, dl = 0;
-#pragma unroll
-            for (int cc = 0; cc < SMALL_ITEMS; ++cc) {
-                const uint32_t e = t + cc * GT;
-                if (e < s.len) {
-                    const Key k = to_key(sk[e]);
-                    dh |= k.hi ^ k0.hi;
-                    dl |= k.lo ^ k0.lo;
-                }
-            }
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) {
-                dh |= __shfl_xor_sync(0xffffffffu, dh, d);
-                dl |= __shfl_xor_sync(0xffffffffu, dl, d);
-            }
-            if (lane == 0) {
-                red[0][w] = dh;
-                red[1][w] = dl;
-            }
-        }
-        group_sync<GT>(gi);
-        uint64_t dh = 0, dl = 0;
-#pragma unroll
-        for (uint32_t q = 0; q < GT / 32; ++q) {
-            dh |= red[0][gi * (GT / 32) + q];
-            dl |= red[1][gi * (GT / 32) + q];
-        }
-        bool packed = false;
-        const uint32_t f = (dh | dl) ? clz128(dh, dl) : 128u;
-        if (f < 128) {
-            // Every warp of the group sorts the packed keys of its own
-            // records (t, t + GT, ...; any split of the records works: the
-            // position in the low bits identifies each one); positions past
-            // the end pad as distinct values above every real one.
-            uint64_t v[SMALL_ITEMS];
-#pragma unroll
-            for (int cc = 0; cc < SMALL_ITEMS; ++cc) {
-                const uint32_t e = t + cc * GT;
-                v[cc] = e < s.len ? sort_key(to_key(sk[e]), f, e) : ((~0ull << POS_BITS) | e);
-            }
-            warp_bitonic64<SMALL_ITEMS>(v, lane);
-#pragma unroll
-            for (int i = 0; i < SMALL_ITEMS; ++i) sv[pad(gw * BLOCK_RUN + lane * SMALL_ITEMS + i)] = v[i];
-            group_sync<GT>(gi);
-            group_merge_passes64<GT>(sv, CAP, t, gi);
-            if (!window_pairs_ok_ind<false>(sk, sv, s.len, t, GT)) ok_flag[gi] = 0;
-            group_sync<GT>(gi);
-            packed = ok_flag[gi] != 0;
-            if (!packed) {
-                if (!window_runs_short(sv, s.len, t, GT)) fix_flag[gi] = 0;
-                group_sync<GT>(gi);
-                packed = fix_flag[gi] != 0;
-                if (packed) {
-                    sort_window_runs<false>(sk, sv, s.len, t, GT);
-                } else {
-                    // Full comparator over the whole group span (rare): the
-                    // slots past the end sort last.
-                    for (uint32_t e = s.len + t; e < CAP; e += GT) {
-                        sk[e] = from_key(key_max());
-                        sx[e] = IDX_MAX;
-                    }
-                    group_sync<GT>(gi);
-                    if (t == 0) full += s.len;
-                    group_sort_full<GT, false>(sk, sx, CAP, t, gi);
-                }
-            }
-        }
-        group_sync<GT>(gi);
-        if (packed)
-            finish_packed<false>(a, s, sk, sx, sv, f, t, GT, N, c);
-        else
-            finish_segment<false, false>(a, s, sk, sx, sv, t, GT, N, c);
-        group_sync<GT>(gi);
+    for (int q = 0; q < G; ++q) {
+        const uint64_t at = pos[q] & ~15ull;
+        const bool in = ii[q] != IDX_MAX && key_words_inside(a.arena_bytes, at);
+        const ulonglong2 *w = reinterpret_cast<const ulonglong2 *>(a.arena + at);
+        v0[q] = in ? __ldg(w) : make_ulonglong2(0, 0);
+        v1[q] = in && (pos[q] & 15) ? __ldg(w + 1) : make_ulonglong2(0, 0);
     }
-    cp_async_wait<0>();
-    if (t == 0 && (fresh | keyed)) {
-        atomicAdd(&c->block_fresh, fresh);
-        atomicAdd(&c->block_keyed, keyed);
-        if (full) atomicAdd(&c->full_sorted, full);
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+        if (key_words_inside(a.arena_bytes, pos[q] & ~15ull))
+            kk[q] = key_of_words(v0[q], v1[q], (uint32_t)pos[q] & 15u);
+        else if (ii[q] != IDX_MAX)
+            kk[q] = load_key_tail(a.arena, a.arena_bytes, pos[q]);
     }
 }
 
+// ---- segments of 33..2048 strings: a group of threads each ------------------
+// A group of GT = 32, 64, 128 or 256 threads sorts one segment of up to
+// ITEMS * GT strings (8 per thread; 2 or 4 for the smallest).  Records (16-byte
+// key, index) sit in shared memory at their positions; what moves is one
+// 32-bit value per record in registers: the first bits in which the segment's
+// keys differ at all, with the position in the low bits.  Bits that every key
+// of the segment shares carry no order, so they are squeezed out (letters
+// leave 5 bits of each byte): the 21 to 26 squeezed bits order most segments
+// completely.  Values whose squeezed bits tie are checked against the full
+// keys; a tied run out of order is put right in place when it is short, else
+// the segment is refined on further bits.
+//
+// The sort is bound by issued instructions and shared-memory latency, not by
+// HBM: 32-bit values make a compare-exchange one min and one max, and an
+// exchange between lanes one shuffle and one select; a neighbour's LCP follows
+// from the first differing bit of two values, so full keys are read for ties
+// only.  24 bytes of shared memory per string let 1024 threads share an SM.
+// Measured on B200 against 64-bit packed keys merged in shared memory (80
+// registers, 768 threads per SM): 10,000 partitioned segments of 400 strings
+// at 55 G strings/s (2290 instructions per warp of 256, 910 of them the
+// network; ALU pipe 65-75 % busy); the CTA-sort launches of 69 M batched
+// strings 2.79 -> 1.53 ms, of 16 M suffixes 4.23 -> 2.59 ms, of 50 M URLs 2.27
+// -> 1.62 ms.
+
+// Barrier among the GT threads of group gi: named barrier 1 + gi (0 is
+// __syncthreads).  Immediate ids, so that a CTA claims only the barriers it
+// uses (at most 5) and the SM's barriers do not limit occupancy.
 template <int GT>
-__global__ void __launch_bounds__(SMALL_THREADS, 2) k_block2(SortArgs a, const Seg *__restrict__ S,
-                                                             Span sp, Seg *N, Counters *c) {
+__device__ __forceinline__ void group_sync(uint32_t gi) {
+    constexpr int G = SMALL_THREADS / GT;
+    if constexpr (GT == 32) {
+        __syncwarp();
+    } else {
+        if (G == 1 || gi == 0)
+            asm volatile("bar.sync 1, %0;" ::"n"(GT) : "memory");
+        else if (G == 2 || gi == 1)
+            asm volatile("bar.sync 2, %0;" ::"n"(GT) : "memory");
+        else if (gi == 2)
+            asm volatile("bar.sync 3, %0;" ::"n"(GT) : "memory");
+        else
+            asm volatile("bar.sync 4, %0;" ::"n"(GT) : "memory");
+    }
+}
+
+// Whether any thread of the group has `want`; a barrier of the group.
+template <int GT>
+__device__ __forceinline__ bool group_any(bool want, uint32_t gi) {
+    if constexpr (GT == 32) {
+        return __any_sync(0xffffffffu, want);
+    } else {
+        constexpr int G = SMALL_THREADS / GT;
+        uint32_t r;
+#define SS_BAR_ANY(id)                                                               \
+    asm volatile("{ .reg .pred p, q; setp.ne.u32 p, %1, 0; bar.red.or.pred q, " #id  \
+                 ", %2, p; selp.u32 %0, 1, 0, q; }"                                  \
+                 : "=r"(r)                                                           \
+                 : "r"((uint32_t)want), "n"(GT)                                      \
+                 : "memory")
+        if (G == 1 || gi == 0)
+            SS_BAR_ANY(1);
+        else if (G == 2 || gi == 1)
+            SS_BAR_ANY(2);
+        else if (gi == 2)
+            SS_BAR_ANY(3);
+        else
+            SS_BAR_ANY(4);
+#undef SS_BAR_ANY
+        return r != 0;
+    }
+}
+
+template <typename V>
+__device__ __forceinline__ void cmp_swap(V &a, V &b) {
+    const V lo = min(a, b), hi = max(a, b);
+    a = lo;
+    b = hi;
+}
+
+// One exchange between threads: the lower one keeps the smaller value, the
+// upper one (up) the larger.
+template <typename V>
+__device__ __forceinline__ V keep_side(V v, V o, bool up) {
+    return (o < v) != up ? o : v;
+}
+
+// Batcher's odd-even merge sort of v[LO .. LO + N), as templates so that every
+// index is a constant and the values stay in registers.
+template <int LO, int N, int R, int ITEMS, typename V>
+__device__ __forceinline__ void net_merge(V (&v)[ITEMS]) {
+    if constexpr (2 * R < N) {
+        net_merge<LO, N, 2 * R>(v);
+        net_merge<LO + R, N, 2 * R>(v);
+#pragma unroll
+        for (int i = LO + R; i + R < LO + N; i += 2 * R) cmp_swap(v[i], v[i + R]);
+    } else {
+        cmp_swap(v[LO], v[LO + R]);
+    }
+}
+
+template <int LO, int N, int ITEMS, typename V>
+__device__ __forceinline__ void net_sort(V (&v)[ITEMS]) {
+    if constexpr (N > 1) {
+        net_sort<LO, N / 2>(v);
+        net_sort<LO + N / 2, N / 2>(v);
+        net_merge<LO, N, 1>(v);
+    }
+}
+
+// Bitonic half-cleaners of strides M, M / 2, .. 1 inside a thread.
+template <int M, int ITEMS, typename V>
+__device__ __forceinline__ void net_clean(V (&v)[ITEMS]) {
+    if constexpr (M >= 1) {
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i)
+            if ((i & M) == 0) cmp_swap(v[i], v[i + M]);
+        net_clean<M / 2>(v);
+    }
+}
+
+// Half-cleaners of lane strides m, m / 2, .. 1, then inside the lanes.  The
+// loop over strides stays a loop: unrolled, the sorts outgrow the
+// instruction cache.
+template <int ITEMS, typename V>
+__device__ __forceinline__ void warp_clean(V (&v)[ITEMS], uint32_t m, uint32_t lane) {
+#pragma unroll 1
+    for (; m >= 1; m /= 2) {
+        const bool up = (lane & m) != 0;
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i)
+            v[i] = keep_side(v[i], __shfl_xor_sync(0xffffffffu, v[i], m), up);
+    }
+    net_clean<ITEMS / 2>(v);
+}
+
+// Every thread stores its values to x (16-byte words, consecutive threads
+// next to each other) and loads those of thread `from`.  Two barriers.
+template <int GT, int ITEMS, typename V>
+__device__ __forceinline__ void swap_values(const V (&v)[ITEMS], V (&o)[ITEMS], void *x,
+                                            uint32_t t, uint32_t from, uint32_t gi) {
+    constexpr int PER = 16 / sizeof(V);  // values per 16-byte word
+    V w[PER];
+#pragma unroll
+    for (int j = 0; j < ITEMS / PER; ++j) {
+#pragma unroll
+        for (int q = 0; q < PER; ++q) w[q] = v[j * PER + q];
+        static_cast<uint4 *>(x)[j * GT + t] = *reinterpret_cast<const uint4 *>(w);
+    }
+    group_sync<GT>(gi);
+#pragma unroll
+    for (int j = 0; j < ITEMS / PER; ++j) {
+        *reinterpret_cast<uint4 *>(w) = static_cast<const uint4 *>(x)[j * GT + from];
+#pragma unroll
+        for (int q = 0; q < PER; ++q) o[j * PER + q] = w[q];
+    }
+    group_sync<GT>(gi);
+}
+
+// Sorts the GT * ITEMS values of a group; thread t ends with ranks t * ITEMS
+// .. t * ITEMS + ITEMS - 1.  Odd-even merge sort inside a thread, then bitonic
+// merges of 2, 4, .. GT threads whose first stage compares mirrored positions,
+// so that every stage sorts ascending; strides of 32 threads and more go
+// through shared memory (x: GT * ITEMS values).
+template <int GT, int ITEMS, typename V>
+__device__ __forceinline__ void group_net_sort(V (&v)[ITEMS], void *x, uint32_t t, uint32_t gi) {
+    const uint32_t lane = t & 31;
+    net_sort<0, ITEMS>(v);
+#pragma unroll 1
+    for (uint32_t half = 1; half < 32; half *= 2) {
+        const bool up = (lane & half) != 0;
+        const uint32_t mirror = 2 * half - 1;
+#pragma unroll
+        for (int i = 0; i < ITEMS / 2; ++i) {
+            const V p = __shfl_xor_sync(0xffffffffu, v[ITEMS - 1 - i], mirror);
+            const V q = __shfl_xor_sync(0xffffffffu, v[i], mirror);
+            v[i] = keep_side(v[i], p, up);
+            v[ITEMS - 1 - i] = keep_side(v[ITEMS - 1 - i], q, up);
+        }
+        warp_clean<ITEMS>(v, half / 2, lane);
+    }
+    if constexpr (GT > 32) {
+#pragma unroll 1
+        for (uint32_t half = 32; half < GT; half *= 2) {
+            V o[ITEMS];
+            swap_values<GT, ITEMS>(v, o, x, t, t ^ (2 * half - 1), gi);
+            const bool up = (t & half) != 0;
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) v[i] = keep_side(v[i], o[ITEMS - 1 - i], up);
+#pragma unroll 1
+            for (uint32_t m = half / 2; m >= 32; m /= 2) {
+                swap_values<GT, ITEMS>(v, o, x, t, t ^ m, gi);
+                const bool um = (t & m) != 0;
+#pragma unroll
+                for (int i = 0; i < ITEMS; ++i) v[i] = keep_side(v[i], o[i], um);
+            }
+            warp_clean<ITEMS>(v, 16, lane);
+        }
+    }
+}
+
+// Shared memory of one group: keys, values (in passing between threads, and
+// the final order), indices.  Values and indices together also hold 64-bit
+// values while a segment is refined.
+template <int GT, int ITEMS>
+struct SegSmem {
+    ulonglong2 key[GT * 8];
+    uint32_t val[GT * 8];
+    uint32_t idx[GT * 8];
+    uint64_t red[GT / 32][2];
+    uint32_t last[GT / 32], first[GT / 32];  // values at the edges of each warp
+    uint32_t fill[GT == 32 ? 2 : 4];  // to a multiple of 16 bytes
+};
+
+// Final order: per rank the record's position and, above it, the key bytes
+// it shares with the record before (SEG_TIE: not known from the values).
+constexpr uint32_t SEG_ORD_BITS = 11, SEG_TIE = 31;
+
+template <int GT, int ITEMS>
+constexpr int SEG_POS_BITS = (ITEMS == 2 ? 1 : ITEMS == 4 ? 2 : 3) +
+                             (GT == 32 ? 5 : GT == 64 ? 6 : GT == 128 ? 7 : 8);
+
+// Takes the next bits of `mask` (most significant first, at most `need`) off
+// it as one run of adjacent bits: `width` bits that start `lead` bits from the
+// top.  False when the mask is empty.
+__device__ __forceinline__ bool next_run(uint64_t &mask, uint32_t need, uint32_t &lead,
+                                         uint32_t &width) {
+    if (!mask || !need) return false;
+    lead = (uint32_t)__clzll((long long)mask);
+    const uint64_t inv = ~(mask << lead);
+    const uint32_t run = inv ? (uint32_t)__clzll((long long)inv) : 64u;
+    width = min(run, need);
+    mask &= ~((width == 64 ? ~0ull : ((1ull << width) - 1)) << (64 - lead - width));
+    return true;
+}
+
+// Orders the records by further differing bits after a first sort whose tied
+// runs were out of order: every pass sorts (first rank of the record's tied
+// run, its next differing bits, position) as 64-bit values; 42 or more bits
+// a pass, so at most four passes for the 128 key bits.  mh, ml: the differing
+// bits not used yet.  On return sm.val holds positions only, in (key,
+// position) order; sm.idx is read again from I.
+template <int GT, int ITEMS>
+__device__ __noinline__ void group_refine(SegSmem<GT, ITEMS> &sm, const uint32_t *I, uint32_t len,
+                                          uint64_t mh, uint64_t ml, uint32_t t, uint32_t gi) {
+    constexpr int PB = SEG_POS_BITS<GT, ITEMS>;
+    constexpr uint32_t PM = (1u << PB) - 1, MORE = 64 - 2 * PB;
+    constexpr int GRP = ITEMS < 4 ? ITEMS : 4;
+    const uint32_t lane = t & 31, gw = t >> 5;
+    uint64_t v[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t r = t * ITEMS + i;
+        v[i] = r < len ? (uint64_t)sm.val[r] : ~0ull;
+    }
+#pragma unroll 1
+    for (int pass = 0; pass < 5; ++pass) {
+        // First rank of each record's tied run (a running maximum of the ranks
+        // at which a run starts), in place of the bits used so far.
+        if (lane == 31) sm.red[gw][0] = v[ITEMS - 1];
+        group_sync<GT>(gi);
+        uint64_t pv = __shfl_up_sync(0xffffffffu, v[ITEMS - 1], 1);
+        if (lane == 0 && gw) pv = sm.red[gw - 1][0];
+        uint32_t h = 0;
+        bool tie = false;
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const uint32_t r = t * ITEMS + i;
+            const uint64_t cur = v[i];
+            const bool start = r == 0 || (cur >> PB) != (pv >> PB);
+            tie |= !start && r < len;
+            if (start) h = r;
+            v[i] = (uint64_t)h << (64 - PB) | ((uint32_t)cur & PM);
+            pv = cur;
+        }
+        uint32_t hm = h;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, hm, d);
+            if (lane >= (uint32_t)d) hm = max(hm, y);
+        }
+        if (lane == 31) sm.red[gw][1] = hm;
+        hm = __shfl_up_sync(0xffffffffu, hm, 1);
+        if (lane == 0) hm = 0;
+        if (!group_any<GT>(tie, gi) || !(mh | ml)) break;
+        for (uint32_t q = 0; q < gw; ++q) hm = max(hm, (uint32_t)sm.red[q][1]);
+        uint64_t nh = mh, nl = ml;
+#pragma unroll
+        for (int g = 0; g < ITEMS; g += GRP) {
+            Key k[GRP];
+            uint64_t acc[GRP];
+#pragma unroll
+            for (int q = 0; q < GRP; ++q) {
+                k[q] = t * ITEMS + g + q < len ? to_key(sm.key[(uint32_t)v[g + q] & PM]) : key_max();
+                acc[q] = 0;
+            }
+            uint32_t need = MORE, lead, width;
+            nh = mh;
+            nl = ml;
+            while (next_run(nh, need, lead, width)) {
+#pragma unroll
+                for (int q = 0; q < GRP; ++q)
+                    acc[q] = (acc[q] << width) | (k[q].hi << lead >> (64 - width));
+                need -= width;
+            }
+            while (next_run(nl, need, lead, width)) {
+#pragma unroll
+                for (int q = 0; q < GRP; ++q)
+                    acc[q] = (acc[q] << width) | (k[q].lo << lead >> (64 - width));
+                need -= width;
+            }
+#pragma unroll
+            for (int q = 0; q < GRP; ++q) {
+                const uint64_t head = max((uint32_t)(v[g + q] >> (64 - PB)), hm);
+                v[g + q] = t * ITEMS + g + q < len
+                               ? head << (64 - PB) | acc[q] << PB | ((uint32_t)v[g + q] & PM)
+                               : ~0ull;
+            }
+        }
+        mh = nh;
+        ml = nl;
+        group_net_sort<GT, ITEMS>(v, sm.val, t, gi);
+        group_sync<GT>(gi);
+    }
+    group_sync<GT>(gi);
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) sm.val[t * ITEMS + i] = (uint32_t)v[i] & PM;
+    for (uint32_t e = t; e < len; e += GT) sm.idx[e] = I[e];
+    group_sync<GT>(gi);
+}
+
+// Puts the tied runs that are out of full-key order right, each by the thread
+// that finds its first inversion (insertion sort; equal keys keep position
+// order).  With a run of more than SEG_FIX records among them nothing is
+// moved: returns 1, or 2 when one is longer than SEG_FULL; else 0.
+constexpr uint32_t SEG_FIX = 12, SEG_FULL = 64;
+
+template <int GT, int ITEMS>
+__device__ __noinline__ uint32_t group_fix_runs(SegSmem<GT, ITEMS> &sm, uint32_t len, uint32_t t,
+                                                uint32_t gi) {
+    constexpr int PB = SEG_POS_BITS<GT, ITEMS>;
+    constexpr uint32_t PM = (1u << PB) - 1;
+    auto val = [&](uint32_t r) -> uint32_t & { return sm.val[r]; };
+    auto key = [&](uint32_t r) -> Key { return to_key(sm.key[val(r) & PM]); };
+    auto tied = [&](uint32_t r) -> bool { return ((val(r) ^ val(r - 1)) >> PB) == 0; };
+    // The run around rank e, as far as SEG_FULL + 1 records.  Sorting a run
+    // moves values of equal squeezed bits only, so what this reads of other
+    // threads' runs (one value past either end) does not change under it.
+    auto extent = [&](uint32_t e, uint32_t &lo, uint32_t &hi) {
+        lo = e - 1;
+        while (lo > 0 && e - lo <= SEG_FULL && tied(lo)) --lo;
+        hi = e + 1;
+        while (hi < len && hi - lo <= SEG_FULL && tied(hi)) ++hi;
+    };
+    uint32_t own = 0, longest = 0;
+#pragma unroll 1
+    for (int q = 0; q < ITEMS; ++q) {
+        const uint32_t e = q * GT + t;
+        if (e == 0 || e >= len || !tied(e) || !key_lt(key(e), key(e - 1))) continue;
+        uint32_t lo, hi;
+        extent(e, lo, hi);
+        longest = max(longest, hi - lo);
+        if (hi - lo > SEG_FIX) continue;
+        bool first = true;  // no earlier inversion in the run
+        for (uint32_t r = lo + 1; first && r < e; ++r) first = !key_lt(key(r), key(r - 1));
+        if (first) own |= 1u << q;
+    }
+    if (group_any<GT>(longest > SEG_FIX, gi)) return group_any<GT>(longest > SEG_FULL, gi) ? 2 : 1;
+    for (; own; own &= own - 1) {
+        uint32_t lo, hi;
+        extent((__ffs(own) - 1) * GT + t, lo, hi);
+        for (uint32_t i = lo + 1; i < hi; ++i) {
+            const uint32_t x = val(i);
+            const Key kx = to_key(sm.key[x & PM]);
+            uint32_t j = i;
+            while (j > lo && key_lt(kx, key(j - 1))) {
+                val(j) = val(j - 1);
+                --j;
+            }
+            val(j) = x;
+        }
+    }
+    group_sync<GT>(gi);
+    return 0;
+}
+
+// Orders a segment of `len` records (at most GT * ITEMS, in sm.key at their
+// positions) whose keys differ in the bits mh, ml (not both 0): writes the
+// final order to sm.val.  Returns whether a run of more than SEG_FULL tied
+// records was out of order.
+template <int GT, int ITEMS>
+__device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint32_t *I,
+                                              uint32_t len, uint64_t mh, uint64_t ml, uint32_t t,
+                                              uint32_t gi) {
+    constexpr int PB = SEG_POS_BITS<GT, ITEMS>;
+    constexpr uint32_t PM = (1u << PB) - 1, WB = 32 - PB;
+    const uint32_t lane = t & 31, gw = t >> 5;
+    // Squeezed bits: the first WB differing bits of the 64 from the first
+    // one (bit f of the key) on, run by run of adjacent ones; lane j keeps the
+    // key byte of squeezed bit j.
+    const uint32_t f = clz128(mh, ml);
+    const uint64_t wm = window64(Key{mh, ml}, f);
+    uint32_t used = 0, byte_of = SEG_TIE;
+    uint32_t v[ITEMS], wh[ITEMS], wl[ITEMS];
+#pragma unroll
+    for (int q = 0; q < ITEMS; ++q) {
+        const uint32_t e = q * GT + t;
+        const Key k = e < len ? to_key(sm.key[e]) : Key{0, 0};
+        // the 96 bits from the 32-bit word that holds bit f on
+        const uint64_t top = f < 64 ? k.hi : k.lo, next = f < 64 ? k.lo : 0;
+        const uint32_t w0 = (uint32_t)(top >> 32), w1 = (uint32_t)top,
+                       w2 = (uint32_t)(next >> 32), w3 = (uint32_t)next;
+        wh[q] = f & 32 ? __funnelshift_l(w2, w1, f) : __funnelshift_l(w1, w0, f);
+        wl[q] = f & 32 ? __funnelshift_l(w3, w2, f) : __funnelshift_l(w2, w1, f);
+        v[q] = 0;
+    }
+    auto squeeze = [&](uint32_t &m, const uint32_t(&w)[ITEMS], uint32_t base) {
+#pragma unroll 1
+        while (m && used < WB) {
+            const uint32_t lead = __clz(m);
+            const uint32_t width = min((uint32_t)__clz(~(m << lead)), WB - used);
+            const uint32_t mul = 1u << width, low = mul - 1, sh = 32 - lead - width;
+#pragma unroll
+            for (int q = 0; q < ITEMS; ++q) v[q] = v[q] * mul + ((w[q] >> sh) & low);
+            if (lane - used < width) byte_of = (f + base + lead + lane - used) >> 3;
+            used += width;
+            m &= ~(low << sh);
+        }
+    };
+    uint32_t m0 = (uint32_t)(wm >> 32), m1 = (uint32_t)wm;
+    squeeze(m0, wh, 0);
+    squeeze(m1, wl, 32);
+#pragma unroll
+    for (int q = 0; q < ITEMS; ++q) {
+        const uint32_t e = q * GT + t;
+        v[q] = e < len ? v[q] << PB | e : ~0u;
+    }
+    group_net_sort<GT, ITEMS>(v, sm.val, t, gi);
+    // Ties on the squeezed bits must be in full-key order.  A pair out of
+    // order that both lie in one thread and tie with nothing else is swapped
+    // on the spot; other runs out of order go through shared memory.
+    uint32_t pv = __shfl_up_sync(0xffffffffu, v[ITEMS - 1], 1);
+    uint32_t nv = __shfl_down_sync(0xffffffffu, v[0], 1);
+    if constexpr (GT > 32) {
+        if (lane == 31) sm.last[gw] = v[ITEMS - 1];
+        if (lane == 0) sm.first[gw] = v[0];
+        group_sync<GT>(gi);
+        if (lane == 0 && gw) pv = sm.last[gw - 1];
+        if (lane == 31 && gw + 1 < GT / 32) nv = sm.first[gw + 1];
+    }
+    if (t == 0) pv = ~v[0];
+    if (t == GT - 1) nv = ~v[ITEMS - 1];
+    bool full = false, bad = false;
+    uint32_t tie = 0;  // bit i: rank t * ITEMS + i ties with the one before
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+        if ((v[i] ^ (i ? v[i ? i - 1 : 0] : pv)) <= PM) tie |= 1u << i;
+    if ((nv ^ v[ITEMS - 1]) <= PM) tie |= 1u << ITEMS;
+    if (tie && t * ITEMS < len) {
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            if ((tie >> i & 1u) && t * ITEMS + i < len) {
+                const uint32_t y = i ? v[i ? i - 1 : 0] : pv;
+                if (key_lt(to_key(sm.key[v[i] & PM]), to_key(sm.key[y & PM]))) {
+                    if (i > 0 && (tie >> (i ? i - 1 : 0) & 7u) == 2u) {
+                        v[i ? i - 1 : 0] = v[i];
+                        v[i] = y;
+                    } else {
+                        bad = true;
+                    }
+                }
+            }
+        }
+    }
+    // (a swap changes no value that another thread compares by more than its
+    // position, and those it does belong to a longer run)
+    if (group_any<GT>(bad, gi)) {
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) sm.val[t * ITEMS + i] = v[i];
+        group_sync<GT>(gi);
+        const uint32_t run = group_fix_runs<GT, ITEMS>(sm, len, t, gi);
+        if (run) {
+            full = run == 2;
+            byte_of = SEG_TIE;  // the values are positions only
+            // The differing bits not used: m0, m1 of the window, and what
+            // lies past the window's 64 bits.
+            const uint64_t m = (uint64_t)m0 << 32 | m1;
+            const uint64_t rh = f < 64 ? m >> f : 0ull;
+            const uint64_t rl = f == 0   ? ml
+                                : f < 64 ? (m << (64 - f)) | ((ml << f) >> f)
+                                         : m >> (f - 64);
+            group_refine<GT, ITEMS>(sm, I, len, rh, rl, t, gi);
+        }
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) v[i] = sm.val[t * ITEMS + i];
+        if (t) pv = sm.val[t * ITEMS - 1];
+        group_sync<GT>(gi);
+    }
+    // The order, with the bytes shared with the neighbour where the first
+    // differing squeezed bit tells (no NUL can precede it in either key).
+    uint32_t o[ITEMS / 2];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t x = (v[i] ^ (i ? v[i ? i - 1 : 0] : pv)) >> PB;
+        const uint32_t l = __shfl_sync(0xffffffffu, byte_of, __clz(x) + used - 32);
+        const uint32_t h = l * (1u << SEG_ORD_BITS) + (v[i] & PM);
+        if (i & 1)
+            o[i / 2] += h * 65536u;
+        else
+            o[i / 2] = h;
+    }
+    if constexpr (ITEMS == 8)
+        reinterpret_cast<uint4 *>(sm.val)[t] = make_uint4(o[0], o[1], o[2], o[3]);
+    else if constexpr (ITEMS == 4)
+        reinterpret_cast<uint2 *>(sm.val)[t] = make_uint2(o[0], o[1]);
+    else
+        sm.val[t] = o[0];
+    return full;
+}
+
+// Sorts segment s (at most 8 * GT strings) with the GT threads of group gi,
+// thread t.  Returns whether a run of more than SEG_FULL tied records was out
+// of order.  One warp (GT = 32) orders up to 64 or 128 strings with 2 or 4
+// per thread.
+template <int GT>
+__device__ __forceinline__ bool sort_segment(const SortArgs &a, const Seg &s, SegSmem<GT, 8> &sm,
+                                             uint32_t t, uint32_t gi, Seg *N, Counters *c) {
+    constexpr int GRP = 4;  // strings at a time
+    const uint32_t lane = t & 31, gw = t >> 5;
+    const int b = s.flags & SEG_BUF1;
+    const uint32_t *I = a.idxb(b) + s.start;
+    // Records into shared memory: asynchronous copies of the partition's keys
+    // (no registers, all in flight at once), or the strings' own bytes through
+    // index and offset.
+    if (s.flags & SEG_KEYS) {
+        const ulonglong2 *K = a.keyb(b) + s.start;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t e = q * GT + t;
+            if (e < s.len) {
+                cp_async16(sm.key + e, K + e);
+                cp_async4(sm.idx + e, I + e);
+            }
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+    } else {
+#pragma unroll 1
+        for (uint32_t e0 = t; e0 < s.len; e0 += GRP * GT) {
+            Key k[GRP];
+            uint32_t id[GRP];
+            gather_keys<GRP>(a, I, s.depth, e0, GT, s.len, k, id);
+#pragma unroll
+            for (int q = 0; q < GRP; ++q)
+                if (e0 + q * GT < s.len) {
+                    sm.key[e0 + q * GT] = from_key(k[q]);
+                    sm.idx[e0 + q * GT] = id[q];
+                }
+        }
+    }
+    group_sync<GT>(gi);
+    // The bits in which the keys differ.
+    uint64_t mh = 0, ml = 0;
+    {
+        const Key k0 = to_key(sm.key[0]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t e = q * GT + t;
+            if (e < s.len) {
+                const Key k = to_key(sm.key[e]);
+                mh |= k.hi ^ k0.hi;
+                ml |= k.lo ^ k0.lo;
+            }
+        }
+        auto wor = [](uint64_t x) -> uint64_t {
+            return (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(x >> 32)) << 32 |
+                   __reduce_or_sync(0xffffffffu, (uint32_t)x);
+        };
+        mh = wor(mh);
+        ml = wor(ml);
+        if constexpr (GT > 32) {
+            if (lane == 0) {
+                sm.red[gw][0] = mh;
+                sm.red[gw][1] = ml;
+            }
+            group_sync<GT>(gi);
+#pragma unroll
+            for (int q = 0; q < GT / 32; ++q) {
+                mh |= sm.red[q][0];
+                ml |= sm.red[q][1];
+            }
+        }
+    }
+    bool full = false;
+    if (mh | ml) {
+        if (GT == 32 && s.len <= 64)
+            full = order_segment<GT, 2>(reinterpret_cast<SegSmem<GT, 2> &>(sm), I, s.len, mh, ml,
+                                        t, gi);
+        else if (GT == 32 && s.len <= 128)
+            full = order_segment<GT, 4>(reinterpret_cast<SegSmem<GT, 4> &>(sm), I, s.len, mh, ml,
+                                        t, gi);
+        else
+            full = order_segment<GT, 8>(sm, I, s.len, mh, ml, t, gi);
+    } else {  // all keys equal: position order
+        for (uint32_t e = t; e < s.len; e += GT)
+            reinterpret_cast<uint16_t *>(sm.val)[e] = (uint16_t)(SEG_TIE << SEG_ORD_BITS | e);
+    }
+    group_sync<GT>(gi);
+    // Results in rank order: indices, LCPs, first and last key, next-round
+    // runs.  Ties read both keys.
+    const uint16_t *ord = reinterpret_cast<const uint16_t *>(sm.val);
+    constexpr uint32_t OM = (1u << SEG_ORD_BITS) - 1;
+    auto key_at = [&](uint32_t r) -> Key { return to_key(sm.key[ord[r] & OM]); };
+    uint32_t *oi = a.idx[0] + s.start + t, *ol = a.lcp + s.start + t;
+    if (t < 2) {
+        const uint32_t r = t ? s.len - 1 : 0;
+        a.key[0][s.start + r] = from_key(key_at(r));
+    }
+#pragma unroll 4
+    for (uint32_t e0 = 0; e0 < s.len; e0 += GT) {
+        const uint32_t e = e0 + t;
+        const bool on = e < s.len;
+        const uint32_t w = on ? ord[e] : 0u;
+        if (on) oi[e0] = sm.idx[w & OM];
+        bool cont = false;  // goes on a run of equal keys that do not end
+        if (on && e) {
+            uint32_t l = w >> SEG_ORD_BITS;
+            if (l == SEG_TIE) {
+                const Key k = to_key(sm.key[w & OM]), kp = key_at(e - 1);
+                const bool same = key_eq(kp, k);
+                cont = same && !key_is_end(k);
+                l = same ? key_len(k) : key_lcp(kp, k);
+            }
+            if (!cont) ol[e0] = s.depth + l;
+        }
+        const uint32_t cm = __ballot_sync(0xffffffffu, cont);
+        if (cm) {  // warp-uniform
+            bool tail = cont && !((cm >> 1) >> lane & 1u);
+            if (tail && lane == 31 && e + 1 < s.len) tail = !key_eq(key_at(e + 1), key_at(e));
+            uint32_t lo = 0;
+            if (tail) {
+                const uint32_t heads = ~cm & lanemask_lt();
+                if (heads) {
+                    lo = e - lane + 31 - __clz(heads);
+                } else {  // the run starts before this warp's ranks
+                    const Key k = key_at(e);
+                    uint32_t hi = e;
+                    while (lo < hi) {
+                        const uint32_t mid = (lo + hi) >> 1;
+                        if (key_lt(key_at(mid), k))
+                            lo = mid + 1;
+                        else
+                            hi = mid;
+                    }
+                }
+            }
+            emit_next_warp(N, c, tail, s.start + lo, e - lo + 1, s.depth + KEY_BYTES);
+        }
+    }
+    group_sync<GT>(gi);
+    return full;
+}
+
+// GT = 32 takes the segments of 33..256 strings and sorts each with 2, 4 or 8
+// strings per thread; 64, 128 and 256 take one size class each.
+template <int GT>
+constexpr size_t SEG_SMEM = (SMALL_THREADS / GT) * sizeof(SegSmem<GT, 8>);
+
+template <int GT>
+__global__ void __launch_bounds__(SMALL_THREADS, 4) k_segsort(SortArgs a,
+                                                              const Seg *__restrict__ T0, Span sp,
+                                                              Seg *N, Counters *c) {
+    constexpr uint32_t G = SMALL_THREADS / GT;
+    extern __shared__ __align__(16) unsigned char seg_smem[];
     const uint32_t lo = count_of(sp.lo);
-    block2_class<GT>(a, S + lo, count_of(sp.hi) - lo, N, c);
+    const Seg *__restrict__ T = T0 + lo;
+    const uint32_t nT = count_of(sp.hi) - lo;
+    const uint32_t gi = threadIdx.x / GT, t = threadIdx.x % GT;
+    auto &sm = reinterpret_cast<SegSmem<GT, 8> *>(seg_smem)[gi];
+    unsigned long long fresh = 0, keyed = 0, full = 0;
+    for (uint32_t g = blockIdx.x * G + gi; g < nT; g += gridDim.x * G) {
+        const Seg s = T[g];
+        if (s.flags & SEG_KEYS)
+            keyed += s.len;
+        else
+            fresh += s.len;
+        if (sort_segment<GT>(a, s, sm, t, gi, N, c)) full += s.len;
+    }
+    if (t == 0 && (fresh | keyed)) {
+        atomicAdd(GT == 32 ? &c->warp8_fresh : &c->block_fresh, fresh);
+        atomicAdd(GT == 32 ? &c->warp8_keyed : &c->block_keyed, keyed);
+        if (full) atomicAdd(&c->full_sorted, full);
+    }
 }
 
 // ---- equality buckets: work items of up to EQ_TILE strings ------------------
@@ -3381,31 +3075,14 @@ static void set_smem_attrs() {
                          (int)sizeof(ScatterSmem));
     cudaFuncSetAttribute(k_scatter2, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(Scatter2Smem));
-    cudaFuncSetAttribute(k_warp8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W8_SMEM);
-    cudaFuncSetAttribute(k_block<64, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK_SMEM);
-    cudaFuncSetAttribute(k_block<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK_SMEM);
-    cudaFuncSetAttribute(k_block<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK_SMEM);
-    cudaFuncSetAttribute(k_block<128, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK_SMEM);
-    cudaFuncSetAttribute(k_block<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK_SMEM);
-    cudaFuncSetAttribute(k_block<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK_SMEM);
-    cudaFuncSetAttribute(k_block<256, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK_SMEM);
-    cudaFuncSetAttribute(k_block<256, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK_SMEM);
-    cudaFuncSetAttribute(k_block<256, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK_SMEM);
-    cudaFuncSetAttribute(k_block2<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK2_SMEM);
-    cudaFuncSetAttribute(k_block2<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK2_SMEM);
-    cudaFuncSetAttribute(k_block2<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)BLOCK2_SMEM);
+    cudaFuncSetAttribute(k_segsort<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)SEG_SMEM<32>);
+    cudaFuncSetAttribute(k_segsort<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)SEG_SMEM<64>);
+    cudaFuncSetAttribute(k_segsort<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)SEG_SMEM<128>);
+    cudaFuncSetAttribute(k_segsort<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)SEG_SMEM<256>);
     done.fetch_or(bit, std::memory_order_release);
 }
 
@@ -3600,38 +3277,19 @@ void launch_warp8(const SortArgs &a, const Seg *W8, Span sp, Seg *N, Counters *c
                   cudaStream_t st) {
     if (span_empty(sp) || grid <= 0) return;
     set_smem_attrs();
-    k_warp8<<<grid, WARP_THREADS, W8_SMEM, st>>>(a, W8, sp, N, c);
+    k_segsort<32><<<grid, SMALL_THREADS, SEG_SMEM<32>, st>>>(a, W8, sp, N, c);
 }
 
 void launch_block(const SortArgs &a, const Seg *S, Span sp, int cls, Seg *N, Counters *c,
-                  int grid, cudaStream_t st, bool prefetch) {
+                  int grid, cudaStream_t st) {
     if (span_empty(sp) || grid <= 0) return;
     set_smem_attrs();
-    if (prefetch) {
-        if (cls == 0)
-            k_block2<64><<<grid, SMALL_THREADS, BLOCK2_SMEM, st>>>(a, S, sp, N, c);
-        else if (cls == 1)
-            k_block2<128><<<grid, SMALL_THREADS, BLOCK2_SMEM, st>>>(a, S, sp, N, c);
-        else
-            k_block2<256><<<grid, SMALL_THREADS, BLOCK2_SMEM, st>>>(a, S, sp, N, c);
-        return;
-    }
-#define SS_BLOCK_LAUNCH(VAR)                                                           \
-    do {                                                                               \
-        if (cls == 0)                                                                  \
-            k_block<64, VAR><<<grid, SMALL_THREADS, BLOCK_SMEM, st>>>(a, S, sp, N, c);  \
-        else if (cls == 1)                                                             \
-            k_block<128, VAR><<<grid, SMALL_THREADS, BLOCK_SMEM, st>>>(a, S, sp, N, c); \
-        else                                                                           \
-            k_block<256, VAR><<<grid, SMALL_THREADS, BLOCK_SMEM, st>>>(a, S, sp, N, c); \
-    } while (0)
-    if (a.block_lean == 2)
-        SS_BLOCK_LAUNCH(2);
-    else if (a.block_lean == 1)
-        SS_BLOCK_LAUNCH(1);
+    if (cls == 0)
+        k_segsort<64><<<grid, SMALL_THREADS, SEG_SMEM<64>, st>>>(a, S, sp, N, c);
+    else if (cls == 1)
+        k_segsort<128><<<grid, SMALL_THREADS, SEG_SMEM<128>, st>>>(a, S, sp, N, c);
     else
-        SS_BLOCK_LAUNCH(0);
-#undef SS_BLOCK_LAUNCH
+        k_segsort<256><<<grid, SMALL_THREADS, SEG_SMEM<256>, st>>>(a, S, sp, N, c);
 }
 
 void launch_equal(const SortArgs &a, const Seg *E, Span sp, Seg *N, Counters *c, int grid,

@@ -1,0 +1,59 @@
+"""The one-warp sort of 33..1024 strings (squeezed 32-bit values): segment
+sizes at the edges of its size classes, and key sets that reach each of its
+branches (no ties, tied runs in order, short and long tied runs out of
+order, all keys equal, runs that continue in the next round)."""
+import numpy as np
+import pytest
+
+import cases
+import pyoracle
+import pyssort
+
+pytestmark = pytest.mark.gpu
+
+SIZES = (33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 2047,
+         2048, 2049)
+
+
+def _strings(kind, n, rng):
+    if kind == "random":  # distinct within the squeezed bits, all byte values
+        return [bytes(rng.integers(1, 256, size=rng.integers(1, 20)).tolist()) for _ in range(n)]
+    if kind == "letters":
+        return [bytes(rng.integers(97, 123, size=rng.integers(1, 24)).tolist()) for _ in range(n)]
+    if kind == "pairs":  # short tied runs: 13 shared letters, then two differing tails
+        return [b"abcdefgh" + bytes(rng.integers(97, 99, size=8).tolist()) + bytes([97 + i % 3])
+                for i in range(n)]
+    if kind == "few":  # long tied runs, distinguished in the last key byte, and equal keys
+        return [b"xyzzyxyz"[:int(rng.integers(4, 9))] + b"q" * int(rng.integers(0, 8)) +
+                bytes([int(rng.integers(97, 100))]) for _ in range(n)]
+    if kind == "late":  # the first 27 differing bits agree for most strings
+        return [(b"\x01\xff" * 7 if rng.random() < 0.9 else b"\xfe\x01" * 7) +
+                bytes([int(rng.integers(1, 256)), int(rng.integers(1, 256))]) for _ in range(n)]
+    if kind == "equal":
+        return [b"the same sixteen bytes and more"] * n
+    if kind == "runs":  # runs of equal 16-byte keys that go on differently
+        return [b"0123456789abcde" + bytes([int(rng.integers(97, 101))]) +
+                bytes(rng.integers(97, 100, size=rng.integers(0, 20)).tolist()) for _ in range(n)]
+    raise ValueError(kind)
+
+
+@pytest.mark.parametrize("kind", ["random", "letters", "pairs", "few", "late", "equal", "runs"])
+def test_one_warp_sort_sizes(sorter, kind):
+    rng = np.random.default_rng(sum(kind.encode()))
+    for n in SIZES:
+        arena, offs = cases.arena_of(_strings(kind, n, rng))
+        p, l = sorter.sort_host(arena, offs)
+        rp, rl = pyoracle.oracle_sort(arena, offs)
+        assert np.array_equal(p, rp), n
+        assert np.array_equal(l, rl), n
+
+
+@pytest.mark.parametrize("kind", ["letters", "pairs", "few", "late", "runs"])
+def test_one_warp_sort_of_partitioned_segments(sorter, kind):
+    """The same key sets behind a sample partition: keys come from the key
+    buffer (asynchronous copies) instead of the arena."""
+    rng = np.random.default_rng(7 + sum(kind.encode()))
+    arena, offs = cases.arena_of(_strings(kind, 60_000, rng))
+    p, l = sorter.sort_host(arena, offs)
+    rp, rl = pyoracle.oracle_sort(arena, offs)
+    assert np.array_equal(p, rp) and np.array_equal(l, rl)
