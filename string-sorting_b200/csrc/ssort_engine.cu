@@ -118,14 +118,15 @@ int ssort_ctx::launch_small(const SortArgs &a, Seg *nxt, SmallDone &d) {
     n = h_ctr->n_w8 - d.w8;
     LAUNCH(this, "warp8", launch_warp8(a, ws.W8, hspan(d.w8, d.w8 + n), nxt, dc, grid(n, 8), s2));
     d.w8 += n;
-    // CTA-sort size classes: groups of 64, 128, 256 threads per segment.
-    Seg *lists[3] = {ws.S, ws.S2, ws.S3};
-    const uint32_t counts[3] = {h_ctr->n_small, h_ctr->n_small2, h_ctr->n_small3};
-    for (int k = 0; k < 3; ++k) {
+    // CTA-sort size classes: groups of 64, 128, 256, 512 threads per segment.
+    const SmallLists lists = ws.small();
+    const uint32_t counts[SMALL_CLASSES] = {h_ctr->n_small, h_ctr->n_small2, h_ctr->n_small3,
+                                            h_ctr->n_small4};
+    for (int k = 0; k < SMALL_CLASSES; ++k) {
         n = counts[k] - d.s[k];
-        const uint32_t per_cta = 4u >> k;
+        const uint32_t per_cta = k < 3 ? 4u >> k : 1u;
         LAUNCH(this, "block",
-               launch_block(a, lists[k], hspan(d.s[k], d.s[k] + n), k, nxt, dc,
+               launch_block(a, lists.s[k], hspan(d.s[k], d.s[k] + n), k, nxt, dc,
                             grid(n, per_cta), s3));
         d.s[k] += n;
     }
@@ -169,7 +170,7 @@ int ssort_ctx::round_body(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt,
     SS_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), st));
     LAUNCH(this, "classify",
            launch_classify(cur, hcount(n_cur), a.warp8_cap, ws.W1, ws.W8,
-                           SmallLists{{ws.S, ws.S2, ws.S3}}, ws.L, dc, 0, st));
+                           ws.small(), ws.L, dc, 0, st));
     SS_TRY(sync_counters());
     if (round_no < SSORT_MAX_ROUNDS) stats.live[round_no] = h_ctr->live_next;
     // The on-chip sorts of the segments known after each host read of the
@@ -214,7 +215,7 @@ int ssort_ctx::round_body(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt,
                               ws.cm, g2, st));
         LAUNCH(this, "emit",
                launch_emit(a, lcur, nl, ws.tile_base, ws.nspl, ws.cm_base, ws.cm, ws.W1, ws.W8,
-                           SmallLists{{ws.S, ws.S2, ws.S3}}, lnext, ws.E, ws.B, nxt, dc, 0, st));
+                           ws.small(), lnext, ws.E, ws.B, nxt, dc, 0, st));
         SS_TRY(launch_small(a, nxt, done));  // segments known before this level
         SS_TRY(sync_counters());
         SS_TRY(fork_small());
@@ -232,7 +233,8 @@ int ssort_ctx::round_body(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt,
     LAUNCH(this, "boundary", launch_boundary(a, ws.B, dc, g4, st));
     SS_TRY(sync_counters());
     stats.small_segments +=
-        h_ctr->n_w1 + h_ctr->n_w8 + h_ctr->n_small + h_ctr->n_small2 + h_ctr->n_small3;
+        h_ctr->n_w1 + h_ctr->n_w8 + h_ctr->n_small + h_ctr->n_small2 + h_ctr->n_small3 +
+        h_ctr->n_small4;
     stats.partitioned += h_ctr->partitioned;
     stats.gather_elems += h_ctr->gather_elems;
     if (fused_gather) stats.gather_fused += h_ctr->gather_elems;
@@ -301,6 +303,7 @@ int ssort_ctx::run_ws(const uint8_t *arena_p, uint64_t arena_bytes, const void *
     a.bkt = ws.bkt;
     a.target_bucket = target_bucket;
     a.warp8_cap = warp8_cap;
+    a.leaf_cap = n >= LEAF_MIN_N ? LEAF_CAP : SMALL_CAP;
     a.warp1_deep = warp1_deep;
     a.l2_prefetch = l2_prefetch ? 1u : 0u;
     a.scatter_staged_idx = scatter_variant;

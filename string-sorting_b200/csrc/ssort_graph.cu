@@ -94,11 +94,12 @@ int ssort_ctx::graph_small(const SortArgs &a, cudaStream_t s) {
     LAUNCH(this, "warp8",
            launch_warp8(a, ws.W8, Span{dcount(&g->cur_w8), dcount(&dc->n_w8)}, nxt, dc,
                         grid_for(6), s));
-    Seg *lists[3] = {ws.S, ws.S2, ws.S3};
-    const uint32_t *counts[3] = {&dc->n_small, &dc->n_small2, &dc->n_small3};
-    for (int k = 0; k < 3; ++k)
+    const SmallLists lists = ws.small();
+    const uint32_t *counts[SMALL_CLASSES] = {&dc->n_small, &dc->n_small2, &dc->n_small3,
+                                             &dc->n_small4};
+    for (int k = 0; k < SMALL_CLASSES; ++k)
         LAUNCH(this, "block",
-               launch_block(a, lists[k], Span{dcount(&g->cur_s[k]), dcount(counts[k])}, k, nxt,
+               launch_block(a, lists.s[k], Span{dcount(&g->cur_s[k]), dcount(counts[k])}, k, nxt,
                             dc, grid_for(6), s));
     LAUNCH(this, "equal",
            launch_equal(a, ws.E, Span{dcount(&g->cur_e), dcount(&dc->n_equal)}, nxt, dc,
@@ -114,7 +115,7 @@ int ssort_ctx::graph_build(const SortArgs &a) {
     Counters *dc = ws.ctr;
     const Count nl = dcount(&g->n_large);
     const int g8 = grid_for(8), g4 = grid_for(4), g2 = grid_for(2);
-    const SmallLists S{{ws.S, ws.S2, ws.S3}};
+    const SmallLists S = ws.small();
     cudaGraph_t top = nullptr;
     SS_CUDA(cudaGraphCreate(&top, 0));
     graph = top;

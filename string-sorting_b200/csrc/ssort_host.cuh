@@ -217,7 +217,7 @@ struct ssort_ctx {
             uint32_t ninst = 0);
     // List entries of the on-chip sorts already launched in this round.
     struct SmallDone {
-        uint32_t w1 = 0, w8 = 0, s[3] = {0, 0, 0}, e = 0;
+        uint32_t w1 = 0, w8 = 0, s[ssort::SMALL_CLASSES] = {0, 0, 0, 0}, e = 0;
     };
     int fork_small();
     int launch_small(const ssort::SortArgs &a, ssort::Seg *nxt, SmallDone &done);

@@ -382,29 +382,33 @@ __global__ void k_iota(uint32_t *idx, uint32_t n) {
 
 // Appends o (when sm) to the CTA-sort list of its size class; warp-collective.
 // Appends segment o (when v) to the list its length selects: one-warp sorts
-// of <= 32 or <= warp8_cap strings, the CTA sorts' three size classes, or the
-// large list L (counter nl).  Warp-collective; the six reservations are all
-// issued before any is waited for.
+// of <= 32 or <= warp8_cap strings, the CTA sorts' four size classes (up to
+// cap strings), or the large list L (counter nl).  Warp-collective; the
+// reservations are all issued before any is waited for.
 __device__ __forceinline__ void append_by_length(const Seg &o, bool v, uint32_t warp8_cap,
-                                                 Seg *W1, Seg *W8, const SmallLists &S, Seg *L,
-                                                 uint32_t *nl, Counters *c) {
+                                                 uint32_t cap, Seg *W1, Seg *W8,
+                                                 const SmallLists &S, Seg *L, uint32_t *nl,
+                                                 Counters *c) {
     const bool w1 = v && o.len <= (uint32_t)WARP1_CAP;
     const bool w8 = v && !w1 && o.len <= warp8_cap;
-    const bool sm = v && !w1 && !w8 && o.len <= (uint32_t)SMALL_CAP;
+    const bool sm = v && !w1 && !w8 && o.len <= cap;
     const bool c0 = sm && o.len <= (uint32_t)BLOCK_CAP1;
     const bool c1 = sm && !c0 && o.len <= (uint32_t)BLOCK_CAP2;
-    const bool c2 = sm && !c0 && !c1;
+    const bool c2 = sm && !c0 && !c1 && o.len <= (uint32_t)SMALL_CAP;
+    const bool c3 = sm && !c0 && !c1 && !c2;
     const bool lg = v && !w1 && !w8 && !sm;
     const WarpRes r1 = warp_reserve(&c->n_w1, w1), r8 = warp_reserve(&c->n_w8, w8),
                   rs0 = warp_reserve(&c->n_small, c0), rs1 = warp_reserve(&c->n_small2, c1),
-                  rs2 = warp_reserve(&c->n_small3, c2), rl = warp_reserve(nl, lg);
+                  rs2 = warp_reserve(&c->n_small3, c2), rs3 = warp_reserve(&c->n_small4, c3),
+                  rl = warp_reserve(nl, lg);
     const uint32_t t1 = warp_slot(r1), t8 = warp_slot(r8), ts0 = warp_slot(rs0),
-                   ts1 = warp_slot(rs1), ts2 = warp_slot(rs2), tl = warp_slot(rl);
+                   ts1 = warp_slot(rs1), ts2 = warp_slot(rs2), ts3 = warp_slot(rs3), tl = warp_slot(rl);
     if (w1) W1[t1] = o;
     if (w8) W8[t8] = o;
     if (c0) S.s[0][ts0] = o;
     if (c1) S.s[1][ts1] = o;
     if (c2) S.s[2][ts2] = o;
+    if (c3) S.s[3][ts3] = o;
     if (lg) L[tl] = o;
 }
 
@@ -416,7 +420,7 @@ __global__ void k_classify(const Seg *__restrict__ R, Count cnt, uint32_t warp8_
     const uint32_t i = b0 + threadIdx.x;
     const bool v = i < nR;
     const Seg s = v ? R[i] : Seg{0, 0, 0, 0};
-    append_by_length(s, v, warp8_cap, W1, W8, S, L, &c->n_large, c);
+    append_by_length(s, v, warp8_cap, SMALL_CAP, W1, W8, S, L, &c->n_large, c);
     const bool lg = v && s.len > (uint32_t)SMALL_CAP && s.len > warp8_cap;
     const unsigned long long live = warp_sum(v ? s.len : 0);
     const unsigned long long big = warp_sum(lg ? s.len : 0);
@@ -1708,8 +1712,8 @@ __global__ void k_emit(SortArgs a, const Seg *__restrict__ L, Count cnt,
         uint32_t ebase = 0;
         if ((threadIdx.x & 31) == 31 && tot) ebase = atomicAdd(&c->n_equal, tot);
         const bool rng = multi && !(b & 1);
-        append_by_length(Seg{p, len, s.depth, flags}, rng, a.warp8_cap, W1, W8, S, L2,
-                         &c->n_large_next, c);
+        append_by_length(Seg{p, len, s.depth, flags}, rng, a.warp8_cap, a.leaf_cap, W1, W8, S,
+                         L2, &c->n_large_next, c);
         const uint32_t tb = warp_slot(rb), tn = warp_slot(rn);
         if (bnd) B[tb] = make_uint2(p, s.depth);
         if (direct) N[tn] = Seg{p, len, s.depth + KEY_BYTES, 0u};
@@ -2096,14 +2100,14 @@ __device__ __forceinline__ void gather_keys(const SortArgs &a, const uint32_t *_
     }
 }
 
-// ---- segments of 33..2048 strings: a group of threads each ------------------
-// A group of GT = 32, 64, 128 or 256 threads sorts one segment of up to
+// ---- segments of 33..4096 strings: a group of threads each ------------------
+// A group of GT = 32, 64, 128, 256 or 512 threads sorts one segment of up to
 // ITEMS * GT strings (8 per thread; 2 or 4 for the smallest).  Records (16-byte
 // key, index) sit in shared memory at their positions; what moves is one
 // 32-bit value per record in registers: the first bits in which the segment's
 // keys differ at all, with the position in the low bits.  Bits that every key
 // of the segment shares carry no order, so they are squeezed out (letters
-// leave 5 bits of each byte): the 21 to 26 squeezed bits order most segments
+// leave 5 bits of each byte): the 20 to 26 squeezed bits order most segments
 // completely.  Values whose squeezed bits tie are checked against the full
 // keys; a tied run out of order is put right in place when it is short, else
 // the segment is refined on further bits.
@@ -2125,7 +2129,7 @@ __device__ __forceinline__ void gather_keys(const SortArgs &a, const uint32_t *_
 // uses (at most 5) and the SM's barriers do not limit occupancy.
 template <int GT>
 __device__ __forceinline__ void group_sync(uint32_t gi) {
-    constexpr int G = SMALL_THREADS / GT;
+    constexpr int G = GT < SMALL_THREADS ? SMALL_THREADS / GT : 1;
     if constexpr (GT == 32) {
         __syncwarp();
     } else {
@@ -2146,7 +2150,7 @@ __device__ __forceinline__ bool group_any(bool want, uint32_t gi) {
     if constexpr (GT == 32) {
         return __any_sync(0xffffffffu, want);
     } else {
-        constexpr int G = SMALL_THREADS / GT;
+        constexpr int G = GT < SMALL_THREADS ? SMALL_THREADS / GT : 1;
         uint32_t r;
 #define SS_BAR_ANY(id)                                                               \
     asm volatile("{ .reg .pred p, q; setp.ne.u32 p, %1, 0; bar.red.or.pred q, " #id  \
@@ -2310,11 +2314,16 @@ struct SegSmem {
 
 // Final order: per rank the record's position and, above it, the key bytes
 // it shares with the record before (SEG_TIE: not known from the values).
-constexpr uint32_t SEG_ORD_BITS = 11, SEG_TIE = 31;
+// The 12-bit positions of the largest groups leave four bits, so that byte 15
+// counts as not known there.
+template <int GT>
+constexpr uint32_t SEG_ORD_BITS = GT == 512 ? 12 : 11;
+template <int GT>
+constexpr uint32_t SEG_TIE = (1u << (16 - SEG_ORD_BITS<GT>)) - 1;
 
 template <int GT, int ITEMS>
 constexpr int SEG_POS_BITS = (ITEMS == 2 ? 1 : ITEMS == 4 ? 2 : 3) +
-                             (GT == 32 ? 5 : GT == 64 ? 6 : GT == 128 ? 7 : 8);
+                             (GT == 32 ? 5 : GT == 64 ? 6 : GT == 128 ? 7 : GT == 256 ? 8 : 9);
 
 // Takes the next bits of `mask` (most significant first, at most `need`) off
 // it as one run of adjacent bits: `width` bits that start `lead` bits from the
@@ -2332,7 +2341,7 @@ __device__ __forceinline__ bool next_run(uint64_t &mask, uint32_t need, uint32_t
 
 // Orders the records by further differing bits after a first sort whose tied
 // runs were out of order: every pass sorts (first rank of the record's tied
-// run, its next differing bits, position) as 64-bit values; 42 or more bits
+// run, its next differing bits, position) as 64-bit values; 40 or more bits
 // a pass, so at most four passes for the 128 key bits.  mh, ml: the differing
 // bits not used yet.  On return sm.val holds positions only, in (key,
 // position) order; sm.idx is read again from I.
@@ -2496,7 +2505,7 @@ __device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint
     // key byte of squeezed bit j.
     const uint32_t f = clz128(mh, ml);
     const uint64_t wm = window64(Key{mh, ml}, f);
-    uint32_t used = 0, byte_of = SEG_TIE;
+    uint32_t used = 0, byte_of = SEG_TIE<GT>;
     uint32_t v[ITEMS], wh[ITEMS], wl[ITEMS];
 #pragma unroll
     for (int q = 0; q < ITEMS; ++q) {
@@ -2577,7 +2586,7 @@ __device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint
         const uint32_t run = group_fix_runs<GT, ITEMS>(sm, len, t, gi);
         if (run) {
             full = run == 2;
-            byte_of = SEG_TIE;  // the values are positions only
+            byte_of = SEG_TIE<GT>;  // the values are positions only
             // The differing bits not used: m0, m1 of the window, and what
             // lies past the window's 64 bits.
             const uint64_t m = (uint64_t)m0 << 32 | m1;
@@ -2599,7 +2608,7 @@ __device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint
     for (int i = 0; i < ITEMS; ++i) {
         const uint32_t x = (v[i] ^ (i ? v[i ? i - 1 : 0] : pv)) >> PB;
         const uint32_t l = __shfl_sync(0xffffffffu, byte_of, __clz(x) + used - 32);
-        const uint32_t h = l * (1u << SEG_ORD_BITS) + (v[i] & PM);
+        const uint32_t h = l * (1u << SEG_ORD_BITS<GT>) + (v[i] & PM);
         if (i & 1)
             o[i / 2] += h * 65536u;
         else
@@ -2699,13 +2708,13 @@ __device__ __forceinline__ bool sort_segment(const SortArgs &a, const Seg &s, Se
             full = order_segment<GT, 8>(sm, I, s.len, mh, ml, t, gi);
     } else {  // all keys equal: position order
         for (uint32_t e = t; e < s.len; e += GT)
-            reinterpret_cast<uint16_t *>(sm.val)[e] = (uint16_t)(SEG_TIE << SEG_ORD_BITS | e);
+            reinterpret_cast<uint16_t *>(sm.val)[e] = (uint16_t)(SEG_TIE<GT> << SEG_ORD_BITS<GT> | e);
     }
     group_sync<GT>(gi);
     // Results in rank order: indices, LCPs, first and last key, next-round
     // runs.  Ties read both keys.
     const uint16_t *ord = reinterpret_cast<const uint16_t *>(sm.val);
-    constexpr uint32_t OM = (1u << SEG_ORD_BITS) - 1;
+    constexpr uint32_t OM = (1u << SEG_ORD_BITS<GT>) - 1;
     auto key_at = [&](uint32_t r) -> Key { return to_key(sm.key[ord[r] & OM]); };
     uint32_t *oi = a.idx[0] + s.start + t, *ol = a.lcp + s.start + t;
     if (t < 2) {
@@ -2720,8 +2729,8 @@ __device__ __forceinline__ bool sort_segment(const SortArgs &a, const Seg &s, Se
         if (on) oi[e0] = sm.idx[w & OM];
         bool cont = false;  // goes on a run of equal keys that do not end
         if (on && e) {
-            uint32_t l = w >> SEG_ORD_BITS;
-            if (l == SEG_TIE) {
+            uint32_t l = w >> SEG_ORD_BITS<GT>;
+            if (l == SEG_TIE<GT>) {
                 const Key k = to_key(sm.key[w & OM]), kp = key_at(e - 1);
                 const bool same = key_eq(kp, k);
                 cont = same && !key_is_end(k);
@@ -2758,15 +2767,16 @@ __device__ __forceinline__ bool sort_segment(const SortArgs &a, const Seg &s, Se
 }
 
 // GT = 32 takes the segments of 33..256 strings and sorts each with 2, 4 or 8
-// strings per thread; 64, 128 and 256 take one size class each.
+// strings per thread; 64, 128, 256 and 512 take one size class each.
 template <int GT>
-constexpr size_t SEG_SMEM = (SMALL_THREADS / GT) * sizeof(SegSmem<GT, 8>);
+constexpr int SEG_CTA = GT < SMALL_THREADS ? SMALL_THREADS : GT;  // threads of a CTA
+template <int GT>
+constexpr size_t SEG_SMEM = (SEG_CTA<GT> / GT) * sizeof(SegSmem<GT, 8>);
 
 template <int GT>
-__global__ void __launch_bounds__(SMALL_THREADS, 4) k_segsort(SortArgs a,
-                                                              const Seg *__restrict__ T0, Span sp,
-                                                              Seg *N, Counters *c) {
-    constexpr uint32_t G = SMALL_THREADS / GT;
+__global__ void __launch_bounds__(SEG_CTA<GT>, 1024 / SEG_CTA<GT>)
+    k_segsort(SortArgs a, const Seg *__restrict__ T0, Span sp, Seg *N, Counters *c) {
+    constexpr uint32_t G = GT < SMALL_THREADS ? SMALL_THREADS / GT : 1;
     extern __shared__ __align__(16) unsigned char seg_smem[];
     const uint32_t lo = count_of(sp.lo);
     const Seg *__restrict__ T = T0 + lo;
@@ -2849,7 +2859,7 @@ __global__ void k_g_round_begin(GraphState *g, Counters *c, cudaGraphConditional
     if (threadIdx.x == 0) {
         cudaGraphSetConditional(h_round, 0u);
         g->cur_w1 = g->cur_w8 = g->cur_e = 0;
-        g->cur_s[0] = g->cur_s[1] = g->cur_s[2] = 0;
+        for (uint32_t &s : g->cur_s) s = 0;
         g->levels = 0;
     }
 }
@@ -2906,6 +2916,7 @@ __global__ void k_g_level_end(GraphState *g, Counters *c, Seg *L, const Seg *__r
     g->cur_s[0] = c->n_small;
     g->cur_s[1] = c->n_small2;
     g->cur_s[2] = c->n_small3;
+    g->cur_s[3] = c->n_small4;
     g->cur_e = c->n_equal;
     bool more = n > 0;
     if (more && g->levels >= g->max_levels) {
@@ -2923,7 +2934,7 @@ __global__ void k_g_round_end(GraphState *g, const Counters *c, Seg *R, const Se
     if (!last_cta(&g->ticket)) return;
     const bool fused = g->fused_round != 0;
     g->small_segments += (unsigned long long)c->n_w1 + c->n_w8 + c->n_small + c->n_small2 +
-                         c->n_small3;
+                         c->n_small3 + c->n_small4;
     g->partitioned += c->partitioned;
     g->gather_elems += c->gather_elems;
     if (fused) g->gather_fused += c->gather_elems;
@@ -3083,6 +3094,8 @@ static void set_smem_attrs() {
                          (int)SEG_SMEM<128>);
     cudaFuncSetAttribute(k_segsort<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)SEG_SMEM<256>);
+    cudaFuncSetAttribute(k_segsort<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)SEG_SMEM<512>);
     done.fetch_or(bit, std::memory_order_release);
 }
 
@@ -3288,8 +3301,10 @@ void launch_block(const SortArgs &a, const Seg *S, Span sp, int cls, Seg *N, Cou
         k_segsort<64><<<grid, SMALL_THREADS, SEG_SMEM<64>, st>>>(a, S, sp, N, c);
     else if (cls == 1)
         k_segsort<128><<<grid, SMALL_THREADS, SEG_SMEM<128>, st>>>(a, S, sp, N, c);
-    else
+    else if (cls == 2)
         k_segsort<256><<<grid, SMALL_THREADS, SEG_SMEM<256>, st>>>(a, S, sp, N, c);
+    else
+        k_segsort<512><<<grid, SEG_CTA<512>, SEG_SMEM<512>, st>>>(a, S, sp, N, c);
 }
 
 void launch_equal(const SortArgs &a, const Seg *E, Span sp, Seg *N, Counters *c, int grid,

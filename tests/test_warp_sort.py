@@ -57,3 +57,23 @@ def test_one_warp_sort_of_partitioned_segments(sorter, kind):
     p, l = sorter.sort_host(arena, offs)
     rp, rl = pyoracle.oracle_sort(arena, offs)
     assert np.array_equal(p, rp) and np.array_equal(l, rl)
+
+
+def test_large_leaf_buckets():
+    """Sorts of at least 4 Mi strings sort range buckets of 2049..4096 strings
+    on chip (with 12-bit positions, so that a difference in key byte 15 is found
+    in the full keys): wide buckets, strings that differ in their last key byte
+    only, and duplicates."""
+    n = 4_300_000
+    rng = np.random.default_rng(5)
+    rows = np.full((n, 17), 97, dtype=np.uint8)
+    rows[:, 0:3] = rng.integers(97, 123, size=(n, 3))
+    rows[:, 13:16] = rng.integers(97, 123, size=(n, 3))
+    rows[:, 16] = 0
+    arena = np.concatenate([rows.ravel(), np.zeros(16, np.uint8)])
+    offs = np.arange(n, dtype=np.uint64) * 17
+    with pyssort.Sorter(0) as s:
+        s.set_param(pyssort.SSORT_PARAM_TARGET_BUCKET, 2048)
+        p, l = s.sort_host(arena, offs)
+    bad, first = pyoracle.oracle_check(arena, offs, p, l)
+    assert bad == 0, (bad, first)
