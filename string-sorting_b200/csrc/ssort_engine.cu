@@ -71,11 +71,11 @@ int ssort_ctx::scan(const uint32_t *in, uint32_t *out, uint32_t cap, Count n) {
 }
 
 // The count-matrix scan on stream s: single-pass with decoupled look-back
-// (SSORT_PARAM_SCAN = 1; its state is cleared first), or reduce-then-scan.
+// (SSORT_PARAM_SCAN = 1; the sample kernel cleared its state), or
+// reduce-then-scan.
 int ssort_ctx::scan_on(const uint32_t *in, uint32_t *out, uint32_t cap, Count n,
                        cudaStream_t s) {
     if (scan_lookback) {
-        SS_CUDA(cudaMemsetAsync(ws.lookback, 0, lookback_state_bytes(cap), s));
         LAUNCH(this, "scan",
                launch_scan_lookback(in, out, cap, n, ws.lookback, &ws.ctr->error, s));
     } else {
@@ -202,10 +202,8 @@ int ssort_ctx::round_body(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt,
         const bool first = fused_gather && levels_this_round == 1;
         const Count nl = hcount(n_large);
         LAUNCH(this, "sample",
-               launch_sample(a, lcur, nl, ws.spl, ws.nspl, ws.tbl, ws.ntiles, ws.cm_size,
-                             first, 0, st));
-        LAUNCH(this, "scan_pair",
-               launch_scan_pair(ws.ntiles, ws.tile_base, ws.cm_size, ws.cm_base, nl, st));
+               launch_sample(a, lcur, nl, ws.spl, ws.nspl, ws.tbl, level_bases(ws), first, dc,
+                             0, st));
         LAUNCH(this, first ? "count_gather" : "count",
                launch_count(a, lcur, nl, ws.tile_base, ws.spl, ws.nspl, ws.tbl, ws.cm_base,
                             ws.cm, dc, first, g2, st));

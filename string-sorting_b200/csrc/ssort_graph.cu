@@ -164,10 +164,8 @@ int ssort_ctx::graph_build(const SortArgs &a) {
                 const bool gather = f == 0;  // body 0 runs when the condition is set
                 SS_CUDA(cudaStreamBeginCaptureToGraph(s2, fb[f], nullptr, nullptr, 0, mode));
                 LAUNCH(this, "sample",
-                       launch_sample(a, ws.L, nl, ws.spl, ws.nspl, ws.tbl, ws.ntiles, ws.cm_size,
-                                     gather, g2, s2));
-                LAUNCH(this, "scan_pair",
-                       launch_scan_pair(ws.ntiles, ws.tile_base, ws.cm_size, ws.cm_base, nl, s2));
+                       launch_sample(a, ws.L, nl, ws.spl, ws.nspl, ws.tbl, level_bases(ws),
+                                     gather, dc, g2, s2));
                 LAUNCH(this, gather ? "count_gather" : "count",
                        launch_count(a, ws.L, nl, ws.tile_base, ws.spl, ws.nspl, ws.tbl,
                                     ws.cm_base, ws.cm, dc, gather, g2, s2));

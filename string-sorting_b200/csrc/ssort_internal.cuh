@@ -95,7 +95,7 @@ struct Counters {
         block_keyed;
     unsigned long long equal_moved, equal_final;  // equality-bucket copies / lcp fills
     uint32_t n_small2, n_small3, n_small4;  // CTA-sort segments of the 2nd to 4th size class
-    uint32_t pad;
+    uint32_t sample_ticket;  // CTAs of the sample kernel that are done (0 between launches)
     unsigned long long warp1_deep;  // strings re-sorted by in-warp refinement steps
     unsigned long long full_sorted;  // strings of segments re-sorted by the full comparator
     unsigned long long window_saved, window_used;  // key2 entries written / read
@@ -353,9 +353,6 @@ void launch_unbase(uint32_t *perm, const ReqJob *jobs, uint32_t njobs, uint32_t 
                    cudaStream_t st);
 void launch_localize(uint32_t *perm, uint32_t n, const uint32_t *inst_start, uint32_t ninst,
                      cudaStream_t st);
-// Single-CTA scans of short per-segment arrays (out*[n] = totals).
-void launch_scan_pair(const uint32_t *in0, uint32_t *out0, const uint32_t *in1, uint32_t *out1,
-                      Count n, cudaStream_t st);
 void launch_seg_tiles(const Seg *segs, Count n, uint32_t tile, uint32_t *out, cudaStream_t st);
 // exclusive scan of in[0..n) into out[0..n); out[n] = total (out has n+1 slots).
 // cap (host) bounds n and sizes the grid; n itself is count_of(n).
@@ -364,18 +361,23 @@ void launch_scan(const uint32_t *in, uint32_t *out, uint32_t cap, Count n, uint3
 uint32_t scan_partials_needed(uint32_t n);
 // The same scan in one pass with decoupled look-back: tiles take their order
 // from a ticket and add up their predecessors' published sums; `state` holds
-// a ticket word and one status word per tile and must be zeroed first
-// (lookback_state_bytes(cap)); a look-back that waits too long sets *err.
-size_t lookback_state_bytes(uint32_t cap);
+// a ticket word and one status word per tile, zeroed by the level's sample
+// kernel; a look-back that waits too long sets *err.
 void launch_scan_lookback(const uint32_t *in, uint32_t *out, uint32_t cap, Count n,
                           unsigned char *state, uint32_t *err, cudaStream_t st);
 void launch_gather(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
                    Counters *c, int grid, cudaStream_t st);
 // from_arena / gather: first partition level of a round, whose keys the
 // count kernel gathers from the arena (the sample reads its strings there).
+// Also the level's per-segment bases and a cleared look-back state.
+struct LevelBases {
+    uint32_t *ntiles, *cm_size;     // per segment: tiles, count-matrix entries
+    uint32_t *tile_base, *cm_base;  // their exclusive scans (totals at [nL])
+    unsigned long long *lookback;
+};
 void launch_sample(const SortArgs &a, const Seg *L, Count nL, ulonglong2 *spl,
-                   uint32_t *nspl, uint16_t *tbl, uint32_t *ntiles, uint32_t *cm_size,
-                   bool from_arena, int grid, cudaStream_t st);
+                   uint32_t *nspl, uint16_t *tbl, const LevelBases &lb, bool from_arena,
+                   Counters *c, int grid, cudaStream_t st);
 void launch_count(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
                   const ulonglong2 *spl, const uint32_t *nspl, const uint16_t *tbl,
                   const uint32_t *cm_base, uint32_t *cm, Counters *c, bool gather, int grid,
@@ -425,5 +427,10 @@ void launch_g_level_end(GraphState *g, Counters *c, Seg *L, const Seg *L2,
 // from N to R, and the round condition is set.
 void launch_g_round_end(GraphState *g, Counters *c, Seg *R, const Seg *N,
                         unsigned long long h_round, int grid, cudaStream_t st);
+
+inline LevelBases level_bases(const Workspace &w) {
+    return LevelBases{w.ntiles, w.cm_size, w.tile_base, w.cm_base,
+                      reinterpret_cast<unsigned long long *>(w.lookback)};
+}
 
 }  // namespace ssort

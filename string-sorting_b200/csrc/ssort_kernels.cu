@@ -13,6 +13,7 @@
 // is_end test, src/util/get_char.h:162-175, and its bucket-skip rule,
 // src/msd_ce.cpp:402) become the next round's segments at depth+16; every
 // other adjacent pair gets its LCP here.
+#include <algorithm>
 #include <atomic>
 
 #include "ssort_internal.cuh"
@@ -265,10 +266,6 @@ __device__ __forceinline__ void prefetch_l2(const void *p, uint64_t bytes) {
     }
 }
 
-// Padded shared-memory index: one spare slot per 8 keeps both the blocked
-// (stride 8) and the striped (stride 1) access patterns free of bank conflicts.
-__device__ __forceinline__ uint32_t pad(uint32_t e) { return e + (e >> 3); }
-
 // ---- packed 64-bit sort keys -------------------------------------------------
 // In a segment of at most 32 strings every key shares its first f bits (f =
 // leading zeros of the OR of key ^ key0).  The 53 bits after them, with the
@@ -293,85 +290,6 @@ __device__ __forceinline__ uint64_t window64(const Key &k, uint32_t f) {
 
 __device__ __forceinline__ uint64_t sort_key(const Key &k, uint32_t f, uint32_t pos) {
     return (window64(k, f) & ~POS_MASK) | pos;
-}
-
-// Merge-path split over two sorted uint64 runs (values distinct).
-__device__ __forceinline__ uint32_t merge_split64(const uint64_t *s, uint32_t a0, uint32_t la,
-                                                  uint32_t b0, uint32_t lb, uint32_t d) {
-    uint32_t lo = d > lb ? d - lb : 0, hi = d < la ? d : la;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (s[pad(a0 + mid)] < s[pad(b0 + d - 1 - mid)])
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    return lo;
-}
-
-// Compare-exchange: afterwards a <= b.
-__device__ __forceinline__ void cas64(uint64_t &a, uint64_t &b) {
-    const bool lt = a < b;
-    const uint64_t lo = lt ? a : b, hi = lt ? b : a;
-    a = lo;
-    b = hi;
-}
-
-// Sorts ITEMS (2, 4 or 8) values held by one thread: optimal sorting networks
-// of 1, 5 and 19 comparators.
-template <int ITEMS>
-__device__ __forceinline__ void sort_local64(uint64_t (&v)[ITEMS]) {
-    if constexpr (ITEMS == 2) {
-        cas64(v[0], v[1]);
-    } else if constexpr (ITEMS == 4) {
-        cas64(v[0], v[1]); cas64(v[2], v[3]);
-        cas64(v[0], v[2]); cas64(v[1], v[3]);
-        cas64(v[1], v[2]);
-    } else {
-        static_assert(ITEMS == 8, "2, 4 or 8 values per thread");
-        cas64(v[0], v[2]); cas64(v[1], v[3]); cas64(v[4], v[6]); cas64(v[5], v[7]);
-        cas64(v[0], v[4]); cas64(v[1], v[5]); cas64(v[2], v[6]); cas64(v[3], v[7]);
-        cas64(v[0], v[1]); cas64(v[2], v[3]); cas64(v[4], v[5]); cas64(v[6], v[7]);
-        cas64(v[2], v[4]); cas64(v[3], v[5]);
-        cas64(v[1], v[4]); cas64(v[3], v[6]);
-        cas64(v[1], v[2]); cas64(v[3], v[4]); cas64(v[5], v[6]);
-    }
-}
-
-// One warp sorts the 32 * ITEMS values v (lane l holds any ITEMS of them)
-// into sv[pad(base .. base + 32 * ITEMS)]: every lane sorts its own values in
-// registers, then merge-path passes (synchronised by __syncwarp only) double
-// the sorted runs up to the whole warp.  Fewer instructions than the bitonic
-// network, whose 15 cross-lane stages each move every value through a
-// shuffle; equal values (the all-ones padding) merge consistently.
-template <int ITEMS>
-__device__ __forceinline__ void warp_merge_sort64(uint64_t (&v)[ITEMS], uint64_t *sv,
-                                                  uint32_t base, uint32_t lane) {
-    sort_local64<ITEMS>(v);
-    const uint32_t o = lane * ITEMS;
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) sv[pad(base + o + i)] = v[i];
-    __syncwarp();
-#pragma unroll
-    for (uint32_t run = ITEMS; run < 32 * ITEMS; run <<= 1) {
-        const uint32_t a0 = base + (o & ~(2 * run - 1)), b0 = a0 + run;
-        const uint32_t d = o & (2 * run - 1);
-        uint32_t ia = merge_split64(sv, a0, run, b0, run, d);
-        uint32_t ib = d - ia;
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) {
-            const uint64_t va = ia < run ? sv[pad(a0 + ia)] : ~0ull;
-            const uint64_t vb = ib < run ? sv[pad(b0 + ib)] : ~0ull;
-            const bool take_a = ib >= run || (ia < run && va < vb);
-            v[i] = take_a ? va : vb;
-            ia += take_a;
-            ib += !take_a;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) sv[pad(base + o + i)] = v[i];
-        __syncwarp();
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -698,6 +616,7 @@ __global__ void k_byte_hist(const uint8_t *__restrict__ arena, uint64_t arena_by
 constexpr int SMALL_SCAN_THREADS = 1024;
 
 // Inclusive scan of v across the CTA; returns the CTA total in `total`.
+template <int THREADS>
 __device__ __forceinline__ uint32_t cta_inclusive_scan(uint32_t v, uint32_t &total,
                                                        uint32_t *warp_sums) {
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -710,40 +629,13 @@ __device__ __forceinline__ uint32_t cta_inclusive_scan(uint32_t v, uint32_t &tot
     __syncthreads();
     uint32_t before = 0;
     total = 0;
-    for (uint32_t q = 0; q < SMALL_SCAN_THREADS / 32; ++q) {
+    for (uint32_t q = 0; q < THREADS / 32; ++q) {
         const uint32_t x = warp_sums[q];
         if (q < w) before += x;
         total += x;
     }
     __syncthreads();
     return v + before;
-}
-
-// out0/out1 = exclusive scans of in0/in1 (n entries); out*[n] = totals.
-__global__ void __launch_bounds__(SMALL_SCAN_THREADS) k_scan_pair(const uint32_t *__restrict__ in0,
-                                                                   uint32_t *out0,
-                                                                   const uint32_t *__restrict__ in1,
-                                                                   uint32_t *out1, Count cnt) {
-    __shared__ uint32_t warp_sums[SMALL_SCAN_THREADS / 32];
-    const uint32_t n = count_of(cnt);
-    uint32_t c0 = 0, c1 = 0;
-    for (uint32_t b = 0; b < n; b += SMALL_SCAN_THREADS) {
-        const uint32_t i = b + threadIdx.x;
-        const uint32_t v0 = i < n ? in0[i] : 0, v1 = i < n ? in1[i] : 0;
-        uint32_t t0, t1;
-        const uint32_t s0 = cta_inclusive_scan(v0, t0, warp_sums);
-        const uint32_t s1 = cta_inclusive_scan(v1, t1, warp_sums);
-        if (i < n) {
-            out0[i] = c0 + s0 - v0;
-            out1[i] = c1 + s1 - v1;
-        }
-        c0 += t0;
-        c1 += t1;
-    }
-    if (threadIdx.x == 0) {
-        out0[n] = c0;
-        out1[n] = c1;
-    }
 }
 
 // out = exclusive scan of ceil(len / tile) over the segments; out[n] = total.
@@ -757,7 +649,7 @@ __global__ void __launch_bounds__(SMALL_SCAN_THREADS) k_seg_tiles(const Seg *__r
         const uint32_t i = b + threadIdx.x;
         const uint32_t v = i < n ? (segs[i].len + tile - 1) / tile : 0;
         uint32_t t;
-        const uint32_t s = cta_inclusive_scan(v, t, warp_sums);
+        const uint32_t s = cta_inclusive_scan<SMALL_SCAN_THREADS>(v, t, warp_sums);
         if (i < n) out[i] = c + s - v;
         c += t;
     }
@@ -909,9 +801,310 @@ __global__ void __launch_bounds__(GATHER_THREADS) k_gather(SortArgs a, const Seg
     }
 }
 
+// Keys at `depth` of up to G strings per thread: elements e0 + q * stride
+// below len, whose indices stand at I[at[q]].  Every step's loads are issued for all G strings
+// before any is used (index, then offset, then the two 16-byte words that
+// hold the key), so that G chains of dependent reads overlap.
+template <int G>
+__device__ __forceinline__ void gather_keys_at(const SortArgs &a, const uint32_t *__restrict__ I,
+                                               uint32_t depth, const uint32_t (&at)[G],
+                                               uint32_t e0, uint32_t stride, uint32_t len,
+                                               Key (&kk)[G], uint32_t (&ii)[G]) {
+    uint64_t pos[G];
+    ulonglong2 v0[G], v1[G];
+#pragma unroll
+    for (int q = 0; q < G; ++q) ii[q] = e0 + q * stride < len ? I[at[q]] : IDX_MAX;
+#pragma unroll
+    for (int q = 0; q < G; ++q)
+        pos[q] = ii[q] != IDX_MAX ? string_offset(a.offs, a.off_width, ii[q]) + depth : 0ull;
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+        const uint64_t base = pos[q] & ~15ull;
+        const bool in = ii[q] != IDX_MAX && key_words_inside(a.arena_bytes, base);
+        const ulonglong2 *w = reinterpret_cast<const ulonglong2 *>(a.arena + base);
+        v0[q] = in ? __ldg(w) : make_ulonglong2(0, 0);
+        v1[q] = in && (pos[q] & 15) ? __ldg(w + 1) : make_ulonglong2(0, 0);
+    }
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+        if (key_words_inside(a.arena_bytes, pos[q] & ~15ull))
+            kk[q] = key_of_words(v0[q], v1[q], (uint32_t)pos[q] & 15u);
+        else if (ii[q] != IDX_MAX)
+            kk[q] = load_key_tail(a.arena, a.arena_bytes, pos[q]);
+    }
+}
+
+// The same for the elements' own places in I.
+template <int G>
+__device__ __forceinline__ void gather_keys(const SortArgs &a, const uint32_t *__restrict__ I,
+                                            uint32_t depth, uint32_t e0, uint32_t stride,
+                                            uint32_t len, Key (&kk)[G], uint32_t (&ii)[G]) {
+    uint32_t at[G];
+#pragma unroll
+    for (int q = 0; q < G; ++q) at[q] = e0 + q * stride;
+    gather_keys_at<G>(a, I, depth, at, e0, stride, len, kk, ii);
+}
+
+// ---- register sorts of 32-bit values (samples and on-chip segments) ---------
+// Barrier among the GT threads of group gi: named barrier 1 + gi (0 is
+// __syncthreads).  Immediate ids, so that a CTA claims only the barriers it
+// uses (at most 5) and the SM's barriers do not limit occupancy.
+template <int GT>
+__device__ __forceinline__ void group_sync(uint32_t gi) {
+    constexpr int G = GT < SMALL_THREADS ? SMALL_THREADS / GT : 1;
+    if constexpr (GT == 32) {
+        __syncwarp();
+    } else {
+        if (G == 1 || gi == 0)
+            asm volatile("bar.sync 1, %0;" ::"n"(GT) : "memory");
+        else if (G == 2 || gi == 1)
+            asm volatile("bar.sync 2, %0;" ::"n"(GT) : "memory");
+        else if (gi == 2)
+            asm volatile("bar.sync 3, %0;" ::"n"(GT) : "memory");
+        else
+            asm volatile("bar.sync 4, %0;" ::"n"(GT) : "memory");
+    }
+}
+
+// Whether any thread of the group has `want`; a barrier of the group.
+template <int GT>
+__device__ __forceinline__ bool group_any(bool want, uint32_t gi) {
+    if constexpr (GT == 32) {
+        return __any_sync(0xffffffffu, want);
+    } else {
+        constexpr int G = GT < SMALL_THREADS ? SMALL_THREADS / GT : 1;
+        uint32_t r;
+#define SS_BAR_ANY(id)                                                               \
+    asm volatile("{ .reg .pred p, q; setp.ne.u32 p, %1, 0; bar.red.or.pred q, " #id  \
+                 ", %2, p; selp.u32 %0, 1, 0, q; }"                                  \
+                 : "=r"(r)                                                           \
+                 : "r"((uint32_t)want), "n"(GT)                                      \
+                 : "memory")
+        if (G == 1 || gi == 0)
+            SS_BAR_ANY(1);
+        else if (G == 2 || gi == 1)
+            SS_BAR_ANY(2);
+        else if (gi == 2)
+            SS_BAR_ANY(3);
+        else
+            SS_BAR_ANY(4);
+#undef SS_BAR_ANY
+        return r != 0;
+    }
+}
+
+template <typename V>
+__device__ __forceinline__ void cmp_swap(V &a, V &b) {
+    const V lo = min(a, b), hi = max(a, b);
+    a = lo;
+    b = hi;
+}
+
+// One exchange between threads: the lower one keeps the smaller value, the
+// upper one (up) the larger.
+template <typename V>
+__device__ __forceinline__ V keep_side(V v, V o, bool up) {
+    return (o < v) != up ? o : v;
+}
+
+// Batcher's odd-even merge sort of v[LO .. LO + N), as templates so that every
+// index is a constant and the values stay in registers.
+template <int LO, int N, int R, int ITEMS, typename V>
+__device__ __forceinline__ void net_merge(V (&v)[ITEMS]) {
+    if constexpr (2 * R < N) {
+        net_merge<LO, N, 2 * R>(v);
+        net_merge<LO + R, N, 2 * R>(v);
+#pragma unroll
+        for (int i = LO + R; i + R < LO + N; i += 2 * R) cmp_swap(v[i], v[i + R]);
+    } else {
+        cmp_swap(v[LO], v[LO + R]);
+    }
+}
+
+template <int LO, int N, int ITEMS, typename V>
+__device__ __forceinline__ void net_sort(V (&v)[ITEMS]) {
+    if constexpr (N > 1) {
+        net_sort<LO, N / 2>(v);
+        net_sort<LO + N / 2, N / 2>(v);
+        net_merge<LO, N, 1>(v);
+    }
+}
+
+// Bitonic half-cleaners of strides M, M / 2, .. 1 inside a thread.
+template <int M, int ITEMS, typename V>
+__device__ __forceinline__ void net_clean(V (&v)[ITEMS]) {
+    if constexpr (M >= 1) {
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i)
+            if ((i & M) == 0) cmp_swap(v[i], v[i + M]);
+        net_clean<M / 2>(v);
+    }
+}
+
+// Half-cleaners of lane strides m, m / 2, .. 1, then inside the lanes.  The
+// loop over strides stays a loop: unrolled, the sorts outgrow the
+// instruction cache.
+template <int ITEMS, typename V>
+__device__ __forceinline__ void warp_clean(V (&v)[ITEMS], uint32_t m, uint32_t lane) {
+#pragma unroll 1
+    for (; m >= 1; m /= 2) {
+        const bool up = (lane & m) != 0;
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i)
+            v[i] = keep_side(v[i], __shfl_xor_sync(0xffffffffu, v[i], m), up);
+    }
+    net_clean<ITEMS / 2>(v);
+}
+
+// Every thread stores its values to x (16-byte words, consecutive threads
+// next to each other) and loads those of thread `from`.  Two barriers.
+template <int GT, int ITEMS, typename V>
+__device__ __forceinline__ void swap_values(const V (&v)[ITEMS], V (&o)[ITEMS], void *x,
+                                            uint32_t t, uint32_t from, uint32_t gi) {
+    constexpr int PER = 16 / sizeof(V);  // values per 16-byte word
+    V w[PER];
+#pragma unroll
+    for (int j = 0; j < ITEMS / PER; ++j) {
+#pragma unroll
+        for (int q = 0; q < PER; ++q) w[q] = v[j * PER + q];
+        static_cast<uint4 *>(x)[j * GT + t] = *reinterpret_cast<const uint4 *>(w);
+    }
+    group_sync<GT>(gi);
+#pragma unroll
+    for (int j = 0; j < ITEMS / PER; ++j) {
+        *reinterpret_cast<uint4 *>(w) = static_cast<const uint4 *>(x)[j * GT + from];
+#pragma unroll
+        for (int q = 0; q < PER; ++q) o[j * PER + q] = w[q];
+    }
+    group_sync<GT>(gi);
+}
+
+// Sorts the GT * ITEMS values of a group; thread t ends with ranks t * ITEMS
+// .. t * ITEMS + ITEMS - 1.  Odd-even merge sort inside a thread, then bitonic
+// merges of 2, 4, .. GT threads whose first stage compares mirrored positions,
+// so that every stage sorts ascending; strides of 32 threads and more go
+// through shared memory (x: GT * ITEMS values).  With `threads` < GT (a power
+// of two, at least 32) aligned blocks of that many threads sort on their own.
+template <int GT, int ITEMS, typename V>
+__device__ __forceinline__ void group_net_sort(V (&v)[ITEMS], void *x, uint32_t t, uint32_t gi,
+                                               uint32_t threads = GT) {
+    const uint32_t lane = t & 31;
+    net_sort<0, ITEMS>(v);
+#pragma unroll 1
+    for (uint32_t half = 1; half < 32; half *= 2) {
+        const bool up = (lane & half) != 0;
+        const uint32_t mirror = 2 * half - 1;
+#pragma unroll
+        for (int i = 0; i < ITEMS / 2; ++i) {
+            const V p = __shfl_xor_sync(0xffffffffu, v[ITEMS - 1 - i], mirror);
+            const V q = __shfl_xor_sync(0xffffffffu, v[i], mirror);
+            v[i] = keep_side(v[i], p, up);
+            v[ITEMS - 1 - i] = keep_side(v[ITEMS - 1 - i], q, up);
+        }
+        warp_clean<ITEMS>(v, half / 2, lane);
+    }
+    if constexpr (GT > 32) {
+#pragma unroll 1
+        for (uint32_t half = 32; half < threads; half *= 2) {
+            V o[ITEMS];
+            swap_values<GT, ITEMS>(v, o, x, t, t ^ (2 * half - 1), gi);
+            const bool up = (t & half) != 0;
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) v[i] = keep_side(v[i], o[ITEMS - 1 - i], up);
+#pragma unroll 1
+            for (uint32_t m = half / 2; m >= 32; m /= 2) {
+                swap_values<GT, ITEMS>(v, o, x, t, t ^ m, gi);
+                const bool um = (t & m) != 0;
+#pragma unroll
+                for (int i = 0; i < ITEMS; ++i) v[i] = keep_side(v[i], o[i], um);
+            }
+            warp_clean<ITEMS>(v, 16, lane);
+        }
+    }
+}
+
+// The first differing bits of a set of keys, as the high bits of 32-bit
+// values: bits that all keys share carry no order and are squeezed out.
+template <int ITEMS>
+struct Squeezed {
+    uint32_t v[ITEMS];  // squeezed bits << pos_bits | position, all ones past the end
+    uint32_t f;         // first differing key bit
+    uint32_t used;      // squeezed bits taken
+    uint32_t byte_of;   // in lane j < used: the key byte of squeezed bit j; else `none`
+    uint32_t m0, m1;    // differing bits of the 64 from bit f on that were not taken
+};
+
+// Squeezes the keys at positions e = q * stride + t < len (q < ITEMS) whose
+// differing bits are mh, ml (not both 0): the first 32 - pos_bits differing
+// ones of the 64 bits from the first on, run by run of adjacent bits.
+template <int ITEMS>
+__device__ __forceinline__ void squeeze_keys(Squeezed<ITEMS> &o, const ulonglong2 *key,
+                                             uint32_t len, uint32_t stride, uint32_t t,
+                                             uint64_t mh, uint64_t ml, uint32_t pos_bits,
+                                             uint32_t none) {
+    const uint32_t lane = t & 31, want = 32 - pos_bits;
+    const uint32_t f = clz128(mh, ml);
+    const uint64_t wm = window64(Key{mh, ml}, f);
+    uint32_t wh[ITEMS], wl[ITEMS];
+#pragma unroll
+    for (int q = 0; q < ITEMS; ++q) {
+        const uint32_t e = q * stride + t;
+        const Key k = e < len ? to_key(key[e]) : Key{0, 0};
+        // the 96 bits from the 32-bit word that holds bit f on
+        const uint64_t top = f < 64 ? k.hi : k.lo, next = f < 64 ? k.lo : 0;
+        const uint32_t w0 = (uint32_t)(top >> 32), w1 = (uint32_t)top,
+                       w2 = (uint32_t)(next >> 32), w3 = (uint32_t)next;
+        wh[q] = f & 32 ? __funnelshift_l(w2, w1, f) : __funnelshift_l(w1, w0, f);
+        wl[q] = f & 32 ? __funnelshift_l(w3, w2, f) : __funnelshift_l(w2, w1, f);
+        o.v[q] = 0;
+    }
+    uint32_t used = 0, byte_of = none;
+    auto squeeze = [&](uint32_t &m, const uint32_t(&w)[ITEMS], uint32_t base) {
+#pragma unroll 1
+        while (m && used < want) {
+            const uint32_t lead = __clz(m);
+            const uint32_t width = min((uint32_t)__clz(~(m << lead)), want - used);
+            const uint32_t mul = 1u << width, low = mul - 1, sh = 32 - lead - width;
+#pragma unroll
+            for (int q = 0; q < ITEMS; ++q) o.v[q] = o.v[q] * mul + ((w[q] >> sh) & low);
+            if (lane - used < width) byte_of = (f + base + lead + lane - used) >> 3;
+            used += width;
+            m &= ~(low << sh);
+        }
+    };
+    o.m0 = (uint32_t)(wm >> 32);
+    o.m1 = (uint32_t)wm;
+    squeeze(o.m0, wh, 0);
+    squeeze(o.m1, wl, 32);
+    o.f = f;
+    o.used = used;
+    o.byte_of = byte_of;
+#pragma unroll
+    for (int q = 0; q < ITEMS; ++q) {
+        const uint32_t e = q * stride + t;
+        o.v[q] = e < len ? o.v[q] << pos_bits | e : ~0u;
+    }
+}
+
+__device__ __forceinline__ uint64_t warp_or64(uint64_t x) {
+    return (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(x >> 32)) << 32 |
+           __reduce_or_sync(0xffffffffu, (uint32_t)x);
+}
+
 // ---- splitter selection: one CTA per large segment ------------------------
 constexpr int SAMPLE_THREADS = 512;
-constexpr uint32_t SAMPLE_KEEP = 1024;  // samples kept in shared memory (16 KB)
+static_assert(SAMPLES_MAX == SAMPLE_THREADS * 8, "8 samples per thread");
+
+// The samples' keys, their sorted values (later the splitters' window bits),
+// the candidates: 89 KB, two CTAs per SM.
+struct SampleSmem {
+    ulonglong2 key[SAMPLES_MAX];
+    ulonglong2 cands[SAMPLE_THREADS];
+    uint32_t val[SAMPLES_MAX];
+    uint64_t red[SAMPLE_THREADS / 32][2];
+    uint32_t warp_cnt[SAMPLE_THREADS / 32 + 1];
+    uint32_t last;
+};
 
 __device__ __forceinline__ uint32_t hash32(uint32_t x) {
     x ^= x >> 16;
@@ -922,41 +1115,20 @@ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
     return x;
 }
 
+// Splitters of segment si.  The samples are ordered as 32-bit values (their
+// first differing bits and the sample number) by the register network of the
+// on-chip sorts: with 4096 samples and 64-bit keys merged in shared memory
+// this CTA took most of the first level's latency (one segment of 10 M URLs
+// 35 us).  The order only picks quantiles: samples that tie on 20 to 24
+// differing bits may stand in any order, and the chosen candidates are put in
+// full-key order below.
 __device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__restrict__ L,
-                                               uint32_t si, ulonglong2 *spl, uint32_t *nspl,
-                                               uint16_t *tbl, uint32_t *ntiles, uint32_t *cm_size,
-                                               bool from_arena);
-
-// One CTA per large segment at a time (segments si = blockIdx.x, + gridDim.x, ...).
-__global__ void __launch_bounds__(SAMPLE_THREADS, 2) k_sample(SortArgs a, const Seg *__restrict__ L,
-                                                           Count cnt, ulonglong2 *spl,
-                                                           uint32_t *nspl, uint16_t *tbl,
-                                                           uint32_t *ntiles, uint32_t *cm_size,
-                                                           bool from_arena) {
-    const uint32_t nL = count_of(cnt);
-    for (uint32_t si = blockIdx.x; si < nL; si += gridDim.x) {
-        sample_segment(a, L, si, spl, nspl, tbl, ntiles, cm_size, from_arena);
-        __syncthreads();  // shared memory is reused by the next segment
-    }
-}
-
-__device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__restrict__ L,
-                                               uint32_t si, ulonglong2 *spl, uint32_t *nspl,
-                                               uint16_t *tbl, uint32_t *ntiles, uint32_t *cm_size,
-                                               bool from_arena) {
-    // sv: the samples' packed sort keys (padded layout).  Up to SAMPLE_KEEP
-    // samples are loaded by all threads into smp and the candidates are read
-    // from there; larger samples stay in registers and only the chosen
-    // candidates are read again.
-    extern __shared__ __align__(16) unsigned char sample_smem[];
-    uint64_t *sv = reinterpret_cast<uint64_t *>(sample_smem);
-    ulonglong2 *smp = reinterpret_cast<ulonglong2 *>(sv + SAMPLES_MAX + SAMPLES_MAX / 8);
-    __shared__ ulonglong2 cands[SAMPLE_THREADS];
-    __shared__ uint32_t warp_cnt[SAMPLE_THREADS / 32 + 1];
-    __shared__ uint64_t red[4][SAMPLE_THREADS / 32];
+                                               uint32_t si, SampleSmem &sm, ulonglong2 *spl,
+                                               uint32_t *nspl, uint16_t *tbl, uint32_t *ntiles,
+                                               uint32_t *cm_size, bool from_arena) {
     const Seg s = L[si];
     const ulonglong2 *K = a.keyb(s.flags & SEG_BUF1) + s.start;
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
     const uint32_t tcls = a.target_by_class[31 - __clz(s.len)];
     const uint32_t tb = tcls ? tcls : a.target_bucket;
     uint32_t k = (s.len + tb - 1) / tb;
@@ -972,125 +1144,77 @@ __device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__r
         const uint32_t r = hash32(s.start * 0x9E3779B1u + i * 0x85EBCA77u + s.len);
         return (uint32_t)(((uint64_t)r * s.len) >> 32);
     };
-    auto key_at = [&](uint32_t e) -> Key {
-        return from_arena ? load_key(a.arena, a.arena_bytes,
-                                     string_offset(a.offs, a.off_width, a.idx[0][s.start + e]) +
-                                         s.depth)
-                          : to_key(K[e]);
-    };
-    // Warp w < S / 256 holds samples w * 256 + lane * 8 + i (i < 8).
-    const bool active = w * 256 < S;
-    const bool kept = S <= SAMPLE_KEEP;  // block-uniform
-    if (kept) {
-        for (uint32_t i = threadIdx.x; i < S; i += SAMPLE_THREADS)
-            smp[i] = from_key(key_at(pos_of(i)));
-        __syncthreads();
-    }
-    Key kk[8];
-    uint64_t oh = 0, ol = 0, ah = ~0ull, al = ~0ull;
-    if (active) {
+    constexpr int G = 4;  // samples in flight per thread
+#pragma unroll 1
+    for (uint32_t e0 = t; e0 < S; e0 += G * SAMPLE_THREADS) {
+        uint32_t at[G];
+        Key kk[G];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t e = w * 256 + lane * 8 + i;
-            kk[i] = kept ? to_key(smp[e]) : key_at(pos_of(e));
+        for (int q = 0; q < G; ++q) at[q] = s.start + pos_of(e0 + q * SAMPLE_THREADS);
+        if (from_arena) {
+            uint32_t id[G];
+            gather_keys_at<G>(a, a.idx[0], s.depth, at, e0, SAMPLE_THREADS, S, kk, id);
+        } else {
+#pragma unroll
+            for (int q = 0; q < G; ++q)
+                kk[q] = e0 + q * SAMPLE_THREADS < S ? to_key(K[at[q] - s.start]) : Key{0, 0};
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            oh |= kk[i].hi;
-            ol |= kk[i].lo;
-            ah &= kk[i].hi;
-            al &= kk[i].lo;
-        }
-    }
-    // fs: the first bit in which the samples differ (where OR and AND differ).
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        oh |= __shfl_xor_sync(0xffffffffu, oh, d);
-        ol |= __shfl_xor_sync(0xffffffffu, ol, d);
-        ah &= __shfl_xor_sync(0xffffffffu, ah, d);
-        al &= __shfl_xor_sync(0xffffffffu, al, d);
-    }
-    if (lane == 0) {
-        red[0][w] = oh;
-        red[1][w] = ol;
-        red[2][w] = ah;
-        red[3][w] = al;
+        for (int q = 0; q < G; ++q)
+            if (e0 + q * SAMPLE_THREADS < S) sm.key[e0 + q * SAMPLE_THREADS] = from_key(kk[q]);
     }
     __syncthreads();
-    uint64_t dh = 0, dl = 0;
+    // The first S / 8 threads order the samples, 8 each.
+    const uint32_t act = S / 8;
+    uint64_t mh = 0, ml = 0;
     {
-        uint64_t h1 = 0, l1 = 0, h0 = ~0ull, l0 = ~0ull;
+        const Key k0 = to_key(sm.key[0]);
+        for (uint32_t e = t; e < S; e += SAMPLE_THREADS) {
+            const Key x = to_key(sm.key[e]);
+            mh |= x.hi ^ k0.hi;
+            ml |= x.lo ^ k0.lo;
+        }
+        mh = warp_or64(mh);
+        ml = warp_or64(ml);
+        if (lane == 0) {
+            sm.red[w][0] = mh;
+            sm.red[w][1] = ml;
+        }
+        __syncthreads();
 #pragma unroll
         for (int q = 0; q < SAMPLE_THREADS / 32; ++q) {
-            h1 |= red[0][q];
-            l1 |= red[1][q];
-            h0 &= red[2][q];
-            l0 &= red[3][q];
+            mh |= sm.red[q][0];
+            ml |= sm.red[q][1];
         }
-        dh = h1 ^ h0;
-        dl = l1 ^ l0;
     }
-    const uint32_t fs = (dh | dl) ? clz128(dh, dl) : 128u;
-    // Order the samples by packed keys (window after the samples' common
-    // prefix, 12-bit sample index): warp runs of 256, then merges.  The order
-    // only picks quantiles; the chosen candidates are sorted by full key below.
-    if (active) {
-        uint64_t v[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t e = w * 256 + lane * 8 + i;
-            v[i] = fs < 128 ? ((window64(kk[i], fs) & ~0xFFFull) | e) : e;
+    if (mh | ml) {
+        Squeezed<8> z;
+        squeeze_keys<8>(z, sm.key, t < act ? S : 0u, act, t, mh, ml, 31 - __clz(S), 0u);
+        group_net_sort<SAMPLE_THREADS, 8>(z.v, sm.val, t, 0, act);
+        if (t < act) {
+            uint4 *o = reinterpret_cast<uint4 *>(sm.val + 8 * t);
+            o[0] = make_uint4(z.v[0], z.v[1], z.v[2], z.v[3]);
+            o[1] = make_uint4(z.v[4], z.v[5], z.v[6], z.v[7]);
         }
-        warp_merge_sort64<8>(v, sv, w * 256, lane);
+    } else {  // all samples equal
+        for (uint32_t e = t; e < S; e += SAMPLE_THREADS) sm.val[e] = e;
     }
     __syncthreads();
-    for (uint32_t run = 256; run < S; run <<= 1) {
-        const uint32_t o = threadIdx.x * 8;
-        uint64_t ov[8];
-        const bool act = o < S;
-        if (act) {
-            const uint32_t a0 = o & ~(2 * run - 1), b0 = a0 + run;  // run: a power of two
-            const uint32_t d = o - a0;
-            uint32_t ia = merge_split64(sv, a0, run, b0, run, d);
-            uint32_t ib = d - ia;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint64_t va = ia < run ? sv[pad(a0 + ia)] : ~0ull;
-                const uint64_t vb = ib < run ? sv[pad(b0 + ib)] : ~0ull;
-                const bool take_a = ib >= run || (ia < run && va < vb);
-                ov[i] = take_a ? va : vb;
-                ia += take_a;
-                ib += !take_a;
-            }
-        }
-        __syncthreads();
-        if (act) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) sv[pad(o + i)] = ov[i];
-        }
-        __syncthreads();
-    }
     // Candidates at ranks (j+1)*S/(k+1), padded with the all-ones key.  They
-    // are in packed-key order, which is full-key order unless two windows
-    // tie; only then a bitonic network over the next power of two >= k slots
-    // sorts them by full key.
-    {
-        const uint32_t j = threadIdx.x;
-        if (j < k) {
-            const uint32_t e = sv[pad(((j + 1) * S) / (k + 1))] & 0xFFF;
-            cands[j] = kept ? smp[e] : from_key(key_at(pos_of(e)));
-        } else {
-            cands[j] = from_key(key_max());
-        }
-    }
+    // are in full-key order unless two values tie; only then a bitonic network
+    // over the next power of two >= k slots sorts them by full key.
+    ulonglong2 *cands = sm.cands;
+    if (t < k)
+        cands[t] = sm.key[sm.val[((t + 1) * S) / (k + 1)] & (S - 1)];
+    else
+        cands[t] = from_key(key_max());
     __syncthreads();
-    const bool out_of_order = threadIdx.x + 1 < k &&
-                              key_lt(to_key(cands[threadIdx.x + 1]), to_key(cands[threadIdx.x]));
+    const bool out_of_order = t + 1 < k && key_lt(to_key(cands[t + 1]), to_key(cands[t]));
     if (__syncthreads_or(out_of_order)) {
         const uint32_t kp = next_pow2(k);
         for (uint32_t kk = 2; kk <= kp; kk <<= 1) {
             for (uint32_t jj = kk >> 1; jj > 0; jj >>= 1) {
-                const uint32_t i = threadIdx.x, l = i ^ jj;
+                const uint32_t i = t, l = i ^ jj;
                 bool take = false;
                 Key y{0, 0};
                 if (i < kp) {
@@ -1109,47 +1233,45 @@ __device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__r
         }
     }
     // Survivors: the distinct candidates, compacted in order.
-    const uint32_t j = threadIdx.x;
     Key cand{0, 0};
     bool keep = false;
-    if (j < k) {
-        cand = to_key(cands[j]);
-        keep = j == 0 || !key_eq(to_key(cands[j - 1]), cand);
+    if (t < k) {
+        cand = to_key(cands[t]);
+        keep = t == 0 || !key_eq(to_key(cands[t - 1]), cand);
     }
     const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-    if (lane == 0) warp_cnt[w] = __popc(bal);
+    if (lane == 0) sm.warp_cnt[w] = __popc(bal);
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (t == 0) {
         uint32_t run = 0;
         for (int q = 0; q < SAMPLE_THREADS / 32; ++q) {
-            const uint32_t v = warp_cnt[q];
-            warp_cnt[q] = run;
+            const uint32_t v = sm.warp_cnt[q];
+            sm.warp_cnt[q] = run;
             run += v;
         }
-        warp_cnt[SAMPLE_THREADS / 32] = run;
+        sm.warp_cnt[SAMPLE_THREADS / 32] = run;
     }
     __syncthreads();
-    const uint32_t u = warp_cnt[SAMPLE_THREADS / 32];
+    const uint32_t u = sm.warp_cnt[SAMPLE_THREADS / 32];
     ulonglong2 *out = spl + (uint64_t)si * SPL_STRIDE;
     if (keep) {
-        const uint32_t pos = warp_cnt[w] + __popc(bal & lanemask_lt());
+        const uint32_t pos = sm.warp_cnt[w] + __popc(bal & lanemask_lt());
         out[pos] = from_key(cand);
         cands[pos] = from_key(cand);  // candidates were read before the barriers
     }
     const uint32_t kp2 = next_pow2(u + 1);
-    for (uint32_t q = u + threadIdx.x; q + 1 < kp2; q += SAMPLE_THREADS)
-        out[q] = from_key(key_max());
+    for (uint32_t q = u + t; q + 1 < kp2; q += SAMPLE_THREADS) out[q] = from_key(key_max());
     __syncthreads();
     // Lookup table over the TBL_BITS bits after the splitters' common prefix.
     const Key s0 = to_key(cands[0]), sl = to_key(cands[u - 1]);
     const uint32_t f = u >= 2 ? clz128(s0.hi ^ sl.hi, s0.lo ^ sl.lo) : 128u;
     if (f < 128) {
         // The splitters' window bits first (non-decreasing, as the splitters
-        // are sorted), into the packed-key area, which is free by now; then
-        // each table entry is the number of splitters whose window bits are
-        // below the entry's value (a binary search over those values).
-        uint16_t *wb = reinterpret_cast<uint16_t *>(sv);
-        for (uint32_t j = threadIdx.x; j < u; j += SAMPLE_THREADS)
+        // are sorted), into the values' area, which is free by now; then each
+        // table entry is the number of splitters whose window bits are below
+        // the entry's value (a binary search over those values).
+        uint16_t *wb = reinterpret_cast<uint16_t *>(sm.val);
+        for (uint32_t j = t; j < u; j += SAMPLE_THREADS)
             wb[j] = (uint16_t)window_bits(to_key(cands[j]), f);
         __syncthreads();
         // Thread t fills entries 8t .. 8t + 7 (and one more thread the last
@@ -1167,7 +1289,7 @@ __device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__r
             return lo;
         };
         static_assert(TBL_N == SAMPLE_THREADS * 8, "table entries per thread");
-        const uint32_t w0 = threadIdx.x * 8;
+        const uint32_t w0 = t * 8;
         uint32_t lo = lower(0, u, w0);
         const uint32_t hi = lower(lo, u, w0 + 8);
         uint32_t tv[4];
@@ -1178,14 +1300,60 @@ __device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__r
             tv[i / 2] = t0 | (lo << 16);
         }
         *reinterpret_cast<uint4 *>(T + w0) = make_uint4(tv[0], tv[1], tv[2], tv[3]);
-        if (threadIdx.x == 0) T[TBL_N] = (uint16_t)lower(0, u, TBL_N);
+        if (t == 0) T[TBL_N] = (uint16_t)lower(0, u, TBL_N);
     }
-    if (threadIdx.x == 0) {
+    if (t == 0) {
         nspl[si] = u | (f << 16);
         const uint32_t nt = (s.len + PART_TILE - 1) / PART_TILE;
         ntiles[si] = nt;
         cm_size[si] = (2 * u + 1) * nt;
     }
+}
+
+// One CTA per large segment at a time (segments si = blockIdx.x, + gridDim.x,
+// ...).  The last CTA to finish turns the segments' tile and count-matrix
+// sizes into bases (exclusive scans, totals at [nL]) and clears the look-back
+// scan's state for the level's total: two launches less per level.
+__global__ void __launch_bounds__(SAMPLE_THREADS, 2)
+    k_sample(SortArgs a, const Seg *__restrict__ L, Count cnt, ulonglong2 *spl, uint32_t *nspl,
+             uint16_t *tbl, LevelBases lb, bool from_arena, Counters *c) {
+    extern __shared__ __align__(16) unsigned char sample_smem[];
+    SampleSmem &sm = *reinterpret_cast<SampleSmem *>(sample_smem);
+    const uint32_t nL = count_of(cnt), t = threadIdx.x;
+    for (uint32_t si = blockIdx.x; si < nL; si += gridDim.x) {
+        sample_segment(a, L, si, sm, spl, nspl, tbl, lb.ntiles, lb.cm_size, from_arena);
+        __syncthreads();  // shared memory is reused by the next segment
+    }
+    __threadfence();
+    __syncthreads();
+    if (t == 0) sm.last = atomicAdd(&c->sample_ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!sm.last) return;
+    __threadfence();
+    uint32_t c0 = 0, c1 = 0;
+    for (uint32_t b = 0; b < nL; b += SAMPLE_THREADS) {
+        const uint32_t i = b + t;
+        const uint32_t v0 = i < nL ? __ldcg(lb.ntiles + i) : 0;
+        const uint32_t v1 = i < nL ? __ldcg(lb.cm_size + i) : 0;
+        uint32_t t0, t1;
+        const uint32_t s0 = cta_inclusive_scan<SAMPLE_THREADS>(v0, t0, sm.warp_cnt);
+        const uint32_t s1 = cta_inclusive_scan<SAMPLE_THREADS>(v1, t1, sm.warp_cnt);
+        if (i < nL) {
+            lb.tile_base[i] = c0 + s0 - v0;
+            lb.cm_base[i] = c1 + s1 - v1;
+        }
+        c0 += t0;
+        c1 += t1;
+    }
+    if (t == 0) {
+        lb.tile_base[nL] = c0;
+        lb.cm_base[nL] = c1;
+        c->sample_ticket = 0;
+    }
+    // ticket word and one status word per scan tile
+    for (uint32_t q = t; q < 1 + (c1 + SCAN_CHUNK_ELEMS - 1) / SCAN_CHUNK_ELEMS;
+         q += SAMPLE_THREADS)
+        lb.lookback[q] = 0;
 }
 
 // ---- partition count: per-tile bucket histograms ---------------------------
@@ -1656,23 +1824,29 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 3) k_scatter2(
     }
 }
 
-// ---- bucket emission: one CTA per partitioned segment ----------------------
+// ---- bucket emission: EMIT_CHUNKS CTAs per partitioned segment --------------
+// A CTA takes 256 buckets of a segment: the reads, the key of an equality
+// bucket and the list appends are one chain of dependent round trips, so that
+// four CTAs side by side take a quarter of the time one takes over 1023
+// buckets (26 -> 8 us for one segment).
+constexpr int EMIT_THREADS = 256;
+constexpr int EMIT_CHUNKS = (NB_MAX + EMIT_THREADS) / EMIT_THREADS;
 __global__ void k_emit(SortArgs a, const Seg *__restrict__ L, Count cnt,
                        const uint32_t *__restrict__ tile_base,
                        const uint32_t *__restrict__ nspl, const uint32_t *__restrict__ cm_base,
                        const uint32_t *__restrict__ cm_scan, Seg *W1, Seg *W8, SmallLists S,
                        Seg *L2, Seg *E, uint2 *B, Seg *N, Counters *c) {
     const uint32_t nL = count_of(cnt);
-    for (uint32_t si = blockIdx.x; si < nL; si += gridDim.x) {
-    const Seg s = L[si];
+    for (uint32_t q = blockIdx.x; q < nL * EMIT_CHUNKS; q += gridDim.x) {
+    const uint32_t si = q / EMIT_CHUNKS, b0 = q % EMIT_CHUNKS * EMIT_THREADS;
     const uint32_t u = nspl[si] & 0xFFFF, nb = 2 * u + 1;
-    const uint32_t nt = tile_base[si + 1] - tile_base[si];
-    const uint32_t cmb = cm_base[si];
-    const uint32_t seg0 = cm_scan[cmb];
-    const uint32_t ob = (s.flags & SEG_BUF1) ^ 1u;
-    const uint32_t flags = ob | SEG_KEYS;
-    // Uniform trip count: every warp reaches the collective appends.
-    for (uint32_t b0 = 0; b0 < nb; b0 += blockDim.x) {
+    if (b0 < nb) {  // the whole CTA reaches the collective appends
+        const Seg s = L[si];
+        const uint32_t nt = tile_base[si + 1] - tile_base[si];
+        const uint32_t cmb = cm_base[si];
+        const uint32_t seg0 = cm_scan[cmb];
+        const uint32_t ob = (s.flags & SEG_BUF1) ^ 1u;
+        const uint32_t flags = ob | SEG_KEYS;
         const uint32_t b = b0 + threadIdx.x;
         uint32_t off = 0, len = 0;
         if (b < nb) {
@@ -1720,8 +1894,8 @@ __global__ void k_emit(SortArgs a, const Seg *__restrict__ L, Count cnt,
         ebase = __shfl_sync(0xffffffffu, ebase, 31) + incl - nch;
         for (uint32_t ch = 0; ch < nch; ++ch)
             E[ebase + ch] = Seg{p, len, s.depth, ob | (ch << SEG_CHUNK_SHIFT)};
+        if (b == 0) atomicAdd(&c->partitioned, (unsigned long long)s.len);
     }
-    if (threadIdx.x == 0) atomicAdd(&c->partitioned, (unsigned long long)s.len);
     }
 }
 
@@ -2068,38 +2242,6 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Keys at `depth` of up to G strings per lane: elements e0 + q * stride below
-// len of the index array I.  Every step's loads are issued for all G strings
-// before any is used (index, then offset, then the two 16-byte words that
-// hold the key), so that G chains of dependent reads overlap.
-template <int G>
-__device__ __forceinline__ void gather_keys(const SortArgs &a, const uint32_t *__restrict__ I,
-                                            uint32_t depth, uint32_t e0, uint32_t stride,
-                                            uint32_t len, Key (&kk)[G], uint32_t (&ii)[G]) {
-    uint64_t pos[G];
-    ulonglong2 v0[G], v1[G];
-#pragma unroll
-    for (int q = 0; q < G; ++q) ii[q] = e0 + q * stride < len ? I[e0 + q * stride] : IDX_MAX;
-#pragma unroll
-    for (int q = 0; q < G; ++q)
-        pos[q] = ii[q] != IDX_MAX ? string_offset(a.offs, a.off_width, ii[q]) + depth : 0ull;
-#pragma unroll
-    for (int q = 0; q < G; ++q) {
-        const uint64_t at = pos[q] & ~15ull;
-        const bool in = ii[q] != IDX_MAX && key_words_inside(a.arena_bytes, at);
-        const ulonglong2 *w = reinterpret_cast<const ulonglong2 *>(a.arena + at);
-        v0[q] = in ? __ldg(w) : make_ulonglong2(0, 0);
-        v1[q] = in && (pos[q] & 15) ? __ldg(w + 1) : make_ulonglong2(0, 0);
-    }
-#pragma unroll
-    for (int q = 0; q < G; ++q) {
-        if (key_words_inside(a.arena_bytes, pos[q] & ~15ull))
-            kk[q] = key_of_words(v0[q], v1[q], (uint32_t)pos[q] & 15u);
-        else if (ii[q] != IDX_MAX)
-            kk[q] = load_key_tail(a.arena, a.arena_bytes, pos[q]);
-    }
-}
-
 // ---- segments of 33..4096 strings: a group of threads each ------------------
 // A group of GT = 32, 64, 128, 256 or 512 threads sorts one segment of up to
 // ITEMS * GT strings (8 per thread; 2 or 4 for the smallest).  Records (16-byte
@@ -2123,181 +2265,6 @@ __device__ __forceinline__ void gather_keys(const SortArgs &a, const uint32_t *_
 // network; ALU pipe 65-75 % busy); the CTA-sort launches of 69 M batched
 // strings 2.79 -> 1.53 ms, of 16 M suffixes 4.23 -> 2.59 ms, of 50 M URLs 2.27
 // -> 1.62 ms.
-
-// Barrier among the GT threads of group gi: named barrier 1 + gi (0 is
-// __syncthreads).  Immediate ids, so that a CTA claims only the barriers it
-// uses (at most 5) and the SM's barriers do not limit occupancy.
-template <int GT>
-__device__ __forceinline__ void group_sync(uint32_t gi) {
-    constexpr int G = GT < SMALL_THREADS ? SMALL_THREADS / GT : 1;
-    if constexpr (GT == 32) {
-        __syncwarp();
-    } else {
-        if (G == 1 || gi == 0)
-            asm volatile("bar.sync 1, %0;" ::"n"(GT) : "memory");
-        else if (G == 2 || gi == 1)
-            asm volatile("bar.sync 2, %0;" ::"n"(GT) : "memory");
-        else if (gi == 2)
-            asm volatile("bar.sync 3, %0;" ::"n"(GT) : "memory");
-        else
-            asm volatile("bar.sync 4, %0;" ::"n"(GT) : "memory");
-    }
-}
-
-// Whether any thread of the group has `want`; a barrier of the group.
-template <int GT>
-__device__ __forceinline__ bool group_any(bool want, uint32_t gi) {
-    if constexpr (GT == 32) {
-        return __any_sync(0xffffffffu, want);
-    } else {
-        constexpr int G = GT < SMALL_THREADS ? SMALL_THREADS / GT : 1;
-        uint32_t r;
-#define SS_BAR_ANY(id)                                                               \
-    asm volatile("{ .reg .pred p, q; setp.ne.u32 p, %1, 0; bar.red.or.pred q, " #id  \
-                 ", %2, p; selp.u32 %0, 1, 0, q; }"                                  \
-                 : "=r"(r)                                                           \
-                 : "r"((uint32_t)want), "n"(GT)                                      \
-                 : "memory")
-        if (G == 1 || gi == 0)
-            SS_BAR_ANY(1);
-        else if (G == 2 || gi == 1)
-            SS_BAR_ANY(2);
-        else if (gi == 2)
-            SS_BAR_ANY(3);
-        else
-            SS_BAR_ANY(4);
-#undef SS_BAR_ANY
-        return r != 0;
-    }
-}
-
-template <typename V>
-__device__ __forceinline__ void cmp_swap(V &a, V &b) {
-    const V lo = min(a, b), hi = max(a, b);
-    a = lo;
-    b = hi;
-}
-
-// One exchange between threads: the lower one keeps the smaller value, the
-// upper one (up) the larger.
-template <typename V>
-__device__ __forceinline__ V keep_side(V v, V o, bool up) {
-    return (o < v) != up ? o : v;
-}
-
-// Batcher's odd-even merge sort of v[LO .. LO + N), as templates so that every
-// index is a constant and the values stay in registers.
-template <int LO, int N, int R, int ITEMS, typename V>
-__device__ __forceinline__ void net_merge(V (&v)[ITEMS]) {
-    if constexpr (2 * R < N) {
-        net_merge<LO, N, 2 * R>(v);
-        net_merge<LO + R, N, 2 * R>(v);
-#pragma unroll
-        for (int i = LO + R; i + R < LO + N; i += 2 * R) cmp_swap(v[i], v[i + R]);
-    } else {
-        cmp_swap(v[LO], v[LO + R]);
-    }
-}
-
-template <int LO, int N, int ITEMS, typename V>
-__device__ __forceinline__ void net_sort(V (&v)[ITEMS]) {
-    if constexpr (N > 1) {
-        net_sort<LO, N / 2>(v);
-        net_sort<LO + N / 2, N / 2>(v);
-        net_merge<LO, N, 1>(v);
-    }
-}
-
-// Bitonic half-cleaners of strides M, M / 2, .. 1 inside a thread.
-template <int M, int ITEMS, typename V>
-__device__ __forceinline__ void net_clean(V (&v)[ITEMS]) {
-    if constexpr (M >= 1) {
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i)
-            if ((i & M) == 0) cmp_swap(v[i], v[i + M]);
-        net_clean<M / 2>(v);
-    }
-}
-
-// Half-cleaners of lane strides m, m / 2, .. 1, then inside the lanes.  The
-// loop over strides stays a loop: unrolled, the sorts outgrow the
-// instruction cache.
-template <int ITEMS, typename V>
-__device__ __forceinline__ void warp_clean(V (&v)[ITEMS], uint32_t m, uint32_t lane) {
-#pragma unroll 1
-    for (; m >= 1; m /= 2) {
-        const bool up = (lane & m) != 0;
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i)
-            v[i] = keep_side(v[i], __shfl_xor_sync(0xffffffffu, v[i], m), up);
-    }
-    net_clean<ITEMS / 2>(v);
-}
-
-// Every thread stores its values to x (16-byte words, consecutive threads
-// next to each other) and loads those of thread `from`.  Two barriers.
-template <int GT, int ITEMS, typename V>
-__device__ __forceinline__ void swap_values(const V (&v)[ITEMS], V (&o)[ITEMS], void *x,
-                                            uint32_t t, uint32_t from, uint32_t gi) {
-    constexpr int PER = 16 / sizeof(V);  // values per 16-byte word
-    V w[PER];
-#pragma unroll
-    for (int j = 0; j < ITEMS / PER; ++j) {
-#pragma unroll
-        for (int q = 0; q < PER; ++q) w[q] = v[j * PER + q];
-        static_cast<uint4 *>(x)[j * GT + t] = *reinterpret_cast<const uint4 *>(w);
-    }
-    group_sync<GT>(gi);
-#pragma unroll
-    for (int j = 0; j < ITEMS / PER; ++j) {
-        *reinterpret_cast<uint4 *>(w) = static_cast<const uint4 *>(x)[j * GT + from];
-#pragma unroll
-        for (int q = 0; q < PER; ++q) o[j * PER + q] = w[q];
-    }
-    group_sync<GT>(gi);
-}
-
-// Sorts the GT * ITEMS values of a group; thread t ends with ranks t * ITEMS
-// .. t * ITEMS + ITEMS - 1.  Odd-even merge sort inside a thread, then bitonic
-// merges of 2, 4, .. GT threads whose first stage compares mirrored positions,
-// so that every stage sorts ascending; strides of 32 threads and more go
-// through shared memory (x: GT * ITEMS values).
-template <int GT, int ITEMS, typename V>
-__device__ __forceinline__ void group_net_sort(V (&v)[ITEMS], void *x, uint32_t t, uint32_t gi) {
-    const uint32_t lane = t & 31;
-    net_sort<0, ITEMS>(v);
-#pragma unroll 1
-    for (uint32_t half = 1; half < 32; half *= 2) {
-        const bool up = (lane & half) != 0;
-        const uint32_t mirror = 2 * half - 1;
-#pragma unroll
-        for (int i = 0; i < ITEMS / 2; ++i) {
-            const V p = __shfl_xor_sync(0xffffffffu, v[ITEMS - 1 - i], mirror);
-            const V q = __shfl_xor_sync(0xffffffffu, v[i], mirror);
-            v[i] = keep_side(v[i], p, up);
-            v[ITEMS - 1 - i] = keep_side(v[ITEMS - 1 - i], q, up);
-        }
-        warp_clean<ITEMS>(v, half / 2, lane);
-    }
-    if constexpr (GT > 32) {
-#pragma unroll 1
-        for (uint32_t half = 32; half < GT; half *= 2) {
-            V o[ITEMS];
-            swap_values<GT, ITEMS>(v, o, x, t, t ^ (2 * half - 1), gi);
-            const bool up = (t & half) != 0;
-#pragma unroll
-            for (int i = 0; i < ITEMS; ++i) v[i] = keep_side(v[i], o[ITEMS - 1 - i], up);
-#pragma unroll 1
-            for (uint32_t m = half / 2; m >= 32; m /= 2) {
-                swap_values<GT, ITEMS>(v, o, x, t, t ^ m, gi);
-                const bool um = (t & m) != 0;
-#pragma unroll
-                for (int i = 0; i < ITEMS; ++i) v[i] = keep_side(v[i], o[i], um);
-            }
-            warp_clean<ITEMS>(v, 16, lane);
-        }
-    }
-}
 
 // Shared memory of one group: keys, values (in passing between threads, and
 // the final order), indices.  Values and indices together also hold 64-bit
@@ -2498,48 +2465,11 @@ __device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint
                                               uint32_t len, uint64_t mh, uint64_t ml, uint32_t t,
                                               uint32_t gi) {
     constexpr int PB = SEG_POS_BITS<GT, ITEMS>;
-    constexpr uint32_t PM = (1u << PB) - 1, WB = 32 - PB;
+    constexpr uint32_t PM = (1u << PB) - 1;
     const uint32_t lane = t & 31, gw = t >> 5;
-    // Squeezed bits: the first WB differing bits of the 64 from the first
-    // one (bit f of the key) on, run by run of adjacent ones; lane j keeps the
-    // key byte of squeezed bit j.
-    const uint32_t f = clz128(mh, ml);
-    const uint64_t wm = window64(Key{mh, ml}, f);
-    uint32_t used = 0, byte_of = SEG_TIE<GT>;
-    uint32_t v[ITEMS], wh[ITEMS], wl[ITEMS];
-#pragma unroll
-    for (int q = 0; q < ITEMS; ++q) {
-        const uint32_t e = q * GT + t;
-        const Key k = e < len ? to_key(sm.key[e]) : Key{0, 0};
-        // the 96 bits from the 32-bit word that holds bit f on
-        const uint64_t top = f < 64 ? k.hi : k.lo, next = f < 64 ? k.lo : 0;
-        const uint32_t w0 = (uint32_t)(top >> 32), w1 = (uint32_t)top,
-                       w2 = (uint32_t)(next >> 32), w3 = (uint32_t)next;
-        wh[q] = f & 32 ? __funnelshift_l(w2, w1, f) : __funnelshift_l(w1, w0, f);
-        wl[q] = f & 32 ? __funnelshift_l(w3, w2, f) : __funnelshift_l(w2, w1, f);
-        v[q] = 0;
-    }
-    auto squeeze = [&](uint32_t &m, const uint32_t(&w)[ITEMS], uint32_t base) {
-#pragma unroll 1
-        while (m && used < WB) {
-            const uint32_t lead = __clz(m);
-            const uint32_t width = min((uint32_t)__clz(~(m << lead)), WB - used);
-            const uint32_t mul = 1u << width, low = mul - 1, sh = 32 - lead - width;
-#pragma unroll
-            for (int q = 0; q < ITEMS; ++q) v[q] = v[q] * mul + ((w[q] >> sh) & low);
-            if (lane - used < width) byte_of = (f + base + lead + lane - used) >> 3;
-            used += width;
-            m &= ~(low << sh);
-        }
-    };
-    uint32_t m0 = (uint32_t)(wm >> 32), m1 = (uint32_t)wm;
-    squeeze(m0, wh, 0);
-    squeeze(m1, wl, 32);
-#pragma unroll
-    for (int q = 0; q < ITEMS; ++q) {
-        const uint32_t e = q * GT + t;
-        v[q] = e < len ? v[q] << PB | e : ~0u;
-    }
+    Squeezed<ITEMS> z;
+    squeeze_keys<ITEMS>(z, sm.key, len, GT, t, mh, ml, PB, SEG_TIE<GT>);
+    uint32_t(&v)[ITEMS] = z.v;
     group_net_sort<GT, ITEMS>(v, sm.val, t, gi);
     // Ties on the squeezed bits must be in full-key order.  A pair out of
     // order that both lie in one thread and tie with nothing else is swapped
@@ -2586,10 +2516,11 @@ __device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint
         const uint32_t run = group_fix_runs<GT, ITEMS>(sm, len, t, gi);
         if (run) {
             full = run == 2;
-            byte_of = SEG_TIE<GT>;  // the values are positions only
+            z.byte_of = SEG_TIE<GT>;  // the values are positions only
             // The differing bits not used: m0, m1 of the window, and what
             // lies past the window's 64 bits.
-            const uint64_t m = (uint64_t)m0 << 32 | m1;
+            const uint32_t f = z.f;
+            const uint64_t m = (uint64_t)z.m0 << 32 | z.m1;
             const uint64_t rh = f < 64 ? m >> f : 0ull;
             const uint64_t rl = f == 0   ? ml
                                 : f < 64 ? (m << (64 - f)) | ((ml << f) >> f)
@@ -2607,7 +2538,7 @@ __device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         const uint32_t x = (v[i] ^ (i ? v[i ? i - 1 : 0] : pv)) >> PB;
-        const uint32_t l = __shfl_sync(0xffffffffu, byte_of, __clz(x) + used - 32);
+        const uint32_t l = __shfl_sync(0xffffffffu, z.byte_of, __clz(x) + z.used - 32);
         const uint32_t h = l * (1u << SEG_ORD_BITS<GT>) + (v[i] & PM);
         if (i & 1)
             o[i / 2] += h * 65536u;
@@ -2677,12 +2608,8 @@ __device__ __forceinline__ bool sort_segment(const SortArgs &a, const Seg &s, Se
                 ml |= k.lo ^ k0.lo;
             }
         }
-        auto wor = [](uint64_t x) -> uint64_t {
-            return (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(x >> 32)) << 32 |
-                   __reduce_or_sync(0xffffffffu, (uint32_t)x);
-        };
-        mh = wor(mh);
-        ml = wor(ml);
+        mh = warp_or64(mh);
+        ml = warp_or64(ml);
         if constexpr (GT > 32) {
             if (lane == 0) {
                 sm.red[gw][0] = mh;
@@ -2961,8 +2888,10 @@ __global__ void k_g_round_end(GraphState *g, const Counters *c, Seg *R, const Se
 }
 
 // ---- exclusive scan (u32), one pass with decoupled look-back ---------------
-// Each CTA takes the next tile from a ticket (so every tile it waits for has
-// started), scans its 4096 values, publishes its sum, and warp 0 walks back
+// A CTA takes tiles from a ticket until none is left (a tile is published
+// before its CTA takes another, so every tile it waits for has started and
+// waits for nothing newer; the host knows only a bound of n, and one CTA per
+// tile of that bound took 10 us to find nothing), scans its 4096 values, publishes its sum, and warp 0 walks back
 // over its predecessors' status words 32 at a time, adding sums until it
 // meets an inclusive prefix; then it publishes its own inclusive prefix.
 // Status word: flag (1 = tile sum, 2 = inclusive prefix) << 32 | value.  The
@@ -2985,14 +2914,16 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_lookback(const uint32_t *
     __shared__ uint32_t s_tile, s_prefix;
     const uint32_t n = count_of(cnt);
     const uint32_t lane = threadIdx.x & 31;
+    if (n == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) out[0] = 0;
+        return;
+    }
+    while (true) {
     if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
     __syncthreads();
     const uint32_t t = s_tile;
     const uint64_t base = (uint64_t)t * SCAN_CHUNK;
-    if (base >= n) {
-        if (n == 0 && t == 0 && threadIdx.x == 0) out[0] = 0;
-        return;
-    }
+    if (base >= n) return;
     for (int k = 0; k < SCAN_ITEMS; ++k) {
         const int j = k * SCAN_THREADS + threadIdx.x;
         const uint64_t i = base + j;
@@ -3056,6 +2987,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_lookback(const uint32_t *
         if (i < n) out[i] = buf[j];
     }
     if (threadIdx.x == 0 && base + SCAN_CHUNK >= n) out[n] = s_prefix + total;
+    __syncthreads();  // shared memory is reused by the CTA's next tile
+    }
 }
 
 }  // namespace
@@ -3067,15 +3000,14 @@ static inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b -
 // it.  The attribute belongs to the function in the current device's context,
 // so it is set once per device (bit d of the mask), for all kernels at once;
 // two threads that race here both set the same values, which is harmless.
-static constexpr int SAMPLE_SMEM =
-    (SAMPLES_MAX + SAMPLES_MAX / 8) * sizeof(uint64_t) + SAMPLE_KEEP * sizeof(ulonglong2);
 static void set_smem_attrs() {
     static std::atomic<uint64_t> done{0};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return;  // the launch reports it
     const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
     if (bit && (done.load(std::memory_order_acquire) & bit)) return;
-    cudaFuncSetAttribute(k_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_SMEM);
+    cudaFuncSetAttribute(k_sample, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(SampleSmem));
     cudaFuncSetAttribute(k_count<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(PartSmem));
     cudaFuncSetAttribute(k_count<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3186,11 +3118,6 @@ void launch_byte_hist(const uint8_t *arena, uint64_t arena_bytes, const void *of
     k_byte_hist<<<1, 256, 0, st>>>(arena, arena_bytes, offs, off_width, n, samples, hist);
 }
 
-void launch_scan_pair(const uint32_t *in0, uint32_t *out0, const uint32_t *in1, uint32_t *out1,
-                      Count n, cudaStream_t st) {
-    k_scan_pair<<<1, SMALL_SCAN_THREADS, 0, st>>>(in0, out0, in1, out1, n);
-}
-
 void launch_seg_tiles(const Seg *segs, Count n, uint32_t tile, uint32_t *out, cudaStream_t st) {
     k_seg_tiles<<<1, SMALL_SCAN_THREADS, 0, st>>>(segs, n, tile, out);
 }
@@ -3201,7 +3128,7 @@ size_t lookback_state_bytes(uint32_t cap) { return 8 + (size_t)cdiv(cap ? cap : 
 
 void launch_scan_lookback(const uint32_t *in, uint32_t *out, uint32_t cap, Count n,
                           unsigned char *state, uint32_t *err, cudaStream_t st) {
-    const uint32_t nb = cdiv(cap ? cap : 1, SCAN_CHUNK);
+    const uint32_t nb = std::min<uint32_t>(cdiv(cap ? cap : 1, SCAN_CHUNK), 148 * 8);
     k_scan_lookback<<<nb, SCAN_THREADS, 0, st>>>(in, out, n,
                                                   reinterpret_cast<unsigned long long *>(state + 8),
                                                   reinterpret_cast<uint32_t *>(state), err);
@@ -3222,13 +3149,13 @@ void launch_gather(const SortArgs &a, const Seg *L, Count nL, const uint32_t *ti
 }
 
 void launch_sample(const SortArgs &a, const Seg *L, Count nL, ulonglong2 *spl, uint32_t *nspl,
-                   uint16_t *tbl, uint32_t *ntiles, uint32_t *cm_size, bool from_arena, int grid,
+                   uint16_t *tbl, const LevelBases &lb, bool from_arena, Counters *c, int grid,
                    cudaStream_t st) {
     const int g = grid_of(grid, nL, 1, 1u << 30);
     if (!g) return;
     set_smem_attrs();
-    k_sample<<<g, SAMPLE_THREADS, SAMPLE_SMEM, st>>>(a, L, nL, spl, nspl, tbl, ntiles, cm_size,
-                                                     from_arena);
+    k_sample<<<g, SAMPLE_THREADS, sizeof(SampleSmem), st>>>(a, L, nL, spl, nspl, tbl, lb,
+                                                            from_arena, c);
 }
 
 void launch_count(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
@@ -3269,9 +3196,9 @@ void launch_emit(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile
                  const uint32_t *nspl, const uint32_t *cm_base, const uint32_t *cm_scan,
                  Seg *W1, Seg *W8, SmallLists S, Seg *L2, Seg *E, uint2 *B, Seg *N,
                  Counters *c, int grid, cudaStream_t st) {
-    const int g = grid_of(grid, nL, 1, 1u << 30);
+    const int g = grid > 0 ? grid : grid_of(grid, nL, 1, 1u << 28) * EMIT_CHUNKS;
     if (!g) return;
-    k_emit<<<g, 256, 0, st>>>(a, L, nL, tile_base, nspl, cm_base, cm_scan, W1, W8, S, L2, E, B,
+    k_emit<<<g, EMIT_THREADS, 0, st>>>(a, L, nL, tile_base, nspl, cm_base, cm_scan, W1, W8, S, L2, E, B,
                               N, c);
 }
 
