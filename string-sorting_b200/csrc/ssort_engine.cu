@@ -6,6 +6,7 @@
 #include "ssort_host.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -37,9 +38,38 @@ int ssort_ctx::reserve(uint32_t n) {
     SS_TRY(ensure(ws_buf, lay.total));
     ws = ws_bind(lay, (unsigned char *)ws_buf.p);
     ws_n = n;
-    if (!h_ctr) {
-        SS_CUDA(cudaHostAlloc((void **)&h_ctr, sizeof(Counters), cudaHostAllocDefault));
+    if (!hc) {
+        SS_CUDA(cudaHostAlloc((void **)&hc, sizeof(HostCounters), cudaHostAllocDefault));
+        std::memset(hc, 0, sizeof(HostCounters));
+        published = true;
+        use_counters(0);
     }
+    return SSORT_OK;
+}
+
+// Waits for the counters of the last kernel given a publish_next(), or copies
+// them.  The wait polls the flag that the kernel's last CTA sets in pinned
+// memory; the stream is queried now and then, so that a failed launch, a
+// fault or a stream that is being captured ends it with an error.
+int ssort_ctx::read_counters() {
+    if (published) {
+        volatile uint32_t *flag = &hc->flag;
+        for (uint32_t spin = 1; *flag != pub_seq; ++spin) {
+            if (spin % 2048) continue;
+            const cudaError_t e = cudaStreamQuery(st);
+            if (e == cudaErrorNotReady) continue;
+            if (e != cudaSuccess) return cuda_fail(e, "waiting for a kernel's counters");
+            if (*flag != pub_seq)
+                return fail(SSORT_EINTERNAL, "a kernel ended without its counters");
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);
+    } else {
+        SS_CUDA(cudaMemcpyAsync(&hc->rc, ws.rc, sizeof(RoundCounters), cudaMemcpyDeviceToHost,
+                                st));
+        SS_CUDA(cudaStreamSynchronize(st));
+    }
+    if (hc->rc.c[0].error || hc->rc.c[1].error)
+        return fail(SSORT_EINTERNAL, "a scan's look-back waited past its bound");
     return SSORT_OK;
 }
 
@@ -77,7 +107,7 @@ int ssort_ctx::scan_on(const uint32_t *in, uint32_t *out, uint32_t cap, Count n,
                        cudaStream_t s) {
     if (scan_lookback) {
         LAUNCH(this, "scan",
-               launch_scan_lookback(in, out, cap, n, ws.lookback, &ws.ctr->error, s));
+               launch_scan_lookback(in, out, cap, n, ws.lookback, &dev_ctr()->error, s));
     } else {
         LAUNCH(this, "scan", launch_scan(in, out, cap, n, ws.partials, s));
     }
@@ -105,7 +135,7 @@ int ssort_ctx::launch_small(const SortArgs &a, Seg *nxt, SmallDone &d) {
         SS_CUDA(cudaStreamWaitEvent(side, ev_fork, 0));  // recorded by fork_small
         SS_CUDA(cudaStreamWaitEvent(side2, ev_fork, 0));
     }
-    Counters *dc = ws.ctr;
+    Counters *dc = dev_ctr();
     // One pass of CTAs over the entries (no CTA loops over several): short
     // CTAs let the scheduler give SMs back to the partition kernels.  The
     // packed warp sort keeps a capped grid: its warps loop over entries.
@@ -136,12 +166,33 @@ int ssort_ctx::launch_small(const SortArgs &a, Seg *nxt, SmallDone &d) {
     return SSORT_OK;
 }
 
+void ssort_ctx::add_stats(const Counters &c) {
+    stats.partitioned += c.partitioned;
+    stats.gather_elems += c.gather_elems;
+    stats.warp1_fresh += c.warp1_fresh;
+    stats.warp1_deep += c.warp1_deep;
+    stats.full_sorted += c.full_sorted;
+    stats.window_saved += c.window_saved;
+    stats.window_used += c.window_used;
+    stats.warp1_keyed += c.warp1_keyed;
+    stats.warp8_fresh += c.warp8_fresh;
+    stats.warp8_keyed += c.warp8_keyed;
+    stats.block_fresh += c.block_fresh;
+    stats.block_keyed += c.block_keyed;
+    stats.equal_moved += c.equal_moved;
+    stats.equal_final += c.equal_final;
+    stats.boundaries += c.n_bound;
+}
+
 // One refinement round over the n_cur segments in `cur`: classification,
 // key gather and sample partitioning of large segments, on-chip sorts,
 // equality buckets and boundary LCPs.  The next round's segments are
 // appended to `nxt`; their count is returned in n_next.
+// classified: the segments are in the lists and counted in h_ctr already.
+// ahead: the round's last kernel also classifies the next round's segments,
+// and h_ctr is left on their counts.
 int ssort_ctx::round(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt, uint32_t &n_next,
-                     uint32_t round_no) {
+                     uint32_t round_no, bool classified, bool ahead) {
     // A fresh round (round 0 of a sort, or by the caller's choice) streams
     // the arena in index order with a separate gather; a deep round gathers
     // keys at random inside the first count.  Every round overlaps its
@@ -149,13 +200,14 @@ int ssort_ctx::round(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt, uint
     // switched off or timing kernels one by one.
     fresh_round = round_mode >= 0 ? round_mode == 0 : round_no == 0;
     overlap_round = side && side2 && hp && !prof && overlap;
-    if (!overlap_round) return round_body(a, cur, n_cur, nxt, n_next, round_no);
+    if (!overlap_round || forked)
+        return round_body(a, cur, n_cur, nxt, n_next, round_no, classified, ahead);
     // Fork the round onto the high-priority stream and join it back.
     cudaStream_t user = st;
     SS_CUDA(cudaEventRecord(ev_round, user));
     SS_CUDA(cudaStreamWaitEvent(hp, ev_round, 0));
     st = hp;
-    const int rc = round_body(a, cur, n_cur, nxt, n_next, round_no);
+    const int rc = round_body(a, cur, n_cur, nxt, n_next, round_no, classified, ahead);
     st = user;
     if (rc != SSORT_OK) return rc;
     SS_CUDA(cudaEventRecord(ev_round, hp));
@@ -164,14 +216,17 @@ int ssort_ctx::round(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt, uint
 }
 
 int ssort_ctx::round_body(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt,
-                          uint32_t &n_next, uint32_t round_no) {
-    Counters *dc = ws.ctr;
+                          uint32_t &n_next, uint32_t round_no, bool classified, bool ahead) {
     const int g8 = grid_for(8), g4 = grid_for(4), g2 = grid_for(2);
-    SS_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), st));
-    LAUNCH(this, "classify",
-           launch_classify(cur, hcount(n_cur), a.warp8_cap, ws.W1, ws.W8,
-                           ws.small(), ws.L, dc, 0, st));
-    SS_TRY(sync_counters());
+    if (!classified) {
+        use_counters(0);
+        SS_CUDA(cudaMemsetAsync(ws.rc, 0, sizeof(RoundCounters), st));
+        LAUNCH(this, "classify",
+               launch_classify(cur, hcount(n_cur), a.warp8_cap, ws.W1, ws.W8, ws.small(), ws.L,
+                               dev_ctr(), 0, st, ws.rc, publish_next()));
+        SS_TRY(read_counters());
+    }
+    Counters *dc = dev_ctr();
     if (round_no < SSORT_MAX_ROUNDS) stats.live[round_no] = h_ctr->live_next;
     // The on-chip sorts of the segments known after each host read of the
     // counters are launched on the side stream after the next partition
@@ -213,12 +268,13 @@ int ssort_ctx::round_body(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt,
                               ws.cm, g2, st));
         LAUNCH(this, "emit",
                launch_emit(a, lcur, nl, ws.tile_base, ws.nspl, ws.cm_base, ws.cm, ws.W1, ws.W8,
-                           ws.small(), lnext, ws.E, ws.B, nxt, dc, 0, st));
+                           ws.small(), lnext, ws.E, ws.B, nxt, dc, 0, st,
+                           ws.rc, publish_next()));
         SS_TRY(launch_small(a, nxt, done));  // segments known before this level
-        SS_TRY(sync_counters());
+        SS_TRY(read_counters());
         SS_TRY(fork_small());
         n_large = h_ctr->n_large_next;
-        SS_CUDA(cudaMemsetAsync(&dc->n_large_next, 0, 4, st));
+        if (!published) SS_CUDA(cudaMemsetAsync(&dc->n_large_next, 0, 4, st));
         std::swap(lcur, lnext);
     }
     SS_TRY(launch_small(a, nxt, done));  // the rest
@@ -228,28 +284,28 @@ int ssort_ctx::round_body(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt,
         SS_CUDA(cudaEventRecord(ev_join2, side2));
         SS_CUDA(cudaStreamWaitEvent(st, ev_join2, 0));
     }
-    LAUNCH(this, "boundary", launch_boundary(a, ws.B, dc, g4, st));
-    SS_TRY(sync_counters());
+    if (ahead) {
+        const int g = (int)std::min<uint64_t>(g4, ((uint64_t)a.n + 255) / 256);
+        LAUNCH(this, "round_end",
+               launch_round_end(a, ws.B, nxt, ws.W1, ws.W8, ws.small(), ws.L, ws.rc, ctr_i,
+                                publish_next(), g, st));
+        SS_TRY(read_counters());
+        if (!published) SS_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), st));
+    } else {
+        LAUNCH(this, "boundary", launch_boundary(a, ws.B, dc, g4, st));
+        SS_CUDA(cudaMemcpyAsync(&hc->rc, ws.rc, sizeof(RoundCounters), cudaMemcpyDeviceToHost,
+                                st));
+        SS_CUDA(cudaStreamSynchronize(st));
+        if (h_ctr->error)
+            return fail(SSORT_EINTERNAL, "a scan's look-back waited past its bound");
+    }
     stats.small_segments +=
         h_ctr->n_w1 + h_ctr->n_w8 + h_ctr->n_small + h_ctr->n_small2 + h_ctr->n_small3 +
         h_ctr->n_small4;
-    stats.partitioned += h_ctr->partitioned;
-    stats.gather_elems += h_ctr->gather_elems;
     if (fused_gather) stats.gather_fused += h_ctr->gather_elems;
-    stats.warp1_fresh += h_ctr->warp1_fresh;
-    stats.warp1_deep += h_ctr->warp1_deep;
-    stats.full_sorted += h_ctr->full_sorted;
-    stats.window_saved += h_ctr->window_saved;
-    stats.window_used += h_ctr->window_used;
-    stats.warp1_keyed += h_ctr->warp1_keyed;
-    stats.warp8_fresh += h_ctr->warp8_fresh;
-    stats.warp8_keyed += h_ctr->warp8_keyed;
-    stats.block_fresh += h_ctr->block_fresh;
-    stats.block_keyed += h_ctr->block_keyed;
-    stats.equal_moved += h_ctr->equal_moved;
-    stats.equal_final += h_ctr->equal_final;
-    stats.boundaries += h_ctr->n_bound;
+    add_stats(*h_ctr);
     n_next = h_ctr->n_next;
+    if (ahead) use_counters(ctr_i ^ 1);
     return SSORT_OK;
 }
 
@@ -316,29 +372,72 @@ int ssort_ctx::run_ws(const uint8_t *arena_p, uint64_t arena_bytes, const void *
         return run_graph(a, n, d_inst, ninst);
 
     Seg *cur = ws.R, *nxt = ws.N;
-    Counters *dc = ws.ctr;
-
-    LAUNCH(this, "iota", launch_iota(d_perm, n, st));
-    SS_CUDA(cudaMemsetAsync(a.lcp, 0, 4, st));
-    uint32_t n_cur = 1;
+    use_counters(0);
+    uint32_t n_cur = 1, round_no = 0;
+    bool classified = true;
     if (d_inst) {
-        SS_CUDA(cudaMemsetAsync(dc, 0, sizeof(Counters), st));
-        LAUNCH(this, "init_batch", launch_init_batch(d_inst, ninst, cur, a.lcp, dc, st));
-        SS_TRY(sync_counters());
-        n_cur = h_ctr->n_next;
-    } else {
+        LAUNCH(this, "begin",
+               launch_begin(d_perm, n, a.lcp, ws.rc, Seg{0, 0, 0, 0}, nullptr, nullptr, st));
+        // The instances are counted in the second counter set and classified
+        // into the first.
+        Counters *made = ws.rc->c + 1;
+        LAUNCH(this, "init_batch", launch_init_batch(d_inst, ninst, cur, a.lcp, made, st));
+        LAUNCH(this, "classify",
+               launch_classify(cur, dcount(&made->n_next), a.warp8_cap, ws.W1, ws.W8, ws.small(),
+                               ws.L, dev_ctr(), (int)((ninst + 255) / 256), st, ws.rc,
+                               publish_next()));
+        SS_TRY(read_counters());
+        n_cur = hc->rc.c[1].n_next;
+        SS_CUDA(cudaMemsetAsync(made, 0, sizeof(Counters), st));
+    } else if (n <= (uint32_t)SMALL_CAP) {
+        // One CTA sorts it all; what it leaves goes on below.
+        LAUNCH(this, "tiny", launch_tiny(a, cur, nxt, ws.rc, publish_next(), st));
         if (n < 2) return SSORT_OK;
-        Seg first{0, n, 0, 0};
-        SS_CUDA(cudaMemcpyAsync(cur, &first, sizeof(Seg), cudaMemcpyHostToDevice, st));
+        SS_TRY(read_counters());
+        const RoundCounters &r = hc->rc;
+        round_no = r.tiny_rounds;
+        std::copy(r.tiny_live, r.tiny_live + round_no, stats.live);
+        stats.small_segments = r.tiny_segments;
+        add_stats(*h_ctr);
+        n_cur = r.tiny_left;
+        if (round_no & 1) std::swap(cur, nxt);
+        classified = false;
+    } else {
+        // The only segment is a large one: its list entry and counts are known.
+        LAUNCH(this, "begin",
+               launch_begin(d_perm, n, a.lcp, ws.rc, Seg{0, n, 0, 0}, ws.L, &ws.rc->c[0].n_large,
+                            st));
+        *h_ctr = Counters{};
+        h_ctr->n_large = 1;
+        h_ctr->live_next = h_ctr->gather_elems = n;
     }
-    uint32_t round_no = 0;
-    while (n_cur) {
+    // The rounds run on `hp` (round() forks its own when called alone).
+    overlap_round = side && side2 && hp && !prof && overlap && n_cur;
+    cudaStream_t user = st;
+    if (overlap_round) {
+        SS_CUDA(cudaEventRecord(ev_round, user));
+        SS_CUDA(cudaStreamWaitEvent(hp, ev_round, 0));
+        st = hp;
+        forked = true;
+    }
+    int rc = SSORT_OK;
+    while (n_cur && rc == SSORT_OK) {
         uint32_t n_next = 0;
-        SS_TRY(round(a, cur, n_cur, nxt, n_next, round_no));
+        rc = round(a, cur, n_cur, nxt, n_next, round_no, classified, true);
         n_cur = n_next;
+        classified = true;
         std::swap(cur, nxt);
         ++round_no;
     }
+    st = user;
+    if (forked) {
+        forked = false;
+        if (rc == SSORT_OK) {
+            SS_CUDA(cudaEventRecord(ev_round, hp));
+            SS_CUDA(cudaStreamWaitEvent(user, ev_round, 0));
+        }
+    }
+    SS_TRY(rc);
     stats.rounds = round_no;
     if (d_inst) LAUNCH(this, "localize", launch_localize(d_perm, n, d_inst, ninst, st));
     return SSORT_OK;
@@ -568,7 +667,7 @@ void ssort_ctx_destroy(ssort_ctx *ctx) {
             if (b->p) cudaFreeHost(b->p);
         for (cudaEvent_t e : ctx->ev_stage)
             if (e) cudaEventDestroy(e);
-        if (ctx->h_ctr) cudaFreeHost(ctx->h_ctr);
+        if (ctx->hc) cudaFreeHost(ctx->hc);
         if (ctx->h_hist) cudaFreeHost(ctx->h_hist);
         if (ctx->hist_buf.p) cudaFree(ctx->hist_buf.p);
         for (auto e : ctx->ev_pool) cudaEventDestroy(e);
@@ -1284,7 +1383,7 @@ struct NoallocDevice {
     bool ready = false;
     unsigned char *scratch = nullptr;  // device address of g_noalloc_scratch
     int num_sms = 0;
-    Counters host_ctr{};               // plain host copy of the round counters
+    HostCounters host_ctr{};           // plain host copy of the round counters
 };
 
 std::mutex g_noalloc_mu;
@@ -1323,7 +1422,8 @@ extern "C" int ssort_sort_device_noalloc(const uint8_t *d_arena, uint64_t arena_
     c.device = dev;
     c.num_sms = d.num_sms;
     c.st = (cudaStream_t)stream;
-    c.h_ctr = &d.host_ctr;
+    c.hc = &d.host_ctr;
+    c.use_counters(0);
     c.graph_mode = 0;  // the host-driven loop: building a graph would allocate
     c.ws = ws_bind(ws_layout(NOALLOC_MAX_N), d.scratch);
     c.ws_n = NOALLOC_MAX_N;
@@ -1332,7 +1432,7 @@ extern "C" int ssort_sort_device_noalloc(const uint8_t *d_arena, uint64_t arena_
     // before an error still use the shared scratch, and the next call (which
     // may start as soon as the lock is released) must not race with them.
     const cudaError_t se = cudaStreamSynchronize(c.st);
-    c.h_ctr = nullptr;
+    c.hc = nullptr;
     if (rc == SSORT_OK && se != cudaSuccess) return cuda_fail(se, "cudaStreamSynchronize");
     return rc;
 }

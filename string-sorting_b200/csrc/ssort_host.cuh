@@ -54,6 +54,7 @@ struct ssort_ctx {
     // sorts fill the SMs the partition's latency-bound passes leave idle.
     cudaStream_t side = nullptr, side2 = nullptr, hp = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr, ev_round = nullptr;
+    bool forked = false;         // the sort's rounds already run on `hp`
     bool overlap_round = false;  // this round runs its on-chip sorts on `side`
     bool fresh_round = false;    // this round gathers round-0 style (see round())
     int round_mode = -1;         // -1: fresh iff round_no == 0; 0: fresh; 1: deep
@@ -73,7 +74,14 @@ struct ssort_ctx {
     ssort::HBuf h_stage[2];
     cudaEvent_t ev_stage[2] = {nullptr, nullptr};
     int copy_pageable(void *d_dst, const void *h_src, uint64_t bytes);
-    ssort::Counters *h_ctr = nullptr;
+    // Host copy of the device counters.  A context's lies in pinned memory,
+    // where the counting kernels publish it (`published`); elsewhere it is
+    // copied.  ctr_i: which of the two counter sets the current round uses.
+    ssort::HostCounters *hc = nullptr;
+    ssort::Counters *h_ctr = nullptr;  // hc->rc.c[ctr_i]
+    bool published = false;
+    uint32_t pub_seq = 0;
+    int ctr_i = 0;
 
     ssort_stats stats{};
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
@@ -199,13 +207,18 @@ struct ssort_ctx {
         return SSORT_OK;
     }
 
-    int sync_counters() {
-        SS_CUDA(cudaMemcpyAsync(h_ctr, ws.ctr, sizeof(ssort::Counters), cudaMemcpyDeviceToHost, st));
-        SS_CUDA(cudaStreamSynchronize(st));
-        if (h_ctr->error)
-            return ssort::fail(SSORT_EINTERNAL, "a scan's look-back waited past its bound");
-        return SSORT_OK;
+    ssort::Counters *dev_ctr() const { return ws.rc->c + ctr_i; }
+    void use_counters(int i) {
+        ctr_i = i;
+        h_ctr = hc->rc.c + i;
     }
+    // For the next kernel that publishes the counters; read_counters waits
+    // for the last one launched.
+    ssort::Publish publish_next() {
+        if (!published) return ssort::Publish{nullptr, 0};
+        return ssort::Publish{reinterpret_cast<uint32_t *>(hc), ++pub_seq};
+    }
+    int read_counters();
 
     int grid_for(int per_sm) const { return num_sms * per_sm; }
 
@@ -220,12 +233,13 @@ struct ssort_ctx {
         uint32_t w1 = 0, w8 = 0, s[ssort::SMALL_CLASSES] = {0, 0, 0, 0}, e = 0;
     };
     int fork_small();
+    void add_stats(const ssort::Counters &c);
     int launch_small(const ssort::SortArgs &a, ssort::Seg *nxt, SmallDone &done);
     int round_body(const ssort::SortArgs &a, ssort::Seg *cur, uint32_t n_cur, ssort::Seg *nxt,
-                   uint32_t &n_next, uint32_t round_no);
+                   uint32_t &n_next, uint32_t round_no, bool classified, bool ahead);
     int round(const ssort::SortArgs &a, ssort::Seg *cur, uint32_t n_cur, ssort::Seg *nxt,
               uint32_t &n_next,
-              uint32_t round_no);
+              uint32_t round_no, bool classified = false, bool ahead = false);
     int run_ws(const uint8_t *arena, uint64_t arena_bytes, const void *offs, int off_width,
                uint32_t n, uint32_t *d_perm, uint32_t *d_lcp, const uint32_t *d_inst = nullptr,
                uint32_t ninst = 0);

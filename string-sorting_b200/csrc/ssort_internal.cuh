@@ -101,6 +101,29 @@ struct Counters {
     unsigned long long window_saved, window_used;  // key2 entries written / read
 };
 
+// The counters of two consecutive rounds (a round classifies the next one's
+// segments while its own counts are still wanted), and what the one-CTA sort
+// of small inputs did in its rounds.
+constexpr uint32_t TINY_ROUNDS = 64;
+struct RoundCounters {
+    Counters c[2];
+    uint32_t ticket;  // CTAs of the publishing kernel that are done (0 between launches)
+    uint32_t tiny_rounds, tiny_segments, tiny_left;  // rounds run, segments sorted / left over
+    uint32_t tiny_live[TINY_ROUNDS];
+};
+
+// Where a kernel's last CTA copies the RoundCounters for the waiting host:
+// pinned host memory, followed by a word that becomes `seq` once the copy is
+// complete.  A null host: the host copies them itself.
+struct Publish {
+    uint32_t *host;
+    uint32_t seq;
+};
+struct HostCounters {
+    RoundCounters rc;
+    uint32_t flag;
+};
+
 // A count the host knows (dev == nullptr: `host`) or only the device knows:
 // *dev, or dev[*at] when `at` is set (a count stored at an index that is
 // itself a device value).  The host-driven round loop passes host counts;
@@ -261,7 +284,7 @@ constexpr WsLayout ws_layout(uint64_t n) {
     o.partials = take((size_t)scan_partials_for(o.cm_cap) * 4);
     // single-pass scan: a ticket word, then one status word per tile
     o.lookback = take(8 + (size_t)scan_partials_for(o.cm_cap) * 8);
-    o.ctr = take(sizeof(Counters));
+    o.ctr = take(sizeof(RoundCounters));
     o.gs = take(sizeof(GraphState));
     o.total = off;
     return o;
@@ -276,7 +299,8 @@ struct Workspace {
     uint2 *B;
     uint16_t *tbl;
     uint32_t *bkt;
-    Counters *ctr;
+    RoundCounters *rc;
+    Counters *ctr;  // rc->c[0]
     GraphState *gs;
     size_t cm_cap;
 };
@@ -311,21 +335,31 @@ inline Workspace ws_bind(const WsLayout &o, unsigned char *base) {
     w.cm = (uint32_t *)(base + o.cm);
     w.partials = (uint32_t *)(base + o.partials);
     w.lookback = base + o.lookback;
-    w.ctr = (Counters *)(base + o.ctr);
+    w.rc = (RoundCounters *)(base + o.ctr);
+    w.ctr = w.rc->c;
     w.gs = (GraphState *)(base + o.gs);
     w.cm_cap = o.cm_cap;
     return w;
 }
 
 // ---- launchers (ssort_kernels.cu) ----------------------------------------
+// Start of a sort: idx = identity, lcp[0] = 0, counters cleared; with first.len
+// also the first round's only segment, appended to *list (counter *count).
+void launch_begin(uint32_t *idx, uint32_t n, uint32_t *lcp, RoundCounters *rc, Seg first,
+                  Seg *list, uint32_t *count, cudaStream_t st);
 void launch_iota(uint32_t *idx, uint32_t n, cudaStream_t st);
+// A whole sort of at most SMALL_CAP strings by one CTA (k_tiny); A, B: segment
+// lists of two rounds.
+void launch_tiny(const SortArgs &a, Seg *A, Seg *B, RoundCounters *rc, Publish pub,
+                 cudaStream_t st);
 // 256-bin histogram of the first 8 key bytes of `samples` strings (tuning).
 void launch_byte_hist(const uint8_t *arena, uint64_t arena_bytes, const void *offs, int off_width,
                       uint32_t n, uint32_t samples, uint32_t *hist, cudaStream_t st);
 // Launchers with a Count take `grid` CTAs (or size the grid from a host count
 // when grid <= 0); their kernels loop over the work they find.
 void launch_classify(const Seg *R, Count nR, uint32_t warp8_cap, Seg *W1, Seg *W8,
-                     SmallLists S, Seg *L, Counters *c, int grid, cudaStream_t st);
+                     SmallLists S, Seg *L, Counters *c, int grid, cudaStream_t st,
+                     RoundCounters *rc = nullptr, Publish pub = Publish{nullptr, 0});
 // Batches: one round-0 segment per instance; instance-local result indices.
 void launch_init_batch(const uint32_t *inst_start, uint32_t ninst, Seg *R, uint32_t *lcp,
                        Counters *c, cudaStream_t st);
@@ -389,7 +423,8 @@ void launch_scatter(const SortArgs &a, const Seg *L, Count nL, const uint32_t *t
 void launch_emit(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
                  const uint32_t *nspl, const uint32_t *cm_base, const uint32_t *cm_scan,
                  Seg *W1, Seg *W8, SmallLists S, Seg *L2, Seg *E, uint2 *B, Seg *N,
-                 Counters *c, int grid, cudaStream_t st);
+                 Counters *c, int grid, cudaStream_t st, RoundCounters *rc = nullptr,
+                 Publish pub = Publish{nullptr, 0});
 // On-chip segment sorts; list lengths are read from the counters on the device.
 // The on-chip sorts take n list entries from the given list pointer (a range
 // of the list), so that they can run while the list is still being appended.
@@ -403,6 +438,11 @@ void launch_block(const SortArgs &a, const Seg *S, Span sp, int cls, Seg *N, Cou
 void launch_equal(const SortArgs &a, const Seg *E, Span sp, Seg *N, Counters *c, int grid,
                   cudaStream_t st);
 void launch_boundary(const SortArgs &a, const uint2 *B, Counters *c, int grid, cudaStream_t st);
+// Boundary LCPs of the round counted in rc->c[i], and the classification of
+// the next round's segments N into the lists and rc->c[i ^ 1].
+void launch_round_end(const SortArgs &a, const uint2 *B, const Seg *N, Seg *W1, Seg *W8,
+                      SmallLists S, Seg *L, RoundCounters *rc, int i, Publish pub, int grid,
+                      cudaStream_t st);
 
 // Control kernels of the device-driven round loop.  Conditions are
 // cudaGraphConditionalHandle values (unsigned long long).

@@ -330,23 +330,75 @@ __device__ __forceinline__ void append_by_length(const Seg &o, bool v, uint32_t 
     if (lg) L[tl] = o;
 }
 
-__global__ void k_classify(const Seg *__restrict__ R, Count cnt, uint32_t warp8_cap, Seg *W1,
-                           Seg *W8, SmallLists S, Seg *L, Counters *c) {
-    const uint32_t nR = count_of(cnt);
+__device__ __forceinline__ void classify_list(const Seg *__restrict__ R, uint32_t nR,
+                                              uint32_t warp8_cap, Seg *W1, Seg *W8,
+                                              const SmallLists &S, Seg *L, Counters *c) {
     // Block-uniform trip count: every warp reaches the collective appends.
     for (uint32_t b0 = blockIdx.x * blockDim.x; b0 < nR; b0 += gridDim.x * blockDim.x) {
-    const uint32_t i = b0 + threadIdx.x;
-    const bool v = i < nR;
-    const Seg s = v ? R[i] : Seg{0, 0, 0, 0};
-    append_by_length(s, v, warp8_cap, SMALL_CAP, W1, W8, S, L, &c->n_large, c);
-    const bool lg = v && s.len > (uint32_t)SMALL_CAP && s.len > warp8_cap;
-    const unsigned long long live = warp_sum(v ? s.len : 0);
-    const unsigned long long big = warp_sum(lg ? s.len : 0);
-    if ((threadIdx.x & 31) == 0) {
-        if (live) atomicAdd(&c->live_next, live);
-        if (big) atomicAdd(&c->gather_elems, big);
+        const uint32_t i = b0 + threadIdx.x;
+        const bool v = i < nR;
+        const Seg s = v ? R[i] : Seg{0, 0, 0, 0};
+        append_by_length(s, v, warp8_cap, SMALL_CAP, W1, W8, S, L, &c->n_large, c);
+        const bool lg = v && s.len > (uint32_t)SMALL_CAP && s.len > warp8_cap;
+        const unsigned long long live = warp_sum(v ? s.len : 0);
+        const unsigned long long big = warp_sum(lg ? s.len : 0);
+        if ((threadIdx.x & 31) == 0) {
+            if (live) atomicAdd(&c->live_next, live);
+            if (big) atomicAdd(&c->gather_elems, big);
+        }
     }
+}
+
+// End of a kernel whose counts the host waits for: the last CTA to get here
+// copies the counters to pinned host memory and sets the host's flag.  The
+// host polls the flag, which saves the copy engine's launch and the stream
+// synchronisation (a round trip of about 4 us instead of 12).  True in the
+// last CTA.
+__device__ __forceinline__ bool publish(const Publish &p, RoundCounters *rc) {
+    if (!p.host) return false;
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&rc->ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(rc);
+    volatile uint32_t *h = p.host;
+    constexpr uint32_t WORDS = sizeof(RoundCounters) / 4;
+    for (uint32_t i = threadIdx.x; i < WORDS; i += blockDim.x) h[i] = __ldcg(w + i);
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        rc->ticket = 0;
+        h[WORDS] = p.seq;
     }
+    return true;
+}
+
+__global__ void k_begin(uint32_t *idx, uint32_t n, uint32_t *lcp, RoundCounters *rc, Seg first,
+                        Seg *list, uint32_t *count) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        idx[i] = i;
+    if (blockIdx.x != 0) return;
+    uint32_t *w = reinterpret_cast<uint32_t *>(rc);
+    for (uint32_t i = threadIdx.x; i < sizeof(RoundCounters) / 4; i += blockDim.x) w[i] = 0;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (n) lcp[0] = 0;
+    if (first.len) {
+        *list = first;
+        *count = 1;
+        rc->c[0].live_next = first.len;
+        if (first.len > (uint32_t)SMALL_CAP) rc->c[0].gather_elems = first.len;
+    }
+}
+
+__global__ void k_classify(const Seg *__restrict__ R, Count cnt, uint32_t warp8_cap, Seg *W1,
+                           Seg *W8, SmallLists S, Seg *L, Counters *c, RoundCounters *rc,
+                           Publish pub) {
+    classify_list(R, count_of(cnt), warp8_cap, W1, W8, S, L, c);
+    publish(pub, rc);
 }
 
 // ---- batches of independent instances ---------------------------------------
@@ -806,7 +858,7 @@ __global__ void __launch_bounds__(GATHER_THREADS) k_gather(SortArgs a, const Seg
 // before any is used (index, then offset, then the two 16-byte words that
 // hold the key), so that G chains of dependent reads overlap.
 template <int G>
-__device__ __forceinline__ void gather_keys_at(const SortArgs &a, const uint32_t *__restrict__ I,
+__device__ __forceinline__ void gather_keys_at(const SortArgs &a, const uint32_t *I,
                                                uint32_t depth, const uint32_t (&at)[G],
                                                uint32_t e0, uint32_t stride, uint32_t len,
                                                Key (&kk)[G], uint32_t (&ii)[G]) {
@@ -836,7 +888,7 @@ __device__ __forceinline__ void gather_keys_at(const SortArgs &a, const uint32_t
 
 // The same for the elements' own places in I.
 template <int G>
-__device__ __forceinline__ void gather_keys(const SortArgs &a, const uint32_t *__restrict__ I,
+__device__ __forceinline__ void gather_keys(const SortArgs &a, const uint32_t *I,
                                             uint32_t depth, uint32_t e0, uint32_t stride,
                                             uint32_t len, Key (&kk)[G], uint32_t (&ii)[G]) {
     uint32_t at[G];
@@ -1835,7 +1887,8 @@ __global__ void k_emit(SortArgs a, const Seg *__restrict__ L, Count cnt,
                        const uint32_t *__restrict__ tile_base,
                        const uint32_t *__restrict__ nspl, const uint32_t *__restrict__ cm_base,
                        const uint32_t *__restrict__ cm_scan, Seg *W1, Seg *W8, SmallLists S,
-                       Seg *L2, Seg *E, uint2 *B, Seg *N, Counters *c) {
+                       Seg *L2, Seg *E, uint2 *B, Seg *N, Counters *c, RoundCounters *rc,
+                       Publish pub) {
     const uint32_t nL = count_of(cnt);
     for (uint32_t q = blockIdx.x; q < nL * EMIT_CHUNKS; q += gridDim.x) {
     const uint32_t si = q / EMIT_CHUNKS, b0 = q % EMIT_CHUNKS * EMIT_THREADS;
@@ -1897,6 +1950,8 @@ __global__ void k_emit(SortArgs a, const Seg *__restrict__ L, Count cnt,
         if (b == 0) atomicAdd(&c->partitioned, (unsigned long long)s.len);
     }
     }
+    // (the count of the level just emitted starts the next one at 0)
+    if (publish(pub, rc) && threadIdx.x == 0) c->n_large_next = 0;
 }
 
 // ---- segments of <= 32 strings: one warp, one string per lane -------------
@@ -2762,12 +2817,117 @@ __global__ void k_equal(SortArgs a, const Seg *__restrict__ E0, Span sp, Seg *N,
     }
 }
 
-__global__ void k_boundary(SortArgs a, const uint2 *__restrict__ B, Counters *c) {
-    const uint32_t nB = c->n_bound;
+__device__ __forceinline__ void boundary_lcps(const SortArgs &a, const uint2 *__restrict__ B,
+                                              uint32_t nB) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nB; i += gridDim.x * blockDim.x) {
         const uint2 e = B[i];
         a.lcp[e.x] = e.y + key_lcp(to_key(a.key[0][e.x - 1]), to_key(a.key[0][e.x]));
     }
+}
+
+__global__ void k_boundary(SortArgs a, const uint2 *__restrict__ B, Counters *c) {
+    boundary_lcps(a, B, c->n_bound);
+}
+
+// End of a round whose next round follows at once: one launch and one host
+// round trip for the boundary LCPs and the next round's classification.  The
+// finished round's counters are cleared for the round after the next.
+__global__ void k_round_end(SortArgs a, const uint2 *__restrict__ B, const Seg *__restrict__ N,
+                            Seg *W1, Seg *W8, SmallLists S, Seg *L, RoundCounters *rc, int i,
+                            Publish pub) {
+    const Counters *old = rc->c + i;
+    boundary_lcps(a, B, old->n_bound);
+    classify_list(N, old->n_next, a.warp8_cap, W1, W8, S, L, rc->c + (i ^ 1));
+    if (publish(pub, rc)) {
+        uint32_t *w = reinterpret_cast<uint32_t *>(rc->c + i);
+        for (uint32_t q = threadIdx.x; q < sizeof(Counters) / 4; q += blockDim.x) w[q] = 0;
+    }
+}
+
+// ---- a whole small sort in one CTA -----------------------------------------
+// At most SMALL_CAP strings need no partition: one CTA sorts them, then keeps
+// refining the runs of equal keys round by round, with the code of the
+// on-chip sorts (the whole CTA on segments of more than 256 strings, a warp on
+// each smaller one).  What the rounds of the general loop cost such a sort is
+// launches and host round trips: 500 words took 134 us.  A round with more
+// segments than TINY_SEGMENTS (which the general loop spreads over the chip),
+// or the TINY_ROUNDS-th, is left to the general loop.
+constexpr uint32_t TINY_SEGMENTS = 128;
+constexpr size_t TINY_SMEM =
+    SEG_SMEM<256> > SEG_SMEM<32> ? SEG_SMEM<256> : SEG_SMEM<32>;
+
+__global__ void __launch_bounds__(SMALL_THREADS, 1)
+    k_tiny(SortArgs a, Seg *A, Seg *B, RoundCounters *rc, Publish pub) {
+    extern __shared__ __align__(16) unsigned char seg_smem[];
+    __shared__ unsigned long long live;
+    const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
+    Counters *c = rc->c;
+    {
+        uint32_t *z = reinterpret_cast<uint32_t *>(rc);
+        for (uint32_t i = t; i < sizeof(RoundCounters) / 4; i += SMALL_THREADS) z[i] = 0;
+    }
+    for (uint32_t i = t; i < a.n; i += SMALL_THREADS) a.idx[0][i] = i;
+    if (t == 0) {
+        a.lcp[0] = 0;
+        A[0] = Seg{0, a.n, 0, 0};
+    }
+    __syncthreads();
+    uint32_t n_cur = 1, round = 0, segments = 0;
+    for (; round < TINY_ROUNDS && n_cur && n_cur <= TINY_SEGMENTS; ++round) {
+        if (t == 0) {
+            live = 0;
+            c->n_next = 0;
+        }
+        __syncthreads();
+        const Seg own = t < n_cur ? A[t] : Seg{0, 0, 0, 0};
+        const unsigned long long sum = warp_sum(own.len);
+        if (lane == 0 && sum) atomicAdd(&live, sum);
+        if (__syncthreads_or(own.len > (uint32_t)WARP8_CAP)) {
+            for (uint32_t g = 0; g < n_cur; ++g) {
+                const Seg s = A[g];
+                if (s.len <= (uint32_t)WARP8_CAP) continue;
+                const bool full = sort_segment<256>(
+                    a, s, *reinterpret_cast<SegSmem<256, 8> *>(seg_smem), t, 0, B, c);
+                if (t == 0) {
+                    c->block_fresh += s.len;
+                    if (full) c->full_sorted += s.len;
+                }
+            }
+            __syncthreads();
+        }
+        unsigned long long deep = 0;
+        for (uint32_t g = w; g < n_cur; g += SMALL_THREADS / 32) {
+            const Seg s = A[g];
+            if (s.len > (uint32_t)WARP8_CAP) continue;
+            if (s.len <= (uint32_t)WARP1_CAP) {
+                deep += warp1_group<32>(a, s, lane, B, c);
+                if (lane == 0) atomicAdd(&c->warp1_fresh, (unsigned long long)s.len);
+            } else {
+                const bool full = sort_segment<32>(
+                    a, s, reinterpret_cast<SegSmem<32, 8> *>(seg_smem)[w], lane, 0, B, c);
+                if (lane == 0) {
+                    atomicAdd(&c->warp8_fresh, (unsigned long long)s.len);
+                    if (full) atomicAdd(&c->full_sorted, (unsigned long long)s.len);
+                }
+            }
+        }
+        deep = warp_sum(deep);
+        if (lane == 0 && deep) atomicAdd(&c->warp1_deep, deep);
+        __syncthreads();
+        if (t == 0) rc->tiny_live[round] = (uint32_t)live;
+        segments += n_cur;
+        n_cur = atomicAdd(&c->n_next, 0u);
+        Seg *x = A;
+        A = B;
+        B = x;
+        __syncthreads();
+    }
+    if (t == 0) {
+        rc->tiny_rounds = round;
+        rc->tiny_segments = segments;
+        rc->tiny_left = n_cur;
+    }
+    publish(pub, rc);
 }
 
 // ---- control kernels of the device-driven round loop --------------------------
@@ -3018,6 +3178,7 @@ static void set_smem_attrs() {
                          (int)sizeof(ScatterSmem));
     cudaFuncSetAttribute(k_scatter2, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(Scatter2Smem));
+    cudaFuncSetAttribute(k_tiny, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TINY_SMEM);
     cudaFuncSetAttribute(k_segsort<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)SEG_SMEM<32>);
     cudaFuncSetAttribute(k_segsort<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3045,11 +3206,30 @@ static int grid_of(int grid, const Count &n, uint32_t per, uint32_t cap) {
     return (int)(g < cap ? g : cap);
 }
 
+void launch_begin(uint32_t *idx, uint32_t n, uint32_t *lcp, RoundCounters *rc, Seg first,
+                  Seg *list, uint32_t *count, cudaStream_t st) {
+    const uint32_t g = cdiv(n, 256) < 148 * 16 ? cdiv(n, 256) : 148 * 16;
+    k_begin<<<g ? g : 1, 256, 0, st>>>(idx, n, lcp, rc, first, list, count);
+}
+
+void launch_tiny(const SortArgs &a, Seg *A, Seg *B, RoundCounters *rc, Publish pub,
+                 cudaStream_t st) {
+    set_smem_attrs();
+    k_tiny<<<1, SMALL_THREADS, TINY_SMEM, st>>>(a, A, B, rc, pub);
+}
+
 void launch_classify(const Seg *R, Count nR, uint32_t warp8_cap, Seg *W1, Seg *W8,
-                     SmallLists S, Seg *L, Counters *c, int grid, cudaStream_t st) {
+                     SmallLists S, Seg *L, Counters *c, int grid, cudaStream_t st,
+                     RoundCounters *rc, Publish pub) {
     const int g = grid_of(grid, nR, 256, 1u << 30);
     if (!g) return;
-    k_classify<<<g, 256, 0, st>>>(R, nR, warp8_cap, W1, W8, S, L, c);
+    k_classify<<<g, 256, 0, st>>>(R, nR, warp8_cap, W1, W8, S, L, c, rc, pub);
+}
+
+void launch_round_end(const SortArgs &a, const uint2 *B, const Seg *N, Seg *W1, Seg *W8,
+                      SmallLists S, Seg *L, RoundCounters *rc, int i, Publish pub, int grid,
+                      cudaStream_t st) {
+    k_round_end<<<grid, 256, 0, st>>>(a, B, N, W1, W8, S, L, rc, i, pub);
 }
 
 void launch_init_batch(const uint32_t *inst_start, uint32_t ninst, Seg *R, uint32_t *lcp,
@@ -3195,11 +3375,11 @@ void launch_scatter(const SortArgs &a, const Seg *L, Count nL, const uint32_t *t
 void launch_emit(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
                  const uint32_t *nspl, const uint32_t *cm_base, const uint32_t *cm_scan,
                  Seg *W1, Seg *W8, SmallLists S, Seg *L2, Seg *E, uint2 *B, Seg *N,
-                 Counters *c, int grid, cudaStream_t st) {
+                 Counters *c, int grid, cudaStream_t st, RoundCounters *rc, Publish pub) {
     const int g = grid > 0 ? grid : grid_of(grid, nL, 1, 1u << 28) * EMIT_CHUNKS;
     if (!g) return;
     k_emit<<<g, EMIT_THREADS, 0, st>>>(a, L, nL, tile_base, nspl, cm_base, cm_scan, W1, W8, S, L2, E, B,
-                              N, c);
+                              N, c, rc, pub);
 }
 
 // A span with host bounds and nothing in it launches nothing.
