@@ -149,17 +149,21 @@ int ssort_ctx::launch_small(const SortArgs &a, Seg *nxt, SmallDone &d) {
     LAUNCH(this, "warp8", launch_warp8(a, ws.W8, hspan(d.w8, d.w8 + n), nxt, dc, grid(n, 8), s2));
     d.w8 += n;
     // CTA-sort size classes: groups of 64, 128, 256, 512 threads per segment.
-    const SmallLists lists = ws.small();
     const uint32_t counts[SMALL_CLASSES] = {h_ctr->n_small, h_ctr->n_small2, h_ctr->n_small3,
                                             h_ctr->n_small4};
+    SmallWork wk{};
+    wk.list = ws.small();
     for (int k = 0; k < SMALL_CLASSES; ++k) {
-        n = counts[k] - d.s[k];
-        const uint32_t per_cta = k < 3 ? 4u >> k : 1u;
-        LAUNCH(this, "block",
-               launch_block(a, lists.s[k], hspan(d.s[k], d.s[k] + n), k, nxt, dc,
-                            grid(n, per_cta), s3));
-        d.s[k] += n;
+        const uint32_t segs = counts[k] - d.s[k];
+        wk.span[k] = hspan(d.s[k], counts[k]);
+        const bool own = segs >= CLASS_MIN_SEGS >> k;
+        if (own)
+            LAUNCH(this, "block",
+                   launch_block_class(a, wk.list.s[k], wk.span[k], k, nxt, dc, s3));
+        wk.cta[k + 1] = wk.cta[k] + (own ? 0 : block_ctas(segs, k));
+        d.s[k] = counts[k];
     }
+    LAUNCH(this, "block", launch_block(a, wk, nxt, dc, s3));
     n = h_ctr->n_equal - d.e;
     LAUNCH(this, "equal", launch_equal(a, ws.E, hspan(d.e, d.e + n), nxt, dc, grid(n, 1), s2));
     d.e += n;
@@ -265,7 +269,7 @@ int ssort_ctx::round_body(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt,
         SS_TRY(scan(ws.cm, ws.cm, (uint32_t)(ws.cm_cap - 1), dcount(ws.cm_base + n_large)));
         LAUNCH(this, "scatter",
                launch_scatter(a, lcur, nl, ws.tile_base, ws.spl, ws.nspl, ws.tbl, ws.cm_base,
-                              ws.cm, g2, st));
+                              ws.cm, dc, g2, st));
         LAUNCH(this, "emit",
                launch_emit(a, lcur, nl, ws.tile_base, ws.nspl, ws.cm_base, ws.cm, ws.W1, ws.W8,
                            ws.small(), lnext, ws.E, ws.B, nxt, dc, 0, st,

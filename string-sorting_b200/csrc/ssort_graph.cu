@@ -94,13 +94,15 @@ int ssort_ctx::graph_small(const SortArgs &a, cudaStream_t s) {
     LAUNCH(this, "warp8",
            launch_warp8(a, ws.W8, Span{dcount(&g->cur_w8), dcount(&dc->n_w8)}, nxt, dc,
                         grid_for(6), s));
-    const SmallLists lists = ws.small();
     const uint32_t *counts[SMALL_CLASSES] = {&dc->n_small, &dc->n_small2, &dc->n_small3,
                                              &dc->n_small4};
-    for (int k = 0; k < SMALL_CLASSES; ++k)
-        LAUNCH(this, "block",
-               launch_block(a, lists.s[k], Span{dcount(&g->cur_s[k]), dcount(counts[k])}, k, nxt,
-                            dc, grid_for(6), s));
+    SmallWork wk{};
+    wk.list = ws.small();
+    for (int k = 0; k < SMALL_CLASSES; ++k) {
+        wk.span[k] = Span{dcount(&g->cur_s[k]), dcount(counts[k])};
+        wk.cta[k + 1] = wk.cta[k] + (uint32_t)grid_for(2);
+    }
+    LAUNCH(this, "block", launch_block(a, wk, nxt, dc, s));
     LAUNCH(this, "equal",
            launch_equal(a, ws.E, Span{dcount(&g->cur_e), dcount(&dc->n_equal)}, nxt, dc,
                         grid_for(8), s));
@@ -175,7 +177,7 @@ int ssort_ctx::graph_build(const SortArgs &a) {
                            dcount(ws.cm_base, &g->n_large), s1));
             LAUNCH(this, "scatter",
                    launch_scatter(a, ws.L, nl, ws.tile_base, ws.spl, ws.nspl, ws.tbl, ws.cm_base,
-                                  ws.cm, g2, s1));
+                                  ws.cm, dc, g2, s1));
             LAUNCH(this, "emit",
                    launch_emit(a, ws.L, nl, ws.tile_base, ws.nspl, ws.cm_base, ws.cm, ws.W1,
                                ws.W8, S, ws.L2, ws.E, ws.B, ws.N, dc, g4, s1));

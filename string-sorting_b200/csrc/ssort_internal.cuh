@@ -95,6 +95,8 @@ struct Counters {
         block_keyed;
     unsigned long long equal_moved, equal_final;  // equality-bucket copies / lcp fills
     uint32_t n_small2, n_small3, n_small4;  // CTA-sort segments of the 2nd to 4th size class
+    uint32_t count_ticket, scatter_ticket;  // tiles handed out (cleared by the level's sample)
+    uint32_t pad;
     uint32_t sample_ticket;  // CTAs of the sample kernel that are done (0 between launches)
     unsigned long long warp1_deep;  // strings re-sorted by in-warp refinement steps
     unsigned long long full_sorted;  // strings of segments re-sorted by the full comparator
@@ -418,7 +420,7 @@ void launch_count(const SortArgs &a, const Seg *L, Count nL, const uint32_t *til
                   cudaStream_t st);
 void launch_scatter(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
                     const ulonglong2 *spl, const uint32_t *nspl, const uint16_t *tbl,
-                    const uint32_t *cm_base, const uint32_t *cm_scan, int grid,
+                    const uint32_t *cm_base, const uint32_t *cm_scan, Counters *c, int grid,
                     cudaStream_t st);
 void launch_emit(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
                  const uint32_t *nspl, const uint32_t *cm_base, const uint32_t *cm_scan,
@@ -432,9 +434,21 @@ void launch_warp1(const SortArgs &a, const Seg *W1, Span sp, Seg *N, Counters *c
                   cudaStream_t st);
 void launch_warp8(const SortArgs &a, const Seg *W8, Span sp, Seg *N, Counters *c, int grid,
                   cudaStream_t st);
-// cls: size class 0 .. 3 (segment list S holds that class)
-void launch_block(const SortArgs &a, const Seg *S, Span sp, int cls, Seg *N, Counters *c,
-                  int grid, cudaStream_t st);
+// The CTA sorts of a level: per size class its list, the entries to sort and
+// the first CTA that works on it (cta[SMALL_CLASSES]: CTAs in all).
+struct SmallWork {
+    SmallLists list;
+    Span span[SMALL_CLASSES];
+    uint32_t cta[SMALL_CLASSES + 1];
+};
+// CTAs that sort n segments of class k in one pass.
+inline uint32_t block_ctas(uint32_t n, int k) { return (n + (8u >> k) - 1) / (8u >> k); }
+void launch_block(const SortArgs &a, const SmallWork &wk, Seg *N, Counters *c, cudaStream_t st);
+// One class by itself (host counts), worth it where it has at least
+// CLASS_MIN_SEGS >> k segments: two waves of its CTAs on every SM.
+constexpr uint32_t CLASS_MIN_SEGS = 148 * 2 * 8 * 2;  // of class 0, halved per class
+void launch_block_class(const SortArgs &a, const Seg *S, Span sp, int cls, Seg *N, Counters *c,
+                        cudaStream_t st);
 void launch_equal(const SortArgs &a, const Seg *E, Span sp, Seg *N, Counters *c, int grid,
                   cudaStream_t st);
 void launch_boundary(const SortArgs &a, const uint2 *B, Counters *c, int grid, cudaStream_t st);

@@ -898,52 +898,43 @@ __device__ __forceinline__ void gather_keys(const SortArgs &a, const uint32_t *I
 }
 
 // ---- register sorts of 32-bit values (samples and on-chip segments) ---------
-// Barrier among the GT threads of group gi: named barrier 1 + gi (0 is
-// __syncthreads).  Immediate ids, so that a CTA claims only the barriers it
-// uses (at most 5) and the SM's barriers do not limit occupancy.
-template <int GT>
-__device__ __forceinline__ void group_sync(uint32_t gi) {
-    constexpr int G = GT < SMALL_THREADS ? SMALL_THREADS / GT : 1;
-    if constexpr (GT == 32) {
-        __syncwarp();
-    } else {
-        if (G == 1 || gi == 0)
-            asm volatile("bar.sync 1, %0;" ::"n"(GT) : "memory");
-        else if (G == 2 || gi == 1)
-            asm volatile("bar.sync 2, %0;" ::"n"(GT) : "memory");
-        else if (gi == 2)
-            asm volatile("bar.sync 3, %0;" ::"n"(GT) : "memory");
-        else
-            asm volatile("bar.sync 4, %0;" ::"n"(GT) : "memory");
-    }
-}
-
-// Whether any thread of the group has `want`; a barrier of the group.
-template <int GT>
-__device__ __forceinline__ bool group_any(bool want, uint32_t gi) {
-    if constexpr (GT == 32) {
+// The threads that sort one set of values together: one warp, or 2 to 16 of a
+// CTA's warps with a named barrier of their own (0 is __syncthreads).  The
+// CTA form holds its size at run time (LOG2 = 0) or as a constant.
+struct WarpGroup {
+    static constexpr bool warp = true;
+    uint32_t t;
+    __device__ __forceinline__ constexpr uint32_t threads() const { return 32; }
+    __device__ __forceinline__ constexpr uint32_t log2() const { return 5; }
+    __device__ __forceinline__ void sync() const { __syncwarp(); }
+    // whether any thread of the group has `want`; a barrier of the group
+    __device__ __forceinline__ bool any(bool want) const {
         return __any_sync(0xffffffffu, want);
-    } else {
-        constexpr int G = GT < SMALL_THREADS ? SMALL_THREADS / GT : 1;
+    }
+};
+
+template <int LOG2 = 0>
+struct CtaGroup {
+    static constexpr bool warp = false;
+    uint32_t t, log2_threads, barrier;
+    __device__ __forceinline__ constexpr uint32_t log2() const {
+        return LOG2 ? LOG2 : log2_threads;
+    }
+    __device__ __forceinline__ constexpr uint32_t threads() const { return 1u << log2(); }
+    __device__ __forceinline__ void sync() const {
+        asm volatile("bar.sync %0, %1;" ::"r"(barrier), "r"(threads()) : "memory");
+    }
+    __device__ __forceinline__ bool any(bool want) const {
         uint32_t r;
-#define SS_BAR_ANY(id)                                                               \
-    asm volatile("{ .reg .pred p, q; setp.ne.u32 p, %1, 0; bar.red.or.pred q, " #id  \
-                 ", %2, p; selp.u32 %0, 1, 0, q; }"                                  \
-                 : "=r"(r)                                                           \
-                 : "r"((uint32_t)want), "n"(GT)                                      \
-                 : "memory")
-        if (G == 1 || gi == 0)
-            SS_BAR_ANY(1);
-        else if (G == 2 || gi == 1)
-            SS_BAR_ANY(2);
-        else if (gi == 2)
-            SS_BAR_ANY(3);
-        else
-            SS_BAR_ANY(4);
-#undef SS_BAR_ANY
+        asm volatile(
+            "{ .reg .pred p, q; setp.ne.u32 p, %1, 0; bar.red.or.pred q, %2, %3, p; "
+            "selp.u32 %0, 1, 0, q; }"
+            : "=r"(r)
+            : "r"((uint32_t)want), "r"(barrier), "r"(threads())
+            : "memory");
         return r != 0;
     }
-}
+};
 
 template <typename V>
 __device__ __forceinline__ void cmp_swap(V &a, V &b) {
@@ -1010,37 +1001,37 @@ __device__ __forceinline__ void warp_clean(V (&v)[ITEMS], uint32_t m, uint32_t l
 
 // Every thread stores its values to x (16-byte words, consecutive threads
 // next to each other) and loads those of thread `from`.  Two barriers.
-template <int GT, int ITEMS, typename V>
-__device__ __forceinline__ void swap_values(const V (&v)[ITEMS], V (&o)[ITEMS], void *x,
-                                            uint32_t t, uint32_t from, uint32_t gi) {
+template <class G, int ITEMS, typename V>
+__device__ __forceinline__ void swap_values(const G &g, const V (&v)[ITEMS], V (&o)[ITEMS],
+                                            void *x, uint32_t from) {
     constexpr int PER = 16 / sizeof(V);  // values per 16-byte word
     V w[PER];
 #pragma unroll
     for (int j = 0; j < ITEMS / PER; ++j) {
 #pragma unroll
         for (int q = 0; q < PER; ++q) w[q] = v[j * PER + q];
-        static_cast<uint4 *>(x)[j * GT + t] = *reinterpret_cast<const uint4 *>(w);
+        static_cast<uint4 *>(x)[j * g.threads() + g.t] = *reinterpret_cast<const uint4 *>(w);
     }
-    group_sync<GT>(gi);
+    g.sync();
 #pragma unroll
     for (int j = 0; j < ITEMS / PER; ++j) {
-        *reinterpret_cast<uint4 *>(w) = static_cast<const uint4 *>(x)[j * GT + from];
+        *reinterpret_cast<uint4 *>(w) = static_cast<const uint4 *>(x)[j * g.threads() + from];
 #pragma unroll
         for (int q = 0; q < PER; ++q) o[j * PER + q] = w[q];
     }
-    group_sync<GT>(gi);
+    g.sync();
 }
 
-// Sorts the GT * ITEMS values of a group; thread t ends with ranks t * ITEMS
-// .. t * ITEMS + ITEMS - 1.  Odd-even merge sort inside a thread, then bitonic
-// merges of 2, 4, .. GT threads whose first stage compares mirrored positions,
-// so that every stage sorts ascending; strides of 32 threads and more go
-// through shared memory (x: GT * ITEMS values).  With `threads` < GT (a power
-// of two, at least 32) aligned blocks of that many threads sort on their own.
-template <int GT, int ITEMS, typename V>
-__device__ __forceinline__ void group_net_sort(V (&v)[ITEMS], void *x, uint32_t t, uint32_t gi,
-                                               uint32_t threads = GT) {
-    const uint32_t lane = t & 31;
+// Sorts the ITEMS values of each of a group's threads; thread t ends with
+// ranks t * ITEMS .. t * ITEMS + ITEMS - 1.  Odd-even merge sort inside a
+// thread, then bitonic merges of 2, 4, .. threads whose first stage compares
+// mirrored positions, so that every stage sorts ascending; strides of 32
+// threads and more go through shared memory (x: a value per thread and item).
+// Aligned blocks of `threads` (a power of two, at least 32) sort on their own.
+template <class G, int ITEMS, typename V>
+__device__ __forceinline__ void group_net_sort(const G &g, V (&v)[ITEMS], void *x,
+                                               uint32_t threads) {
+    const uint32_t t = g.t, lane = t & 31;
     net_sort<0, ITEMS>(v);
 #pragma unroll 1
     for (uint32_t half = 1; half < 32; half *= 2) {
@@ -1055,17 +1046,17 @@ __device__ __forceinline__ void group_net_sort(V (&v)[ITEMS], void *x, uint32_t 
         }
         warp_clean<ITEMS>(v, half / 2, lane);
     }
-    if constexpr (GT > 32) {
+    if constexpr (!G::warp) {
 #pragma unroll 1
         for (uint32_t half = 32; half < threads; half *= 2) {
             V o[ITEMS];
-            swap_values<GT, ITEMS>(v, o, x, t, t ^ (2 * half - 1), gi);
+            swap_values<G, ITEMS>(g, v, o, x, t ^ (2 * half - 1));
             const bool up = (t & half) != 0;
 #pragma unroll
             for (int i = 0; i < ITEMS; ++i) v[i] = keep_side(v[i], o[ITEMS - 1 - i], up);
 #pragma unroll 1
             for (uint32_t m = half / 2; m >= 32; m /= 2) {
-                swap_values<GT, ITEMS>(v, o, x, t, t ^ m, gi);
+                swap_values<G, ITEMS>(g, v, o, x, t ^ m);
                 const bool um = (t & m) != 0;
 #pragma unroll
                 for (int i = 0; i < ITEMS; ++i) v[i] = keep_side(v[i], o[i], um);
@@ -1145,7 +1136,8 @@ __device__ __forceinline__ uint64_t warp_or64(uint64_t x) {
 
 // ---- splitter selection: one CTA per large segment ------------------------
 constexpr int SAMPLE_THREADS = 512;
-static_assert(SAMPLES_MAX == SAMPLE_THREADS * 8, "8 samples per thread");
+static_assert(SAMPLE_THREADS == 1 << 9 && SAMPLES_MAX == SAMPLE_THREADS * 8,
+              "8 samples per thread");
 
 // The samples' keys, their sorted values (later the splitters' window bits),
 // the candidates: 89 KB, two CTAs per SM.
@@ -1242,7 +1234,7 @@ __device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__r
     if (mh | ml) {
         Squeezed<8> z;
         squeeze_keys<8>(z, sm.key, t < act ? S : 0u, act, t, mh, ml, 31 - __clz(S), 0u);
-        group_net_sort<SAMPLE_THREADS, 8>(z.v, sm.val, t, 0, act);
+        group_net_sort<CtaGroup<9>, 8>(CtaGroup<9>{t, 9, 1}, z.v, sm.val, act);
         if (t < act) {
             uint4 *o = reinterpret_cast<uint4 *>(sm.val + 8 * t);
             o[0] = make_uint4(z.v[0], z.v[1], z.v[2], z.v[3]);
@@ -1402,6 +1394,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
         lb.cm_base[nL] = c1;
         c->sample_ticket = 0;
     }
+    if (t == 0) c->count_ticket = c->scatter_ticket = 0;
     // ticket word and one status word per scan tile
     for (uint32_t q = t; q < 1 + (c1 + SCAN_CHUNK_ELEMS - 1) / SCAN_CHUNK_ELEMS;
          q += SAMPLE_THREADS)
@@ -1432,6 +1425,29 @@ __device__ __forceinline__ void load_splitters(PartSmem &sm, const ulonglong2 *_
     }
 }
 
+// Tiles for a CTA of the partition kernels, in ticket order: the first is its
+// own index, later ones come from a counter, asked for while the current tile
+// is worked on.  The kernels share the chip with the on-chip sorts, so a CTA
+// may start late; with a fixed stride it would keep the whole kernel waiting.
+// Called by all threads; a tile's work holds at least one __syncthreads.
+struct TileQueue {
+    uint32_t *ticket;
+    uint32_t turn;
+    __device__ __forceinline__ explicit TileQueue(uint32_t *t) : ticket(t), turn(0) {}
+    __device__ __forceinline__ static uint32_t *slots() {
+        __shared__ uint32_t s[2];
+        return s;
+    }
+    __device__ __forceinline__ void ask() {
+        if (threadIdx.x == 0) slots()[turn] = atomicAdd(ticket, 1u) + gridDim.x;
+    }
+    __device__ __forceinline__ uint32_t next() {
+        const uint32_t t = slots()[turn];
+        turn ^= 1;
+        return t;
+    }
+};
+
 // GATHER (first partition level of a round): the keys are loaded from the
 // arena through idx and offsets and stored to the key buffer here, so the
 // key gather's random arena reads overlap the classification work.
@@ -1453,7 +1469,9 @@ __global__ void __launch_bounds__(PART_THREADS, 2) k_count(SortArgs a, const Seg
     const uint32_t total_tiles = tile_base[nL];
     const uint32_t lt = lanemask_lt();
     uint32_t loaded = ~0u;
-    for (uint32_t t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+    TileQueue tiles(&cnt_ctr->count_ticket);
+    for (uint32_t t = blockIdx.x; t < total_tiles; t = tiles.next()) {
+        tiles.ask();
         const uint32_t si = find_seg(tile_base, nL, t);
         const Seg s = L[si];
         const uint32_t u = nspl[si] & 0xFFFF, f = nspl[si] >> 16, nb = 2 * u + 1;
@@ -1616,7 +1634,8 @@ __global__ void __launch_bounds__(SCATTER_THREADS) k_scatter(SortArgs a, const S
                                                              const uint32_t *__restrict__ tile_base,
                                                              const uint32_t *__restrict__ nspl,
                                                              const uint32_t *__restrict__ cm_base,
-                                                             const uint32_t *__restrict__ cm_scan) {
+                                                             const uint32_t *__restrict__ cm_scan,
+                                                             Counters *ctr) {
     extern __shared__ __align__(16) unsigned char scatter_smem[];
     ScatterSmem &sm = *reinterpret_cast<ScatterSmem *>(scatter_smem);
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1624,7 +1643,9 @@ __global__ void __launch_bounds__(SCATTER_THREADS) k_scatter(SortArgs a, const S
     const uint32_t nL = count_of(cnt);
     const uint32_t total_tiles = tile_base[nL];
     bool any_bulk = false;  // this thread issued bulk copies (BULK)
-    for (uint32_t t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+    TileQueue tiles(&ctr->scatter_ticket);
+    for (uint32_t t = blockIdx.x; t < total_tiles; t = tiles.next()) {
+        tiles.ask();
         const uint32_t si = find_seg(tile_base, nL, t);
         const Seg s = L[si];
         const uint32_t u = nspl[si] & 0xFFFF, nb = 2 * u + 1;
@@ -1769,14 +1790,16 @@ constexpr int SCATTER2_BATCH = 4;  // keys in flight per thread in the write-out
 __global__ void __launch_bounds__(SCATTER_THREADS, 3) k_scatter2(
     SortArgs a, const Seg *__restrict__ L, Count cnt, const uint32_t *__restrict__ tile_base,
     const uint32_t *__restrict__ nspl, const uint32_t *__restrict__ cm_base,
-    const uint32_t *__restrict__ cm_scan) {
+    const uint32_t *__restrict__ cm_scan, Counters *ctr) {
     extern __shared__ __align__(16) unsigned char scatter_smem[];
     Scatter2Smem &sm = *reinterpret_cast<Scatter2Smem *>(scatter_smem);
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     constexpr uint32_t QPT = (NB_MAX + 1) / SCATTER_THREADS;  // buckets per thread (4)
     const uint32_t nL = count_of(cnt);
     const uint32_t total_tiles = tile_base[nL];
-    for (uint32_t t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+    TileQueue tiles(&ctr->scatter_ticket);
+    for (uint32_t t = blockIdx.x; t < total_tiles; t = tiles.next()) {
+        tiles.ask();
         const uint32_t si = find_seg(tile_base, nL, t);
         const Seg s = L[si];
         const uint32_t u = nspl[si] & 0xFFFF, nb = 2 * u + 1;
@@ -2321,31 +2344,40 @@ __device__ __forceinline__ void cp_async_wait() {
 // strings 2.79 -> 1.53 ms, of 16 M suffixes 4.23 -> 2.59 ms, of 50 M URLs 2.27
 // -> 1.62 ms.
 
-// Shared memory of one group: keys, values (in passing between threads, and
-// the final order), indices.  Values and indices together also hold 64-bit
-// values while a segment is refined.
-template <int GT, int ITEMS>
-struct SegSmem {
-    ulonglong2 key[GT * 8];
-    uint32_t val[GT * 8];
-    uint32_t idx[GT * 8];
-    uint64_t red[GT / 32][2];
-    uint32_t last[GT / 32], first[GT / 32];  // values at the edges of each warp
-    uint32_t fill[GT == 32 ? 2 : 4];  // to a multiple of 16 bytes
+// Shared memory of one group, for 8 strings per thread: keys, values (in
+// passing between threads, and the final order), indices, and what its warps
+// tell each other.  Values and indices together also hold 64-bit values while
+// a segment is refined.
+struct SegMem {
+    ulonglong2 *key;
+    uint32_t *val, *idx;
+    uint64_t *red;          // two per warp
+    uint32_t *last, *first; // values at the edges of each warp
 };
+constexpr __host__ __device__ size_t seg_bytes(uint32_t threads) {
+    return threads * 8 * 24 + (threads + 31) / 32 * 32;
+}
+__device__ __forceinline__ SegMem seg_mem(unsigned char *base, uint32_t threads) {
+    SegMem m;
+    m.key = reinterpret_cast<ulonglong2 *>(base);
+    m.val = reinterpret_cast<uint32_t *>(base + threads * 128);
+    m.idx = m.val + threads * 8;
+    m.red = reinterpret_cast<uint64_t *>(base + threads * 192);
+    m.last = reinterpret_cast<uint32_t *>(base + threads * 192 + threads / 32 * 16);
+    m.first = m.last + threads / 32;
+    return m;
+}
 
 // Final order: per rank the record's position and, above it, the key bytes
-// it shares with the record before (SEG_TIE: not known from the values).
-// The 12-bit positions of the largest groups leave four bits, so that byte 15
-// counts as not known there.
-template <int GT>
-constexpr uint32_t SEG_ORD_BITS = GT == 512 ? 12 : 11;
-template <int GT>
-constexpr uint32_t SEG_TIE = (1u << (16 - SEG_ORD_BITS<GT>)) - 1;
+// it shares with the record before, up to 14 (SEG_TIE: 15 or not known from
+// the values).
+constexpr uint32_t SEG_ORD_BITS = 12, SEG_TIE = 15;
 
-template <int GT, int ITEMS>
-constexpr int SEG_POS_BITS = (ITEMS == 2 ? 1 : ITEMS == 4 ? 2 : 3) +
-                             (GT == 32 ? 5 : GT == 64 ? 6 : GT == 128 ? 7 : GT == 256 ? 8 : 9);
+// Bits of a position among threads * ITEMS.
+template <int ITEMS, class G>
+__device__ __forceinline__ constexpr uint32_t pos_bits(const G &g) {
+    return g.log2() + (ITEMS == 2 ? 1 : ITEMS == 4 ? 2 : 3);
+}
 
 // Takes the next bits of `mask` (most significant first, at most `need`) off
 // it as one run of adjacent bits: `width` bits that start `lead` bits from the
@@ -2367,13 +2399,12 @@ __device__ __forceinline__ bool next_run(uint64_t &mask, uint32_t need, uint32_t
 // a pass, so at most four passes for the 128 key bits.  mh, ml: the differing
 // bits not used yet.  On return sm.val holds positions only, in (key,
 // position) order; sm.idx is read again from I.
-template <int GT, int ITEMS>
-__device__ __noinline__ void group_refine(SegSmem<GT, ITEMS> &sm, const uint32_t *I, uint32_t len,
-                                          uint64_t mh, uint64_t ml, uint32_t t, uint32_t gi) {
-    constexpr int PB = SEG_POS_BITS<GT, ITEMS>;
-    constexpr uint32_t PM = (1u << PB) - 1, MORE = 64 - 2 * PB;
+template <class G, int ITEMS>
+__device__ __noinline__ void group_refine(G g, SegMem sm, const uint32_t *I, uint32_t len,
+                                          uint64_t mh, uint64_t ml) {
+    const uint32_t PB = pos_bits<ITEMS>(g), PM = (1u << PB) - 1, MORE = 64 - 2 * PB;
     constexpr int GRP = ITEMS < 4 ? ITEMS : 4;
-    const uint32_t lane = t & 31, gw = t >> 5;
+    const uint32_t t = g.t, lane = t & 31, gw = t >> 5;
     uint64_t v[ITEMS];
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
@@ -2384,10 +2415,10 @@ __device__ __noinline__ void group_refine(SegSmem<GT, ITEMS> &sm, const uint32_t
     for (int pass = 0; pass < 5; ++pass) {
         // First rank of each record's tied run (a running maximum of the ranks
         // at which a run starts), in place of the bits used so far.
-        if (lane == 31) sm.red[gw][0] = v[ITEMS - 1];
-        group_sync<GT>(gi);
+        if (lane == 31) sm.red[2 * gw] = v[ITEMS - 1];
+        g.sync();
         uint64_t pv = __shfl_up_sync(0xffffffffu, v[ITEMS - 1], 1);
-        if (lane == 0 && gw) pv = sm.red[gw - 1][0];
+        if (lane == 0 && gw) pv = sm.red[2 * gw - 2];
         uint32_t h = 0;
         bool tie = false;
 #pragma unroll
@@ -2406,11 +2437,11 @@ __device__ __noinline__ void group_refine(SegSmem<GT, ITEMS> &sm, const uint32_t
             const uint32_t y = __shfl_up_sync(0xffffffffu, hm, d);
             if (lane >= (uint32_t)d) hm = max(hm, y);
         }
-        if (lane == 31) sm.red[gw][1] = hm;
+        if (lane == 31) sm.red[2 * gw + 1] = hm;
         hm = __shfl_up_sync(0xffffffffu, hm, 1);
         if (lane == 0) hm = 0;
-        if (!group_any<GT>(tie, gi) || !(mh | ml)) break;
-        for (uint32_t q = 0; q < gw; ++q) hm = max(hm, (uint32_t)sm.red[q][1]);
+        if (!g.any(tie) || !(mh | ml)) break;
+        for (uint32_t q = 0; q < gw; ++q) hm = max(hm, (uint32_t)sm.red[2 * q + 1]);
         uint64_t nh = mh, nl = ml;
 #pragma unroll
         for (int g = 0; g < ITEMS; g += GRP) {
@@ -2446,14 +2477,14 @@ __device__ __noinline__ void group_refine(SegSmem<GT, ITEMS> &sm, const uint32_t
         }
         mh = nh;
         ml = nl;
-        group_net_sort<GT, ITEMS>(v, sm.val, t, gi);
-        group_sync<GT>(gi);
+        group_net_sort<G, ITEMS>(g, v, sm.val, g.threads());
+        g.sync();
     }
-    group_sync<GT>(gi);
+    g.sync();
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) sm.val[t * ITEMS + i] = (uint32_t)v[i] & PM;
-    for (uint32_t e = t; e < len; e += GT) sm.idx[e] = I[e];
-    group_sync<GT>(gi);
+    for (uint32_t e = t; e < len; e += g.threads()) sm.idx[e] = I[e];
+    g.sync();
 }
 
 // Puts the tied runs that are out of full-key order right, each by the thread
@@ -2462,11 +2493,9 @@ __device__ __noinline__ void group_refine(SegSmem<GT, ITEMS> &sm, const uint32_t
 // moved: returns 1, or 2 when one is longer than SEG_FULL; else 0.
 constexpr uint32_t SEG_FIX = 12, SEG_FULL = 64;
 
-template <int GT, int ITEMS>
-__device__ __noinline__ uint32_t group_fix_runs(SegSmem<GT, ITEMS> &sm, uint32_t len, uint32_t t,
-                                                uint32_t gi) {
-    constexpr int PB = SEG_POS_BITS<GT, ITEMS>;
-    constexpr uint32_t PM = (1u << PB) - 1;
+template <class G, int ITEMS>
+__device__ __noinline__ uint32_t group_fix_runs(G g, SegMem sm, uint32_t len) {
+    const uint32_t PB = pos_bits<ITEMS>(g), PM = (1u << PB) - 1, t = g.t;
     auto val = [&](uint32_t r) -> uint32_t & { return sm.val[r]; };
     auto key = [&](uint32_t r) -> Key { return to_key(sm.key[val(r) & PM]); };
     auto tied = [&](uint32_t r) -> bool { return ((val(r) ^ val(r - 1)) >> PB) == 0; };
@@ -2482,7 +2511,7 @@ __device__ __noinline__ uint32_t group_fix_runs(SegSmem<GT, ITEMS> &sm, uint32_t
     uint32_t own = 0, longest = 0;
 #pragma unroll 1
     for (int q = 0; q < ITEMS; ++q) {
-        const uint32_t e = q * GT + t;
+        const uint32_t e = q * g.threads() + t;
         if (e == 0 || e >= len || !tied(e) || !key_lt(key(e), key(e - 1))) continue;
         uint32_t lo, hi;
         extent(e, lo, hi);
@@ -2492,10 +2521,10 @@ __device__ __noinline__ uint32_t group_fix_runs(SegSmem<GT, ITEMS> &sm, uint32_t
         for (uint32_t r = lo + 1; first && r < e; ++r) first = !key_lt(key(r), key(r - 1));
         if (first) own |= 1u << q;
     }
-    if (group_any<GT>(longest > SEG_FIX, gi)) return group_any<GT>(longest > SEG_FULL, gi) ? 2 : 1;
+    if (g.any(longest > SEG_FIX)) return g.any(longest > SEG_FULL) ? 2 : 1;
     for (; own; own &= own - 1) {
         uint32_t lo, hi;
-        extent((__ffs(own) - 1) * GT + t, lo, hi);
+        extent((__ffs(own) - 1) * g.threads() + t, lo, hi);
         for (uint32_t i = lo + 1; i < hi; ++i) {
             const uint32_t x = val(i);
             const Key kx = to_key(sm.key[x & PM]);
@@ -2507,7 +2536,7 @@ __device__ __noinline__ uint32_t group_fix_runs(SegSmem<GT, ITEMS> &sm, uint32_t
             val(j) = x;
         }
     }
-    group_sync<GT>(gi);
+    g.sync();
     return 0;
 }
 
@@ -2515,31 +2544,29 @@ __device__ __noinline__ uint32_t group_fix_runs(SegSmem<GT, ITEMS> &sm, uint32_t
 // positions) whose keys differ in the bits mh, ml (not both 0): writes the
 // final order to sm.val.  Returns whether a run of more than SEG_FULL tied
 // records was out of order.
-template <int GT, int ITEMS>
-__device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint32_t *I,
-                                              uint32_t len, uint64_t mh, uint64_t ml, uint32_t t,
-                                              uint32_t gi) {
-    constexpr int PB = SEG_POS_BITS<GT, ITEMS>;
-    constexpr uint32_t PM = (1u << PB) - 1;
-    const uint32_t lane = t & 31, gw = t >> 5;
+template <class G, int ITEMS>
+__device__ __forceinline__ bool order_segment(const G &g, const SegMem &sm, const uint32_t *I,
+                                              uint32_t len, uint64_t mh, uint64_t ml) {
+    const uint32_t PB = pos_bits<ITEMS>(g), PM = (1u << PB) - 1;
+    const uint32_t t = g.t, lane = t & 31, gw = t >> 5;
     Squeezed<ITEMS> z;
-    squeeze_keys<ITEMS>(z, sm.key, len, GT, t, mh, ml, PB, SEG_TIE<GT>);
+    squeeze_keys<ITEMS>(z, sm.key, len, g.threads(), t, mh, ml, PB, SEG_TIE);
     uint32_t(&v)[ITEMS] = z.v;
-    group_net_sort<GT, ITEMS>(v, sm.val, t, gi);
+    group_net_sort<G, ITEMS>(g, v, sm.val, g.threads());
     // Ties on the squeezed bits must be in full-key order.  A pair out of
     // order that both lie in one thread and tie with nothing else is swapped
     // on the spot; other runs out of order go through shared memory.
     uint32_t pv = __shfl_up_sync(0xffffffffu, v[ITEMS - 1], 1);
     uint32_t nv = __shfl_down_sync(0xffffffffu, v[0], 1);
-    if constexpr (GT > 32) {
+    if constexpr (!G::warp) {
         if (lane == 31) sm.last[gw] = v[ITEMS - 1];
         if (lane == 0) sm.first[gw] = v[0];
-        group_sync<GT>(gi);
+        g.sync();
         if (lane == 0 && gw) pv = sm.last[gw - 1];
-        if (lane == 31 && gw + 1 < GT / 32) nv = sm.first[gw + 1];
+        if (lane == 31 && gw + 1 < g.threads() / 32) nv = sm.first[gw + 1];
     }
     if (t == 0) pv = ~v[0];
-    if (t == GT - 1) nv = ~v[ITEMS - 1];
+    if (t == g.threads() - 1) nv = ~v[ITEMS - 1];
     bool full = false, bad = false;
     uint32_t tie = 0;  // bit i: rank t * ITEMS + i ties with the one before
 #pragma unroll
@@ -2564,14 +2591,14 @@ __device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint
     }
     // (a swap changes no value that another thread compares by more than its
     // position, and those it does belong to a longer run)
-    if (group_any<GT>(bad, gi)) {
+    if (g.any(bad)) {
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) sm.val[t * ITEMS + i] = v[i];
-        group_sync<GT>(gi);
-        const uint32_t run = group_fix_runs<GT, ITEMS>(sm, len, t, gi);
+        g.sync();
+        const uint32_t run = group_fix_runs<G, ITEMS>(g, sm, len);
         if (run) {
             full = run == 2;
-            z.byte_of = SEG_TIE<GT>;  // the values are positions only
+            z.byte_of = SEG_TIE;  // the values are positions only
             // The differing bits not used: m0, m1 of the window, and what
             // lies past the window's 64 bits.
             const uint32_t f = z.f;
@@ -2580,12 +2607,12 @@ __device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint
             const uint64_t rl = f == 0   ? ml
                                 : f < 64 ? (m << (64 - f)) | ((ml << f) >> f)
                                          : m >> (f - 64);
-            group_refine<GT, ITEMS>(sm, I, len, rh, rl, t, gi);
+            group_refine<G, ITEMS>(g, sm, I, len, rh, rl);
         }
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) v[i] = sm.val[t * ITEMS + i];
         if (t) pv = sm.val[t * ITEMS - 1];
-        group_sync<GT>(gi);
+        g.sync();
     }
     // The order, with the bytes shared with the neighbour where the first
     // differing squeezed bit tells (no NUL can precede it in either key).
@@ -2594,7 +2621,7 @@ __device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint
     for (int i = 0; i < ITEMS; ++i) {
         const uint32_t x = (v[i] ^ (i ? v[i ? i - 1 : 0] : pv)) >> PB;
         const uint32_t l = __shfl_sync(0xffffffffu, z.byte_of, __clz(x) + z.used - 32);
-        const uint32_t h = l * (1u << SEG_ORD_BITS<GT>) + (v[i] & PM);
+        const uint32_t h = l * (1u << SEG_ORD_BITS) + (v[i] & PM);
         if (i & 1)
             o[i / 2] += h * 65536u;
         else
@@ -2609,13 +2636,13 @@ __device__ __forceinline__ bool order_segment(SegSmem<GT, ITEMS> &sm, const uint
     return full;
 }
 
-// Sorts segment s (at most 8 * GT strings) with the GT threads of group gi,
-// thread t.  Returns whether a run of more than SEG_FULL tied records was out
-// of order.  One warp (GT = 32) orders up to 64 or 128 strings with 2 or 4
-// per thread.
-template <int GT>
-__device__ __forceinline__ bool sort_segment(const SortArgs &a, const Seg &s, SegSmem<GT, 8> &sm,
-                                             uint32_t t, uint32_t gi, Seg *N, Counters *c) {
+// Sorts segment s (at most 8 strings per thread) with a group of threads.
+// Returns whether a run of more than SEG_FULL tied records was out of order.
+// One warp orders up to 64 or 128 strings with 2 or 4 per thread.
+template <class G>
+__device__ __forceinline__ bool sort_segment(const G &g, const SortArgs &a, const Seg &s,
+                                             const SegMem &sm, Seg *N, Counters *c) {
+    const uint32_t t = g.t, GT = g.threads();
     constexpr int GRP = 4;  // strings at a time
     const uint32_t lane = t & 31, gw = t >> 5;
     const int b = s.flags & SEG_BUF1;
@@ -2627,7 +2654,7 @@ __device__ __forceinline__ bool sort_segment(const SortArgs &a, const Seg &s, Se
         const ulonglong2 *K = a.keyb(b) + s.start;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const uint32_t e = q * GT + t;
+            const uint32_t e = q * g.threads() + t;
             if (e < s.len) {
                 cp_async16(sm.key + e, K + e);
                 cp_async4(sm.idx + e, I + e);
@@ -2649,14 +2676,14 @@ __device__ __forceinline__ bool sort_segment(const SortArgs &a, const Seg &s, Se
                 }
         }
     }
-    group_sync<GT>(gi);
+    g.sync();
     // The bits in which the keys differ.
     uint64_t mh = 0, ml = 0;
     {
         const Key k0 = to_key(sm.key[0]);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const uint32_t e = q * GT + t;
+            const uint32_t e = q * g.threads() + t;
             if (e < s.len) {
                 const Key k = to_key(sm.key[e]);
                 mh |= k.hi ^ k0.hi;
@@ -2665,38 +2692,35 @@ __device__ __forceinline__ bool sort_segment(const SortArgs &a, const Seg &s, Se
         }
         mh = warp_or64(mh);
         ml = warp_or64(ml);
-        if constexpr (GT > 32) {
+        if constexpr (!G::warp) {
             if (lane == 0) {
-                sm.red[gw][0] = mh;
-                sm.red[gw][1] = ml;
+                sm.red[2 * gw] = mh;
+                sm.red[2 * gw + 1] = ml;
             }
-            group_sync<GT>(gi);
-#pragma unroll
-            for (int q = 0; q < GT / 32; ++q) {
-                mh |= sm.red[q][0];
-                ml |= sm.red[q][1];
+            g.sync();
+            for (uint32_t q = 0; q < GT / 32; ++q) {
+                mh |= sm.red[2 * q];
+                ml |= sm.red[2 * q + 1];
             }
         }
     }
     bool full = false;
     if (mh | ml) {
-        if (GT == 32 && s.len <= 64)
-            full = order_segment<GT, 2>(reinterpret_cast<SegSmem<GT, 2> &>(sm), I, s.len, mh, ml,
-                                        t, gi);
-        else if (GT == 32 && s.len <= 128)
-            full = order_segment<GT, 4>(reinterpret_cast<SegSmem<GT, 4> &>(sm), I, s.len, mh, ml,
-                                        t, gi);
+        if (G::warp && s.len <= 64)
+            full = order_segment<G, G::warp ? 2 : 8>(g, sm, I, s.len, mh, ml);
+        else if (G::warp && s.len <= 128)
+            full = order_segment<G, G::warp ? 4 : 8>(g, sm, I, s.len, mh, ml);
         else
-            full = order_segment<GT, 8>(sm, I, s.len, mh, ml, t, gi);
+            full = order_segment<G, 8>(g, sm, I, s.len, mh, ml);
     } else {  // all keys equal: position order
         for (uint32_t e = t; e < s.len; e += GT)
-            reinterpret_cast<uint16_t *>(sm.val)[e] = (uint16_t)(SEG_TIE<GT> << SEG_ORD_BITS<GT> | e);
+            reinterpret_cast<uint16_t *>(sm.val)[e] = (uint16_t)(SEG_TIE << SEG_ORD_BITS | e);
     }
-    group_sync<GT>(gi);
+    g.sync();
     // Results in rank order: indices, LCPs, first and last key, next-round
     // runs.  Ties read both keys.
     const uint16_t *ord = reinterpret_cast<const uint16_t *>(sm.val);
-    constexpr uint32_t OM = (1u << SEG_ORD_BITS<GT>) - 1;
+    constexpr uint32_t OM = (1u << SEG_ORD_BITS) - 1;
     auto key_at = [&](uint32_t r) -> Key { return to_key(sm.key[ord[r] & OM]); };
     uint32_t *oi = a.idx[0] + s.start + t, *ol = a.lcp + s.start + t;
     if (t < 2) {
@@ -2711,8 +2735,8 @@ __device__ __forceinline__ bool sort_segment(const SortArgs &a, const Seg &s, Se
         if (on) oi[e0] = sm.idx[w & OM];
         bool cont = false;  // goes on a run of equal keys that do not end
         if (on && e) {
-            uint32_t l = w >> SEG_ORD_BITS<GT>;
-            if (l == SEG_TIE<GT>) {
+            uint32_t l = w >> SEG_ORD_BITS;
+            if (l == SEG_TIE) {
                 const Key k = to_key(sm.key[w & OM]), kp = key_at(e - 1);
                 const bool same = key_eq(kp, k);
                 cont = same && !key_is_end(k);
@@ -2744,41 +2768,87 @@ __device__ __forceinline__ bool sort_segment(const SortArgs &a, const Seg &s, Se
             emit_next_warp(N, c, tail, s.start + lo, e - lo + 1, s.depth + KEY_BYTES);
         }
     }
-    group_sync<GT>(gi);
+    g.sync();
     return full;
 }
 
-// GT = 32 takes the segments of 33..256 strings and sorts each with 2, 4 or 8
-// strings per thread; 64, 128, 256 and 512 take one size class each.
-template <int GT>
-constexpr int SEG_CTA = GT < SMALL_THREADS ? SMALL_THREADS : GT;  // threads of a CTA
-template <int GT>
-constexpr size_t SEG_SMEM = (SEG_CTA<GT> / GT) * sizeof(SegSmem<GT, 8>);
-
-template <int GT>
-__global__ void __launch_bounds__(SEG_CTA<GT>, 1024 / SEG_CTA<GT>)
-    k_segsort(SortArgs a, const Seg *__restrict__ T0, Span sp, Seg *N, Counters *c) {
-    constexpr uint32_t G = GT < SMALL_THREADS ? SMALL_THREADS / GT : 1;
-    extern __shared__ __align__(16) unsigned char seg_smem[];
-    const uint32_t lo = count_of(sp.lo);
-    const Seg *__restrict__ T = T0 + lo;
-    const uint32_t nT = count_of(sp.hi) - lo;
-    const uint32_t gi = threadIdx.x / GT, t = threadIdx.x % GT;
-    auto &sm = reinterpret_cast<SegSmem<GT, 8> *>(seg_smem)[gi];
+// Sorts segments lo + g, g = first, first + step, .. < nT of list T with the
+// thread group grp.
+template <class G>
+__device__ __forceinline__ void sort_list(const G &grp, const SortArgs &a,
+                                          const Seg *__restrict__ T, uint32_t nT, uint32_t first,
+                                          uint32_t step, const SegMem &sm, Seg *N, Counters *c) {
     unsigned long long fresh = 0, keyed = 0, full = 0;
-    for (uint32_t g = blockIdx.x * G + gi; g < nT; g += gridDim.x * G) {
+    for (uint32_t g = first; g < nT; g += step) {
         const Seg s = T[g];
         if (s.flags & SEG_KEYS)
             keyed += s.len;
         else
             fresh += s.len;
-        if (sort_segment<GT>(a, s, sm, t, gi, N, c)) full += s.len;
+        if (sort_segment(grp, a, s, sm, N, c)) full += s.len;
     }
-    if (t == 0 && (fresh | keyed)) {
-        atomicAdd(GT == 32 ? &c->warp8_fresh : &c->block_fresh, fresh);
-        atomicAdd(GT == 32 ? &c->warp8_keyed : &c->block_keyed, keyed);
+    if (grp.t == 0 && (fresh | keyed)) {
+        atomicAdd(G::warp ? &c->warp8_fresh : &c->block_fresh, fresh);
+        atomicAdd(G::warp ? &c->warp8_keyed : &c->block_keyed, keyed);
         if (full) atomicAdd(&c->full_sorted, full);
     }
+}
+
+// Segments of 33..256 strings: one warp each.
+constexpr size_t WARPSORT_SMEM = SMALL_THREADS / 32 * seg_bytes(32);
+
+__global__ void __launch_bounds__(SMALL_THREADS, 4)
+    k_warpsort(SortArgs a, const Seg *__restrict__ T0, Span sp, Seg *N, Counters *c) {
+    extern __shared__ __align__(16) unsigned char seg_smem[];
+    const uint32_t lo = count_of(sp.lo), w = threadIdx.x / 32, per = SMALL_THREADS / 32;
+    sort_list(WarpGroup{threadIdx.x & 31}, a, T0 + lo, count_of(sp.hi) - lo, blockIdx.x * per + w,
+              gridDim.x * per, seg_mem(seg_smem + w * seg_bytes(32), 32), N, c);
+}
+
+// Classes with few segments, in one launch: class k's segments (up to 512 << k
+// strings, 64 << k threads each) are taken by CTAs cta[k] .. cta[k + 1] - 1 of
+// SEG_CTA threads, 8 >> k segments side by side.  Such a launch spends most of
+// its time fetching instructions, which the classes share here, and a level's
+// classes run side by side: 3 M URLs 1.08 -> 0.94 ms, 200 small instances 201
+// -> 171 us.
+constexpr int SEG_CTA = 512;
+constexpr size_t SEG_SMEM = SEG_CTA / 64 * seg_bytes(64);
+static_assert(SEG_SMEM >= seg_bytes(512) && SEG_SMEM >= 2 * seg_bytes(256), "group slots");
+
+__global__ void __launch_bounds__(SEG_CTA, 2)
+    k_segsort(SortArgs a, SmallWork wk, Seg *N, Counters *c) {
+    extern __shared__ __align__(16) unsigned char seg_smem[];
+    uint32_t k = 0;
+    while (k + 1 < SMALL_CLASSES && blockIdx.x >= wk.cta[k + 1]) ++k;
+    const uint32_t log2_threads = 6 + k, per = SEG_CTA >> log2_threads;
+    const uint32_t lo = count_of(wk.span[k].lo), nT = count_of(wk.span[k].hi) - lo;
+    const Seg *__restrict__ T = wk.list.s[k] + lo;
+    const uint32_t gi = threadIdx.x >> log2_threads;
+    const CtaGroup<> grp{threadIdx.x & ((1u << log2_threads) - 1), log2_threads, 1 + gi};
+    const SegMem sm = seg_mem(seg_smem + gi * seg_bytes(grp.threads()), grp.threads());
+    sort_list(grp, a, T, nT, (blockIdx.x - wk.cta[k]) * per + gi,
+              (wk.cta[k + 1] - wk.cta[k]) * per, sm, N, c);
+}
+
+// A class with many segments: its group size is a constant (fewer
+// instructions: 69 M batched strings 5.80 -> 5.53 ms against the shared
+// launch).  CTAs of 512 threads, although four of 256 per SM sort alone
+// faster (5.40 ms): these sorts run beside the partition, whose CTAs have 512
+// threads and whose next kernel waits for room on every SM; small CTAs keep
+// filling each half that comes free (50 M URLs 7.33 ms with 512, 7.86 with
+// 256).
+template <int K>
+constexpr size_t CLASS_SMEM = SEG_CTA / (64 << K) * seg_bytes(64 << K);
+
+template <int K>
+__global__ void __launch_bounds__(SEG_CTA, 2)
+    k_segsort_class(SortArgs a, const Seg *__restrict__ T0, Span sp, Seg *N, Counters *c) {
+    extern __shared__ __align__(16) unsigned char seg_smem[];
+    constexpr uint32_t GT = 64u << K, per = SEG_CTA / GT;
+    const uint32_t lo = count_of(sp.lo), gi = threadIdx.x / GT;
+    const CtaGroup<6 + K> grp{threadIdx.x % GT, 6 + K, 1 + gi};
+    sort_list(grp, a, T0 + lo, count_of(sp.hi) - lo, blockIdx.x * per + gi, gridDim.x * per,
+              seg_mem(seg_smem + gi * seg_bytes(GT), GT), N, c);
 }
 
 // ---- equality buckets: work items of up to EQ_TILE strings ------------------
@@ -2854,7 +2924,7 @@ __global__ void k_round_end(SortArgs a, const uint2 *__restrict__ B, const Seg *
 // or the TINY_ROUNDS-th, is left to the general loop.
 constexpr uint32_t TINY_SEGMENTS = 128;
 constexpr size_t TINY_SMEM =
-    SEG_SMEM<256> > SEG_SMEM<32> ? SEG_SMEM<256> : SEG_SMEM<32>;
+    seg_bytes(SMALL_THREADS) > WARPSORT_SMEM ? seg_bytes(SMALL_THREADS) : WARPSORT_SMEM;
 
 __global__ void __launch_bounds__(SMALL_THREADS, 1)
     k_tiny(SortArgs a, Seg *A, Seg *B, RoundCounters *rc, Publish pub) {
@@ -2886,8 +2956,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1)
             for (uint32_t g = 0; g < n_cur; ++g) {
                 const Seg s = A[g];
                 if (s.len <= (uint32_t)WARP8_CAP) continue;
-                const bool full = sort_segment<256>(
-                    a, s, *reinterpret_cast<SegSmem<256, 8> *>(seg_smem), t, 0, B, c);
+                const bool full = sort_segment(CtaGroup<8>{t, 8, 1}, a, s,
+                                               seg_mem(seg_smem, SMALL_THREADS), B, c);
                 if (t == 0) {
                     c->block_fresh += s.len;
                     if (full) c->full_sorted += s.len;
@@ -2903,8 +2973,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1)
                 deep += warp1_group<32>(a, s, lane, B, c);
                 if (lane == 0) atomicAdd(&c->warp1_fresh, (unsigned long long)s.len);
             } else {
-                const bool full = sort_segment<32>(
-                    a, s, reinterpret_cast<SegSmem<32, 8> *>(seg_smem)[w], lane, 0, B, c);
+                const bool full = sort_segment(WarpGroup{lane}, a, s,
+                                               seg_mem(seg_smem + w * seg_bytes(32), 32), B, c);
                 if (lane == 0) {
                     atomicAdd(&c->warp8_fresh, (unsigned long long)s.len);
                     if (full) atomicAdd(&c->full_sorted, (unsigned long long)s.len);
@@ -3179,16 +3249,17 @@ static void set_smem_attrs() {
     cudaFuncSetAttribute(k_scatter2, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(Scatter2Smem));
     cudaFuncSetAttribute(k_tiny, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TINY_SMEM);
-    cudaFuncSetAttribute(k_segsort<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)SEG_SMEM<32>);
-    cudaFuncSetAttribute(k_segsort<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)SEG_SMEM<64>);
-    cudaFuncSetAttribute(k_segsort<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)SEG_SMEM<128>);
-    cudaFuncSetAttribute(k_segsort<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)SEG_SMEM<256>);
-    cudaFuncSetAttribute(k_segsort<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)SEG_SMEM<512>);
+    cudaFuncSetAttribute(k_warpsort, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)WARPSORT_SMEM);
+    cudaFuncSetAttribute(k_segsort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SEG_SMEM);
+    cudaFuncSetAttribute(k_segsort_class<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)CLASS_SMEM<0>);
+    cudaFuncSetAttribute(k_segsort_class<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)CLASS_SMEM<1>);
+    cudaFuncSetAttribute(k_segsort_class<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)CLASS_SMEM<2>);
+    cudaFuncSetAttribute(k_segsort_class<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)CLASS_SMEM<3>);
     done.fetch_or(bit, std::memory_order_release);
 }
 
@@ -3354,22 +3425,23 @@ void launch_count(const SortArgs &a, const Seg *L, Count nL, const uint32_t *til
 
 void launch_scatter(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
                     const ulonglong2 *spl, const uint32_t *nspl, const uint16_t *tbl,
-                    const uint32_t *cm_base, const uint32_t *cm_scan, int grid, cudaStream_t st) {
+                    const uint32_t *cm_base, const uint32_t *cm_scan, Counters *c, int grid,
+                    cudaStream_t st) {
     if (!nL.dev && !nL.host) return;
     set_smem_attrs();
     if (a.scatter_staged_idx == 2) {
         k_scatter<true><<<grid, SCATTER_THREADS, sizeof(ScatterSmem), st>>>(
-            a, L, nL, tile_base, nspl, cm_base, cm_scan);
+            a, L, nL, tile_base, nspl, cm_base, cm_scan, c);
         return;
     }
     if (a.scatter_staged_idx) {
         // three CTAs per SM where k_scatter fits two (grid: two per SM)
         k_scatter2<<<grid / 2 * 3, SCATTER_THREADS, sizeof(Scatter2Smem), st>>>(
-            a, L, nL, tile_base, nspl, cm_base, cm_scan);
+            a, L, nL, tile_base, nspl, cm_base, cm_scan, c);
         return;
     }
     k_scatter<false><<<grid, SCATTER_THREADS, sizeof(ScatterSmem), st>>>(
-        a, L, nL, tile_base, nspl, cm_base, cm_scan);
+        a, L, nL, tile_base, nspl, cm_base, cm_scan, c);
 }
 
 void launch_emit(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
@@ -3397,21 +3469,36 @@ void launch_warp8(const SortArgs &a, const Seg *W8, Span sp, Seg *N, Counters *c
                   cudaStream_t st) {
     if (span_empty(sp) || grid <= 0) return;
     set_smem_attrs();
-    k_segsort<32><<<grid, SMALL_THREADS, SEG_SMEM<32>, st>>>(a, W8, sp, N, c);
+    k_warpsort<<<grid, SMALL_THREADS, WARPSORT_SMEM, st>>>(a, W8, sp, N, c);
 }
 
-void launch_block(const SortArgs &a, const Seg *S, Span sp, int cls, Seg *N, Counters *c,
-                  int grid, cudaStream_t st) {
-    if (span_empty(sp) || grid <= 0) return;
+void launch_block(const SortArgs &a, const SmallWork &wk, Seg *N, Counters *c, cudaStream_t st) {
+    const uint32_t grid = wk.cta[SMALL_CLASSES];
+    if (!grid) return;
+    set_smem_attrs();
+    k_segsort<<<grid, SEG_CTA, SEG_SMEM, st>>>(a, wk, N, c);
+}
+
+template <int K>
+static void class_launch(const SortArgs &a, const Seg *S, Span sp, Seg *N, Counters *c,
+                         cudaStream_t st) {
+    constexpr uint32_t per = SEG_CTA / (64 << K);
+    k_segsort_class<K><<<cdiv(sp.hi.host - sp.lo.host, per), SEG_CTA, CLASS_SMEM<K>, st>>>(
+        a, S, sp, N, c);
+}
+
+void launch_block_class(const SortArgs &a, const Seg *S, Span sp, int cls, Seg *N, Counters *c,
+                        cudaStream_t st) {
+    if (span_empty(sp)) return;
     set_smem_attrs();
     if (cls == 0)
-        k_segsort<64><<<grid, SMALL_THREADS, SEG_SMEM<64>, st>>>(a, S, sp, N, c);
+        class_launch<0>(a, S, sp, N, c, st);
     else if (cls == 1)
-        k_segsort<128><<<grid, SMALL_THREADS, SEG_SMEM<128>, st>>>(a, S, sp, N, c);
+        class_launch<1>(a, S, sp, N, c, st);
     else if (cls == 2)
-        k_segsort<256><<<grid, SMALL_THREADS, SEG_SMEM<256>, st>>>(a, S, sp, N, c);
+        class_launch<2>(a, S, sp, N, c, st);
     else
-        k_segsort<512><<<grid, SEG_CTA<512>, SEG_SMEM<512>, st>>>(a, S, sp, N, c);
+        class_launch<3>(a, S, sp, N, c, st);
 }
 
 void launch_equal(const SortArgs &a, const Seg *E, Span sp, Seg *N, Counters *c, int grid,
