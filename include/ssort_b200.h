@@ -256,9 +256,9 @@ int ssort_get_stats(const ssort_ctx *ctx, ssort_stats *out);
                                        the next round; 0: every run waits for the next round */
 #define SSORT_PARAM_BLOCK_PREFETCH 6 /* 0 or 1; no effect (the CTA sort always copies its
                                         records asynchronously) */
-#define SSORT_PARAM_MATCH_VOTE 13    /* 1: the partition's count kernel finds the lanes of a
-                                        warp that share a bucket with one ballot per
-                                        bucket-id bit; 0 (default): with __match_any_sync */
+#define SSORT_PARAM_MATCH_VOTE 13    /* 0 or 1; no effect (the partition's count kernel finds
+                                        the lanes that share a bucket with the match unit
+                                        and with ballots side by side) */
 #define SSORT_PARAM_SCAN 15          /* 1 (default): the partition's count-matrix scan runs
                                         in one pass with decoupled look-back (tiles in
                                         ticket order add up their predecessors' published

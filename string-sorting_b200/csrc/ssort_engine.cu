@@ -365,7 +365,6 @@ int ssort_ctx::run_ws(const uint8_t *arena_p, uint64_t arena_bytes, const void *
     a.warp1_deep = warp1_deep;
     a.l2_prefetch = l2_prefetch ? 1u : 0u;
     a.scatter_staged_idx = scatter_variant;
-    a.match_vote = match_vote ? 1u : 0u;
     a.max_splitters = (1u << (digit_bits - 1)) - 1;
     std::copy(std::begin(class_targets), std::end(class_targets), std::begin(a.target_by_class));
     a.key2 = key2;
@@ -979,8 +978,7 @@ int ssort_set_param(ssort_ctx *ctx, int param, int64_t value) {
             return SSORT_OK;  // one warp-level sort is left: nothing to choose
         case SSORT_PARAM_MATCH_VOTE:
             if (value != 0 && value != 1) return fail(SSORT_EINVAL, "match_vote must be 0 or 1");
-            ctx->match_vote = value != 0;
-            return SSORT_OK;
+            return SSORT_OK;  // the count kernel uses both ways side by side
         case SSORT_PARAM_BLOCK_LEAN:
             if (value < 0 || value > 2) return fail(SSORT_EINVAL, "block_lean must be 0, 1 or 2");
             return SSORT_OK;  // one finish is left: nothing to choose

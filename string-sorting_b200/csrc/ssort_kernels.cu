@@ -149,31 +149,20 @@ __device__ __forceinline__ uint32_t next_pow2(uint32_t x) {
     return x <= 1 ? 1u : 1u << (32 - __clz(x - 1));
 }
 
-// Largest i in [0, n) with base[i] <= t (base ascending, base[0] = 0).
+// Largest i in [0, n) with base[i] <= t (base ascending, base[0] = 0), found by
+// a whole warp together: 32 probes a step, so two dependent reads for up to
+// 1024 segments where a binary search takes ten.
 __device__ __forceinline__ uint32_t find_seg(const uint32_t *base, uint32_t n, uint32_t t) {
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(base + mid) <= t)
-            lo = mid;
-        else
-            hi = mid;
+    uint32_t lo = 0;
+    while (n > 1) {
+        const uint32_t step = (n + 31) / 32, i = (threadIdx.x & 31) * step;
+        const uint32_t below =
+            __ballot_sync(0xffffffffu, i < n && __ldg(base + lo + i) <= t);  // a prefix, lane 0 set
+        const uint32_t at = (31 - __clz(below)) * step;
+        lo += at;
+        n = min(step, n - at);
     }
     return lo;
-}
-
-// Lanes of the warp whose value v equals this lane's, for values below
-// 2^bits: one ballot per bit (lanes agreeing on every bit are the peers).
-// The same set as __match_any_sync(full, v), from vote and logic
-// instructions instead of the match unit.  Warp-collective; bits is
-// warp-uniform.
-__device__ __forceinline__ uint32_t match_bits(uint32_t v, uint32_t bits) {
-    uint32_t peers = 0xffffffffu;
-    for (uint32_t k = 0; k < bits; ++k) {
-        const uint32_t m = __ballot_sync(0xffffffffu, (v >> k) & 1u);
-        peers &= ((v >> k) & 1u) ? m : ~m;
-    }
-    return peers;
 }
 
 // Warp-aggregated append to a list counter: all 32 lanes call it together;
@@ -221,42 +210,19 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
     return v;
 }
 
-// Bucket of `key` among u sorted distinct splitters s[0..u): range bucket 2j
-// holds s[j-1] < key < s[j], equality bucket 2j+1 holds key == s[j].  Found
-// through the lookup table T: splitters share their first f bits; T[w] counts
-// the splitters whose next TBL_BITS bits are below w, so a key strictly
-// between the first and last splitter (and hence sharing those f bits) only
-// needs a search among the splitters with its own window.
 __device__ __forceinline__ uint64_t window64(const Key &k, uint32_t f);
 
 __device__ __forceinline__ uint32_t window_bits(const Key &k, uint32_t f) {
     return (uint32_t)(window64(k, f) >> (64 - TBL_BITS));
 }
 
-__device__ __forceinline__ uint32_t classify_tbl(const ulonglong2 *s, const uint16_t *T,
-                                                 uint32_t u, uint32_t f, const Key &key) {
-    const Key s0 = to_key(s[0]), sl = to_key(s[u - 1]);
-    if (key_lt(key, s0)) return 0;
-    if (key_eq(key, s0)) return 1;
-    if (key_lt(sl, key)) return 2 * u;
-    if (key_eq(key, sl)) return 2 * u - 1;
-    const uint32_t w = window_bits(key, f);
-    uint32_t lo = T[w], hi = T[w + 1];
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (key_lt(to_key(s[mid]), key))
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    return (lo < u && key_eq(to_key(s[lo]), key)) ? 2 * lo + 1 : 2 * lo;
-}
-
 // Asks the memory system to stream the bytes of [p, p + bytes) into L2 (a
 // TMA bulk prefetch: no registers, nothing to wait for).  The start is
 // rounded up and the end down to 16-byte boundaries, so nothing outside the
-// range is touched; ranges are issued in pieces of at most 1 MB.
+// range is touched; ranges are issued in pieces of at most 1 MB.  Called by
+// the CTA's first warp; its first thread asks.
 __device__ __forceinline__ void prefetch_l2(const void *p, uint64_t bytes) {
+    if (threadIdx.x != 0) return;
     uint64_t a = ((uint64_t)(uintptr_t)p + 15) & ~15ull;
     const uint64_t e = ((uint64_t)(uintptr_t)p + bytes) & ~15ull;
     while (a < e) {
@@ -1402,27 +1368,104 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
 }
 
 // ---- partition count: per-tile bucket histograms ---------------------------
-// Each warp counts its own 512 consecutive keys into a private row, one
-// shared-memory update per distinct bucket per 32 keys (__match_any_sync).
-// Shared memory of the partition kernels.
+// Each warp counts its own 256 consecutive keys into a private row, one
+// shared-memory update per distinct bucket per 32 keys.  Bound by issued
+// instructions (ALU pipe) and by the latency of its phases.  Measured, launches
+// of one sort: 100 M words 1.78 -> 1.66 ms, 50 M URLs 0.79 -> 0.73 ms (1.33 ->
+// 1.19 ms where it gathers), 69 M batched strings 0.95 -> 0.81 ms, against
+// 16-byte compares with both end splitters, all ranks by the match unit and
+// two CTAs per SM.
+// Shared memory of the count kernel.
 struct PartSmem {
-    ulonglong2 spl[SPL_STRIDE];              // the segment's splitters
-    uint16_t tbl[TBL_N + 8];                 // splitter lookup table
-    uint16_t cnt[PART_WARPS][NB_MAX + 1];    // per-warp bucket counters
-    uint32_t gbase[NB_MAX + 1];              // tile's global base per bucket
+    ulonglong2 spl[SPL_STRIDE];            // the segment's splitters
+    uint64_t win[SPL_STRIDE];              // their 64 bits after the common prefix
+    uint32_t tbl[TBL_N];                   // per window value: first and end splitter
+    uint16_t cnt[PART_WARPS][NB_MAX + 1];  // per-warp bucket counters
 };
 
-// Splitters (and the lookup table when f < 128) of segment si into smem.
+// Keys of a lane (of PART_ITEMS) worked on at a time, and how many of these the
+// match unit ranks.  Two at a time let three CTAs share an SM (40 registers);
+// while gathering, four random reads in flight per lane and two CTAs are
+// better.
+template <bool GATHER>
+constexpr int PART_HALF = GATHER ? 4 : 2;
+template <bool GATHER>
+constexpr int MATCH_ITEMS = GATHER ? 2 : 1;
+template <bool GATHER>
+constexpr int COUNT_CTAS = GATHER ? 2 : 3;
+
+// What classification needs of a segment besides shared memory: its u
+// splitters share their first f bits, the bits (ph, pl) under the mask
+// (mh, ml).
+struct Splitters {
+    uint32_t u, f;
+    uint64_t ph, pl, mh, ml;
+};
+
+// Splitters, their windows and (when f < 128) the lookup table of segment si.
 __device__ __forceinline__ void load_splitters(PartSmem &sm, const ulonglong2 *__restrict__ spl,
                                                const uint16_t *__restrict__ tbl, uint32_t si,
                                                uint32_t u, uint32_t f) {
-    for (uint32_t q = threadIdx.x; q < u; q += PART_THREADS)
-        sm.spl[q] = spl[(uint64_t)si * SPL_STRIDE + q];
-    if (f < 128) {
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(tbl + (uint64_t)si * TBL_STRIDE);
-        uint32_t *dst = reinterpret_cast<uint32_t *>(sm.tbl);
-        for (uint32_t q = threadIdx.x; q < (TBL_N + 2) / 2; q += PART_THREADS) dst[q] = src[q];
+    for (uint32_t q = threadIdx.x; q < u; q += PART_THREADS) {
+        const ulonglong2 x = spl[(uint64_t)si * SPL_STRIDE + q];
+        sm.spl[q] = x;
+        if (f < 128) sm.win[q] = window64(to_key(x), f);
     }
+    if (f < 128) {
+        const uint16_t *src = tbl + (uint64_t)si * TBL_STRIDE;
+        for (uint32_t q = threadIdx.x * 8; q < TBL_N; q += PART_THREADS * 8) {
+            const uint4 x = *reinterpret_cast<const uint4 *>(src + q);
+            const uint32_t e = src[q + 8];
+            uint4 *d = reinterpret_cast<uint4 *>(sm.tbl + q);
+            // entry i: T[i] | T[i + 1] << 16
+            d[0] = make_uint4(x.x, __funnelshift_r(x.x, x.y, 16), x.y,
+                              __funnelshift_r(x.y, x.z, 16));
+            d[1] = make_uint4(x.z, __funnelshift_r(x.z, x.w, 16), x.w,
+                              __funnelshift_r(x.w, e, 16));
+        }
+    }
+}
+
+// Bucket of `key` among the u sorted distinct splitters s[0..u): range bucket
+// 2j holds s[j-1] < key < s[j], equality bucket 2j+1 holds key == s[j].  A key
+// without the splitters' common prefix lies before or after all of them.
+// Any other is placed by the 64 bits after the prefix: the table bounds the
+// splitters with its first TBL_BITS bits, and full keys are compared only
+// with splitters whose 64 bits tie.
+__device__ __forceinline__ uint32_t classify(const PartSmem &sm, const Splitters &p,
+                                             const Key &key) {
+    uint64_t off = (key.hi ^ p.ph) & p.mh;
+    if (p.f > 64) off |= (key.lo ^ p.pl) & p.ml;  // the same branch for the whole CTA
+    if (off) return key_lt(key, Key{p.ph, p.pl}) ? 0 : 2 * p.u;
+    if (p.f >= 128) return 1;  // one splitter, all of whose bits are the prefix
+    // the 64 bits from bit f on, as two shifts across 32-bit words
+    const uint64_t top = p.f < 64 ? key.hi : key.lo, next = p.f < 64 ? key.lo : 0;
+    const uint32_t w0 = (uint32_t)(top >> 32), w1 = (uint32_t)top, w2 = (uint32_t)(next >> 32),
+                   w3 = (uint32_t)next;
+    const uint32_t wh = p.f & 32 ? __funnelshift_l(w2, w1, p.f) : __funnelshift_l(w1, w0, p.f);
+    const uint32_t wl = p.f & 32 ? __funnelshift_l(w3, w2, p.f) : __funnelshift_l(w2, w1, p.f);
+    const uint64_t w = (uint64_t)wh << 32 | wl;
+    const uint32_t r = sm.tbl[wh >> (32 - TBL_BITS)];
+    uint32_t lo = r & 0xFFFF, hi = r >> 16;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (sm.win[mid] < w)
+            lo = mid + 1;
+        else
+            hi = mid;
+    }
+    hi = r >> 16;
+    if (lo < hi && sm.win[lo] == w) {
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (key_lt(to_key(sm.spl[mid]), key))
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        if (lo < p.u && key_eq(to_key(sm.spl[lo]), key)) return 2 * lo + 1;
+    }
+    return 2 * lo;
 }
 
 // Tiles for a CTA of the partition kernels, in ticket order: the first is its
@@ -1452,7 +1495,7 @@ struct TileQueue {
 // arena through idx and offsets and stored to the key buffer here, so the
 // key gather's random arena reads overlap the classification work.
 template <bool GATHER>
-__global__ void __launch_bounds__(PART_THREADS, 2) k_count(SortArgs a, const Seg *__restrict__ L,
+__global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(SortArgs a, const Seg *__restrict__ L,
                                                         Count cnt,
                                                         const uint32_t *__restrict__ tile_base,
                                                         const ulonglong2 *__restrict__ spl,
@@ -1476,7 +1519,7 @@ __global__ void __launch_bounds__(PART_THREADS, 2) k_count(SortArgs a, const Seg
         const Seg s = L[si];
         const uint32_t u = nspl[si] & 0xFFFF, f = nspl[si] >> 16, nb = 2 * u + 1;
         const uint32_t bbits = 32 - __clz(nb);  // bucket ids are 0..nb
-        if (a.l2_prefetch && threadIdx.x == 0 && t + gridDim.x < total_tiles) {
+        if (a.l2_prefetch && threadIdx.x < 32 && t + gridDim.x < total_tiles) {
             // the keys (or, when gathering, the indices) of this CTA's next tile
             const uint32_t t2 = t + gridDim.x;
             const uint32_t s2i = find_seg(tile_base, nL, t2);
@@ -1493,103 +1536,123 @@ __global__ void __launch_bounds__(PART_THREADS, 2) k_count(SortArgs a, const Seg
             loaded = si;
         }
         {
-            uint32_t *h32 = reinterpret_cast<uint32_t *>(&hist[0][0]);
-            for (uint32_t q = threadIdx.x; q < PART_WARPS * (NB_MAX + 1) / 2; q += PART_THREADS)
-                h32[q] = 0;
+            uint4 *h = reinterpret_cast<uint4 *>(&hist[0][0]);
+            for (uint32_t q = threadIdx.x; q < PART_WARPS * (NB_MAX + 1) / 8; q += PART_THREADS)
+                h[q] = make_uint4(0, 0, 0, 0);
         }
         __syncthreads();
+        Splitters sp{u, f, 0, 0, 0, 0};
+        sp.mh = f >= 64 ? ~0ull : f ? ~0ull << (64 - f) : 0ull;
+        sp.ml = f >= 128 ? ~0ull : f > 64 ? ~0ull << (128 - f) : 0ull;
+        sp.ph = sm.spl[0].x & sp.mh;
+        sp.pl = sm.spl[0].y & sp.ml;
         const uint32_t tl = t - tile_base[si];
         const uint32_t nt = tile_base[si + 1] - tile_base[si];
         const uint32_t lo = tl * PART_TILE + w * SUB;
-        Key kk[PART_ITEMS];
-        if (GATHER) {
-            // round-start segments live in buffer 0
-            const uint32_t *I = a.idx[0] + s.start;
-            ulonglong2 *KW = a.key[0] + s.start;
-            if (a.key2 && s.depth == KEY_BYTES) {
-                // round 1: the keys round 0's gather kept, by string id
-                uint32_t got = 0;
+        // Keys and their buckets, HALF keys of a lane at a time.
+        constexpr int HALF = PART_HALF<GATHER>, MATCH = MATCH_ITEMS<GATHER>;
+        const bool kept = GATHER && a.key2 && s.depth == KEY_BYTES;
+        const bool save = GATHER && a.key2 && s.depth == 0;
+        uint32_t bk[PART_ITEMS];
 #pragma unroll
-                for (int c = 0; c < PART_ITEMS; ++c) {
-                    const uint32_t e = lo + c * 32 + lane;
-                    if (e < s.len) {
-                        const ulonglong2 k2 = a.key2[I[e]];
-                        kk[c] = to_key(k2);
-                        KW[e] = k2;
-                        ++got;
-                    } else {
-                        kk[c] = key_max();
+        for (int h = 0; h < PART_ITEMS; h += HALF) {
+            const uint32_t e0 = lo + h * 32 + lane;
+            Key kk[HALF];
+            if (GATHER) {
+                // round-start segments live in buffer 0
+                const uint32_t *I = a.idx[0] + s.start;
+                ulonglong2 *KW = a.key[0] + s.start;
+                if (kept) {
+                    // round 1: the keys round 0's gather kept, by string id
+#pragma unroll
+                    for (int q = 0; q < HALF; ++q)
+                        if (e0 + q * 32 < s.len) kk[q] = to_key(a.key2[I[e0 + q * 32]]);
+                } else {
+                    uint32_t id[HALF];
+                    gather_keys<HALF>(a, I, s.depth, e0, 32, s.len, kk, id);
+                    // Depth 0 with a.key2 (a fresh round gathered here): also
+                    // keep key bytes 16..31 for round 1, as k_gather does.
+                    if (save) {
+#pragma unroll
+                        for (int q = 0; q < HALF; ++q)
+                            if (e0 + q * 32 < s.len)
+                                a.key2[id[q]] = from_key(
+                                    load_key(a.arena, a.arena_bytes,
+                                             string_offset(a.offs, a.off_width, id[q]) +
+                                                 KEY_BYTES));
                     }
                 }
-                const unsigned long long g = warp_sum((unsigned long long)got);
-                if (lane == 0 && g) atomicAdd(&cnt_ctr->window_used, g);
+#pragma unroll
+                for (int q = 0; q < HALF; ++q)
+                    if (e0 + q * 32 < s.len) KW[e0 + q * 32] = from_key(kk[q]);
             } else {
-                // Depth 0 with a.key2 (a fresh round gathered here): also keep
-                // key bytes 16..31 for round 1, as k_gather does.
-                const bool save = a.key2 && s.depth == 0;
-                uint64_t off[PART_ITEMS];
+                const ulonglong2 *K = a.keyb(s.flags & SEG_BUF1) + s.start;
 #pragma unroll
-                for (int c = 0; c < PART_ITEMS; ++c) {
-                    const uint32_t e = lo + c * 32 + lane;
-                    off[c] = e < s.len ? string_offset(a.offs, a.off_width, I[e]) + s.depth : 0;
-                }
-                uint32_t got = 0;
-#pragma unroll
-                for (int c = 0; c < PART_ITEMS; ++c) {
-                    const uint32_t e = lo + c * 32 + lane;
-                    if (e < s.len) {
-                        kk[c] = load_key(a.arena, a.arena_bytes, off[c]);
-                        KW[e] = from_key(kk[c]);
-                        if (save) {
-                            a.key2[I[e]] =
-                                from_key(load_key(a.arena, a.arena_bytes, off[c] + KEY_BYTES));
-                            ++got;
-                        }
-                    } else {
-                        kk[c] = key_max();
-                    }
-                }
-                if (save) {
-                    const unsigned long long g = warp_sum((unsigned long long)got);
-                    if (lane == 0 && g) atomicAdd(&cnt_ctr->window_saved, g);
-                }
+                for (int q = 0; q < HALF; ++q)
+                    if (e0 + q * 32 < s.len) kk[q] = to_key(K[e0 + q * 32]);
             }
-        } else {
-            const ulonglong2 *K = a.keyb(s.flags & SEG_BUF1) + s.start;
 #pragma unroll
-            for (int c = 0; c < PART_ITEMS; ++c) {
-                const uint32_t e = lo + c * 32 + lane;
-                kk[c] = e < s.len ? to_key(K[e]) : key_max();
-            }
+            for (int q = 0; q < HALF; ++q)
+                bk[h + q] = e0 + q * 32 < s.len ? classify(sm, sp, kk[q]) : nb;
         }
-        // Bucket and rank among the warp's earlier keys of the same bucket
-        // (keys are visited in position order: the scatter stays stable).
-        uint32_t br[PART_ITEMS];
+        if ((kept || save) && lane == 0 && lo < s.len)
+            atomicAdd(kept ? &cnt_ctr->window_used : &cnt_ctr->window_saved,
+                      (unsigned long long)min((uint32_t)SUB, s.len - lo));
+        // The lanes of the warp that share each key's bucket: for some keys
+        // from the match unit, for the others by a ballot per bucket-id bit.
+        // The match unit alone (one result every 60 cycles per SM) took 60 % of
+        // this kernel's time; the ballots load the ALU, which classification
+        // keeps busy.  Then each key's rank among the warp's earlier keys of
+        // the same bucket (keys are visited in position order: the scatter
+        // stays stable).
 #pragma unroll
-        for (int c = 0; c < PART_ITEMS; ++c) {
-            const uint32_t e = lo + c * 32 + lane;
-            const uint32_t b = e < s.len ? classify_tbl(sm.spl, sm.tbl, u, f, kk[c]) : nb;
-            const uint32_t peers =
-                a.match_vote ? match_bits(b, bbits) : __match_any_sync(0xffffffffu, b);
-            const uint32_t r = __popc(peers & lt);
-            const uint32_t base = hist[w][b];
-            __syncwarp();
-            if (r == 0) hist[w][b] = (uint16_t)(base + __popc(peers));
-            __syncwarp();
-            br[c] = (b << 16) | (base + r);
+        for (int h = 0; h < PART_ITEMS; h += HALF) {
+            uint32_t peers[HALF], sh[HALF];
+#pragma unroll
+            for (int q = 0; q < HALF; ++q) {
+                if (q < MATCH) {
+                    peers[q] = __match_any_sync(0xffffffffu, bk[h + q]);
+                } else {
+                    peers[q] = 0xffffffffu;
+                    sh[q] = bk[h + q] << (32 - bbits);  // the highest id bit is the sign
+                }
+            }
+#pragma unroll 1
+            for (uint32_t k = 0; k < bbits; ++k) {
+#pragma unroll
+                for (int q = MATCH; q < HALF; ++q) {
+                    const uint32_t m = __ballot_sync(0xffffffffu, (int32_t)sh[q] < 0);
+                    peers[q] &= ~(m ^ (uint32_t)((int32_t)sh[q] >> 31));
+                    sh[q] += sh[q];
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < HALF; ++q) {
+                const uint32_t b = bk[h + q], r = __popc(peers[q] & lt), base = hist[w][b];
+                __syncwarp();
+                if (r == 0) hist[w][b] = (uint16_t)(base + __popc(peers[q]));
+                __syncwarp();
+                bk[h + q] = (b << 16) | (base + r);
+            }
         }
         __syncthreads();
         // Per bucket: the tile's count (to the count matrix) and each warp's
-        // offset inside the tile's run of that bucket.
-        for (uint32_t q = threadIdx.x; q < nb; q += PART_THREADS) {
-            uint32_t run = 0;
+        // offset inside the tile's run of that bucket; two buckets at a time
+        // (counts stay below 2^16).
+        {
+            uint32_t *h = reinterpret_cast<uint32_t *>(&hist[0][0]);
+            for (uint32_t q = threadIdx.x; 2 * q < nb; q += PART_THREADS) {
+                uint32_t run = 0;
 #pragma unroll
-            for (int ww = 0; ww < PART_WARPS; ++ww) {
-                const uint32_t x = hist[ww][q];
-                hist[ww][q] = (uint16_t)run;
-                run += x;
+                for (int ww = 0; ww < PART_WARPS; ++ww) {
+                    const uint32_t x = h[ww * (NB_MAX + 1) / 2 + q];
+                    h[ww * (NB_MAX + 1) / 2 + q] = run;
+                    run += x;
+                }
+                uint32_t *d = cm + cm_base[si] + (uint64_t)(2 * q) * nt + tl;
+                d[0] = run & 0xFFFF;
+                if (2 * q + 1 < nb) d[nt] = run >> 16;
             }
-            cm[cm_base[si] + (uint64_t)q * nt + tl] = run;
         }
         __syncthreads();
         // Packed destination for the scatter: bucket << 12 | offset in the
@@ -1598,8 +1661,8 @@ __global__ void __launch_bounds__(PART_THREADS, 2) k_count(SortArgs a, const Seg
         for (int c = 0; c < PART_ITEMS; ++c) {
             const uint32_t e = lo + c * 32 + lane;
             if (e < s.len) {
-                const uint32_t b = br[c] >> 16;
-                a.bkt[s.start + e] = (b << 12) | (hist[w][b] + (br[c] & 0xFFFF));
+                const uint32_t b = bk[c] >> 16;
+                a.bkt[s.start + e] = (b << 12) | (hist[w][b] + (bk[c] & 0xFFFF));
             }
         }
         __syncthreads();
@@ -1649,7 +1712,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS) k_scatter(SortArgs a, const S
         const uint32_t si = find_seg(tile_base, nL, t);
         const Seg s = L[si];
         const uint32_t u = nspl[si] & 0xFFFF, nb = 2 * u + 1;
-        if (a.l2_prefetch && threadIdx.x == 0 && t + gridDim.x < total_tiles) {
+        if (a.l2_prefetch && threadIdx.x < 32 && t + gridDim.x < total_tiles) {
             // keys, indices and destinations of this CTA's next tile
             const uint32_t t2 = t + gridDim.x;
             const uint32_t s2i = find_seg(tile_base, nL, t2);
@@ -1803,7 +1866,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 3) k_scatter2(
         const uint32_t si = find_seg(tile_base, nL, t);
         const Seg s = L[si];
         const uint32_t u = nspl[si] & 0xFFFF, nb = 2 * u + 1;
-        if (a.l2_prefetch && threadIdx.x == 0 && t + gridDim.x < total_tiles) {
+        if (a.l2_prefetch && threadIdx.x < 32 && t + gridDim.x < total_tiles) {
             const uint32_t t2 = t + gridDim.x;
             const uint32_t s2i = find_seg(tile_base, nL, t2);
             const Seg s2 = L[s2i];
@@ -3419,7 +3482,7 @@ void launch_count(const SortArgs &a, const Seg *L, Count nL, const uint32_t *til
         k_count<true><<<grid, PART_THREADS, sizeof(PartSmem), st>>>(a, L, nL, tile_base, spl, nspl,
                                                                     tbl, cm_base, cm, c);
     else
-        k_count<false><<<grid, PART_THREADS, sizeof(PartSmem), st>>>(a, L, nL, tile_base, spl,
+        k_count<false><<<grid / 2 * COUNT_CTAS<false>, PART_THREADS, sizeof(PartSmem), st>>>(a, L, nL, tile_base, spl,
                                                                      nspl, tbl, cm_base, cm, c);
 }
 

@@ -164,7 +164,6 @@ struct ssort_server {
         a.warp1_deep = ctx->warp1_deep;
         a.l2_prefetch = ctx->l2_prefetch ? 1u : 0u;
         a.scatter_staged_idx = ctx->scatter_variant;
-        a.match_vote = ctx->match_vote ? 1u : 0u;
         a.max_splitters = (1u << (ctx->digit_bits - 1)) - 1;
         return a;
     }

@@ -77,3 +77,28 @@ def test_large_leaf_buckets():
         p, l = s.sort_host(arena, offs)
     bad, first = pyoracle.oracle_check(arena, offs, p, l)
     assert bad == 0, (bad, first)
+
+
+@pytest.mark.parametrize("kind", ["tied_windows", "one_splitter", "outside_prefix", "bytes15"])
+def test_partition_classification(sorter, kind):
+    """Splitter classification at its branches: splitters that share their first
+    64 differing bits, one distinct splitter, keys without the splitters'
+    common prefix on either side, and splitters that differ in the last byte."""
+    rng = np.random.default_rng(sum(kind.encode()))
+    n = 30_000
+    def tail(k):
+        return bytes(rng.integers(97, 123, size=k).tolist())
+    if kind == "tied_windows":
+        strings = [bytes([97 + int(rng.integers(0, 2))]) + b"mmmmmmmmmm" + tail(5) for _ in range(n)]
+    elif kind == "one_splitter":
+        strings = [b"the same key all over"] * n + [b"the", b"thf"]
+    elif kind == "outside_prefix":
+        strings = [b"middle/" + tail(9) for _ in range(n)] + \
+            [tail(3) for _ in range(40)] + [b"", b"\xff\xff", b"middle", b"middle/"]
+    else:
+        strings = [b"fifteen bytes15" + bytes([int(rng.integers(1, 256))]) + tail(2)
+                   for _ in range(n)]
+    arena, offs = cases.arena_of(strings)
+    p, l = sorter.sort_host(arena, offs)
+    rp, rl = pyoracle.oracle_sort(arena, offs)
+    assert np.array_equal(p, rp) and np.array_equal(l, rl)
