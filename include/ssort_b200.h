@@ -274,12 +274,9 @@ int ssort_get_stats(const ssort_ctx *ctx, ssort_stats *out);
                                         partition pass, i.e. a pass splits a segment into
                                         at most 2^bits buckets (2^(bits-1) - 1 sampled
                                         splitters and the buckets between and at them) */
-#define SSORT_PARAM_SCATTER 11       /* 0 (default): the partition scatter lays each tile out
-                                        in shared memory in output order; 1: it stages only
-                                        indices and destinations and reads each key from the
-                                        tile (in L2) in output order, at more CTAs per SM;
-                                        2: as 0, with each bucket run of keys written by one
-                                        asynchronous bulk copy from shared memory */
+#define SSORT_PARAM_SCATTER 11       /* 0, 1 or 2; no effect (the partition scatter stages
+                                        indices and destinations in shared memory and reads
+                                        each key from its tile in output order) */
 #define SSORT_PARAM_GRAPH 7          /* 1: device-driven round loop: the sort runs as a CUDA
                                         graph whose rounds and partition levels are
                                         conditional loops (no host round trip between

@@ -364,7 +364,6 @@ int ssort_ctx::run_ws(const uint8_t *arena_p, uint64_t arena_bytes, const void *
     a.leaf_cap = n >= LEAF_MIN_N ? LEAF_CAP : SMALL_CAP;
     a.warp1_deep = warp1_deep;
     a.l2_prefetch = l2_prefetch ? 1u : 0u;
-    a.scatter_staged_idx = scatter_variant;
     a.max_splitters = (1u << (digit_bits - 1)) - 1;
     std::copy(std::begin(class_targets), std::end(class_targets), std::begin(a.target_by_class));
     a.key2 = key2;
@@ -984,8 +983,7 @@ int ssort_set_param(ssort_ctx *ctx, int param, int64_t value) {
             return SSORT_OK;  // one finish is left: nothing to choose
         case SSORT_PARAM_SCATTER:
             if (value < 0 || value > 2) return fail(SSORT_EINVAL, "scatter must be 0, 1 or 2");
-            ctx->scatter_variant = (uint32_t)value;
-            return SSORT_OK;
+            return SSORT_OK;  // one scatter is left: nothing to choose
         case SSORT_PARAM_L2_PREFETCH:
             if (value != 0 && value != 1) return fail(SSORT_EINVAL, "l2_prefetch must be 0 or 1");
             ctx->l2_prefetch = value != 0;

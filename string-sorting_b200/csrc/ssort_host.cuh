@@ -95,7 +95,6 @@ struct ssort_ctx {
     uint32_t fused_gather = 1;  // 1: rounds >= 1 gather inside the first count; 2: all rounds
     bool l2_prefetch = false;    // partition kernels prefetch their next tile into L2
     uint32_t digit_bits = 10;    // a partition pass makes at most 2^digit_bits buckets
-    uint32_t scatter_variant = 0;  // 1: the scatter stages indices only (k_scatter2)
     bool scan_lookback = true;     // count-matrix scan in one pass (decoupled look-back)
     // Device-driven round loop (ssort_graph.cu): the instantiated graph, the
     // key it was built for, three streams to capture nested conditional

@@ -173,7 +173,6 @@ struct SortArgs {
     uint32_t leaf_cap;       // largest range bucket that is not partitioned again
     uint32_t warp1_deep;     // in-warp refinement steps of the one-per-lane sort
     uint32_t l2_prefetch;    // partition kernels stream their next tile into L2 ahead
-    uint32_t scatter_staged_idx;  // 0: k_scatter; 1: indices only (k_scatter2); 2: bulk key runs
     uint32_t max_splitters;  // splitters per partition pass, 2^(digit bits - 1) - 1 <= KMAX
     // Per segment size class (floor(log2 len)): the wanted strings per range
     // bucket autotuned for that class (0: target_bucket).  Set for batched

@@ -1672,175 +1672,21 @@ __global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(Sort
 // ---- partition scatter: a copy to precomputed destinations --------------------
 // k_count left every key's bucket and its offset inside the tile's run of that
 // bucket; the run's start comes from the scanned count matrix.  Tile order
-// and within-tile order follow positions, so the scatter is stable.  Each
-// tile is first laid out in shared memory in output order (its bucket runs
-// back to back), so consecutive threads store to consecutive addresses within
-// every run.
-constexpr int SCATTER_THREADS = 256;  // 512 x 8 items measured slower
-constexpr int SCATTER_ITEMS = PART_TILE / SCATTER_THREADS;  // 16
+// and within-tile order follow positions, so the scatter is stable.  A tile's
+// indices and destinations are laid out in shared memory in output order (its
+// bucket runs back to back), with each record's place in the tile; the
+// write-out reads the keys from there (the tile's 64 KB, which the CTA is
+// about to leave in L2) and stores consecutive records to consecutive
+// addresses within every run.
+// Bound by how the memory system takes the scattered stores, not by latency:
+// more stores in flight are slower.  100 M words, scatter time of a sort with
+// 256 threads and 1, 2, 3, 4 CTAs per SM: 2.36, 1.82, 1.84, 3.5 ms; with 512
+// threads and 1 or 2: 2.11, 1.80; with the keys staged in shared memory too
+// (98 KB, 1 or 2 CTAs): 2.03, 2.45; each record stored straight to its place:
+// 4.1 to 4.7.
+constexpr int SCATTER_THREADS = 512;
+constexpr int SCATTER_ITEMS = PART_TILE / SCATTER_THREADS;  // 8
 struct ScatterSmem {
-    ulonglong2 key[PART_TILE];
-    uint32_t idx[PART_TILE];
-    uint32_t dst[PART_TILE];
-    uint32_t gbase[NB_MAX + 1];
-    uint32_t tstart[NB_MAX + 1];
-    uint32_t wsum[SCATTER_THREADS / 32];
-};
-
-// BULK: each bucket run of keys leaves shared memory as one asynchronous bulk
-// copy to global memory (cp.async.bulk, issued by the thread that owns the
-// bucket; keys are 16 bytes, so every run starts and ends on a 16-byte
-// boundary at both ends); the indices are stored by the threads as before.
-template <bool BULK>
-__global__ void __launch_bounds__(SCATTER_THREADS) k_scatter(SortArgs a, const Seg *__restrict__ L,
-                                                             Count cnt,
-                                                             const uint32_t *__restrict__ tile_base,
-                                                             const uint32_t *__restrict__ nspl,
-                                                             const uint32_t *__restrict__ cm_base,
-                                                             const uint32_t *__restrict__ cm_scan,
-                                                             Counters *ctr) {
-    extern __shared__ __align__(16) unsigned char scatter_smem[];
-    ScatterSmem &sm = *reinterpret_cast<ScatterSmem *>(scatter_smem);
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    constexpr uint32_t QPT = (NB_MAX + 1) / SCATTER_THREADS;  // buckets per thread (4)
-    const uint32_t nL = count_of(cnt);
-    const uint32_t total_tiles = tile_base[nL];
-    bool any_bulk = false;  // this thread issued bulk copies (BULK)
-    TileQueue tiles(&ctr->scatter_ticket);
-    for (uint32_t t = blockIdx.x; t < total_tiles; t = tiles.next()) {
-        tiles.ask();
-        const uint32_t si = find_seg(tile_base, nL, t);
-        const Seg s = L[si];
-        const uint32_t u = nspl[si] & 0xFFFF, nb = 2 * u + 1;
-        if (a.l2_prefetch && threadIdx.x < 32 && t + gridDim.x < total_tiles) {
-            // keys, indices and destinations of this CTA's next tile
-            const uint32_t t2 = t + gridDim.x;
-            const uint32_t s2i = find_seg(tile_base, nL, t2);
-            const Seg s2 = L[s2i];
-            const uint32_t lo2 = (t2 - tile_base[s2i]) * PART_TILE;
-            const uint32_t len2 = min((uint32_t)PART_TILE, s2.len - lo2);
-            const int b2 = s2.flags & SEG_BUF1;
-            prefetch_l2(a.keyb(b2) + s2.start + lo2, (uint64_t)len2 * 16);
-            prefetch_l2(a.idxb(b2) + s2.start + lo2, (uint64_t)len2 * 4);
-            prefetch_l2(a.bkt + s2.start + lo2, (uint64_t)len2 * 4);
-        }
-        const uint32_t tl = t - tile_base[si];
-        const uint32_t nt = tile_base[si + 1] - tile_base[si];
-        const uint32_t cmb = cm_base[si];
-        const uint32_t seg0 = cm_scan[cmb];
-        const uint32_t lo = tl * PART_TILE;
-        const uint32_t tlen = min((uint32_t)PART_TILE, s.len - lo);
-        const int ib = s.flags & SEG_BUF1;
-        const ulonglong2 *Kin = a.keyb(ib) + s.start;
-        const uint32_t *Iin = a.idxb(ib) + s.start;
-        const uint32_t *Din = a.bkt + s.start;
-        // Element loads first (they overlap the count-matrix reads below).
-        ulonglong2 kk[SCATTER_ITEMS];
-        uint32_t ii[SCATTER_ITEMS], dd[SCATTER_ITEMS];
-#pragma unroll
-        for (int c = 0; c < SCATTER_ITEMS; ++c) {
-            const uint32_t e = c * SCATTER_THREADS + threadIdx.x;
-            if (e < tlen) {
-                kk[c] = Kin[lo + e];
-                ii[c] = Iin[lo + e];
-                dd[c] = Din[lo + e];
-            }
-        }
-        // Per bucket: the tile's run start in the segment and the tile's
-        // count (difference of consecutive scanned entries), then an exclusive
-        // scan of the counts gives each run's start inside the tile.
-        uint32_t cnt[QPT];
-        uint32_t mysum = 0;
-#pragma unroll
-        for (uint32_t j = 0; j < QPT; ++j) {
-            const uint32_t q = threadIdx.x * QPT + j;
-            uint32_t c0 = 0;
-            if (q < nb) {
-                const uint64_t at = cmb + (uint64_t)q * nt + tl;
-                const uint32_t g = cm_scan[at];
-                c0 = cm_scan[at + 1] - g;  // next tile, or next bucket's first tile
-                sm.gbase[q] = g - seg0;
-            }
-            cnt[j] = c0;
-            mysum += c0;
-        }
-        uint32_t incl = mysum;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= (uint32_t)d) incl += y;
-        }
-        if (lane == 31) sm.wsum[w] = incl;
-        __syncthreads();
-        uint32_t run = incl - mysum;
-        for (uint32_t q = 0; q < w; ++q) run += sm.wsum[q];
-#pragma unroll
-        for (uint32_t j = 0; j < QPT; ++j) {
-            sm.tstart[threadIdx.x * QPT + j] = run;
-            run += cnt[j];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < SCATTER_ITEMS; ++c) {
-            const uint32_t e = c * SCATTER_THREADS + threadIdx.x;
-            if (e < tlen) {
-                const uint32_t b = dd[c] >> 12, off = dd[c] & (PART_TILE - 1);
-                const uint32_t slot = sm.tstart[b] + off;
-                sm.key[slot] = kk[c];
-                sm.idx[slot] = ii[c];
-                sm.dst[slot] = sm.gbase[b] + off;
-            }
-        }
-        __syncthreads();
-        ulonglong2 *Kout = a.keyb(ib ^ 1) + s.start;
-        uint32_t *Iout = a.idxb(ib ^ 1) + s.start;
-        if constexpr (BULK) {
-            // The staged keys were written by other threads through the
-            // generic proxy; make them visible to the bulk copies' async proxy.
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            bool issued = false;
-#pragma unroll
-            for (uint32_t j = 0; j < QPT; ++j) {
-                const uint32_t q = threadIdx.x * QPT + j;
-                if (cnt[j]) {
-                    const uint32_t src =
-                        (uint32_t)__cvta_generic_to_shared(&sm.key[sm.tstart[q]]);
-                    asm volatile(
-                        "cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
-                            Kout + sm.gbase[q]),
-                        "r"(src), "r"(cnt[j] * 16u)
-                        : "memory");
-                    issued = true;
-                }
-            }
-            if (issued) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            for (uint32_t i = threadIdx.x; i < tlen; i += SCATTER_THREADS)
-                Iout[sm.dst[i]] = sm.idx[i];
-            // The next tile restages into sm.key: wait until the copies have
-            // read it (their global writes complete by the kernel's end).
-            if (issued) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            any_bulk |= issued;
-        } else {
-            for (uint32_t i = threadIdx.x; i < tlen; i += SCATTER_THREADS) {
-                const uint32_t o = sm.dst[i];
-                Kout[o] = sm.key[i];
-                Iout[o] = sm.idx[i];
-            }
-        }
-        __syncthreads();
-    }
-    // Every bulk copy's writes complete before the thread exits.
-    if (BULK && any_bulk) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-}
-
-
-// The same scatter with only indices and destinations staged: the slots of
-// the tile in output order record where each record sits in the tile, and
-// the write-out reads the keys from there (the tile was just read, and with
-// SortArgs::l2_prefetch also streamed into L2 ahead; the reads stay inside
-// the tile's 64 KB).  48 KB of shared memory and about half the registers of
-// k_scatter, so three or four CTAs share an SM instead of two.
-struct Scatter2Smem {
     uint32_t idx[PART_TILE];    // indices in output order
     uint32_t dst[PART_TILE];    // destinations in output order
     uint16_t src[PART_TILE];    // tile position of the record at each output slot
@@ -1848,16 +1694,16 @@ struct Scatter2Smem {
     uint32_t tstart[NB_MAX + 1];
     uint32_t wsum[SCATTER_THREADS / 32];
 };
-constexpr int SCATTER2_BATCH = 4;  // keys in flight per thread in the write-out
+constexpr int SCATTER_BATCH = 4;  // keys in flight per thread in the write-out
 
-__global__ void __launch_bounds__(SCATTER_THREADS, 3) k_scatter2(
+__global__ void __launch_bounds__(SCATTER_THREADS, 2) k_scatter(
     SortArgs a, const Seg *__restrict__ L, Count cnt, const uint32_t *__restrict__ tile_base,
     const uint32_t *__restrict__ nspl, const uint32_t *__restrict__ cm_base,
     const uint32_t *__restrict__ cm_scan, Counters *ctr) {
     extern __shared__ __align__(16) unsigned char scatter_smem[];
-    Scatter2Smem &sm = *reinterpret_cast<Scatter2Smem *>(scatter_smem);
+    ScatterSmem &sm = *reinterpret_cast<ScatterSmem *>(scatter_smem);
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    constexpr uint32_t QPT = (NB_MAX + 1) / SCATTER_THREADS;  // buckets per thread (4)
+    constexpr uint32_t QPT = (NB_MAX + 1) / SCATTER_THREADS;  // buckets per thread (2)
     const uint32_t nL = count_of(cnt);
     const uint32_t total_tiles = tile_base[nL];
     TileQueue tiles(&ctr->scatter_ticket);
@@ -1941,15 +1787,15 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 3) k_scatter2(
         __syncthreads();
         ulonglong2 *Kout = a.keyb(ib ^ 1) + s.start;
         uint32_t *Iout = a.idxb(ib ^ 1) + s.start;
-        for (uint32_t i0 = 0; i0 < tlen; i0 += SCATTER2_BATCH * SCATTER_THREADS) {
-            ulonglong2 kv[SCATTER2_BATCH];
+        for (uint32_t i0 = 0; i0 < tlen; i0 += SCATTER_BATCH * SCATTER_THREADS) {
+            ulonglong2 kv[SCATTER_BATCH];
 #pragma unroll
-            for (int q = 0; q < SCATTER2_BATCH; ++q) {
+            for (int q = 0; q < SCATTER_BATCH; ++q) {
                 const uint32_t i = i0 + q * SCATTER_THREADS + threadIdx.x;
                 if (i < tlen) kv[q] = __ldg(Kin + sm.src[i]);
             }
 #pragma unroll
-            for (int q = 0; q < SCATTER2_BATCH; ++q) {
+            for (int q = 0; q < SCATTER_BATCH; ++q) {
                 const uint32_t i = i0 + q * SCATTER_THREADS + threadIdx.x;
                 if (i < tlen) {
                     const uint32_t o = sm.dst[i];
@@ -3305,12 +3151,8 @@ static void set_smem_attrs() {
                          (int)sizeof(PartSmem));
     cudaFuncSetAttribute(k_count<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(PartSmem));
-    cudaFuncSetAttribute(k_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(ScatterSmem));
-    cudaFuncSetAttribute(k_scatter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(ScatterSmem));
-    cudaFuncSetAttribute(k_scatter2, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(Scatter2Smem));
     cudaFuncSetAttribute(k_tiny, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TINY_SMEM);
     cudaFuncSetAttribute(k_warpsort, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)WARPSORT_SMEM);
@@ -3492,19 +3334,8 @@ void launch_scatter(const SortArgs &a, const Seg *L, Count nL, const uint32_t *t
                     cudaStream_t st) {
     if (!nL.dev && !nL.host) return;
     set_smem_attrs();
-    if (a.scatter_staged_idx == 2) {
-        k_scatter<true><<<grid, SCATTER_THREADS, sizeof(ScatterSmem), st>>>(
-            a, L, nL, tile_base, nspl, cm_base, cm_scan, c);
-        return;
-    }
-    if (a.scatter_staged_idx) {
-        // three CTAs per SM where k_scatter fits two (grid: two per SM)
-        k_scatter2<<<grid / 2 * 3, SCATTER_THREADS, sizeof(Scatter2Smem), st>>>(
-            a, L, nL, tile_base, nspl, cm_base, cm_scan, c);
-        return;
-    }
-    k_scatter<false><<<grid, SCATTER_THREADS, sizeof(ScatterSmem), st>>>(
-        a, L, nL, tile_base, nspl, cm_base, cm_scan, c);
+    k_scatter<<<grid, SCATTER_THREADS, sizeof(ScatterSmem), st>>>(a, L, nL, tile_base, nspl,
+                                                                  cm_base, cm_scan, c);
 }
 
 void launch_emit(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,

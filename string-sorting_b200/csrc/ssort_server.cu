@@ -163,7 +163,6 @@ struct ssort_server {
         a.leaf_cap = max_strings >= LEAF_MIN_N ? LEAF_CAP : SMALL_CAP;
         a.warp1_deep = ctx->warp1_deep;
         a.l2_prefetch = ctx->l2_prefetch ? 1u : 0u;
-        a.scatter_staged_idx = ctx->scatter_variant;
         a.max_splitters = (1u << (ctx->digit_bits - 1)) - 1;
         return a;
     }
