@@ -381,19 +381,33 @@ __global__ void k_init_batch(const uint32_t *__restrict__ inst_start, uint32_t n
     if (seg) R[slot] = Seg{s, e - s, 0, 0};
 }
 
+// The three kernels below give every position the instance or request it lies
+// in.  A warp takes SPAN_ITEMS * 32 consecutive positions: one search for the
+// first, then every lane only steps over range ends it passes (a search per
+// position took 0.37 ms over 69 M positions in 286 instances; reading and
+// writing them takes 0.09).
+constexpr uint32_t SPAN_ITEMS = 8;
+
 // Global positions -> indices within each position's instance.
 __global__ void k_localize(uint32_t *perm, uint32_t n, const uint32_t *__restrict__ inst_start,
                            uint32_t ninst) {
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        uint32_t lo = 0, hi = ninst;  // largest i with inst_start[i] <= p
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(inst_start + mid) <= p)
-                lo = mid;
-            else
-                hi = mid;
+    const uint32_t lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint64_t p0 = (uint64_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32 * SPAN_ITEMS;
+         p0 < n; p0 += (uint64_t)warps * 32 * SPAN_ITEMS) {
+        uint32_t i = find_seg(inst_start, ninst, (uint32_t)p0);
+        uint32_t end = __ldg(inst_start + i + 1), start = __ldg(inst_start + i);
+#pragma unroll
+        for (uint32_t k = 0; k < SPAN_ITEMS; ++k) {
+            const uint64_t p = p0 + k * 32 + lane;
+            if (p < n) {
+                while (p >= end && i + 1 < ninst) {
+                    ++i;
+                    start = end;
+                    end = __ldg(inst_start + i + 1);
+                }
+                perm[p] -= start;
+            }
         }
-        perm[p] -= __ldg(inst_start + lo);
     }
 }
 
@@ -425,18 +439,26 @@ __device__ __forceinline__ uint32_t find_job(const ReqJob *__restrict__ jobs, ui
 // R[slot].
 __global__ void k_join(uint64_t *goffs, uint32_t *lcp, uint32_t *perm,
                        const ReqJob *__restrict__ jobs, uint32_t njobs, uint32_t total, Seg *R) {
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < total;
-         q += gridDim.x * blockDim.x) {
-        const ReqJob jb = jobs[find_job(jobs, njobs, q)];
-        const uint32_t i = q - jb.first;
-        const uint32_t p = jb.pos + i;
-        uint64_t o = jb.off_width == 4 ? (uint64_t)lcp[p] : goffs[p];
-        if (o > jb.arena_bytes) o = jb.arena_bytes;
-        goffs[p] = jb.region_base + o;
-        perm[p] = p;
-        if (i == 0) {
-            lcp[p] = 0;
-            if (jb.n >= 2) R[jb.slot] = Seg{jb.pos, jb.n, 0, 0};
+    const uint32_t lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint64_t q0 = (uint64_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32 * SPAN_ITEMS;
+         q0 < total; q0 += (uint64_t)warps * 32 * SPAN_ITEMS) {
+        uint32_t j = find_job(jobs, njobs, (uint32_t)q0);
+#pragma unroll
+        for (uint32_t k = 0; k < SPAN_ITEMS; ++k) {
+            const uint64_t q = q0 + k * 32 + lane;
+            if (q >= total) break;
+            while (j + 1 < njobs && jobs[j + 1].first <= q) ++j;
+            const ReqJob jb = jobs[j];
+            const uint32_t i = (uint32_t)q - jb.first;
+            const uint32_t p = jb.pos + i;
+            uint64_t o = jb.off_width == 4 ? (uint64_t)lcp[p] : goffs[p];
+            if (o > jb.arena_bytes) o = jb.arena_bytes;
+            goffs[p] = jb.region_base + o;
+            perm[p] = p;
+            if (i == 0) {
+                lcp[p] = 0;
+                if (jb.n >= 2) R[jb.slot] = Seg{jb.pos, jb.n, 0, 0};
+            }
         }
     }
 }
@@ -463,10 +485,18 @@ __global__ void k_mark(const Seg *__restrict__ R, uint32_t nR, const uint32_t *_
 // Global positions of finished requests -> indices within each request.
 __global__ void k_unbase(uint32_t *perm, const ReqJob *__restrict__ jobs, uint32_t njobs,
                          uint32_t total) {
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < total;
-         q += gridDim.x * blockDim.x) {
-        const ReqJob jb = jobs[find_job(jobs, njobs, q)];
-        perm[jb.pos + (q - jb.first)] -= jb.pos;
+    const uint32_t lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint64_t q0 = (uint64_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32 * SPAN_ITEMS;
+         q0 < total; q0 += (uint64_t)warps * 32 * SPAN_ITEMS) {
+        uint32_t j = find_job(jobs, njobs, (uint32_t)q0);
+#pragma unroll
+        for (uint32_t k = 0; k < SPAN_ITEMS; ++k) {
+            const uint64_t q = q0 + k * 32 + lane;
+            if (q >= total) break;
+            while (j + 1 < njobs && jobs[j + 1].first <= q) ++j;
+            const uint32_t pos = jobs[j].pos;
+            perm[pos + ((uint32_t)q - jobs[j].first)] -= pos;
+        }
     }
 }
 
