@@ -379,6 +379,16 @@ struct ReqJob {
     uint32_t slot;   // segment slot in the round list (requests of >= 2 strings)
     uint32_t off_width, pad;
 };
+// One copy of a batch: dst[0 .. bytes) = src, dst[bytes .. bytes + fill) = 0.
+// `first`: chunks of COPY_CHUNK bytes of the copies before this one.
+constexpr uint32_t COPY_CHUNK = 32768;
+struct CopyJob {
+    const uint8_t *src;
+    uint8_t *dst;
+    uint64_t bytes, fill;
+    uint32_t first, pad;
+};
+void launch_copies(const CopyJob *jobs, uint32_t njobs, uint32_t chunks, cudaStream_t st);
 void launch_join(uint64_t *goffs, uint32_t *lcp, uint32_t *perm, const ReqJob *jobs,
                  uint32_t njobs, uint32_t total, Seg *R, cudaStream_t st);
 void launch_mark(const Seg *R, uint32_t nR, const uint32_t *base, uint32_t nact, uint32_t *flag,

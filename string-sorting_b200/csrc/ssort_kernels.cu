@@ -428,6 +428,45 @@ __device__ __forceinline__ uint32_t find_job(const ReqJob *__restrict__ jobs, ui
     return lo;
 }
 
+// The copies of many requests in one launch, between buffers of this device.
+// A copy per buffer kept the copy streams busy with launches instead: 24
+// requests took 72 copies and fills in, 48 out, at 3 to 4 us each.  A CTA moves
+// one chunk, in the widest words that both ends' alignment allows.
+template <typename W>
+__device__ __forceinline__ void copy_words(uint8_t *dst, const uint8_t *src, uint64_t bytes) {
+    const uint64_t n = bytes / sizeof(W);
+    for (uint64_t i = threadIdx.x; i < n; i += blockDim.x)
+        reinterpret_cast<W *>(dst)[i] = reinterpret_cast<const W *>(src)[i];
+    for (uint64_t i = n * sizeof(W) + threadIdx.x; i < bytes; i += blockDim.x) dst[i] = src[i];
+}
+
+__global__ void __launch_bounds__(512) k_copies(const CopyJob *__restrict__ jobs, uint32_t njobs) {
+    uint32_t lo = 0, hi = njobs;  // largest j with jobs[j].first <= chunk
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (jobs[mid].first <= blockIdx.x)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    const CopyJob jb = jobs[lo];
+    const uint64_t at = (uint64_t)(blockIdx.x - jb.first) * COPY_CHUNK;
+    const uint64_t end = min(at + COPY_CHUNK, jb.bytes + jb.fill);
+    const uint64_t stop = min(end, jb.bytes);
+    if (at < stop) {
+        const uint8_t *s = jb.src + at;
+        uint8_t *d = jb.dst + at;
+        const uint32_t both = (uint32_t)((uintptr_t)s | (uintptr_t)d);
+        if ((both & 15) == 0)
+            copy_words<uint4>(d, s, stop - at);
+        else if ((both & 3) == 0)
+            copy_words<uint32_t>(d, s, stop - at);
+        else
+            copy_words<uint8_t>(d, s, stop - at);
+    }
+    for (uint64_t i = max(at, jb.bytes) + threadIdx.x; i < end; i += blockDim.x) jb.dst[i] = 0;
+}
+
 // Joins admitted requests: request j occupies positions [pos, pos + n) and its
 // bytes sit at region_base in the pool arena.  Its offsets arrive either as
 // uint64 in place in goffs or as uint32 staged in lcp at its positions; each
@@ -3248,6 +3287,10 @@ void launch_localize(uint32_t *perm, uint32_t n, const uint32_t *inst_start, uin
                      cudaStream_t st) {
     const uint32_t g = cdiv(n, 256) < 148 * 8 ? cdiv(n, 256) : 148 * 8;
     k_localize<<<g ? g : 1, 256, 0, st>>>(perm, n, inst_start, ninst);
+}
+
+void launch_copies(const CopyJob *jobs, uint32_t njobs, uint32_t chunks, cudaStream_t st) {
+    if (njobs && chunks) k_copies<<<chunks, 512, 0, st>>>(jobs, njobs);
 }
 
 void launch_join(uint64_t *goffs, uint32_t *lcp, uint32_t *perm, const ReqJob *jobs,

@@ -97,6 +97,62 @@ struct Request {
     uint64_t region = 0, region_size = 0;
     uint64_t pos = 0;
     cudaEvent_t ev = nullptr;  // copy-in done, then copy-out done
+    bool dev_in = false, dev_out = false;  // inputs / outputs in this device's memory
+};
+
+// Whether p lies in device memory of `device` (null counts as there).
+bool on_device(const void *p, int device) {
+    if (!p) return true;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeDevice && at.device == device;
+}
+
+// Copies between device buffers, gathered and run as one launch: a pinned
+// table, its device copy, and the event after which the table may be refilled.
+struct CopyBatch {
+    static constexpr uint32_t CAP = 1024;
+    CopyJob *h = nullptr;
+    DBuf d;
+    cudaEvent_t ev = nullptr;
+    bool pending = false;
+    uint32_t n = 0, chunks = 0;
+
+    int create(ssort_ctx *ctx) {
+        SS_CUDA(cudaHostAlloc((void **)&h, CAP * sizeof(CopyJob), cudaHostAllocDefault));
+        SS_TRY(ctx->ensure(d, CAP * sizeof(CopyJob)));
+        SS_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        return SSORT_OK;
+    }
+    void destroy() {
+        if (h) cudaFreeHost(h);
+        if (d.p) cudaFree(d.p);
+        if (ev) cudaEventDestroy(ev);
+    }
+    int add(void *dst, const void *src, uint64_t bytes, uint64_t fill, cudaStream_t st) {
+        const uint64_t c = (bytes + fill + COPY_CHUNK - 1) / COPY_CHUNK;
+        if (n == CAP || chunks + c > (1u << 30)) SS_TRY(run(st));
+        if (!n && pending) {
+            SS_CUDA(cudaEventSynchronize(ev));
+            pending = false;
+        }
+        h[n++] = CopyJob{(const uint8_t *)src, (uint8_t *)dst, bytes, fill, chunks, 0};
+        chunks += (uint32_t)c;
+        return SSORT_OK;
+    }
+    int run(cudaStream_t st) {
+        if (!n) return SSORT_OK;
+        SS_CUDA(cudaMemcpyAsync(d.p, h, n * sizeof(CopyJob), cudaMemcpyHostToDevice, st));
+        launch_copies((const CopyJob *)d.p, n, chunks, st);
+        SS_CUDA(cudaGetLastError());
+        SS_CUDA(cudaEventRecord(ev, st));
+        pending = true;
+        n = chunks = 0;
+        return SSORT_OK;
+    }
 };
 
 }  // namespace
@@ -112,6 +168,7 @@ struct ssort_server {
     ReqJob *h_join = nullptr, *h_done = nullptr;  // pinned job tables
     cudaEvent_t ev_join_jobs = nullptr, ev_done_jobs = nullptr, ev_unbased = nullptr;
     bool join_jobs_pending = false, done_jobs_pending = false;
+    CopyBatch in, out;  // copies of requests whose buffers lie on the device
     RangeAlloc arena_alloc, pos_alloc;
     std::deque<Request *> queue;
     std::vector<Request *> loading, active, draining;
@@ -185,6 +242,7 @@ struct ssort_server {
 // FIFO admission: the head of the queue is admitted when its pool region and
 // position range fit; later requests wait behind it.
 int ssort_server::admit() {
+    const size_t before = loading.size();
     while (!queue.empty()) {
         Request *r = queue.front();
         if (loading.size() + active.size() + draining.size() >= MAX_SLOTS) break;
@@ -202,17 +260,24 @@ int ssort_server::admit() {
         r->ev = take_event();
         if (!r->ev) return fail(SSORT_ECUDA, "event creation failed");
         uint8_t *dst = (uint8_t *)pool.p + region;
-        if (r->arena_bytes)
-            SS_CUDA(cudaMemcpyAsync(dst, r->arena, r->arena_bytes, cudaMemcpyDefault, h2d));
-        SS_CUDA(cudaMemsetAsync(dst + r->arena_bytes, 0, rsz - r->arena_bytes, h2d));
         void *odst = r->off_width == 8 ? (void *)((uint64_t *)goffs.p + pos)
                                        : (void *)(ctx->ws.lcp + pos);
-        SS_CUDA(cudaMemcpyAsync(odst, r->offs, (size_t)r->n * r->off_width, cudaMemcpyDefault,
-                                h2d));
-        SS_CUDA(cudaEventRecord(r->ev, h2d));
+        if (r->dev_in) {
+            SS_TRY(in.add(dst, r->arena, r->arena_bytes, rsz - r->arena_bytes, h2d));
+            SS_TRY(in.add(odst, r->offs, (uint64_t)r->n * r->off_width, 0, h2d));
+        } else {
+            if (r->arena_bytes)
+                SS_CUDA(cudaMemcpyAsync(dst, r->arena, r->arena_bytes, cudaMemcpyDefault, h2d));
+            SS_CUDA(cudaMemsetAsync(dst + r->arena_bytes, 0, rsz - r->arena_bytes, h2d));
+            SS_CUDA(cudaMemcpyAsync(odst, r->offs, (size_t)r->n * r->off_width, cudaMemcpyDefault,
+                                    h2d));
+        }
         r->state = SSORT_REQ_LOADING;
         loading.push_back(r);
     }
+    SS_TRY(in.run(h2d));
+    for (size_t k = before; k < loading.size(); ++k)
+        SS_CUDA(cudaEventRecord(loading[k]->ev, h2d));
     return SSORT_OK;
 }
 
@@ -296,7 +361,15 @@ int ssort_server::finish(const std::vector<Request *> &done) {
     SS_CUDA(cudaEventRecord(ev_unbased, ctx->st));
     SS_CUDA(cudaStreamWaitEvent(d2h, ev_unbased, 0));
     for (Request *r : done) {
-        if (r->n) {
+        if (r->dev_out) {
+            SS_TRY(out.add(r->perm_out, (uint32_t *)perm.p + r->pos, (uint64_t)r->n * 4, 0, d2h));
+            if (r->lcp_out)
+                SS_TRY(out.add(r->lcp_out, ctx->ws.lcp + r->pos, (uint64_t)r->n * 4, 0, d2h));
+        }
+    }
+    SS_TRY(out.run(d2h));
+    for (Request *r : done) {
+        if (r->n && !r->dev_out) {
             SS_CUDA(cudaMemcpyAsync(r->perm_out, (uint32_t *)perm.p + r->pos, (size_t)r->n * 4,
                                     cudaMemcpyDefault, d2h));
             if (r->lcp_out)
@@ -395,6 +468,8 @@ void server_free(ssort_server *srv) {
             for (DBuf *b : {&srv->pool, &srv->goffs, &srv->perm, &srv->bases, &srv->flags,
                             &srv->d_join, &srv->d_done})
                 if (b->p) cudaFree(b->p);
+            srv->in.destroy();
+            srv->out.destroy();
             if (srv->h_bases) cudaFreeHost(srv->h_bases);
             if (srv->h_flags) cudaFreeHost(srv->h_flags);
             if (srv->h_join) cudaFreeHost(srv->h_join);
@@ -450,6 +525,8 @@ int ssort_server_create(int device, uint64_t arena_budget_bytes, uint64_t max_st
                               cudaHostAllocDefault));
         SS_CUDA(cudaHostAlloc((void **)&srv->h_done, (size_t)MAX_SLOTS * sizeof(ReqJob),
                               cudaHostAllocDefault));
+        SS_TRY(srv->in.create(ctx));
+        SS_TRY(srv->out.create(ctx));
         SS_CUDA(cudaEventCreateWithFlags(&srv->ev_join_jobs, cudaEventDisableTiming));
         SS_CUDA(cudaEventCreateWithFlags(&srv->ev_done_jobs, cudaEventDisableTiming));
         SS_CUDA(cudaEventCreateWithFlags(&srv->ev_unbased, cudaEventDisableTiming));
@@ -493,6 +570,8 @@ int ssort_server_submit(ssort_server *srv, const uint8_t *arena, uint64_t arena_
     r->n = (uint32_t)n;
     r->perm_out = perm_out;
     r->lcp_out = lcp_out;
+    r->dev_in = n && on_device(arena, srv->ctx->device) && on_device(offs, srv->ctx->device);
+    r->dev_out = n && on_device(perm_out, srv->ctx->device) && on_device(lcp_out, srv->ctx->device);
     *id_out = r->id;
     if (n == 0) {
         srv->done_ids.push_back(r->id);
