@@ -361,6 +361,7 @@ int ssort_ctx::run_ws(const uint8_t *arena_p, uint64_t arena_bytes, const void *
     a.bkt = ws.bkt;
     a.target_bucket = target_bucket;
     a.warp8_cap = warp8_cap;
+    a.tile = part_tile(n);
     a.leaf_cap = n >= LEAF_MIN_N ? LEAF_CAP : SMALL_CAP;
     a.warp1_deep = warp1_deep;
     a.l2_prefetch = l2_prefetch ? 1u : 0u;

@@ -76,7 +76,25 @@ constexpr int TARGET_BUCKET = 512;      // default wanted strings per range buck
 constexpr int PART_THREADS = 512;
 constexpr int PART_WARPS = PART_THREADS / 32;
 constexpr int PART_ITEMS = 8;
-constexpr int PART_TILE = PART_THREADS * PART_ITEMS;  // 4096 keys per tile
+constexpr int PART_TILE = PART_THREADS * PART_ITEMS;  // most keys per tile: 4096
+// Keys per tile of a sort of n strings: a small sort has too few tiles of 4096
+// to fill the chip, and one CTA's time for its only tile is what counts (20 k
+// URLs 249 -> 236 us with tiles of 1024; 500 k URLs 390 -> 370 us with 2048).
+// With more tiles than CTAs the larger tile is better again (1 M uniform
+// strings 230 us with 4096, 237 with 2048; 256 k strings 137 with 4096 or
+// 2048, 142 with 1024).
+constexpr uint64_t TILE_1024_MAX_N = 148 * 512, TILE_2048_MAX_N = 148 * 4096;
+constexpr uint32_t part_tile(uint64_t n) {
+    return n <= TILE_1024_MAX_N ? 1024 : n <= TILE_2048_MAX_N ? 2048 : PART_TILE;
+}
+// Most tiles of any sort of at most n strings, its segments' last ones aside.
+constexpr uint64_t most_tiles(uint64_t n) {
+    uint64_t t = n / PART_TILE;
+    const uint64_t a = (n < TILE_1024_MAX_N ? n : TILE_1024_MAX_N) / 1024;
+    const uint64_t b = (n < TILE_2048_MAX_N ? n : TILE_2048_MAX_N) / 2048;
+    if (a > t) t = a;
+    return b > t ? b : t;
+}
 
 constexpr int GATHER_TILE = 4096;
 constexpr int GATHER_THREADS = 256;
@@ -173,6 +191,7 @@ struct SortArgs {
     uint32_t leaf_cap;       // largest range bucket that is not partitioned again
     uint32_t warp1_deep;     // in-warp refinement steps of the one-per-lane sort
     uint32_t l2_prefetch;    // partition kernels stream their next tile into L2 ahead
+    uint32_t tile;           // keys per partition tile, part_tile()
     uint32_t max_splitters;  // splitters per partition pass, 2^(digit bits - 1) - 1 <= KMAX
     // Per segment size class (floor(log2 len)): the wanted strings per range
     // bucket autotuned for that class (0: target_bucket).  Set for batched
@@ -279,7 +298,7 @@ constexpr WsLayout ws_layout(uint64_t n) {
     o.tile_base = take((nlarge + 1) * 4);
     o.tmp = take((nlarge + 1) * 4);
     // bucket-count matrix: at most NB_MAX buckets per tile of each segment
-    o.cm_cap = (size_t)NB_MAX * (n / PART_TILE + nlarge + 1) + 1;
+    o.cm_cap = (size_t)NB_MAX * (most_tiles(n) + nlarge + 1) + 1;
     o.cm = take(o.cm_cap * 4);
     o.partials = take((size_t)scan_partials_for(o.cm_cap) * 4);
     // single-pass scan: a ticket word, then one status word per tile

@@ -1394,7 +1394,7 @@ __device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__r
     }
     if (t == 0) {
         nspl[si] = u | (f << 16);
-        const uint32_t nt = (s.len + PART_TILE - 1) / PART_TILE;
+        const uint32_t nt = (s.len + a.tile - 1) / a.tile;
         ntiles[si] = nt;
         cm_size[si] = (2 * u + 1) * nt;
     }
@@ -1589,7 +1589,7 @@ __global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(Sort
     PartSmem &sm = *reinterpret_cast<PartSmem *>(part_smem);
     auto &hist = sm.cnt;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    constexpr int SUB = PART_TILE / PART_WARPS;
+    const uint32_t SUB = a.tile / PART_WARPS;
     const uint32_t nL = count_of(cnt);
     const uint32_t total_tiles = tile_base[nL];
     const uint32_t lt = lanemask_lt();
@@ -1606,8 +1606,8 @@ __global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(Sort
             const uint32_t t2 = t + gridDim.x;
             const uint32_t s2i = find_seg(tile_base, nL, t2);
             const Seg s2 = L[s2i];
-            const uint32_t lo2 = (t2 - tile_base[s2i]) * PART_TILE;
-            const uint32_t len2 = min((uint32_t)PART_TILE, s2.len - lo2);
+            const uint32_t lo2 = (t2 - tile_base[s2i]) * a.tile;
+            const uint32_t len2 = min(a.tile, s2.len - lo2);
             if (GATHER)
                 prefetch_l2(a.idx[0] + s2.start + lo2, (uint64_t)len2 * 4);
             else
@@ -1630,7 +1630,7 @@ __global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(Sort
         sp.pl = sm.spl[0].y & sp.ml;
         const uint32_t tl = t - tile_base[si];
         const uint32_t nt = tile_base[si + 1] - tile_base[si];
-        const uint32_t lo = tl * PART_TILE + w * SUB;
+        const uint32_t lo = tl * a.tile + w * SUB, end = min(s.len, lo + SUB);
         // Keys and their buckets, HALF keys of a lane at a time.
         constexpr int HALF = PART_HALF<GATHER>, MATCH = MATCH_ITEMS<GATHER>;
         const bool kept = GATHER && a.key2 && s.depth == KEY_BYTES;
@@ -1638,6 +1638,7 @@ __global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(Sort
         uint32_t bk[PART_ITEMS];
 #pragma unroll
         for (int h = 0; h < PART_ITEMS; h += HALF) {
+            if (h * 32 >= SUB) break;  // a smaller tile
             const uint32_t e0 = lo + h * 32 + lane;
             Key kk[HALF];
             if (GATHER) {
@@ -1648,16 +1649,16 @@ __global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(Sort
                     // round 1: the keys round 0's gather kept, by string id
 #pragma unroll
                     for (int q = 0; q < HALF; ++q)
-                        if (e0 + q * 32 < s.len) kk[q] = to_key(a.key2[I[e0 + q * 32]]);
+                        if (e0 + q * 32 < end) kk[q] = to_key(a.key2[I[e0 + q * 32]]);
                 } else {
                     uint32_t id[HALF];
-                    gather_keys<HALF>(a, I, s.depth, e0, 32, s.len, kk, id);
+                    gather_keys<HALF>(a, I, s.depth, e0, 32, end, kk, id);
                     // Depth 0 with a.key2 (a fresh round gathered here): also
                     // keep key bytes 16..31 for round 1, as k_gather does.
                     if (save) {
 #pragma unroll
                         for (int q = 0; q < HALF; ++q)
-                            if (e0 + q * 32 < s.len)
+                            if (e0 + q * 32 < end)
                                 a.key2[id[q]] = from_key(
                                     load_key(a.arena, a.arena_bytes,
                                              string_offset(a.offs, a.off_width, id[q]) +
@@ -1666,20 +1667,20 @@ __global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(Sort
                 }
 #pragma unroll
                 for (int q = 0; q < HALF; ++q)
-                    if (e0 + q * 32 < s.len) KW[e0 + q * 32] = from_key(kk[q]);
+                    if (e0 + q * 32 < end) KW[e0 + q * 32] = from_key(kk[q]);
             } else {
                 const ulonglong2 *K = a.keyb(s.flags & SEG_BUF1) + s.start;
 #pragma unroll
                 for (int q = 0; q < HALF; ++q)
-                    if (e0 + q * 32 < s.len) kk[q] = to_key(K[e0 + q * 32]);
+                    if (e0 + q * 32 < end) kk[q] = to_key(K[e0 + q * 32]);
             }
 #pragma unroll
             for (int q = 0; q < HALF; ++q)
-                bk[h + q] = e0 + q * 32 < s.len ? classify(sm, sp, kk[q]) : nb;
+                bk[h + q] = e0 + q * 32 < end ? classify(sm, sp, kk[q]) : nb;
         }
-        if ((kept || save) && lane == 0 && lo < s.len)
+        if ((kept || save) && lane == 0 && lo < end)
             atomicAdd(kept ? &cnt_ctr->window_used : &cnt_ctr->window_saved,
-                      (unsigned long long)min((uint32_t)SUB, s.len - lo));
+                      (unsigned long long)(end - lo));
         // The lanes of the warp that share each key's bucket: for some keys
         // from the match unit, for the others by a ballot per bucket-id bit.
         // The match unit alone (one result every 60 cycles per SM) took 60 % of
@@ -1689,6 +1690,7 @@ __global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(Sort
         // stays stable).
 #pragma unroll
         for (int h = 0; h < PART_ITEMS; h += HALF) {
+            if (h * 32 >= SUB) break;
             uint32_t peers[HALF], sh[HALF];
 #pragma unroll
             for (int q = 0; q < HALF; ++q) {
@@ -1742,7 +1744,7 @@ __global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(Sort
 #pragma unroll
         for (int c = 0; c < PART_ITEMS; ++c) {
             const uint32_t e = lo + c * 32 + lane;
-            if (e < s.len) {
+            if (e < end) {
                 const uint32_t b = bk[c] >> 16;
                 a.bkt[s.start + e] = (b << 12) | (hist[w][b] + (bk[c] & 0xFFFF));
             }
@@ -1799,8 +1801,8 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 2) k_scatter(
             const uint32_t t2 = t + gridDim.x;
             const uint32_t s2i = find_seg(tile_base, nL, t2);
             const Seg s2 = L[s2i];
-            const uint32_t lo2 = (t2 - tile_base[s2i]) * PART_TILE;
-            const uint32_t len2 = min((uint32_t)PART_TILE, s2.len - lo2);
+            const uint32_t lo2 = (t2 - tile_base[s2i]) * a.tile;
+            const uint32_t len2 = min(a.tile, s2.len - lo2);
             const int b2 = s2.flags & SEG_BUF1;
             prefetch_l2(a.keyb(b2) + s2.start + lo2, (uint64_t)len2 * 16);
             prefetch_l2(a.idxb(b2) + s2.start + lo2, (uint64_t)len2 * 4);
@@ -1810,8 +1812,8 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 2) k_scatter(
         const uint32_t nt = tile_base[si + 1] - tile_base[si];
         const uint32_t cmb = cm_base[si];
         const uint32_t seg0 = cm_scan[cmb];
-        const uint32_t lo = tl * PART_TILE;
-        const uint32_t tlen = min((uint32_t)PART_TILE, s.len - lo);
+        const uint32_t lo = tl * a.tile;
+        const uint32_t tlen = min(a.tile, s.len - lo);
         const int ib = s.flags & SEG_BUF1;
         const ulonglong2 *__restrict__ Kin = a.keyb(ib) + s.start + lo;
         const uint32_t *Iin = a.idxb(ib) + s.start;

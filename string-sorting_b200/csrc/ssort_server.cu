@@ -217,6 +217,7 @@ struct ssort_server {
         a.bkt = ctx->ws.bkt;
         a.target_bucket = ctx->target_bucket;
         a.warp8_cap = ctx->warp8_cap;
+        a.tile = part_tile(max_strings);
         a.leaf_cap = max_strings >= LEAF_MIN_N ? LEAF_CAP : SMALL_CAP;
         a.warp1_deep = ctx->warp1_deep;
         a.l2_prefetch = ctx->l2_prefetch ? 1u : 0u;

@@ -102,3 +102,13 @@ def test_partition_classification(sorter, kind):
     p, l = sorter.sort_host(arena, offs)
     rp, rl = pyoracle.oracle_sort(arena, offs)
     assert np.array_equal(p, rp) and np.array_equal(l, rl)
+
+
+@pytest.mark.parametrize("n", [75_775, 75_776, 75_777, 606_208, 606_209])
+def test_tile_size_limits(sorter, n):
+    """Sorts on either side of the sizes at which partition tiles grow (1024,
+    2048 and 4096 strings per tile)."""
+    ss = pyssort.gen_uniform(n, 1, 12, ord("a"), 26, n)
+    p, l = sorter.sort_host(ss.arena, ss.offs)
+    rp, rl = pyoracle.oracle_sort(ss.arena, ss.offs)
+    assert np.array_equal(p, rp) and np.array_equal(l, rl)
