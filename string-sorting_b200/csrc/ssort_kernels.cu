@@ -1180,6 +1180,24 @@ __device__ __forceinline__ uint64_t warp_or64(uint64_t x) {
            __reduce_or_sync(0xffffffffu, (uint32_t)x);
 }
 
+// ---- asynchronous copies into shared memory -----------------------------------
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+// Waits until at most N of this thread's committed copy groups are pending.
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // ---- splitter selection: one CTA per large segment ------------------------
 constexpr int SAMPLE_THREADS = 512;
 static_assert(SAMPLE_THREADS == 1 << 9 && SAMPLES_MAX == SAMPLE_THREADS * 8,
@@ -1224,7 +1242,14 @@ __device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__r
     uint32_t k = (s.len + tb - 1) / tb;
     if (k > a.max_splitters) k = a.max_splitters;
     if (k < 1) k = 1;
-    uint32_t S = next_pow2(8 * (k + 1));
+    // Eight samples per splitter keep a bucket's size within about a third of
+    // its mean.  In a sort that one CTA's time counts in (below LEAF_MIN_N
+    // strings), four do where the most splitters still leave buckets that are
+    // mostly split again: the CTA's sort, the longest part of a level's first
+    // kernel, halves (1 M uniform strings 252 -> 239 us; with four in every
+    // sort 69 M batched strings 4.94 -> 4.97 ms).
+    const uint32_t per = a.n < LEAF_MIN_N && s.len / (k + 1) > 2 * tb ? 4 : 8;
+    uint32_t S = next_pow2(per * (k + 1));
     if (S < 256) S = 256;
     if (S > (uint32_t)SAMPLES_MAX) S = SAMPLES_MAX;
     // Sample i is the string at position pos_of(i) of the segment.  On the
@@ -1234,24 +1259,28 @@ __device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__r
         const uint32_t r = hash32(s.start * 0x9E3779B1u + i * 0x85EBCA77u + s.len);
         return (uint32_t)(((uint64_t)r * s.len) >> 32);
     };
-    constexpr int G = 4;  // samples in flight per thread
+    if (from_arena) {
+        constexpr int G = 4;  // strings in flight per thread
 #pragma unroll 1
-    for (uint32_t e0 = t; e0 < S; e0 += G * SAMPLE_THREADS) {
-        uint32_t at[G];
-        Key kk[G];
+        for (uint32_t e0 = t; e0 < S; e0 += G * SAMPLE_THREADS) {
+            uint32_t at[G], id[G];
+            Key kk[G];
 #pragma unroll
-        for (int q = 0; q < G; ++q) at[q] = s.start + pos_of(e0 + q * SAMPLE_THREADS);
-        if (from_arena) {
-            uint32_t id[G];
+            for (int q = 0; q < G; ++q) at[q] = s.start + pos_of(e0 + q * SAMPLE_THREADS);
             gather_keys_at<G>(a, a.idx[0], s.depth, at, e0, SAMPLE_THREADS, S, kk, id);
-        } else {
 #pragma unroll
             for (int q = 0; q < G; ++q)
-                kk[q] = e0 + q * SAMPLE_THREADS < S ? to_key(K[at[q] - s.start]) : Key{0, 0};
+                if (e0 + q * SAMPLE_THREADS < S) sm.key[e0 + q * SAMPLE_THREADS] = from_key(kk[q]);
         }
+    } else {
+        // all of a thread's reads in flight at once, past the registers
 #pragma unroll
-        for (int q = 0; q < G; ++q)
-            if (e0 + q * SAMPLE_THREADS < S) sm.key[e0 + q * SAMPLE_THREADS] = from_key(kk[q]);
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t e = t + q * SAMPLE_THREADS;
+            if (e < S) cp_async16(sm.key + e, K + pos_of(e));
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
     }
     __syncthreads();
     // The first S / 8 threads order the samples, 8 each.
@@ -1356,41 +1385,33 @@ __device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__r
     const Key s0 = to_key(cands[0]), sl = to_key(cands[u - 1]);
     const uint32_t f = u >= 2 ? clz128(s0.hi ^ sl.hi, s0.lo ^ sl.lo) : 128u;
     if (f < 128) {
-        // The splitters' window bits first (non-decreasing, as the splitters
-        // are sorted), into the values' area, which is free by now; then each
-        // table entry is the number of splitters whose window bits are below
-        // the entry's value (a binary search over those values).
-        uint16_t *wb = reinterpret_cast<uint16_t *>(sm.val);
-        for (uint32_t j = t; j < u; j += SAMPLE_THREADS)
-            wb[j] = (uint16_t)window_bits(to_key(cands[j]), f);
+        // Entry w is the number of splitters whose window bits are below w: a
+        // histogram of the splitters' window bits (in the values' area, which
+        // is free by now) and its exclusive scan, 8 entries per thread.
+        static_assert(TBL_N == SAMPLE_THREADS * 8 && TBL_N <= SAMPLES_MAX, "table entries");
+        uint4 *h = reinterpret_cast<uint4 *>(sm.val + 8 * t);
+        h[0] = h[1] = make_uint4(0, 0, 0, 0);
         __syncthreads();
-        // Thread t fills entries 8t .. 8t + 7 (and one more thread the last
-        // entry): two searches bound the splitters of its 8 window values,
-        // then each entry searches only between them.
+        for (uint32_t j = t; j < u; j += SAMPLE_THREADS)
+            atomicAdd(&sm.val[window_bits(to_key(cands[j]), f)], 1u);
+        __syncthreads();
+        uint32_t e[8], sum = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t x = sm.val[8 * t + i];
+            e[i] = sum;
+            sum += x;
+        }
+        uint32_t total;
+        const uint32_t before =
+            cta_inclusive_scan<SAMPLE_THREADS>(sum, total, sm.warp_cnt) - sum;
         uint16_t *T = tbl + (uint64_t)si * TBL_STRIDE;
-        auto lower = [&](uint32_t lo, uint32_t hi, uint32_t wv) -> uint32_t {
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (wb[mid] < wv)
-                    lo = mid + 1;
-                else
-                    hi = mid;
-            }
-            return lo;
-        };
-        static_assert(TBL_N == SAMPLE_THREADS * 8, "table entries per thread");
-        const uint32_t w0 = t * 8;
-        uint32_t lo = lower(0, u, w0);
-        const uint32_t hi = lower(lo, u, w0 + 8);
         uint32_t tv[4];
 #pragma unroll
-        for (int i = 0; i < 8; i += 2) {
-            const uint32_t t0 = lower(lo, hi, w0 + i);
-            lo = lower(t0, hi, w0 + i + 1);
-            tv[i / 2] = t0 | (lo << 16);
-        }
-        *reinterpret_cast<uint4 *>(T + w0) = make_uint4(tv[0], tv[1], tv[2], tv[3]);
-        if (t == 0) T[TBL_N] = (uint16_t)lower(0, u, TBL_N);
+        for (int i = 0; i < 8; i += 2)
+            tv[i / 2] = (before + e[i]) | (before + e[i + 1]) << 16;
+        *reinterpret_cast<uint4 *>(T + 8 * t) = make_uint4(tv[0], tv[1], tv[2], tv[3]);
+        if (t == 0) T[TBL_N] = (uint16_t)u;
     }
     if (t == 0) {
         nspl[si] = u | (f << 16);
@@ -1421,23 +1442,34 @@ __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
     __syncthreads();
     if (!sm.last) return;
     __threadfence();
-    uint32_t c0 = 0, c1 = 0;
+    // both scans at once: tiles in the upper half, matrix entries in the lower
+    uint64_t carry = 0;
     for (uint32_t b = 0; b < nL; b += SAMPLE_THREADS) {
         const uint32_t i = b + t;
-        const uint32_t v0 = i < nL ? __ldcg(lb.ntiles + i) : 0;
-        const uint32_t v1 = i < nL ? __ldcg(lb.cm_size + i) : 0;
-        uint32_t t0, t1;
-        const uint32_t s0 = cta_inclusive_scan<SAMPLE_THREADS>(v0, t0, sm.warp_cnt);
-        const uint32_t s1 = cta_inclusive_scan<SAMPLE_THREADS>(v1, t1, sm.warp_cnt);
-        if (i < nL) {
-            lb.tile_base[i] = c0 + s0 - v0;
-            lb.cm_base[i] = c1 + s1 - v1;
+        const uint64_t v =
+            i < nL ? (uint64_t)__ldcg(lb.ntiles + i) << 32 | __ldcg(lb.cm_size + i) : 0;
+        uint64_t x = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint64_t y = __shfl_up_sync(0xffffffffu, x, d);
+            if ((t & 31) >= (uint32_t)d) x += y;
         }
-        c0 += t0;
-        c1 += t1;
+        if ((t & 31) == 31) sm.red[t >> 5][0] = x;
+        __syncthreads();
+        uint64_t before = carry;
+        for (uint32_t q = 0; q < SAMPLE_THREADS / 32; ++q) {
+            if (q < t >> 5) before += sm.red[q][0];
+            carry += sm.red[q][0];
+        }
+        __syncthreads();
+        if (i < nL) {
+            lb.tile_base[i] = (uint32_t)((before + x - v) >> 32);
+            lb.cm_base[i] = (uint32_t)(before + x - v);
+        }
     }
+    const uint32_t c1 = (uint32_t)carry;
     if (t == 0) {
-        lb.tile_base[nL] = c0;
+        lb.tile_base[nL] = (uint32_t)(carry >> 32);
         lb.cm_base[nL] = c1;
         c->sample_ticket = 0;
     }
@@ -2296,24 +2328,6 @@ __global__ void __launch_bounds__(WARP_THREADS) k_warp1(SortArgs a, const Seg *_
     }
     deep = warp_sum(deep);
     if (lane == 0 && deep) atomicAdd(&c->warp1_deep, deep);
-}
-
-// ---- asynchronous copies into shared memory -----------------------------------
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-// Waits until at most N of this thread's committed copy groups are pending.
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // ---- segments of 33..4096 strings: a group of threads each ------------------
