@@ -98,7 +98,6 @@ constexpr uint64_t most_tiles(uint64_t n) {
 
 constexpr int GATHER_TILE = 4096;
 constexpr int GATHER_THREADS = 256;
-constexpr int GATHER_ITEMS = 8;
 constexpr int EQ_TILE = 8192;
 
 struct Counters {

@@ -846,16 +846,26 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t *in, 
 }
 
 // ---- key gather for large segments ----------------------------------------
-__global__ void __launch_bounds__(GATHER_THREADS) k_gather(SortArgs a, const Seg *__restrict__ L,
-                                                          Count cnt,
-                                                          const uint32_t *__restrict__ tile_base,
-                                                          Counters *ctr) {
+// KEEP (a.key2 given): depth 0 also keeps key bytes 16..31 for round 1 (their
+// sectors are read here anyway), depth 16 reads those copies.
+// Bound by memory: index, offset, the strings' sectors and the 16 (KEEP: 32)
+// bytes written.  Without copies, 4 strings a thread and 8 CTAs per SM keep
+// more reads in flight than 8 strings in 4 CTAs: 100 M words 0.92 -> 0.73 ms
+// (5.2 TB/s), a 16 MB text's suffixes 127 -> 97 us.  With copies the longer
+// batches stay the faster form: 50 M URLs 0.86 ms, with 4 strings a thread 0.94.
+// Reading both key words of a batch before the first use took 1.0 and 1.4 ms
+// (80 registers, 3 CTAs).
+template <bool KEEP>
+__global__ void __launch_bounds__(GATHER_THREADS, KEEP ? 4 : 8)
+    k_gather(SortArgs a, const Seg *__restrict__ L, Count cnt,
+             const uint32_t *__restrict__ tile_base, Counters *ctr) {
     after_predecessor();
     const uint32_t nL = count_of(cnt);
-    constexpr int U = GATHER_ITEMS;
-    static_assert(GATHER_TILE % (GATHER_THREADS * GATHER_ITEMS) == 0, "tile shape");
-    const uint32_t total_tiles = tile_base[nL] * (GATHER_TILE / (GATHER_THREADS * U));
+    constexpr int U = KEEP ? 8 : 4;
+    static_assert(GATHER_TILE % (GATHER_THREADS * U) == 0, "tile shape");
     constexpr uint32_t SUBT = GATHER_TILE / (GATHER_THREADS * U);
+    const uint32_t total_tiles = tile_base[nL] * SUBT;
+    unsigned long long n_save = 0, n_used = 0;
     for (uint32_t t2 = blockIdx.x; t2 < total_tiles; t2 += gridDim.x) {
         const uint32_t t = t2 / SUBT;
         const uint32_t si = find_seg(tile_base, nL, t);
@@ -863,10 +873,7 @@ __global__ void __launch_bounds__(GATHER_THREADS) k_gather(SortArgs a, const Seg
         const uint32_t lo = (t - tile_base[si]) * GATHER_TILE + (t2 % SUBT) * GATHER_THREADS * U;
         if (lo >= s.len) continue;
         const uint32_t *I = a.idx[0];
-        // Depth 0 with a.key2: also keep key bytes 16..31 for round 1 (their
-        // sectors are read here anyway); depth 16: read those copies.
-        const bool save = a.key2 && s.depth == 0;
-        const bool saved = a.key2 && s.depth == KEY_BYTES;
+        const bool save = KEEP && s.depth == 0, saved = KEEP && s.depth == KEY_BYTES;
         uint32_t id[U];
         uint64_t off[U];
 #pragma unroll
@@ -891,11 +898,14 @@ __global__ void __launch_bounds__(GATHER_THREADS) k_gather(SortArgs a, const Seg
                 ++kept;
             }
         }
-        if (save || saved) {
-            const unsigned long long k = warp_sum((unsigned long long)kept);
-            if ((threadIdx.x & 31) == 0 && k)
-                atomicAdd(save ? &ctr->window_saved : &ctr->window_used, k);
-        }
+        if (save) n_save += kept;
+        if (saved) n_used += kept;
+    }
+    if (KEEP) {
+        n_save = warp_sum(n_save);
+        n_used = warp_sum(n_used);
+        if ((threadIdx.x & 31) == 0 && n_save) atomicAdd(&ctr->window_saved, n_save);
+        if ((threadIdx.x & 31) == 0 && n_used) atomicAdd(&ctr->window_used, n_used);
     }
 }
 
@@ -3429,7 +3439,8 @@ void launch_scan(const uint32_t *in, uint32_t *out, uint32_t cap, Count n, uint3
 void launch_gather(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
                    Counters *c, int grid, cudaStream_t st) {
     if (!nL.dev && !nL.host) return;
-    launch_next(k_gather, grid, GATHER_THREADS, 0, st, a, L, nL, tile_base, c);
+    launch_next(a.key2 ? k_gather<true> : k_gather<false>, grid, GATHER_THREADS, 0, st, a, L, nL,
+                tile_base, c);
 }
 
 void launch_sample(const SortArgs &a, const Seg *L, Count nL, ulonglong2 *spl, uint32_t *nspl,

@@ -61,3 +61,15 @@ def test_repeated_and_interleaved_contexts():
                 sa, sb = _check(a, s), _check(b, s[::-1])
                 assert sa.live[0] == sb.live[0] == len(s)
                 assert sa.rounds == sb.rounds
+
+
+@pytest.mark.parametrize("n", [4096, 4097, 8191, 9215, 9217])
+def test_separate_gather(n):
+    """The key gather as a kernel of its own at the edges of its 4096-string
+    tiles and 1024-string steps, two rounds deep."""
+    rng = np.random.default_rng(n)
+    strings = [bytes(rng.integers(97, 99, size=rng.integers(0, 24)).tolist()) for _ in range(n)]
+    with pyssort.Sorter(0) as s:
+        s.set_param(pyssort.SSORT_PARAM_FUSED_GATHER, 0)
+        st = _check(s, strings)
+    assert st.gather_fused == 0 and st.partitioned > 0
