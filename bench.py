@@ -225,13 +225,13 @@ KB = 16  # key bytes per round
 # L2 until a later kernel evicts them are not counted here.
 TRAFFIC_WORKLOAD = "urls_50m"
 TRAFFIC_PER_STRING = {
-    "count_gather": 120.3,  # round 1 from the kept copies, round 2 random offset + key reads
+    "count_gather": 128.3,  # round 1 from the kept copies, round 2 random offset + key reads
     "gather": 95.0,         # round 0: the arena streamed in order, bytes 16..31 kept
-    "count": 17.9,
-    "scatter": 36.3,
-    "block": 57.2,
-    "warp8": 195.0,
-    "warp1": 261.0,
+    "count": 17.8,
+    "scatter": 37.1,
+    "block": 60.6,
+    "warp8": 203.5,
+    "warp1": 260.0,
 }
 
 

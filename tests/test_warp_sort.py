@@ -1,4 +1,4 @@
-"""The one-warp sort of 33..1024 strings (squeezed 32-bit values): segment
+"""The on-chip sorts of 33..4096 strings (squeezed 32-bit values): segment
 sizes at the edges of its size classes, and key sets that reach each of its
 branches (no ties, tied runs in order, short and long tied runs out of
 order, all keys equal, runs that continue in the next round)."""
