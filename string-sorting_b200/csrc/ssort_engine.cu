@@ -407,9 +407,12 @@ int ssort_ctx::run_ws(const uint8_t *arena_p, uint64_t arena_bytes, const void *
         classified = false;
     } else {
         // The only segment is a large one: its list entry and counts are known.
+        // Identity indices are written only where a first level that gathers
+        // its own keys reads them (round_body decides by the same rule).
+        const bool reads_idx = gather_fused(fused_gather, round_mode <= 0, n);
         LAUNCH(this, "begin",
-               launch_begin(d_perm, n, a.lcp, ws.rc, Seg{0, n, 0, 0}, ws.L, &ws.rc->c[0].n_large,
-                            st));
+               launch_begin(d_perm, reads_idx ? n : 0, a.lcp, ws.rc, Seg{0, n, 0, SEG_IOTA}, ws.L,
+                            &ws.rc->c[0].n_large, st));
         *h_ctr = Counters{};
         h_ctr->n_large = 1;
         h_ctr->live_next = h_ctr->gather_elems = n;

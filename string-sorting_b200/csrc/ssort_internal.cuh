@@ -28,6 +28,12 @@ constexpr uint32_t KEY_BYTES = 16;
 // Seg.flags
 constexpr uint32_t SEG_BUF1 = 1u;   // idx/keys of this segment live in buffer 1
 constexpr uint32_t SEG_KEYS = 2u;   // key[buf] already holds this depth's keys
+// Round 0: the index at position p is p.  The separate gather and the scatter
+// count instead of reading idx[0], which then need not be written for a sort
+// whose only segment is gathered that way.  12 bytes per string saved: 100 M
+// words 6.28 -> 6.20 ms, 50 M URLs 6.88 -> 6.81, a batch of 55 M strings (whose
+// small instances still read idx[0]) 4.82 -> 4.76.
+constexpr uint32_t SEG_IOTA = 4u;
 constexpr uint32_t SEG_CHUNK_SHIFT = 8;  // equality work items: chunk index << 8
 
 struct Seg {
@@ -361,9 +367,10 @@ inline Workspace ws_bind(const WsLayout &o, unsigned char *base) {
 }
 
 // ---- launchers (ssort_kernels.cu) ----------------------------------------
-// Start of a sort: idx = identity, lcp[0] = 0, counters cleared; with first.len
-// also the first round's only segment, appended to *list (counter *count).
-void launch_begin(uint32_t *idx, uint32_t n, uint32_t *lcp, RoundCounters *rc, Seg first,
+// Start of a sort: idx[0..n_idx) = identity, lcp[0] = 0, counters cleared; with
+// first.len also the first round's only segment, appended to *list (counter
+// *count).
+void launch_begin(uint32_t *idx, uint32_t n_idx, uint32_t *lcp, RoundCounters *rc, Seg first,
                   Seg *list, uint32_t *count, cudaStream_t st);
 void launch_iota(uint32_t *idx, uint32_t n, cudaStream_t st);
 // A whole sort of at most SMALL_CAP strings by one CTA (k_tiny); A, B: segment

@@ -351,16 +351,17 @@ __device__ __forceinline__ bool publish(const Publish &p, RoundCounters *rc) {
     return true;
 }
 
-__global__ void k_begin(uint32_t *idx, uint32_t n, uint32_t *lcp, RoundCounters *rc, Seg first,
-                        Seg *list, uint32_t *count) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+__global__ void k_begin(uint32_t *idx, uint32_t n_idx, uint32_t *lcp, RoundCounters *rc,
+                        Seg first, Seg *list, uint32_t *count) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_idx;
+         i += gridDim.x * blockDim.x)
         idx[i] = i;
     if (blockIdx.x != 0) return;
     uint32_t *w = reinterpret_cast<uint32_t *>(rc);
     for (uint32_t i = threadIdx.x; i < sizeof(RoundCounters) / 4; i += blockDim.x) w[i] = 0;
     __syncthreads();
     if (threadIdx.x != 0) return;
-    if (n) lcp[0] = 0;
+    if (n_idx || first.len) lcp[0] = 0;
     if (first.len) {
         *list = first;
         *count = 1;
@@ -387,7 +388,7 @@ __global__ void k_init_batch(const uint32_t *__restrict__ inst_start, uint32_t n
     if (v && e > s) lcp[s] = 0;
     const bool seg = v && e - s >= 2;
     const uint32_t slot = warp_append(&c->n_next, seg);
-    if (seg) R[slot] = Seg{s, e - s, 0, 0};
+    if (seg) R[slot] = Seg{s, e - s, 0, SEG_IOTA};
 }
 
 // The three kernels below give every position the instance or request it lies
@@ -874,12 +875,13 @@ __global__ void __launch_bounds__(GATHER_THREADS, KEEP ? 4 : 8)
         if (lo >= s.len) continue;
         const uint32_t *I = a.idx[0];
         const bool save = KEEP && s.depth == 0, saved = KEEP && s.depth == KEY_BYTES;
+        const bool iota = s.flags & SEG_IOTA;
         uint32_t id[U];
         uint64_t off[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint32_t i = lo + u * GATHER_THREADS + threadIdx.x;
-            id[u] = i < s.len ? I[s.start + i] : IDX_MAX;
+            id[u] = i >= s.len ? IDX_MAX : iota ? s.start + i : I[s.start + i];
         }
 #pragma unroll
         for (int u = 0; u < U; ++u)
@@ -1847,7 +1849,8 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 2) k_scatter(
             const uint32_t len2 = min(a.tile, s2.len - lo2);
             const int b2 = s2.flags & SEG_BUF1;
             prefetch_l2(a.keyb(b2) + s2.start + lo2, (uint64_t)len2 * 16);
-            prefetch_l2(a.idxb(b2) + s2.start + lo2, (uint64_t)len2 * 4);
+            if (!(s2.flags & SEG_IOTA))
+                prefetch_l2(a.idxb(b2) + s2.start + lo2, (uint64_t)len2 * 4);
             prefetch_l2(a.bkt + s2.start + lo2, (uint64_t)len2 * 4);
         }
         const uint32_t tl = t - tile_base[si];
@@ -1859,13 +1862,14 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 2) k_scatter(
         const int ib = s.flags & SEG_BUF1;
         const ulonglong2 *__restrict__ Kin = a.keyb(ib) + s.start + lo;
         const uint32_t *Iin = a.idxb(ib) + s.start;
+        const bool iota = s.flags & SEG_IOTA;
         const uint32_t *Din = a.bkt + s.start;
         uint32_t ii[SCATTER_ITEMS], dd[SCATTER_ITEMS];
 #pragma unroll
         for (int c = 0; c < SCATTER_ITEMS; ++c) {
             const uint32_t e = c * SCATTER_THREADS + threadIdx.x;
             if (e < tlen) {
-                ii[c] = Iin[lo + e];
+                ii[c] = iota ? s.start + lo + e : Iin[lo + e];
                 dd[c] = Din[lo + e];
             }
         }
@@ -3317,10 +3321,10 @@ static int grid_of(int grid, const Count &n, uint32_t per, uint32_t cap) {
     return (int)(g < cap ? g : cap);
 }
 
-void launch_begin(uint32_t *idx, uint32_t n, uint32_t *lcp, RoundCounters *rc, Seg first,
+void launch_begin(uint32_t *idx, uint32_t n_idx, uint32_t *lcp, RoundCounters *rc, Seg first,
                   Seg *list, uint32_t *count, cudaStream_t st) {
-    const uint32_t g = cdiv(n, 256) < 148 * 16 ? cdiv(n, 256) : 148 * 16;
-    k_begin<<<g ? g : 1, 256, 0, st>>>(idx, n, lcp, rc, first, list, count);
+    const uint32_t g = cdiv(n_idx, 256) < 148 * 16 ? cdiv(n_idx, 256) : 148 * 16;
+    k_begin<<<g ? g : 1, 256, 0, st>>>(idx, n_idx, lcp, rc, first, list, count);
 }
 
 void launch_tiny(const SortArgs &a, Seg *A, Seg *B, RoundCounters *rc, Publish pub,

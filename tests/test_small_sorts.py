@@ -73,3 +73,24 @@ def test_separate_gather(n):
         s.set_param(pyssort.SSORT_PARAM_FUSED_GATHER, 0)
         st = _check(s, strings)
     assert st.gather_fused == 0 and st.partitioned > 0
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+def test_batch_with_separate_gather(graph):
+    """Large instances whose indices the first level counts, beside small ones
+    that read them: several starts, tile remainders and empty instances."""
+    rng = np.random.default_rng(17)
+    sizes = [5000, 0, 1, 4097, 300, 9217, 2, 2049, 0, 2048, 33]
+    inst = np.concatenate([[0], np.cumsum(sizes)]).astype(np.uint32)
+    strings = [bytes(rng.integers(97, 99, size=rng.integers(0, 24)).tolist())
+               for _ in range(int(inst[-1]))]
+    arena, offs = cases.arena_of(strings)
+    with pyssort.Sorter(0) as s:
+        s.set_param(pyssort.SSORT_PARAM_FUSED_GATHER, 0)
+        s.set_param(pyssort.SSORT_PARAM_GRAPH, graph)
+        p, l = s.sort_batch_host(arena, offs, inst)
+    for a, b in zip(inst[:-1], inst[1:]):
+        if a == b:
+            continue
+        rp, rl = pyoracle.oracle_sort(arena, offs[a:b])
+        assert np.array_equal(p[a:b], rp) and np.array_equal(l[a:b], rl)
