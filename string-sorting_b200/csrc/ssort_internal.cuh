@@ -31,7 +31,7 @@ constexpr uint32_t SEG_KEYS = 2u;   // key[buf] already holds this depth's keys
 // Round 0: the index at position p is p.  The separate gather and the scatter
 // count instead of reading idx[0], which then need not be written for a sort
 // whose only segment is gathered that way.  12 bytes per string saved: 100 M
-// words 6.28 -> 6.20 ms, 50 M URLs 6.88 -> 6.81, a batch of 55 M strings (whose
+// words 6.28 -> 6.20 ms, 50 M URLs 6.88 -> 6.81, a batch of 69 M strings (whose
 // small instances still read idx[0]) 4.82 -> 4.76.
 constexpr uint32_t SEG_IOTA = 4u;
 constexpr uint32_t SEG_CHUNK_SHIFT = 8;  // equality work items: chunk index << 8
