@@ -253,7 +253,8 @@ def kernel_bytes(st, w):
     (16); later levels' count reads keys (16); scatter reads and writes key+idx
     (2x20); on-chip sorts read idx (4) + offset (w) + key bytes when they
     gather themselves, or key+idx (20) otherwise, and write idx + lcp (8);
-    equality buckets copy idx (8) and/or write lcp (4)."""
+    equality buckets copy idx (8) and/or write lcp (4).  Round 0's indices are
+    included where the kernels count them instead of reading them."""
     def sort_bytes(fresh, keyed):
         return fresh * (4 + w + KB) + keyed * (KB + 4) + (fresh + keyed) * 8
     # Round 0's gather may also keep key bytes 16..31 per string (read 16 more,
