@@ -28,10 +28,16 @@ constexpr uint32_t IDX_MAX = ~0u;
 // ---- kernels launched before their predecessor has ended -----------------------
 // The kernels of a round follow each other on one stream, each needing all of
 // what the last one wrote, and in small sorts most of them are short.  They are
-// launched with programmatic stream serialization, so that a kernel's CTAs
-// are set up while its predecessor's last ones run, and wait here, before
-// their first access to memory, until it has ended: 1 M uniform strings 267 ->
-// 254 us, 20 k URLs 277 -> 259 us, 3 M URLs 920 -> 885 us.
+// launched with programmatic stream serialization and wait here, before their
+// first access to what a sort writes, until the predecessor has ended.  No kernel
+// signals early, so a successor's CTAs start once every CTA of the predecessor
+// has exited; what overlaps their start is the predecessor's final flush and
+// the stream's hand-over: 1 M uniform strings 267 -> 254 us, 20 k URLs 277 ->
+// 259 us, 3 M URLs 920 -> 885 us.
+// Such a kernel's lifetime begins before its inputs are complete.  Everything
+// that a sort writes is therefore read by ordinary loads: no __ldg and no
+// const __restrict__ pointer, whose read-only loads the compiler may also move
+// above the wait.  The arena and the offsets are inputs and may use them.
 __device__ __forceinline__ void after_predecessor() { cudaGridDependencySynchronize(); }
 
 // ---- 16-byte keys -----------------------------------------------------------
@@ -166,7 +172,7 @@ __device__ __forceinline__ uint32_t find_seg(const uint32_t *base, uint32_t n, u
     while (n > 1) {
         const uint32_t step = (n + 31) / 32, i = (threadIdx.x & 31) * step;
         const uint32_t below =
-            __ballot_sync(0xffffffffu, i < n && __ldg(base + lo + i) <= t);  // a prefix, lane 0 set
+            __ballot_sync(0xffffffffu, i < n && base[lo + i] <= t);  // a prefix, lane 0 set
         const uint32_t at = (31 - __clz(below)) * step;
         lo += at;
         n = min(step, n - at);
@@ -305,7 +311,7 @@ __device__ __forceinline__ void append_by_length(const Seg &o, bool v, uint32_t 
     if (lg) L[tl] = o;
 }
 
-__device__ __forceinline__ void classify_list(const Seg *__restrict__ R, uint32_t nR,
+__device__ __forceinline__ void classify_list(const Seg *R, uint32_t nR,
                                               uint32_t warp8_cap, Seg *W1, Seg *W8,
                                               const SmallLists &S, Seg *L, Counters *c) {
     // Block-uniform trip count: every warp reaches the collective appends.
@@ -750,7 +756,7 @@ __device__ __forceinline__ uint32_t cta_inclusive_scan(uint32_t v, uint32_t &tot
 }
 
 // out = exclusive scan of ceil(len / tile) over the segments; out[n] = total.
-__global__ void __launch_bounds__(SMALL_SCAN_THREADS) k_seg_tiles(const Seg *__restrict__ segs,
+__global__ void __launch_bounds__(SMALL_SCAN_THREADS) k_seg_tiles(const Seg *segs,
                                                                    Count cnt, uint32_t tile,
                                                                    uint32_t *out) {
     after_predecessor();
@@ -872,8 +878,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(const uint32_t *in, 
 // (80 registers, 3 CTAs).
 template <bool KEEP>
 __global__ void __launch_bounds__(GATHER_THREADS, KEEP ? 4 : 8)
-    k_gather(SortArgs a, const Seg *__restrict__ L, Count cnt,
-             const uint32_t *__restrict__ tile_base, Counters *ctr) {
+    k_gather(SortArgs a, const Seg *L, Count cnt,
+             const uint32_t *tile_base, Counters *ctr) {
     after_predecessor();
     const uint32_t nL = count_of(cnt);
     constexpr int U = KEEP ? 8 : 4;
@@ -1256,7 +1262,7 @@ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
 // 35 us).  The order only picks quantiles: samples that tie on 20 to 24
 // differing bits may stand in any order, and the chosen candidates are put in
 // full-key order below.
-__device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__restrict__ L,
+__device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *L,
                                                uint32_t si, SampleSmem &sm, ulonglong2 *spl,
                                                uint32_t *nspl, uint16_t *tbl, uint32_t *ntiles,
                                                uint32_t *cm_size, bool from_arena) {
@@ -1452,7 +1458,7 @@ __device__ __forceinline__ void sample_segment(const SortArgs &a, const Seg *__r
 // sizes into bases (exclusive scans, totals at [nL]) and clears the look-back
 // scan's state for the level's total: two launches less per level.
 __global__ void __launch_bounds__(SAMPLE_THREADS, 2)
-    k_sample(SortArgs a, const Seg *__restrict__ L, Count cnt, ulonglong2 *spl, uint32_t *nspl,
+    k_sample(SortArgs a, const Seg *L, Count cnt, ulonglong2 *spl, uint32_t *nspl,
              uint16_t *tbl, LevelBases lb, bool from_arena, Counters *c) {
     after_predecessor();
     extern __shared__ __align__(16) unsigned char sample_smem[];
@@ -1542,8 +1548,8 @@ struct Splitters {
 };
 
 // Splitters, their windows and (when f < 128) the lookup table of segment si.
-__device__ __forceinline__ void load_splitters(PartSmem &sm, const ulonglong2 *__restrict__ spl,
-                                               const uint16_t *__restrict__ tbl, uint32_t si,
+__device__ __forceinline__ void load_splitters(PartSmem &sm, const ulonglong2 *spl,
+                                               const uint16_t *tbl, uint32_t si,
                                                uint32_t u, uint32_t f) {
     for (uint32_t q = threadIdx.x; q < u; q += PART_THREADS) {
         const ulonglong2 x = spl[(uint64_t)si * SPL_STRIDE + q];
@@ -1634,13 +1640,13 @@ struct TileQueue {
 // arena through idx and offsets and stored to the key buffer here, so the
 // key gather's random arena reads overlap the classification work.
 template <bool GATHER>
-__global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(SortArgs a, const Seg *__restrict__ L,
+__global__ void __launch_bounds__(PART_THREADS, COUNT_CTAS<GATHER>) k_count(SortArgs a, const Seg *L,
                                                         Count cnt,
-                                                        const uint32_t *__restrict__ tile_base,
-                                                        const ulonglong2 *__restrict__ spl,
-                                                        const uint32_t *__restrict__ nspl,
-                                                        const uint16_t *__restrict__ tbl,
-                                                        const uint32_t *__restrict__ cm_base,
+                                                        const uint32_t *tile_base,
+                                                        const ulonglong2 *spl,
+                                                        const uint32_t *nspl,
+                                                        const uint16_t *tbl,
+                                                        const uint32_t *cm_base,
                                                         uint32_t *cm, Counters *cnt_ctr) {
     after_predecessor();
     extern __shared__ __align__(16) unsigned char part_smem[];
@@ -1839,9 +1845,9 @@ struct ScatterSmem {
 constexpr int SCATTER_BATCH = 4;  // keys in flight per thread in the write-out
 
 __global__ void __launch_bounds__(SCATTER_THREADS, 2) k_scatter(
-    SortArgs a, const Seg *__restrict__ L, Count cnt, const uint32_t *__restrict__ tile_base,
-    const uint32_t *__restrict__ nspl, const uint32_t *__restrict__ cm_base,
-    const uint32_t *__restrict__ cm_scan, Counters *ctr) {
+    SortArgs a, const Seg *L, Count cnt, const uint32_t *tile_base,
+    const uint32_t *nspl, const uint32_t *cm_base,
+    const uint32_t *cm_scan, Counters *ctr) {
     after_predecessor();
     extern __shared__ __align__(16) unsigned char scatter_smem[];
     ScatterSmem &sm = *reinterpret_cast<ScatterSmem *>(scatter_smem);
@@ -1874,7 +1880,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 2) k_scatter(
         const uint32_t lo = tl * a.tile;
         const uint32_t tlen = min(a.tile, s.len - lo);
         const int ib = s.flags & SEG_BUF1;
-        const ulonglong2 *__restrict__ Kin = a.keyb(ib) + s.start + lo;
+        const ulonglong2 *Kin = a.keyb(ib) + s.start + lo;
         const uint32_t *Iin = a.idxb(ib) + s.start;
         const bool iota = s.flags & SEG_IOTA;
         const uint32_t *Din = a.bkt + s.start;
@@ -1937,7 +1943,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 2) k_scatter(
 #pragma unroll
             for (int q = 0; q < SCATTER_BATCH; ++q) {
                 const uint32_t i = i0 + q * SCATTER_THREADS + threadIdx.x;
-                if (i < tlen) kv[q] = __ldg(Kin + sm.src[i]);
+                if (i < tlen) kv[q] = Kin[sm.src[i]];
             }
 #pragma unroll
             for (int q = 0; q < SCATTER_BATCH; ++q) {
@@ -1960,10 +1966,10 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 2) k_scatter(
 // buckets (26 -> 8 us for one segment).
 constexpr int EMIT_THREADS = 256;
 constexpr int EMIT_CHUNKS = (NB_MAX + EMIT_THREADS) / EMIT_THREADS;
-__global__ void k_emit(SortArgs a, const Seg *__restrict__ L, Count cnt,
-                       const uint32_t *__restrict__ tile_base,
-                       const uint32_t *__restrict__ nspl, const uint32_t *__restrict__ cm_base,
-                       const uint32_t *__restrict__ cm_scan, Seg *W1, Seg *W8, SmallLists S,
+__global__ void k_emit(SortArgs a, const Seg *L, Count cnt,
+                       const uint32_t *tile_base,
+                       const uint32_t *nspl, const uint32_t *cm_base,
+                       const uint32_t *cm_scan, Seg *W1, Seg *W8, SmallLists S,
                        Seg *L2, Seg *E, uint2 *B, Seg *N, Counters *c, RoundCounters *rc,
                        Publish pub) {
     after_predecessor();
@@ -2323,11 +2329,11 @@ __device__ __forceinline__ uint32_t warp1_group(const SortArgs &a, const Seg &s,
 // remaining segment.
 constexpr uint32_t W1_PACK = 4;
 
-__global__ void __launch_bounds__(WARP_THREADS) k_warp1(SortArgs a, const Seg *__restrict__ T0,
+__global__ void __launch_bounds__(WARP_THREADS) k_warp1(SortArgs a, const Seg *T0,
                                                         Span sp, Seg *N, Counters *c) {
     after_predecessor();
     const uint32_t lo = count_of(sp.lo);
-    const Seg *__restrict__ T = T0 + lo;
+    const Seg *T = T0 + lo;
     const uint32_t nT = count_of(sp.hi) - lo;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -2814,7 +2820,7 @@ __device__ __forceinline__ bool sort_segment(const G &g, const SortArgs &a, cons
 // thread group grp.
 template <class G>
 __device__ __forceinline__ void sort_list(const G &grp, const SortArgs &a,
-                                          const Seg *__restrict__ T, uint32_t nT, uint32_t first,
+                                          const Seg *T, uint32_t nT, uint32_t first,
                                           uint32_t step, const SegMem &sm, Seg *N, Counters *c) {
     unsigned long long fresh = 0, keyed = 0, full = 0;
     for (uint32_t g = first; g < nT; g += step) {
@@ -2836,7 +2842,7 @@ __device__ __forceinline__ void sort_list(const G &grp, const SortArgs &a,
 constexpr size_t WARPSORT_SMEM = SMALL_THREADS / 32 * seg_bytes(32);
 
 __global__ void __launch_bounds__(SMALL_THREADS, 4)
-    k_warpsort(SortArgs a, const Seg *__restrict__ T0, Span sp, Seg *N, Counters *c) {
+    k_warpsort(SortArgs a, const Seg *T0, Span sp, Seg *N, Counters *c) {
     after_predecessor();
     extern __shared__ __align__(16) unsigned char seg_smem[];
     const uint32_t lo = count_of(sp.lo), w = threadIdx.x / 32, per = SMALL_THREADS / 32;
@@ -2862,7 +2868,7 @@ __global__ void __launch_bounds__(SEG_CTA, 2)
     while (k + 1 < SMALL_CLASSES && blockIdx.x >= wk.cta[k + 1]) ++k;
     const uint32_t log2_threads = 6 + k, per = SEG_CTA >> log2_threads;
     const uint32_t lo = count_of(wk.span[k].lo), nT = count_of(wk.span[k].hi) - lo;
-    const Seg *__restrict__ T = wk.list.s[k] + lo;
+    const Seg *T = wk.list.s[k] + lo;
     const uint32_t gi = threadIdx.x >> log2_threads;
     const CtaGroup<> grp{threadIdx.x & ((1u << log2_threads) - 1), log2_threads, 1 + gi};
     const SegMem sm = seg_mem(seg_smem + gi * seg_bytes(grp.threads()), grp.threads());
@@ -2882,7 +2888,7 @@ constexpr size_t CLASS_SMEM = SEG_CTA / (64 << K) * seg_bytes(64 << K);
 
 template <int K>
 __global__ void __launch_bounds__(SEG_CTA, 2)
-    k_segsort_class(SortArgs a, const Seg *__restrict__ T0, Span sp, Seg *N, Counters *c) {
+    k_segsort_class(SortArgs a, const Seg *T0, Span sp, Seg *N, Counters *c) {
     after_predecessor();
     extern __shared__ __align__(16) unsigned char seg_smem[];
     constexpr uint32_t GT = 64u << K, per = SEG_CTA / GT;
@@ -2896,10 +2902,10 @@ __global__ void __launch_bounds__(SEG_CTA, 2)
 // Bound by memory (12 bytes per string).  A thread's four reads go out before
 // its stores, which the compiler may not pass: 3 M URLs 61 -> 40 us, 100 M
 // words 237 -> 231 us (4.4 TB/s); eight in flight 262.
-__global__ void k_equal(SortArgs a, const Seg *__restrict__ E0, Span sp, Seg *N, Counters *c) {
+__global__ void k_equal(SortArgs a, const Seg *E0, Span sp, Seg *N, Counters *c) {
     after_predecessor();
     const uint32_t lo = count_of(sp.lo);
-    const Seg *__restrict__ E = E0 + lo;
+    const Seg *E = E0 + lo;
     const uint32_t nE = count_of(sp.hi) - lo;
     unsigned long long moved = 0, fin = 0;
     for (uint32_t g = blockIdx.x; g < nE; g += gridDim.x) {
@@ -2942,7 +2948,7 @@ __global__ void k_equal(SortArgs a, const Seg *__restrict__ E0, Span sp, Seg *N,
     }
 }
 
-__device__ __forceinline__ void boundary_lcps(const SortArgs &a, const uint2 *__restrict__ B,
+__device__ __forceinline__ void boundary_lcps(const SortArgs &a, const uint2 *B,
                                               uint32_t nB) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nB; i += gridDim.x * blockDim.x) {
         const uint2 e = B[i];
@@ -2957,7 +2963,7 @@ __global__ void k_boundary(SortArgs a, const uint2 *__restrict__ B, Counters *c)
 // End of a round whose next round follows at once: one launch and one host
 // round trip for the boundary LCPs and the next round's classification.  The
 // finished round's counters are cleared for the round after the next.
-__global__ void k_round_end(SortArgs a, const uint2 *__restrict__ B, const Seg *__restrict__ N,
+__global__ void k_round_end(SortArgs a, const uint2 *B, const Seg *N,
                             Seg *W1, Seg *W8, SmallLists S, Seg *L, RoundCounters *rc, int i,
                             Publish pub) {
     after_predecessor();
