@@ -42,15 +42,15 @@ int ssort_ctx::reserve(uint32_t n) {
         SS_CUDA(cudaHostAlloc((void **)&hc, sizeof(HostCounters), cudaHostAllocDefault));
         std::memset(hc, 0, sizeof(HostCounters));
         published = true;
-        use_counters(0);
     }
     return SSORT_OK;
 }
 
-// Waits for the counters of the last kernel given a publish_next(), or copies
-// them.  The wait polls the flag that the kernel's last CTA sets in pinned
-// memory; the stream is queried now and then, so that a failed launch, a
-// fault or a stream that is being captured ends it with an error.
+// Reads the counters into `seen`: waits for those of the last kernel given a
+// publish_next(), or copies them.  The wait polls the flag that the kernel's
+// last CTA sets in pinned memory; the stream is queried now and then, so that
+// a failed launch, a fault or a stream that is being captured ends it with an
+// error.
 int ssort_ctx::read_counters() {
     if (published) {
         volatile uint32_t *flag = &hc->flag;
@@ -63,12 +63,12 @@ int ssort_ctx::read_counters() {
                 return fail(SSORT_EINTERNAL, "a kernel ended without its counters");
         }
         std::atomic_thread_fence(std::memory_order_acquire);
+        seen = hc->rc;
     } else {
-        SS_CUDA(cudaMemcpyAsync(&hc->rc, ws.rc, sizeof(RoundCounters), cudaMemcpyDeviceToHost,
-                                st));
+        SS_CUDA(cudaMemcpyAsync(&seen, ws.rc, sizeof(RoundCounters), cudaMemcpyDeviceToHost, st));
         SS_CUDA(cudaStreamSynchronize(st));
     }
-    if (hc->rc.c[0].error || hc->rc.c[1].error)
+    if (seen.c[0].error || seen.c[1].error)
         return fail(SSORT_EINTERNAL, "a scan's look-back waited past its bound");
     return SSORT_OK;
 }
@@ -300,6 +300,7 @@ int ssort_ctx::round_body(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt,
         SS_CUDA(cudaMemcpyAsync(&hc->rc, ws.rc, sizeof(RoundCounters), cudaMemcpyDeviceToHost,
                                 st));
         SS_CUDA(cudaStreamSynchronize(st));
+        seen = hc->rc;
         if (h_ctr->error)
             return fail(SSORT_EINTERNAL, "a scan's look-back waited past its bound");
     }
@@ -340,8 +341,10 @@ int ssort_ctx::run(const uint8_t *arena_p, uint64_t arena_bytes, const void *off
 // final index lands in d_perm (= idx[0]); every lcp entry is written exactly
 // once: inside an on-chip sort or an equality bucket for pairs in the same
 // leaf, by the boundary pass for pairs split by a partition, and lcp[0] = 0 up
-// front.  The host waits for the device twice per round (segment counts after
-// classification, and the next round's count) plus once per partition level.
+// front.  The host waits for the device once per partition level and once at
+// the end of each round, whose last kernel also counts the next round's
+// segments; before that once more in a batch and in a sort of at most SMALL_CAP
+// strings, whose first counts come from the device.
 // With an instance table (d_inst, ninst > 0) every instance starts as its own
 // round-0 segment and the result indices are made instance-local at the end.
 int ssort_ctx::run_ws(const uint8_t *arena_p, uint64_t arena_bytes, const void *offs_p,
@@ -390,14 +393,14 @@ int ssort_ctx::run_ws(const uint8_t *arena_p, uint64_t arena_bytes, const void *
                                ws.L, dev_ctr(), (int)((ninst + 255) / 256), st, ws.rc,
                                publish_next()));
         SS_TRY(read_counters());
-        n_cur = hc->rc.c[1].n_next;
+        n_cur = seen.c[1].n_next;
         SS_CUDA(cudaMemsetAsync(made, 0, sizeof(Counters), st));
     } else if (n <= (uint32_t)SMALL_CAP) {
         // One CTA sorts it all; what it leaves goes on below.
         LAUNCH(this, "tiny", launch_tiny(a, cur, nxt, ws.rc, publish_next(), st));
         if (n < 2) return SSORT_OK;
         SS_TRY(read_counters());
-        const RoundCounters &r = hc->rc;
+        const RoundCounters &r = seen;
         round_no = r.tiny_rounds;
         std::copy(r.tiny_live, r.tiny_live + round_no, stats.live);
         stats.small_segments = r.tiny_segments;
@@ -1387,7 +1390,6 @@ struct NoallocDevice {
     bool ready = false;
     unsigned char *scratch = nullptr;  // device address of g_noalloc_scratch
     int num_sms = 0;
-    HostCounters host_ctr{};           // plain host copy of the round counters
 };
 
 std::mutex g_noalloc_mu;
@@ -1426,8 +1428,6 @@ extern "C" int ssort_sort_device_noalloc(const uint8_t *d_arena, uint64_t arena_
     c.device = dev;
     c.num_sms = d.num_sms;
     c.st = (cudaStream_t)stream;
-    c.hc = &d.host_ctr;
-    c.use_counters(0);
     c.graph_mode = 0;  // the host-driven loop: building a graph would allocate
     c.ws = ws_bind(ws_layout(NOALLOC_MAX_N), d.scratch);
     c.ws_n = NOALLOC_MAX_N;
@@ -1436,7 +1436,6 @@ extern "C" int ssort_sort_device_noalloc(const uint8_t *d_arena, uint64_t arena_
     // before an error still use the shared scratch, and the next call (which
     // may start as soon as the lock is released) must not race with them.
     const cudaError_t se = cudaStreamSynchronize(c.st);
-    c.hc = nullptr;
     if (rc == SSORT_OK && se != cudaSuccess) return cuda_fail(se, "cudaStreamSynchronize");
     return rc;
 }

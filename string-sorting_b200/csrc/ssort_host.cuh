@@ -74,11 +74,14 @@ struct ssort_ctx {
     ssort::HBuf h_stage[2];
     cudaEvent_t ev_stage[2] = {nullptr, nullptr};
     int copy_pageable(void *d_dst, const void *h_src, uint64_t bytes);
-    // Host copy of the device counters.  A context's lies in pinned memory,
-    // where the counting kernels publish it (`published`); elsewhere it is
-    // copied.  ctr_i: which of the two counter sets the current round uses.
+    // The device counters as last read (read_counters), in memory of the host's
+    // own: a kernel may already be publishing newer ones while the host works
+    // with these.  hc: the pinned page where the counting kernels publish them
+    // (`published`); without it they are copied.  ctr_i: which of the two
+    // counter sets the current round uses.
     ssort::HostCounters *hc = nullptr;
-    ssort::Counters *h_ctr = nullptr;  // hc->rc.c[ctr_i]
+    ssort::RoundCounters seen{};
+    ssort::Counters *h_ctr = seen.c;  // seen.c + ctr_i
     bool published = false;
     uint32_t pub_seq = 0;
     int ctr_i = 0;
@@ -208,7 +211,7 @@ struct ssort_ctx {
     ssort::Counters *dev_ctr() const { return ws.rc->c + ctr_i; }
     void use_counters(int i) {
         ctr_i = i;
-        h_ctr = hc->rc.c + i;
+        h_ctr = seen.c + i;
     }
     // For the next kernel that publishes the counters; read_counters waits
     // for the last one launched.
