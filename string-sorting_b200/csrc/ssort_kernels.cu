@@ -399,10 +399,27 @@ __global__ void k_init_batch(const uint32_t *__restrict__ inst_start, uint32_t n
 
 // The three kernels below give every position the instance or request it lies
 // in.  A warp takes SPAN_ITEMS * 32 consecutive positions: one search for the
-// first, then every lane only steps over range ends it passes (a search per
+// first, then every lane only passes on to a later range (a search per
 // position took 0.37 ms over 69 M positions in 353 instances; reading and
 // writing them takes 0.09).
 constexpr uint32_t SPAN_ITEMS = 8;
+
+// Largest j in [i, n) with first[j] <= p (first ascending, first[i] <= p): in
+// doubling steps, then back in halving ones.  As many reads as one step at a
+// time takes to pass a few ranges, and few where many empty ones follow each
+// other, of which a batch may hold any number (100,000 in a row: one step at a
+// time the batch took 5.9 ms, now 0.27, as without them).
+__device__ __forceinline__ uint32_t pass_on(const uint32_t *first, uint32_t n, uint32_t i,
+                                            uint32_t p) {
+    uint64_t d = 1;
+    while (d < n - i && first[i + d] <= p) {
+        i += (uint32_t)d;
+        d *= 2;
+    }
+    while (d /= 2)
+        if (d < n - i && first[i + d] <= p) i += (uint32_t)d;
+    return i;
+}
 
 // Global positions -> indices within each position's instance.
 __global__ void k_localize(uint32_t *perm, uint32_t n, const uint32_t *__restrict__ inst_start,
@@ -424,9 +441,9 @@ __global__ void k_localize(uint32_t *perm, uint32_t n, const uint32_t *__restric
         for (uint32_t k = 0; k < SPAN_ITEMS; ++k) {
             const uint64_t p = p0 + k * 32 + lane;
             if (p < n) {
-                while (p >= end && i + 1 < ninst) {
-                    ++i;
-                    start = end;
+                if (p >= end) {
+                    i = pass_on(inst_start, ninst, i, (uint32_t)p);
+                    start = __ldg(inst_start + i);
                     end = __ldg(inst_start + i + 1);
                 }
                 perm[p] = v[k] - start;
