@@ -2238,7 +2238,7 @@ __device__ __forceinline__ uint32_t warp1_deepen(const uint8_t *__restrict__ are
 // warp-collective.
 template <int W>
 __device__ __forceinline__ uint32_t warp1_group(const SortArgs &a, const Seg &s, uint32_t lane,
-                                                Seg *N, Counters *c) {
+                                                uint32_t steps, Seg *N, Counters *c) {
     const uint32_t li = lane & (W - 1), base = lane & ~(uint32_t)(W - 1);
     const bool v = li < s.len;
     uint32_t id = IDX_MAX;
@@ -2331,9 +2331,9 @@ __device__ __forceinline__ uint32_t warp1_group(const SortArgs &a, const Seg &s,
     bool run = v && !key_is_end(k) && (!head || eq_next);
     const uint32_t m = lane == 31 ? 0xffffffffu : ((2u << lane) - 1u);
     uint32_t h = run ? 31 - __clz(heads & m) : lane;
-    if (a.warp1_deep && __any_sync(0xffffffffu, run))
+    if (steps && __any_sync(0xffffffffu, run))
         return warp1_deepen<W>(a.arena, a.arena_bytes, a.offs, a.off_width, a.idx[0], a.lcp,
-                               a.warp1_deep, s.start, s.depth + KEY_BYTES, lane, id, run, h, N,
+                               steps, s.start, s.depth + KEY_BYTES, lane, id, run, h, N,
                                c);
     const bool tail = run && !eq_next;  // a run's last lane
     emit_next_warp(N, c, tail, s.start + (h - base), lane - h + 1, s.depth + KEY_BYTES);
@@ -2344,7 +2344,7 @@ __device__ __forceinline__ uint32_t warp1_group(const SortArgs &a, const Seg &s,
 // consecutive list entries and sorts those of at most 8 strings together, one
 // per 8-lane group, so that their loads overlap.  Second pass: one warp per
 // remaining segment.
-constexpr uint32_t W1_PACK = 4;
+constexpr uint32_t W1_PACK = 4, W1_SMALL = 8;
 
 __global__ void __launch_bounds__(WARP_THREADS) k_warp1(SortArgs a, const Seg *T0,
                                                         Span sp, Seg *N, Counters *c) {
@@ -2359,7 +2359,7 @@ __global__ void __launch_bounds__(WARP_THREADS) k_warp1(SortArgs a, const Seg *T
     for (uint32_t g0 = warp0 * W1_PACK; g0 < nT; g0 += nwarps * W1_PACK) {
         const uint32_t j = lane >> 3;
         const Seg sj = g0 + j < nT ? T[g0 + j] : Seg{0, 0, 0, 0};
-        const bool small = sj.len <= 8;
+        const bool small = sj.len <= W1_SMALL;
         if ((lane & 7) == 0) {
             if (sj.flags & SEG_KEYS)
                 keyed += sj.len;
@@ -2367,11 +2367,11 @@ __global__ void __launch_bounds__(WARP_THREADS) k_warp1(SortArgs a, const Seg *T
                 fresh += sj.len;
         }
         if (__any_sync(0xffffffffu, small && sj.len > 0))
-            deep += warp1_group<8>(a, small ? sj : Seg{0, 0, 0, 0}, lane, N, c);
+            deep += warp1_group<8>(a, small ? sj : Seg{0, 0, 0, 0}, lane, a.warp1_deep, N, c);
     }
     for (uint32_t g = warp0; g < nT; g += nwarps) {
         const Seg s = T[g];
-        if (s.len > 8) deep += warp1_group<32>(a, s, lane, N, c);
+        if (s.len > W1_SMALL) deep += warp1_group<32>(a, s, lane, a.warp1_deep, N, c);
     }
     if ((lane & 7) == 0 && (fresh | keyed)) {  // each 8-lane group's leader
         atomicAdd(&c->warp1_fresh, fresh);
@@ -2998,17 +2998,27 @@ __global__ void k_round_end(SortArgs a, const uint2 *B, const Seg *N,
 // refining the runs of equal keys round by round, with the code of the
 // on-chip sorts (the whole CTA on segments of more than 256 strings, a warp on
 // each smaller one).  What the rounds of the general loop cost such a sort is
-// launches and host round trips: 500 words took 134 us.  A round with more
-// segments than TINY_SEGMENTS (which the general loop spreads over the chip),
-// or the TINY_ROUNDS-th, is left to the general loop.
+// launches and host round trips: 500 words took 134 us, now 39.  A round with
+// more segments than TINY_SEGMENTS (which the general loop spreads over the
+// chip), or the TINY_ROUNDS-th, is left to the general loop.
+// So are many runs that stay equal for long: in-warp refinement takes about
+// 4 us per 16 bytes and run, and this CTA's eight warps take the runs in turn.
+// A round whose runs of at most 32 strings are more than the warps gets
+// TINY_STEPS steps in all, and where the next one is as crowded that is left to
+// the general loop: by then this CTA has spent about what a round of that loop
+// costs.  16 strings in each of 128 groups, sharing 1000, 100, 40 bytes: 1047,
+// 189, 127 us; the general loop from the start 1074, 223, 164; without a limit
+// 3784, 378, 139.  With TINY_STEPS 128: 1105, 236, 138; leaving every crowded
+// round at once: 1030, 170, 110, but 500 URLs 89 us instead of 57.
 constexpr uint32_t TINY_SEGMENTS = 128;
+constexpr uint32_t TINY_STEPS = 64;
 constexpr size_t TINY_SMEM =
     seg_bytes(SMALL_THREADS) > WARPSORT_SMEM ? seg_bytes(SMALL_THREADS) : WARPSORT_SMEM;
 
 __global__ void __launch_bounds__(SMALL_THREADS, 1)
     k_tiny(SortArgs a, Seg *A, Seg *B, RoundCounters *rc, Publish pub) {
     extern __shared__ __align__(16) unsigned char seg_smem[];
-    __shared__ unsigned long long live;
+    __shared__ unsigned long long sums;
     const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
     Counters *c = rc->c;
     {
@@ -3022,16 +3032,29 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1)
     }
     __syncthreads();
     uint32_t n_cur = 1, round = 0, segments = 0;
+    bool crowded = false;
     for (; round < TINY_ROUNDS && n_cur && n_cur <= TINY_SEGMENTS; ++round) {
         if (t == 0) {
-            live = 0;
+            sums = 0;
             c->n_next = 0;
         }
         __syncthreads();
         const Seg own = t < n_cur ? A[t] : Seg{0, 0, 0, 0};
-        const unsigned long long sum = warp_sum(own.len);
-        if (lane == 0 && sum) atomicAdd(&live, sum);
-        if (__syncthreads_or(own.len > (uint32_t)WARP8_CAP)) {
+        // live strings, segments of 9..32 strings, segments of up to 8
+        const bool few = own.len && own.len <= W1_SMALL;
+        const bool one = own.len > W1_SMALL && own.len <= (uint32_t)WARP1_CAP;
+        const unsigned long long sum =
+            warp_sum(own.len | (unsigned long long)one << 32 | (unsigned long long)few << 48);
+        if (lane == 0 && sum) atomicAdd(&sums, sum);
+        const bool any_large = __syncthreads_or(own.len > (uint32_t)WARP8_CAP);
+        const uint32_t live = (uint32_t)sums, n_few = (uint32_t)(sums >> 48);
+        const uint32_t tasks =
+            ((uint32_t)(sums >> 32) & 0xFFFFu) + (n_few + W1_PACK - 1) / W1_PACK;
+        const bool again = crowded;
+        crowded = tasks > SMALL_THREADS / 32;
+        if (crowded && again) break;
+        const uint32_t steps = crowded ? min(a.warp1_deep, TINY_STEPS / tasks) : a.warp1_deep;
+        if (any_large) {
             for (uint32_t g = 0; g < n_cur; ++g) {
                 const Seg s = A[g];
                 if (s.len <= (uint32_t)WARP8_CAP) continue;
@@ -3044,13 +3067,22 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1)
             }
             __syncthreads();
         }
-        unsigned long long deep = 0;
+        unsigned long long deep = 0, fresh = 0;
+        // As in k_warp1: up to W1_PACK segments of at most 8 strings together.
+        for (uint32_t g0 = w * W1_PACK; n_few && g0 < n_cur;
+             g0 += SMALL_THREADS / 32 * W1_PACK) {
+            const uint32_t j = lane >> 3;
+            Seg s = g0 + j < n_cur ? A[g0 + j] : Seg{0, 0, 0, 0};
+            if (s.len > W1_SMALL) s.len = 0;
+            if ((lane & 7) == 0) fresh += s.len;
+            if (__any_sync(0xffffffffu, s.len > 0)) deep += warp1_group<8>(a, s, lane, steps, B, c);
+        }
         for (uint32_t g = w; g < n_cur; g += SMALL_THREADS / 32) {
             const Seg s = A[g];
-            if (s.len > (uint32_t)WARP8_CAP) continue;
+            if (s.len <= W1_SMALL || s.len > (uint32_t)WARP8_CAP) continue;
             if (s.len <= (uint32_t)WARP1_CAP) {
-                deep += warp1_group<32>(a, s, lane, B, c);
-                if (lane == 0) atomicAdd(&c->warp1_fresh, (unsigned long long)s.len);
+                deep += warp1_group<32>(a, s, lane, steps, B, c);
+                if (lane == 0) fresh += s.len;
             } else {
                 const bool full = sort_segment(WarpGroup{lane}, a, s,
                                                seg_mem(seg_smem + w * seg_bytes(32), 32), B, c);
@@ -3060,10 +3092,11 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1)
                 }
             }
         }
+        if (fresh) atomicAdd(&c->warp1_fresh, fresh);
         deep = warp_sum(deep);
         if (lane == 0 && deep) atomicAdd(&c->warp1_deep, deep);
         __syncthreads();
-        if (t == 0) rc->tiny_live[round] = (uint32_t)live;
+        if (t == 0) rc->tiny_live[round] = live;
         segments += n_cur;
         n_cur = atomicAdd(&c->n_next, 0u);
         Seg *x = A;
