@@ -97,7 +97,10 @@ struct Request {
     uint64_t region = 0, region_size = 0;
     uint64_t pos = 0;
     cudaEvent_t ev = nullptr;  // copy-in done, then copy-out done
-    bool dev_in = false, dev_out = false;  // inputs / outputs in this device's memory
+    // Inputs / outputs in this device's memory: found out at admission, where the
+    // server's device is current (submit makes no CUDA call, which might bring up
+    // a context on another device).
+    bool dev_in = false, dev_out = false;
 };
 
 // Whether p lies in device memory of `device` (null counts as there).
@@ -263,6 +266,8 @@ int ssort_server::admit() {
         uint8_t *dst = (uint8_t *)pool.p + region;
         void *odst = r->off_width == 8 ? (void *)((uint64_t *)goffs.p + pos)
                                        : (void *)(ctx->ws.lcp + pos);
+        r->dev_in = on_device(r->arena, ctx->device) && on_device(r->offs, ctx->device);
+        r->dev_out = on_device(r->perm_out, ctx->device) && on_device(r->lcp_out, ctx->device);
         if (r->dev_in) {
             SS_TRY(in.add(dst, r->arena, r->arena_bytes, rsz - r->arena_bytes, h2d));
             SS_TRY(in.add(odst, r->offs, (uint64_t)r->n * r->off_width, 0, h2d));
@@ -571,8 +576,6 @@ int ssort_server_submit(ssort_server *srv, const uint8_t *arena, uint64_t arena_
     r->n = (uint32_t)n;
     r->perm_out = perm_out;
     r->lcp_out = lcp_out;
-    r->dev_in = n && on_device(arena, srv->ctx->device) && on_device(offs, srv->ctx->device);
-    r->dev_out = n && on_device(perm_out, srv->ctx->device) && on_device(lcp_out, srv->ctx->device);
     *id_out = r->id;
     if (n == 0) {
         srv->done_ids.push_back(r->id);

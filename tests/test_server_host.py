@@ -1,0 +1,129 @@
+"""The request server's host side, without a GPU: its source is compiled into a
+small program in which the CUDA calls it makes are recorded."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "string-sorting_b200")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+PRELUDE = r"""
+#include <cuda_runtime.h>
+#include <cstdint>
+#include <cstdio>
+#include <string>
+#include <vector>
+
+static std::vector<std::string> calls;  // what the server asked of the device
+static int failed = 0;
+#define CHECK(x) \
+    if (!(x)) std::printf("line %d: %s\n", __LINE__, #x), failed = 1
+
+// Pointers below 1 << 20 stand for memory of device 0.
+static bool is_device(const void *p) { return (uintptr_t)p < (1 << 20); }
+static cudaError_t fake_attributes(cudaPointerAttributes *at, const void *p) {
+    calls.push_back("attributes");
+    *at = cudaPointerAttributes{};
+    at->type = is_device(p) ? cudaMemoryTypeDevice : cudaMemoryTypeHost;
+    return cudaSuccess;
+}
+static cudaError_t fake_copy(void *, const void *, size_t n, cudaMemcpyKind, cudaStream_t) {
+    calls.push_back("copy " + std::to_string(n));
+    return cudaSuccess;
+}
+static cudaError_t fake_set(void *, int, size_t n, cudaStream_t) {
+    calls.push_back("set " + std::to_string(n));
+    return cudaSuccess;
+}
+static cudaError_t fake_record(cudaEvent_t e, cudaStream_t) {
+    calls.push_back("record " + std::to_string((uintptr_t)e));
+    return cudaSuccess;
+}
+static cudaError_t fake_create(cudaEvent_t *e, unsigned) {
+    static uintptr_t made = 0;
+    *e = (cudaEvent_t)++made;
+    return cudaSuccess;
+}
+static cudaError_t fake_sync(cudaEvent_t) { return cudaSuccess; }
+static cudaError_t fake_last() { return cudaSuccess; }
+#define cudaPointerGetAttributes fake_attributes
+#define cudaMemcpyAsync fake_copy
+#define cudaMemsetAsync fake_set
+#define cudaEventRecord fake_record
+#define cudaEventCreateWithFlags fake_create
+#define cudaEventSynchronize fake_sync
+#define cudaGetLastError fake_last
+#include "ssort_server.cu"
+
+namespace ssort {
+void launch_copies(const CopyJob *, uint32_t njobs, uint32_t, cudaStream_t) {
+    calls.push_back("copies " + std::to_string(njobs));
+}
+}  // namespace ssort
+
+template <class T = uint8_t>
+static T *at(uintptr_t p) { return (T *)p; }
+
+// A server of 1 MB and `strings` positions that has seen no device.
+struct Made {
+    ssort_ctx ctx;
+    ssort_server srv;
+    std::vector<CopyJob> jobs[2];
+    explicit Made(uint32_t strings = 100000) {
+        srv.ctx = &ctx;
+        srv.budget = 1 << 20;
+        srv.max_strings = strings;
+        srv.arena_alloc.init(srv.budget);
+        srv.pos_alloc.init(strings);
+        ctx.num_sms = 148;
+        for (int k = 0; k < 2; ++k) {
+            jobs[k].resize(CopyBatch::CAP);
+            (k ? srv.out : srv.in).h = jobs[k].data();
+        }
+    }
+    uint64_t submit(const uint8_t *arena, uint64_t bytes, const void *offs, uint64_t n,
+                    uint32_t *perm, uint32_t *lcp = nullptr) {
+        uint64_t id = 0;
+        CHECK(ssort_server_submit(&srv, arena, bytes, offs, 8, n, perm, lcp, &id) == SSORT_OK);
+        return id;
+    }
+};
+static std::string joined() {
+    std::string s;
+    for (auto &c : calls) s += c + ", ";
+    return s;
+}
+"""
+
+
+def run(tmp_path, body):
+    if not os.path.exists(os.path.join(CUDA, "lib64", "libcudart_static.a")):
+        pytest.skip("no CUDA toolkit")
+    src = tmp_path / "server.cpp"
+    src.write_text(PRELUDE + "int main() {\n" + body + "\n    return failed;\n}\n")
+    exe = tmp_path / "server"
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-w", "-I", os.path.join(CUDA, "include"),
+                    "-I", os.path.join(ROOT, "include"), "-I", os.path.join(PKG, "csrc"),
+                    str(src), "-o", str(exe), os.path.join(PKG, "libssort_b200.so"),
+                    "-Wl,-rpath," + PKG, "-L", os.path.join(CUDA, "lib64"), "-lcudart_static",
+                    "-ldl", "-lrt", "-lpthread"], check=True)
+    r = subprocess.run([str(exe)], stdout=subprocess.PIPE, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout
+
+
+def test_submit_asks_nothing_of_the_device(tmp_path):
+    """A submit from a thread that has made no CUDA call must not bring up a
+    context on whichever device is current there: where the buffers lie is found
+    out when the request is admitted, on the server's device."""
+    run(tmp_path, r"""
+    Made m;
+    m.submit(at(0x1000), 100, at(0x2000), 5, at<uint32_t>(0x3000), at<uint32_t>(0x4000));
+    m.submit(at(1ull << 40), 100, at(2ull << 40), 5, at<uint32_t>(3ull << 40));
+    CHECK(calls.empty());
+    CHECK(m.srv.admit() == SSORT_OK);
+    CHECK(m.srv.loading.size() == 2);
+    CHECK(m.srv.loading[0]->dev_in && m.srv.loading[0]->dev_out);
+    CHECK(!m.srv.loading[1]->dev_in && !m.srv.loading[1]->dev_out);
+    """)
