@@ -22,6 +22,8 @@
 // on what it shared the rounds with.
 #include "ssort_host.cuh"
 
+#include <cudaTypedefs.h>
+
 #include <deque>
 #include <mutex>
 #include <unordered_map>
@@ -103,15 +105,39 @@ struct Request {
     bool dev_in = false, dev_out = false;
 };
 
-// Whether p lies in device memory of `device` (null counts as there).
-bool on_device(const void *p, int device) {
+// The driver's record of the allocation that holds an address (null if this
+// driver has none).
+PFN_cuMemGetAddressRange_v3020 address_range() {
+    static const auto range = []() -> PFN_cuMemGetAddressRange_v3020 {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 3020, cudaEnableDefault,
+                                             &q) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return q == cudaDriverEntryPointSuccess ? (PFN_cuMemGetAddressRange_v3020)f : nullptr;
+    }();
+    return range;
+}
+
+// Whether the `bytes` bytes at p lie in device memory of `device` and inside
+// one allocation there, so that a kernel may copy them (null counts as there).
+// Any other copy goes through cudaMemcpyAsync, which refuses a range that
+// leaves its allocation.
+bool on_device(const void *p, uint64_t bytes, int device) {
     if (!p) return true;
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return at.type == cudaMemoryTypeDevice && at.device == device;
+    if (at.type != cudaMemoryTypeDevice || at.device != device) return false;
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const auto range = address_range();
+    return range && range(&base, &size, (CUdeviceptr)p) == CUDA_SUCCESS &&
+           bytes <= base + size - (CUdeviceptr)p;
 }
 
 // Copies between device buffers, gathered and run as one launch: a pinned
@@ -266,8 +292,10 @@ int ssort_server::admit() {
         uint8_t *dst = (uint8_t *)pool.p + region;
         void *odst = r->off_width == 8 ? (void *)((uint64_t *)goffs.p + pos)
                                        : (void *)(ctx->ws.lcp + pos);
-        r->dev_in = on_device(r->arena, ctx->device) && on_device(r->offs, ctx->device);
-        r->dev_out = on_device(r->perm_out, ctx->device) && on_device(r->lcp_out, ctx->device);
+        r->dev_in = on_device(r->arena, r->arena_bytes, ctx->device) &&
+                    on_device(r->offs, (uint64_t)r->n * r->off_width, ctx->device);
+        r->dev_out = on_device(r->perm_out, (uint64_t)r->n * 4, ctx->device) &&
+                     on_device(r->lcp_out, (uint64_t)r->n * 4, ctx->device);
         if (r->dev_in) {
             SS_TRY(in.add(dst, r->arena, r->arena_bytes, rsz - r->arena_bytes, h2d));
             SS_TRY(in.add(odst, r->offs, (uint64_t)r->n * r->off_width, 0, h2d));

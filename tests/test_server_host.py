@@ -10,6 +10,7 @@ PKG = os.path.join(ROOT, "string-sorting_b200")
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 
 PRELUDE = r"""
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstdio>
@@ -48,6 +49,20 @@ static cudaError_t fake_create(cudaEvent_t *e, unsigned) {
 }
 static cudaError_t fake_sync(cudaEvent_t) { return cudaSuccess; }
 static cudaError_t fake_last() { return cudaSuccess; }
+// Their allocations: 100 bytes at every multiple of 4096.
+static CUresult fake_range(CUdeviceptr *base, size_t *size, CUdeviceptr p) {
+    *base = p & ~4095ull;
+    *size = 100;
+    return p - *base < 100 ? CUDA_SUCCESS : CUDA_ERROR_NOT_FOUND;
+}
+static cudaError_t fake_entry(const char *name, void **f, unsigned, unsigned long long,
+                              cudaDriverEntryPointQueryResult *q) {
+    CHECK(std::string(name) == "cuMemGetAddressRange");
+    *f = (void *)fake_range;
+    *q = cudaDriverEntryPointSuccess;
+    return cudaSuccess;
+}
+#define cudaGetDriverEntryPointByVersion fake_entry
 #define cudaPointerGetAttributes fake_attributes
 #define cudaMemcpyAsync fake_copy
 #define cudaMemsetAsync fake_set
@@ -126,4 +141,44 @@ def test_submit_asks_nothing_of_the_device(tmp_path):
     CHECK(m.srv.loading.size() == 2);
     CHECK(m.srv.loading[0]->dev_in && m.srv.loading[0]->dev_out);
     CHECK(!m.srv.loading[1]->dev_in && !m.srv.loading[1]->dev_out);
+    """)
+
+
+def test_copies_beyond_an_allocation_go_through_the_driver(tmp_path):
+    """cudaMemcpyAsync refuses a range that leaves its allocation; a kernel that
+    copies does not.  Only buffers that lie inside their allocations in full are
+    copied by the server's kernel, inputs and outputs apart."""
+    run(tmp_path, r"""
+    // allocations of 100 bytes at every multiple of 4096
+    {
+        Made m;
+        // n = 10: 80 bytes of offsets, 40 of results
+        m.submit(at(0x1000), 100, at(0x2000 + 20), 10, at<uint32_t>(0x3000 + 60),
+                 at<uint32_t>(0x4000));
+        CHECK(m.srv.admit() == SSORT_OK);
+        CHECK(m.srv.loading[0]->dev_in && m.srv.loading[0]->dev_out);
+        CHECK(joined().find("copies 2") != std::string::npos);
+    }
+    struct { uintptr_t arena, bytes, offs, perm, lcp; bool in, out; } bad[] = {
+        {0x1000, 101, 0x2000, 0x3000, 0x4000, false, true},
+        {0x1000 + 1, 100, 0x2000, 0x3000, 0x4000, false, true},
+        {0x1000, 100, 0x2000 + 21, 0x3000, 0x4000, false, true},
+        {0x1000, 100, 0x2000, 0x3000 + 61, 0x4000, true, false},
+        {0x1000, 100, 0x2000, 0x3000, 0x4000 + 61, true, false},
+        {0x1000, ~0ull >> 45, 0x2000, 0x3000, 0x4000, false, true},
+        {0x1000 + 200, 1, 0x2000, 0x3000, 0x4000, false, true},  // in none
+    };
+    for (auto &b : bad) {
+        calls.clear();
+        Made m;
+        m.submit(at(b.arena), b.bytes, at(b.offs), 10, at<uint32_t>(b.perm),
+                 at<uint32_t>(b.lcp));
+        CHECK(m.srv.admit() == SSORT_OK);
+        CHECK(m.srv.loading[0]->dev_in == b.in);
+        CHECK(m.srv.loading[0]->dev_out == b.out);
+        const bool plain = joined().find("copy " + std::to_string(b.bytes) + ",") !=
+                           std::string::npos;
+        CHECK(plain == !b.in);
+        CHECK((joined().find("copies 2") != std::string::npos) == b.in);
+    }
     """)
