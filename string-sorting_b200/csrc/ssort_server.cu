@@ -270,9 +270,19 @@ struct ssort_server {
 };
 
 // FIFO admission: the head of the queue is admitted when its pool region and
-// position range fit; later requests wait behind it.
+// position range fit; later requests wait behind it.  A host request's event
+// follows its own copies, and those of the device requests before it are on
+// their way by then: while a round is in progress a request joins as soon as
+// its own copies have landed.  Device requests next to each other share a
+// launch and its completion.
 int ssort_server::admit() {
-    const size_t before = loading.size();
+    size_t gathered = loading.size();  // from here on, requests whose copies wait in `in`
+    auto flush = [&]() -> int {
+        SS_TRY(in.run(h2d));
+        for (; gathered < loading.size(); ++gathered)
+            SS_CUDA(cudaEventRecord(loading[gathered]->ev, h2d));
+        return SSORT_OK;
+    };
     while (!queue.empty()) {
         Request *r = queue.front();
         if (loading.size() + active.size() + draining.size() >= MAX_SLOTS) break;
@@ -300,6 +310,7 @@ int ssort_server::admit() {
             SS_TRY(in.add(dst, r->arena, r->arena_bytes, rsz - r->arena_bytes, h2d));
             SS_TRY(in.add(odst, r->offs, (uint64_t)r->n * r->off_width, 0, h2d));
         } else {
+            SS_TRY(flush());
             if (r->arena_bytes)
                 SS_CUDA(cudaMemcpyAsync(dst, r->arena, r->arena_bytes, cudaMemcpyDefault, h2d));
             SS_CUDA(cudaMemsetAsync(dst + r->arena_bytes, 0, rsz - r->arena_bytes, h2d));
@@ -308,11 +319,9 @@ int ssort_server::admit() {
         }
         r->state = SSORT_REQ_LOADING;
         loading.push_back(r);
+        if (!r->dev_in) SS_TRY(flush());
     }
-    SS_TRY(in.run(h2d));
-    for (size_t k = before; k < loading.size(); ++k)
-        SS_CUDA(cudaEventRecord(loading[k]->ev, h2d));
-    return SSORT_OK;
+    return flush();
 }
 
 // Waits until the previous host-to-device copy out of a job table has run,

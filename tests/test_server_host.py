@@ -182,3 +182,34 @@ def test_copies_beyond_an_allocation_go_through_the_driver(tmp_path):
         CHECK((joined().find("copies 2") != std::string::npos) == b.in);
     }
     """)
+
+
+def test_a_host_request_waits_for_its_own_copies_only(tmp_path):
+    """Requests admitted in one step: a host request's event follows its own
+    copies and comes before the next one's; device requests next to each other
+    share a launch, whose events come before the copies of a later host request."""
+    run(tmp_path, r"""
+    const uintptr_t H = 1ull << 40;
+    Made m;
+    // host, host, device, device, host, device; n = 1, 2, .. marks the offsets' copies
+    for (int i = 1; i <= 6; ++i) {
+        const bool dev = i == 3 || i == 4 || i == 6;
+        const uintptr_t base = dev ? 0 : H;
+        m.submit(at(base + 0x1000 * i), 10 * i, at(base + 0x10000), i,
+                 at<uint32_t>(base + 0x20000));
+    }
+    CHECK(m.srv.admit() == SSORT_OK);
+    CHECK(m.srv.loading.size() == 6);
+    std::vector<std::string> seen;  // without the queries and the table's own copy and event
+    for (auto &c : calls)
+        if (c != "attributes" && c != "record 0" && c.compare(0, 3, "set") &&
+            c != "copy " + std::to_string(4 * sizeof(CopyJob)) &&
+            c != "copy " + std::to_string(2 * sizeof(CopyJob)))
+            seen.push_back(c);
+    const std::vector<std::string> want = {
+        "copy 10", "copy 8", "record 1", "copy 20", "copy 16", "record 2",
+        "copies 4", "record 3", "record 4",
+        "copy 50", "copy 40", "record 5", "copies 2", "record 6"};
+    CHECK(seen == want);
+    if (seen != want) for (auto &c : seen) std::printf("%s, ", c.c_str());
+    """)
