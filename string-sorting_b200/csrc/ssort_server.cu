@@ -231,13 +231,20 @@ struct ssort_server {
         if (e) spare_events.push_back(e);
     }
 
+    // Arguments of a round over the active requests.  The rules by size (tiles,
+    // leaves, samples per splitter) go by the strings these hold, as in a sort
+    // of as many, not by what the server could hold: in a server of 16 M
+    // positions one request of 5 k, 20 k, 1 M strings takes 154, 167, 307 us; by
+    // the latter it took 168, 180, 314.
     SortArgs args() const {
+        uint32_t held = 0;
+        for (const Request *r : active) held += r->n;
         SortArgs a{};
         a.arena = (const uint8_t *)pool.p;
         a.arena_bytes = budget;
         a.offs = goffs.p;
         a.off_width = 8;
-        a.n = max_strings;
+        a.n = held;
         a.idx[0] = (uint32_t *)perm.p;
         a.idx[1] = ctx->ws.idx1;
         a.key[0] = ctx->ws.key0;
@@ -246,8 +253,8 @@ struct ssort_server {
         a.bkt = ctx->ws.bkt;
         a.target_bucket = ctx->target_bucket;
         a.warp8_cap = ctx->warp8_cap;
-        a.tile = part_tile(max_strings);
-        a.leaf_cap = max_strings >= LEAF_MIN_N ? LEAF_CAP : SMALL_CAP;
+        a.tile = part_tile(held);
+        a.leaf_cap = held >= LEAF_MIN_N ? LEAF_CAP : SMALL_CAP;
         a.warp1_deep = ctx->warp1_deep;
         a.l2_prefetch = ctx->l2_prefetch ? 1u : 0u;
         a.max_splitters = (1u << (ctx->digit_bits - 1)) - 1;

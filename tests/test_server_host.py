@@ -213,3 +213,33 @@ def test_a_host_request_waits_for_its_own_copies_only(tmp_path):
     CHECK(seen == want);
     if (seen != want) for (auto &c : seen) std::printf("%s, ", c.c_str());
     """)
+
+
+def test_rules_by_size_go_by_the_requests_held(tmp_path):
+    """A round's tile and leaf sizes and samples per splitter are those of a sort
+    of as many strings as the active requests hold, whatever the server could
+    hold; the count matrix, sized for the latter, has room for them."""
+    run(tmp_path, r"""
+    const uint32_t CAPS[] = {50000, 300000, 1u << 20, 16u << 20, 100u << 20};
+    const uint32_t SIZES[] = {2049, 75776, 75777, 300000, 606208, 606209, 1u << 20,
+                              LEAF_MIN_N - 1, LEAF_MIN_N, 16u << 20, 100u << 20};
+    for (uint32_t cap : CAPS) {
+        Made m(cap);
+        const WsLayout lay = ws_layout(cap);
+        for (uint32_t n : SIZES) {
+            if (n > cap) continue;
+            Request a, b;
+            a.n = n / 3;
+            b.n = n - n / 3;
+            m.srv.active = {&a, &b};
+            const SortArgs s = m.srv.args();
+            CHECK(s.n == n);
+            CHECK(s.tile == part_tile(n));
+            CHECK(s.leaf_cap == (n >= LEAF_MIN_N ? LEAF_CAP : SMALL_CAP));
+            // tiles: one more for the remainder of each large segment
+            const uint64_t tiles = n / s.tile + n / (SMALL_CAP + 1) + 1;
+            CHECK(tiles * NB_MAX < lay.cm_cap);
+        }
+        m.srv.active.clear();
+    }
+    """)
