@@ -1240,20 +1240,23 @@ int ssort_autotune(ssort_ctx *ctx, const uint8_t *d_arena, uint64_t arena_bytes,
             struct Knob {
                 int param;
                 std::vector<int64_t> values;
+                bool decides = true;
             };
             // Coordinate descent over: range-bucket size, digit width of a
             // partition pass (splitters per pass), the small-segment cutoff,
             // the gather and overlap choices, the partition's L2 prefetch and
-            // the device-driven loop.  (The two parameters without effect
-            // keep their trials, so that a call times as many sorts as ever.)
+            // the device-driven loop.  The two parameters without effect
+            // keep their trials, so that a call times as many sorts as ever,
+            // but these decide nothing: a lucky time there would be one that
+            // the parameters after it had to beat.
             const Knob knobs[] = {{SSORT_PARAM_TARGET_BUCKET, {256, 512, 1024}},
                                   {SSORT_PARAM_DIGIT_BITS, {10, 9, 8}},
                                   {SSORT_PARAM_WARP8_CAP, {64, 128, 256}},
                                   {SSORT_PARAM_FUSED_GATHER, {1, 0}},
                                   {SSORT_PARAM_OVERLAP, {1, 0}},
-                                  {SSORT_PARAM_BLOCK_PREFETCH, {1, 0}},
+                                  {SSORT_PARAM_BLOCK_PREFETCH, {1, 0}, false},
                                   {SSORT_PARAM_L2_PREFETCH, {1, 0}},
-                                  {SSORT_PARAM_BLOCK_LEAN, {0, 1, 2}},
+                                  {SSORT_PARAM_BLOCK_LEAN, {0, 1, 2}, false},
                                   {SSORT_PARAM_GRAPH, {0, 1}}};
             auto get = [&](int p) -> int64_t {
                 switch (p) {
@@ -1276,7 +1279,7 @@ int ssort_autotune(ssort_ctx *ctx, const uint8_t *d_arena, uint64_t arena_bytes,
                     SS_TRY(ssort_set_param(ctx, k.param, v));
                     double ms = 0;
                     SS_TRY(time_it(ms));
-                    if (ms < best * 0.99) {
+                    if (k.decides && ms < best * 0.99) {
                         best = ms;
                         keep = v;
                     }
