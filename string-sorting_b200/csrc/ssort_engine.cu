@@ -573,9 +573,7 @@ int sort_device_impl(ssort_ctx *ctx, const uint8_t *d_arena, uint64_t arena_byte
     ctx->stats.device_ms = ms;
     if (ctx->prof) ctx->prof_collect();
     size_t held = 0;
-    for (DBuf *b : {&ctx->ws_buf, &ctx->arena, &ctx->offs, &ctx->perm, &ctx->inst, &ctx->aux,
-                     &ctx->aux2})
-        held += b->cap;
+    for (DBuf *b : ctx->device_buffers()) held += b->cap;
     ctx->stats.device_bytes = held;
     return SSORT_OK;
 }
@@ -668,8 +666,7 @@ void ssort_ctx_destroy(ssort_ctx *ctx) {
         for (cudaStream_t c : ctx->cap)
             if (c) cudaStreamDestroy(c);
         if (ctx->h_gs) cudaFreeHost(ctx->h_gs);
-        for (DBuf *b : {&ctx->ws_buf, &ctx->arena, &ctx->offs, &ctx->perm, &ctx->inst, &ctx->aux,
-                     &ctx->aux2})
+        for (DBuf *b : ctx->device_buffers())
             if (b->p) cudaFree(b->p);
         for (HBuf *b : {&ctx->h_offs, &ctx->h_arena, &ctx->h_perm, &ctx->h_stage[0],
                         &ctx->h_stage[1]})
@@ -678,7 +675,6 @@ void ssort_ctx_destroy(ssort_ctx *ctx) {
             if (e) cudaEventDestroy(e);
         if (ctx->hc) cudaFreeHost(ctx->hc);
         if (ctx->h_hist) cudaFreeHost(ctx->h_hist);
-        if (ctx->hist_buf.p) cudaFree(ctx->hist_buf.p);
         for (auto e : ctx->ev_pool) cudaEventDestroy(e);
         if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
         if (ctx->ev_stop) cudaEventDestroy(ctx->ev_stop);

@@ -139,6 +139,11 @@ struct ssort_ctx {
     size_t ev_used = 0;
     std::map<std::string, std::pair<double, uint64_t>> ktimes;
 
+    // Every device buffer of the context.
+    std::vector<ssort::DBuf *> device_buffers() {
+        return {&ws_buf, &arena, &offs, &perm, &inst, &aux, &aux2, &key2_buf, &hist_buf};
+    }
+
     int ensure(ssort::DBuf &b, size_t bytes) {
         if (b.cap >= bytes) return SSORT_OK;
         if (b.p) cudaFree(b.p);

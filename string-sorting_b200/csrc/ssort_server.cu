@@ -686,9 +686,10 @@ int ssort_server_get_info(ssort_server *srv, ssort_server_info *out) {
     i.strings_in_use = srv->pos_alloc.used();
     i.arena_budget = srv->budget;
     i.max_strings = srv->max_strings;
-    size_t held = srv->ctx->ws_buf.cap;
+    size_t held = 0;
+    for (DBuf *b : srv->ctx->device_buffers()) held += b->cap;
     for (DBuf *b : {&srv->pool, &srv->goffs, &srv->perm, &srv->bases, &srv->flags, &srv->d_join,
-                    &srv->d_done})
+                    &srv->d_done, &srv->in.d, &srv->out.d})
         held += b->cap;
     i.device_bytes = held;
     *out = i;

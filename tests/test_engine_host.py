@@ -118,3 +118,25 @@ def test_parameters_without_effect_decide_nothing(tmp_path):
     CHECK(t.default_ms == 100);
     CHECK(t.tuned_ms == 98);
     """)
+
+
+def test_a_context_gives_back_all_its_memory_and_counts_it(tmp_path):
+    """Every device buffer of a context, the key copies and the tuner's histogram
+    among them, is in the size that a sort reports and is freed with it."""
+    run(tmp_path, r"""
+    ssort_ctx *c = new ssort_ctx();
+    CHECK(c->ensure(c->key2_buf, 16 << 20) == SSORT_OK);
+    CHECK(c->ensure(c->hist_buf, 1024) == SSORT_OK);
+    for (DBuf *b : {&c->arena, &c->offs, &c->perm, &c->inst, &c->aux, &c->aux2})
+        CHECK(c->ensure(*b, 1000) == SSORT_OK);
+    uint32_t perm[128];
+    CHECK(ssort_sort_device(c, text, sizeof text, offs, 8, 100, perm, nullptr, nullptr) ==
+          SSORT_OK);
+    size_t all = 0;
+    for (auto &h : held) all += h.second;
+    ssort_stats st{};
+    CHECK(ssort_get_stats(c, &st) == SSORT_OK);
+    CHECK(st.device_bytes == all);
+    ssort_ctx_destroy(c);
+    CHECK(held.empty());
+    """)
