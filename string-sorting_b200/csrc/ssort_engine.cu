@@ -268,8 +268,8 @@ int ssort_ctx::round_body(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt,
                             ws.cm, dc, first, g2, st));
         SS_TRY(scan(ws.cm, ws.cm, (uint32_t)(ws.cm_cap - 1), dcount(ws.cm_base + n_large)));
         LAUNCH(this, "scatter",
-               launch_scatter(a, lcur, nl, ws.tile_base, ws.spl, ws.nspl, ws.tbl, ws.cm_base,
-                              ws.cm, dc, g2, st));
+               launch_scatter(a, lcur, nl, ws.tile_base, ws.nspl, ws.cm_base, ws.cm, dc, g2,
+                              st));
         LAUNCH(this, "emit",
                launch_emit(a, lcur, nl, ws.tile_base, ws.nspl, ws.cm_base, ws.cm, ws.W1, ws.W8,
                            ws.small(), lnext, ws.E, ws.B, nxt, dc, 0, st,

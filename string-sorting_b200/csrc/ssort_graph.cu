@@ -176,8 +176,8 @@ int ssort_ctx::graph_build(const SortArgs &a) {
             SS_TRY(scan_on(ws.cm, ws.cm, (uint32_t)(ws.cm_cap - 1),
                            dcount(ws.cm_base, &g->n_large), s1));
             LAUNCH(this, "scatter",
-                   launch_scatter(a, ws.L, nl, ws.tile_base, ws.spl, ws.nspl, ws.tbl, ws.cm_base,
-                                  ws.cm, dc, g2, s1));
+                   launch_scatter(a, ws.L, nl, ws.tile_base, ws.nspl, ws.cm_base, ws.cm, dc, g2,
+                                  s1));
             LAUNCH(this, "emit",
                    launch_emit(a, ws.L, nl, ws.tile_base, ws.nspl, ws.cm_base, ws.cm, ws.W1,
                                ws.W8, S, ws.L2, ws.E, ws.B, ws.N, dc, g4, s1));

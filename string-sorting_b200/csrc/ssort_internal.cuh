@@ -261,7 +261,7 @@ constexpr uint32_t scan_partials_for(uint64_t n) {
 
 struct WsLayout {
     size_t idx1, key0, key1, lcp, bkt, R, N, W1, W8, S, S2, S3, S4, E, B, L, L2, spl, nspl, tbl, ntiles,
-        cm_size, cm_base, tile_base, tmp, cm, partials, ctr, gs, lookback;
+        cm_size, cm_base, tile_base, cm, partials, ctr, gs, lookback;
     size_t cm_cap, total;
 };
 
@@ -301,7 +301,6 @@ constexpr WsLayout ws_layout(uint64_t n) {
     o.cm_size = take(nlarge * 4);
     o.cm_base = take((nlarge + 1) * 4);
     o.tile_base = take((nlarge + 1) * 4);
-    o.tmp = take((nlarge + 1) * 4);
     // bucket-count matrix: at most NB_MAX buckets per tile of each segment
     o.cm_cap = (size_t)NB_MAX * (most_tiles(n) + nlarge + 1) + 1;
     o.cm = take(o.cm_cap * 4);
@@ -315,7 +314,7 @@ constexpr WsLayout ws_layout(uint64_t n) {
 }
 
 struct Workspace {
-    uint32_t *idx1, *lcp, *nspl, *ntiles, *cm_size, *cm_base, *tile_base, *tmp, *cm, *partials;
+    uint32_t *idx1, *lcp, *nspl, *ntiles, *cm_size, *cm_base, *tile_base, *cm, *partials;
     unsigned char *lookback;  // ticket + tile status words of the single-pass scan
     ulonglong2 *key0, *key1, *spl;
     Seg *R, *N, *W1, *W8, *S, *S2, *S3, *S4, *E, *L, *L2;
@@ -355,7 +354,6 @@ inline Workspace ws_bind(const WsLayout &o, unsigned char *base) {
     w.cm_size = (uint32_t *)(base + o.cm_size);
     w.cm_base = (uint32_t *)(base + o.cm_base);
     w.tile_base = (uint32_t *)(base + o.tile_base);
-    w.tmp = (uint32_t *)(base + o.tmp);
     w.cm = (uint32_t *)(base + o.cm);
     w.partials = (uint32_t *)(base + o.partials);
     w.lookback = base + o.lookback;
@@ -452,9 +450,8 @@ void launch_count(const SortArgs &a, const Seg *L, Count nL, const uint32_t *til
                   const uint32_t *cm_base, uint32_t *cm, Counters *c, bool gather, int grid,
                   cudaStream_t st);
 void launch_scatter(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
-                    const ulonglong2 *spl, const uint32_t *nspl, const uint16_t *tbl,
-                    const uint32_t *cm_base, const uint32_t *cm_scan, Counters *c, int grid,
-                    cudaStream_t st);
+                    const uint32_t *nspl, const uint32_t *cm_base, const uint32_t *cm_scan,
+                    Counters *c, int grid, cudaStream_t st);
 void launch_emit(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
                  const uint32_t *nspl, const uint32_t *cm_base, const uint32_t *cm_scan,
                  Seg *W1, Seg *W8, SmallLists S, Seg *L2, Seg *E, uint2 *B, Seg *N,

@@ -3506,8 +3506,6 @@ void launch_seg_tiles(const Seg *segs, Count n, uint32_t tile, uint32_t *out, cu
 
 uint32_t scan_partials_needed(uint32_t n) { return cdiv(n ? n : 1, SCAN_CHUNK) + 1; }
 
-size_t lookback_state_bytes(uint32_t cap) { return 8 + (size_t)cdiv(cap ? cap : 1, SCAN_CHUNK) * 8; }
-
 void launch_scan_lookback(const uint32_t *in, uint32_t *out, uint32_t cap, Count n,
                           unsigned char *state, uint32_t *err, cudaStream_t st) {
     const uint32_t nb = std::min<uint32_t>(cdiv(cap ? cap : 1, SCAN_CHUNK), 148 * 8);
@@ -3555,9 +3553,8 @@ void launch_count(const SortArgs &a, const Seg *L, Count nL, const uint32_t *til
 }
 
 void launch_scatter(const SortArgs &a, const Seg *L, Count nL, const uint32_t *tile_base,
-                    const ulonglong2 *spl, const uint32_t *nspl, const uint16_t *tbl,
-                    const uint32_t *cm_base, const uint32_t *cm_scan, Counters *c, int grid,
-                    cudaStream_t st) {
+                    const uint32_t *nspl, const uint32_t *cm_base, const uint32_t *cm_scan,
+                    Counters *c, int grid, cudaStream_t st) {
     if (!nL.dev && !nL.host) return;
     set_smem_attrs();
     launch_next(k_scatter, grid, SCATTER_THREADS, sizeof(ScatterSmem), st, a, L, nL, tile_base,
