@@ -81,7 +81,7 @@ int ssort_sort_device(ssort_ctx *ctx, const uint8_t *d_arena, uint64_t arena_byt
  * library allocate device memory: cudaMalloc/cudaFree synchronise the device
  * and can fail when the application has already budgeted all memory to its
  * own pool.  All scratch lives in one fixed device array inside the library
- * (SSORT_NOALLOC_MAX_N strings' worth, about 24 MB), which every GPU that
+ * (SSORT_NOALLOC_MAX_N strings' worth, about 25 MB), which every GPU that
  * loads the library holds until the process exits; larger n is rejected with
  * SSORT_EINVAL.  The caller still passes the inputs and the perm (and
  * optional lcp) outputs, and a cudaStream_t (NULL = the legacy default

@@ -206,7 +206,7 @@ int ssort_ctx::round(const SortArgs &a, Seg *cur, uint32_t n_cur, Seg *nxt, uint
     overlap_round = side && side2 && hp && !prof && overlap;
     if (!overlap_round || forked)
         return round_body(a, cur, n_cur, nxt, n_next, round_no, classified, ahead);
-    // Fork the round onto the high-priority stream and join it back.
+    // Fork the round onto the partition's stream and join it back.
     cudaStream_t user = st;
     SS_CUDA(cudaEventRecord(ev_round, user));
     SS_CUDA(cudaStreamWaitEvent(hp, ev_round, 0));

@@ -54,17 +54,21 @@ constexpr uint32_t KEY2_MIN_BYTES_PER_STRING = 24;  // ... when the arena has th
 constexpr double KEY2_MIN_ROUND1_LIVE = 0.25;       // ... and the last sort's round-1 share
 constexpr int SMALL_CAP = 2048;
 constexpr int SMALL_THREADS = 256;
-// The CTA sort splits its segments into three size classes, sorted by groups
-// of 64, 128 and 256 threads (8 strings per thread): <= BLOCK_CAP1,
-// <= BLOCK_CAP2 and <= SMALL_CAP strings.
+// The CTA sort splits its segments into four size classes, sorted by groups of
+// 64, 128, 256 and 512 threads (8 strings per thread): <= BLOCK_CAP1,
+// <= BLOCK_CAP2, <= SMALL_CAP and <= LEAF_CAP strings.
 constexpr int BLOCK_CAP1 = 512;
 constexpr int BLOCK_CAP2 = 1024;
 // In sorts of at least LEAF_MIN_N strings a range bucket of up to LEAF_CAP
-// strings is sorted by 512 threads (a fourth class) instead of being
-// partitioned again: that level would move every string once more.  Measured:
-// 69 M batched strings 6.23 -> 5.79 ms.  A smaller sort has too few such
-// buckets to fill the chip, and one CTA takes longer over 4096 strings than a
-// level and a smaller sort: 1 M uniform strings 0.36 -> 0.41 ms.
+// strings is sorted by 512 threads (the fourth class) instead of being
+// partitioned again: that level would move every string once more.  69 M batched
+// strings 6.23 -> 5.74 ms.  A smaller sort has too few such buckets to fill the
+// chip, and one CTA takes longer over 4096 strings than a level and a smaller
+// sort.  The samples per splitter go by the same line (sample_segment).  Both
+// rules as above the line / as below it, ms per sort on either side of it:
+// uniform strings 1 M 0.274 / 0.212, 3 M 0.417 / 0.407, 4.3 M 0.507 / 0.510, 16 M
+// 1.293 / 1.291; Zipf words 3 M 0.580 / 0.497, 4.3 M 0.636 / 0.639, 16 M 1.358 /
+// 1.377; URLs 3 M 0.821 / 0.849, 4.3 M 0.970 / 1.004, 16 M 2.355 / 2.371.
 constexpr int LEAF_CAP = 4096;
 constexpr uint32_t LEAF_MIN_N = 1u << 22;
 

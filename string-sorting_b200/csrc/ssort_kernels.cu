@@ -7,12 +7,13 @@
 // with unsigned shifts; the reference's int-promoted 64-bit form sign-extends
 // bytes >= 0x80, :82, and is not reproduced).  Each segment is then sorted by
 // (key, index): segments of <= 32 strings by one warp in registers (four
-// segments of <= 8 per warp), <= SMALL_CAP by a group of 32 to 256 threads of
-// a CTA (by size), larger ones are first split by sample partitioning into range buckets and
-// equality buckets with a stable scatter.  Equal runs whose key holds no NUL (the reference's
-// is_end test, src/util/get_char.h:162-175, and its bucket-skip rule,
-// src/msd_ce.cpp:402) become the next round's segments at depth+16; every
-// other adjacent pair gets its LCP here.
+// segments of <= 8 per warp), those of up to SMALL_CAP (in large sorts LEAF_CAP)
+// by a group of 32 to 512 threads of a CTA (by size), larger ones are first split
+// by sample partitioning into range buckets and equality buckets with a stable
+// scatter.  Equal runs whose key holds no NUL (the reference's is_end test,
+// src/util/get_char.h:162-175, and its bucket-skip rule, src/msd_ce.cpp:402)
+// become the next round's segments at depth+16; every other adjacent pair gets
+// its LCP here.
 #include <algorithm>
 #include <atomic>
 
@@ -279,7 +280,6 @@ __global__ void k_iota(uint32_t *idx, uint32_t n) {
         idx[i] = i;
 }
 
-// Appends o (when sm) to the CTA-sort list of its size class; warp-collective.
 // Appends segment o (when v) to the list its length selects: one-warp sorts
 // of <= 32 or <= warp8_cap strings, the CTA sorts' four size classes (up to
 // cap strings), or the large list L (counter nl).  Warp-collective; the
@@ -2400,10 +2400,16 @@ __global__ void __launch_bounds__(WARP_THREADS) k_warp1(SortArgs a, const Seg *T
 // only.  24 bytes of shared memory per string let 1024 threads share an SM.
 // Measured on B200 against 64-bit packed keys merged in shared memory (80
 // registers, 768 threads per SM): 10,000 partitioned segments of 400 strings
-// at 55 G strings/s (2290 instructions per warp of 256, 910 of them the
-// network; ALU pipe 65-75 % busy); the CTA-sort launches of 69 M batched
-// strings 2.79 -> 1.53 ms, of 16 M suffixes 4.23 -> 2.59 ms, of 50 M URLs 2.27
-// -> 1.62 ms.
+// at 55 G strings/s; the CTA-sort launches of 69 M batched strings 2.79 -> 1.53
+// ms, of 16 M suffixes 4.23 -> 2.59 ms, of 50 M URLs 2.27 -> 1.62 ms.  In a sort
+// of 10 M URLs a warp of 256 strings issues 2400 instructions, the ALU pipe is
+// active 66 % of the time and DRAM 11 %.
+// The other side: strings that begin with one of a few prefixes use the bits up
+// on these, tie in long runs and are sorted twice.  Lists of 250 to 2000 strings
+// whose first 6 letters come from 5 to 100 groups take 0.78 to 0.9 of the 64-bit
+// sorts' speed (prefixes of 3, 9, 12 letters 1.1 to 6 times).  Sorting on 64-bit
+// values at once where a sample of records ties mends most of these and costs
+// 1.5 % of the 69 M batched strings' time.
 
 // Shared memory of one group, for 8 strings per thread: keys, values (in
 // passing between threads, and the final order), indices, and what its warps
